@@ -26,7 +26,7 @@ F64 = torch.float64
 def listed():
     return [
         # One local window as the mapper adjusts it after each new view: the smallest call.
-        {"name": "window", "op": "solve", "kind": "arc", "C": 7, "P": 611, "fixed": 2, "shared": False,
+        {"name": "window", "op": "solve", "kind": "arc", "C": 7, "P": 611, "fixed": 0, "shared": False,
          "precision": "fp64", "iterations": 6},
         # A small turntable scene with its focal length refined (the benchmark's configuration 0).
         {"name": "ring", "op": "solve", "kind": "ring", "C": 10, "P": 2000, "fixed": 1, "shared": True,
@@ -35,8 +35,8 @@ def listed():
         {"name": "sequence", "op": "solve", "kind": "sphere", "C": 61, "P": 12345, "fixed": 1, "shared": False,
          "precision": "fp64", "iterations": 10},
         # A medium map, 200 views and 100k points (configuration 1), badly conditioned.
-        {"name": "helix", "op": "solve", "kind": "helix", "C": 200, "P": 100000, "fixed": 1, "shared": True,
-         "precision": "fp64", "iterations": 5},
+        {"name": "helix", "op": "solve", "kind": "helix", "C": 200, "P": 100000, "fixed": 1, "shared": False,
+         "precision": "fp64", "iterations": 6},
         # A map kept on the device, adjusted twice as it grows, with bearings and several fixed views.
         {"name": "resident", "op": "resident", "kind": "sphere", "C": 317, "P": 41003, "fixed": 3, "bearings": 64,
          "shared": False, "precision": "fp64", "iterations": 6},
@@ -84,8 +84,10 @@ def draw(rng):
             "shared": rng.random() < 0.5, "precision": "fp64", "iterations": rng.randint(4, 10)}
     if C > 800 and rng.random() < 0.5:  # the mixed form is for large maps
         case.update(shared=False, precision="mixed")
-    if kind in ("helix", "arc"):
-        case["iterations"] = min(case["iterations"], 5)
+    if kind == "helix":
+        case.update(shared=False, iterations=min(case["iterations"], 6))
+    if kind == "arc":
+        case.update(fixed=0, iterations=min(case["iterations"], 6))
     if kind == "sphere" and rng.random() < 0.3:
         case["bearings"] = rng.randint(3, 64)
     return case
@@ -254,8 +256,8 @@ def scene(case, seed):
     t0 = t + 0.01 * t.norm(dim=1, keepdim=True) * torch.nn.functional.normalize(rnd.normal(C, 3), dim=1)
     poses0 = torch.cat([R0.reshape(-1, 9), t0], dim=1)
     active = torch.ones(C, device="cuda", dtype=torch.int64)
-    fixed = case.get("fixed", 1)  # the first two views, then the last ones
-    fixed = list(range(min(fixed, 2))) + [C - 1 - j for j in range(fixed - 2)]
+    fixed = case.get("fixed", 1)  # the first two views, then the last ones; 0: every fourth view
+    fixed = list(range(min(fixed, 2))) + [C - 1 - j for j in range(fixed - 2)] or [1] + list(range(0, C, 4))
     poses0[fixed], active[fixed] = poses[fixed], 0
     X0 = X + 0.01 * rnd.normal(len(X), 3)
     if D:
@@ -312,7 +314,7 @@ def control_of(case, s):
 
 
 def window_sizes(case):
-    """The windows of a batch: 5 to 40 views (four of them fixed), 500 to 20,000 points over their logarithm."""
+    """The windows of a batch: 5 to 40 views (every fourth of them fixed, as the views around a window are), 500 to 20,000 points over their logarithm."""
     r = np.random.default_rng(case["count"])
     C = r.integers(5, 41, size=case["count"])
     P = np.rint(np.exp(r.uniform(math.log(500), math.log(20000), size=case["count"]))).astype(int)
@@ -320,7 +322,7 @@ def window_sizes(case):
 
 
 def windows(case, seed):
-    return [scene({"op": "batch", "kind": "arc", "C": C, "P": P, "shared": case["shared"], "fixed": 4}, 1000003 * int(seed) + k)
+    return [scene({"op": "batch", "kind": "arc", "C": C, "P": P, "shared": case["shared"], "fixed": 0}, 1000003 * int(seed) + k)
             for k, (C, P) in enumerate(window_sizes(case))]
 
 
