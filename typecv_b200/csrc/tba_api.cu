@@ -26,6 +26,8 @@
 #include "tba_engine.cuh"
 #include "tba_checks.cuh"
 #include "tba_observations.cuh"
+#include "tba_pcg.cuh"
+#include "tba_schur.cuh"
 
 using tba::Params;
 
@@ -57,6 +59,9 @@ struct tba_device {
   std::string error;
   char* arena = nullptr;
   size_t capacity = 0;
+  // The explicit reduced camera system's structure and blocks (grown as needed, like the arena).
+  char* schur = nullptr;
+  size_t schur_capacity = 0;
   double* pinned = nullptr;  // small host buffer for flag reads
   std::vector<cudaEvent_t> events;
   // Polls of each main-loop wait of the inverse-depth linearisation (tba_device_set_wait_limit).
@@ -345,11 +350,93 @@ Chunks build_chunks(const uint32_t* cs, uint32_t C, uint32_t M, int sms) {
   return ch;
 }
 
-// Reads the first 40 state words into the pinned buffer; returns word `word`.
+// Reads the state words into the pinned buffer; returns word `word`.
 double read_word(tba_device* d, const double* state, int word) {
-  CUDA_TRY(cudaMemcpyAsync(d->pinned, state, 40 * sizeof(double), cudaMemcpyDeviceToHost, d->stream));
+  CUDA_TRY(cudaMemcpyAsync(d->pinned, state, tba::S_READ * sizeof(double), cudaMemcpyDeviceToHost, d->stream));
   CUDA_TRY(cudaStreamSynchronize(d->stream));
+  if (d->pinned[tba::S_WAIT] != 0) throw Fail{TBA_ERROR_CUDA, "GPU BA: a wait between the PCG's blocks ran out"};
   return d->pinned[word];
+}
+
+// ---- the explicit reduced camera system ------------------------------------------------------------
+
+// Pairs of observations of one point (all cameras counted as variable).
+uint64_t count_pairs(const uint32_t* ps, uint32_t P) {
+  uint64_t squares = 0, sum = 0;
+  for (uint32_t p = 0; p < P; p++) {
+    const uint64_t n = uint32_t(ps[p + 1] - ps[p]);
+    squares += n * n;
+    sum += n;
+  }
+  return (squares - sum) / 2;
+}
+
+// 6x6 blocks of S at most.
+uint64_t schur_block_bound(uint64_t C, uint64_t pairs) { return std::min(C * C, 2 * pairs + C); }
+
+// Whether a solve forms the reduced system explicitly: its values cost about 0.04 ns a pair of
+// observations of one point, once per LM iteration, and a PCG step then a pass over the blocks (here a
+// quarter of their bound, at 5 TB/s) and two grid barriers, against a pass over every observation (0.03
+// ns each) and five launches; compared over 16 PCG steps.
+bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t max_cg) {
+  if (pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
+  const double steps = std::min<uint32_t>(max_cg, 16);
+  const double blocks = double(schur_block_bound(C, pairs)) / 4;
+  return 4e-5 * double(pairs) + steps * (5 + 288e-6 / 5 * blocks) < steps * (14 + 3e-5 * double(M));
+}
+
+// Device memory of a solve's explicit system beside the workspace: structure, segment sums, blocks.
+// `blocks` and `camera_pairs` bound the blocks of S and the camera pairs.
+struct SchurLayout {
+  Layout L;
+  size_t counts, bits, row_blk, row_pair, row_ptr, col, pairs, begin, rc, dst, seg_block, totals, part, S;
+  size_t share, uni, uni_n, local, pbuf, zx, slots;  // the persistent PCG's
+  uint32_t seg = 0, grid = 1;
+  SchurLayout(uint32_t C, uint64_t npairs, uint32_t nchunks, uint64_t blocks, uint64_t camera_pairs, int sms) {
+    // Pairs per warp of the block sums: a few warps' worth of segments on every SM.
+    seg = tba::kPairSegMin;
+    while (seg < tba::kPairSegMax && npairs / seg > uint64_t(64) * uint64_t(sms)) seg *= 2;
+    const size_t segs = size_t((npairs + seg - 1) / seg);
+    const size_t bwords = (C + 31) / 32;
+    counts = L.take<uint32_t>(size_t(nchunks) * C);
+    bits = L.take<uint32_t>(C * bwords);
+    row_blk = L.take<uint32_t>(C + 1);
+    row_pair = L.take<uint32_t>(C + 1);
+    row_ptr = L.take<uint32_t>(C + 1);
+    col = L.take<uint32_t>(blocks);
+    pairs = L.take<uint2>(npairs);
+    begin = L.take<uint32_t>(camera_pairs + 1);
+    rc = L.take<uint2>(camera_pairs);
+    dst = L.take<uint2>(camera_pairs);
+    seg_block = L.take<uint32_t>(segs);
+    totals = L.take<uint32_t>(4);
+    grid = tba::pcg_grid(blocks, C, sms);
+    share = L.take<uint32_t>(grid + 1);
+    uni = L.take<uint32_t>(size_t(grid) * C);
+    uni_n = L.take<uint32_t>(grid);
+    local = L.take<uint32_t>(blocks);
+    pbuf = L.take<double>(size_t(grid) * 6 * C);
+    zx = L.take<tba::Flagged>(6 * size_t(C));
+    slots = L.take<tba::Flagged>(4 * size_t(grid));
+    part = L.take<double>(72 * segs);
+    S = L.take<double>(36 * blocks);
+  }
+};
+
+// Grows a device buffer kept by the handle to `bytes` (its old contents are dropped).
+void grow(char*& buffer, size_t& capacity, size_t bytes, const char* what) {
+  if (capacity >= bytes) return;
+  if (buffer) CUDA_TRY(cudaFree(buffer));
+  buffer = nullptr;
+  capacity = 0;
+  size_t free_bytes = 0, total_bytes = 0;
+  CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (bytes > free_bytes)
+    throw Fail{TBA_ERROR_BUDGET, std::string(what) + " needs " + std::to_string(bytes) +
+                                     " bytes of device memory, more than the working budget of " +
+                                     std::to_string(free_bytes) + " bytes"};
+  CUDA_TRY(cudaMalloc(&buffer, bytes));
+  capacity = bytes;
 }
 
 // Makes `loop` a graph of one while node whose body `capture(handle, stream)` records (returning its
@@ -450,6 +537,7 @@ struct HostPlan {
   std::vector<uint32_t> tasks, task_obs;
   Chunks chunks;
   uint32_t fixed = 0;
+  uint64_t pairs = 0;  // pairs of observations of one point
   // The arrays a solve uploads, in the order of a resident scene's device copy.
   std::vector<const std::vector<uint32_t>*> sections() const {
     return {&tasks, &task_obs, &chunks.cam, &chunks.beg, &chunks.cam_first};
@@ -467,6 +555,7 @@ HostPlan make_plan(const tba_control* ctl, const uint32_t* index, int sms) {
   for (size_t t = 0; t < plan.tasks.size(); t++) plan.task_obs[t] = ps[plan.tasks[t]];
   plan.chunks = build_chunks(cs, C, M, sms);
   for (uint32_t c = 0; c < C; c++) plan.fixed += active[c] == 0;
+  plan.pairs = count_pairs(ps, P);
   return plan;
 }
 
@@ -514,60 +603,93 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   p.huber = ctl->huber;
   p.tol = ctl->cg_tolerance;
   p.stall = ctl->stall_tolerance;
-  // The mixed form's inner PCG runs stop at a relative residual the FP32 product can reach; the
-  // FP64 refinement then measures the true residual against the caller's tolerance.
-  p.tol_inner = ctl->precision == TBA_PRECISION_MIXED ? std::max(ctl->cg_tolerance, 1e-6) : ctl->cg_tolerance;
   const uint32_t max_task_blocks = std::max<uint32_t>(1, 4 * uint32_t(d->sms));
   const uint32_t fblocks = tba::product_finish_blocks(p);
   // The one-pass product over stored factors when its camera sums fit shared memory; the two-pass
   // recompute form otherwise.  The mixed form stores FP32 factors for its PCG and FP64 factors for
   // its refinement residual, its FP64 tail and the back-substitution.
-  const bool mixed = ctl->precision == TBA_PRECISION_MIXED;
   p.factored = m <= tba::product_max_unknowns();
   p.Mpad = (M + 31) / 32 * 32;
-  const size_t factor_bytes = p.factored ? size_t(tba::kFactors) * p.Mpad * 8 : 0;
-  const size_t factor32_bytes = p.factored && mixed ? size_t(tba::kFactors) * p.Mpad * 4 : 0;
-  p.F = nullptr;
-  p.F32 = mixed && p.factored ? reinterpret_cast<float*>(1) : nullptr;  // set below; selects the occupancy query
-  const int per_sm = p.factored ? tba::product_blocks_per_sm(p) : 1;
-  const uint32_t max_prod_blocks = std::max<uint32_t>(1, uint32_t(per_sm * d->sms));
+  // The explicit reduced system takes the place of the product over stored factors where it costs less
+  // and fits the device; it is FP64, so a mixed request then needs no refinement.
+  const uint64_t npairs = io.plan ? io.plan->pairs : count_pairs(index + 2 * size_t(M), P);
+  bool schur = p.factored && prefer_schur(C, M, npairs, ctl->max_cg);
+  bool mixed = false;
+  size_t factor_bytes = 0, factor32_bytes = 0;
+  uint32_t max_prod_blocks = 1;
   Layout L;
-  const size_t o_poses = L.take<double>(12 * size_t(C)), o_points = L.take<double>(3 * size_t(P)),
-               o_cams = L.take<double>(6 * size_t(C)), o_pixels = L.take<double>(2 * size_t(M)),
-               o_tposes = L.take<double>(12 * size_t(C)), o_tpoints = L.take<double>(3 * size_t(P)),
-               o_index = L.take<uint32_t>(3 * size_t(M) + P + 2 * size_t(C) + 2),
-               o_pblk32 = L.take<float>(mixed && p.factored ? 6 * size_t(P) : 0),
-               o_tasks = L.take<uint32_t>(max_tasks), o_tobs = L.take<uint32_t>(max_tasks),
-               o_ccam = L.take<uint32_t>(max_chunks),
-               o_cbeg = L.take<uint32_t>(max_chunks + 1), o_cfirst = L.take<uint32_t>(C + 1),
-               o_rlim = L.take<double>(C), o_cmp = L.take<uint32_t>(M), o_cmx = L.take<double>(2 * size_t(M)),
-               o_pblk = L.take<double>(12 * size_t(P)), o_y = L.take<double>(4 * size_t(P)),
-               o_cprod = L.take<double>(8 * max_chunks), o_F = L.take<char>(factor_bytes),
-               o_F32 = L.take<char>(factor32_bytes),
-               o_pw = L.take<double>(6 * size_t(C)), o_xw = L.take<double>(6 * size_t(C)),
-               o_acc = L.take<double>(p.factored ? size_t(max_prod_blocks) * m : 0), o_U = L.take<double>(21 * size_t(C)),
-               o_Minv = L.take<double>(36 * size_t(C)), o_rhs = L.take<double>(6 * size_t(C)),
-               o_hcf = L.take<double>(6 * size_t(C)),
-               o_chunk = L.take<double>(size_t(tba::kCameraPartials) * max_chunks),
-               o_vec = L.take<double>(5 * size_t(m)), o_blk = L.take<double>(4 * size_t(fblocks)),
-               o_scal = L.take<double>(size_t(tba::kScalarPartials) * max_task_blocks),
-               o_cost = L.take<double>(4 * size_t(max_task_blocks)), o_ticket = L.take<uint32_t>(8),
-               o_state = L.take<double>(tba::S_WORDS), o_out = L.take<double>(12 * size_t(C) + 3 * size_t(P) + 27),
-               o_keys = L.take<unsigned long long>(tba::CK_WORDS),
-               o_diag = L.take<double>((ctl->flags & TBA_FLAG_PRODUCT_ERROR) ? 2 * size_t(m) : 0);
-  if (d->capacity < L.bytes) {
-    if (d->arena) CUDA_TRY(cudaFree(d->arena));
-    d->arena = nullptr;
-    d->capacity = 0;
-    size_t free_bytes = 0, total_bytes = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
-    if (L.bytes > free_bytes)
-      throw Fail{TBA_ERROR_BUDGET, "GPU BA needs " + std::to_string(L.bytes) +
-                                       " bytes of device memory, more than the working budget of " +
-                                       std::to_string(free_bytes) + " bytes"};
-    CUDA_TRY(cudaMalloc(&d->arena, L.bytes));
-    d->capacity = L.bytes;
+  size_t o_poses, o_points, o_cams, o_pixels, o_tposes, o_tpoints, o_index, o_pblk32, o_tasks, o_tobs, o_ccam, o_cbeg,
+      o_cfirst, o_rlim, o_cmp, o_cmx, o_pblk, o_y, o_cprod, o_F, o_F32, o_pw, o_xw, o_acc, o_U, o_Minv, o_rhs, o_hcf,
+      o_scf, o_chunk, o_vec, o_blk, o_scal, o_cost, o_ticket, o_state, o_out, o_keys, o_diag;
+  auto lay_out = [&]() {
+    mixed = ctl->precision == TBA_PRECISION_MIXED && !schur;
+    factor_bytes = schur ? 18 * size_t(M) * 8 : (p.factored ? size_t(tba::kFactors) * p.Mpad * 8 : 0);
+    factor32_bytes = p.factored && mixed ? size_t(tba::kFactors) * p.Mpad * 4 : 0;
+    p.F = nullptr;
+    p.F32 = mixed && p.factored ? reinterpret_cast<float*>(1) : nullptr;  // set below; selects the occupancy query
+    const int per_sm = p.factored && !schur ? tba::product_blocks_per_sm(p) : 1;
+    max_prod_blocks = schur ? 0 : std::max<uint32_t>(1, uint32_t(per_sm * d->sms));
+    L = Layout();
+    o_poses = L.take<double>(12 * size_t(C));
+    o_points = L.take<double>(3 * size_t(P));
+    o_cams = L.take<double>(6 * size_t(C));
+    o_pixels = L.take<double>(2 * size_t(M));
+    o_tposes = L.take<double>(12 * size_t(C));
+    o_tpoints = L.take<double>(3 * size_t(P));
+    o_index = L.take<uint32_t>(3 * size_t(M) + P + 2 * size_t(C) + 2);
+    o_pblk32 = L.take<float>(mixed && p.factored ? 6 * size_t(P) : 0);
+    o_tasks = L.take<uint32_t>(max_tasks);
+    o_tobs = L.take<uint32_t>(max_tasks);
+    o_ccam = L.take<uint32_t>(max_chunks);
+    o_cbeg = L.take<uint32_t>(max_chunks + 1);
+    o_cfirst = L.take<uint32_t>(C + 1);
+    o_rlim = L.take<double>(C);
+    o_cmp = L.take<uint32_t>(M);
+    o_cmx = L.take<double>(2 * size_t(M));
+    o_pblk = L.take<double>(12 * size_t(P));
+    o_y = L.take<double>(4 * size_t(P));
+    o_cprod = L.take<double>(8 * max_chunks);
+    o_F = L.take<char>(factor_bytes);
+    o_F32 = L.take<char>(factor32_bytes);
+    o_pw = L.take<double>(6 * size_t(C));
+    o_xw = L.take<double>(6 * size_t(C));
+    o_acc = L.take<double>(p.factored ? size_t(max_prod_blocks) * m : 0);
+    o_U = L.take<double>(21 * size_t(C));
+    o_Minv = L.take<double>(36 * size_t(C));
+    o_rhs = L.take<double>(6 * size_t(C));
+    o_hcf = L.take<double>(6 * size_t(C));
+    o_scf = L.take<double>(6 * size_t(C));
+    o_chunk = L.take<double>(size_t(schur ? tba::kCameraPartialsExplicit : tba::kCameraPartials) * max_chunks);
+    o_vec = L.take<double>(5 * size_t(m));
+    o_blk = L.take<double>(4 * size_t(fblocks));
+    o_scal = L.take<double>(size_t(tba::kScalarPartials) * max_task_blocks);
+    o_cost = L.take<double>(4 * size_t(max_task_blocks));
+    o_ticket = L.take<uint32_t>(8);
+    o_state = L.take<double>(tba::S_WORDS);
+    o_out = L.take<double>(12 * size_t(C) + 3 * size_t(P) + 27);
+    o_keys = L.take<unsigned long long>(tba::CK_WORDS);
+    o_diag = L.take<double>((ctl->flags & TBA_FLAG_PRODUCT_ERROR) ? 2 * size_t(m) : 0);
+  };
+  lay_out();
+  if (schur) {
+    // What the explicit system would add: when it does not fit, the product over stored factors.
+    const uint64_t bound = schur_block_bound(C, npairs), camera_pairs = std::min<uint64_t>(npairs, uint64_t(C) * (C + 1) / 2);
+    const size_t more = SchurLayout(C, npairs, uint32_t(max_chunks), bound, camera_pairs, d->sms).L.bytes;
+    if (d->capacity < L.bytes || d->schur_capacity < more) {
+      size_t free_bytes = 0, total_bytes = 0;
+      CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+      if (L.bytes + more > free_bytes + d->capacity + d->schur_capacity) {
+        schur = false;
+        lay_out();
+      }
+    }
   }
+  if (d->capacity < L.bytes && d->schur && !schur) {  // the workspace may need the explicit system's memory
+    CUDA_TRY(cudaFree(d->schur));
+    d->schur = nullptr;
+    d->schur_capacity = 0;
+  }
+  grow(d->arena, d->capacity, L.bytes, "GPU BA");
   char* a = d->arena;
   auto D = [&](size_t off) { return reinterpret_cast<double*>(a + off); };
   auto U32 = [&](size_t off) { return reinterpret_cast<uint32_t*>(a + off); };
@@ -596,7 +718,10 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   p.pblk = D(o_pblk);
   p.y = D(o_y);
   p.chunk_prod = D(o_cprod);
-  p.F = p.factored ? D(o_F) : nullptr;
+  p.F = p.factored && !schur ? D(o_F) : nullptr;
+  p.schur = schur;
+  p.A = schur ? D(o_F) : nullptr;
+  p.camScf = D(o_scf);
   p.F32 = p.factored && mixed ? reinterpret_cast<float*>(a + o_F32) : nullptr;
   p.pw = D(o_pw);
   p.xw = D(o_xw);
@@ -618,6 +743,10 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   p.ticket = U32(o_ticket);
   p.state = D(o_state);
   p.output = D(o_out);
+
+  // The mixed form's inner PCG runs stop at a relative residual the FP32 product can reach; the
+  // FP64 refinement then measures the true residual against the caller's tolerance.
+  p.tol_inner = mixed ? std::max(ctl->cg_tolerance, 1e-6) : ctl->cg_tolerance;
 
   cudaStream_t s = d->stream;
   size_t ev = 0;
@@ -702,6 +831,90 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   }
 
   uint32_t launches = 0, lm_done = 0, refinements = 0, fp64_iterations = 0;
+  tba::SchurParams sq{};
+  tba::PcgSystem ps{};
+  uint32_t pcg_blocks = 0;
+  if (schur) {
+    // The structure of S.  Where the bound on its blocks is far above what scenes have (a local
+    // covisibility), the counted structure sizes the blocks.
+    uint64_t blocks = schur_block_bound(C, npairs), camera_pairs = std::min<uint64_t>(npairs, uint64_t(C) * (C + 1) / 2);
+    const SchurLayout Q(C, npairs, nchunks, blocks, camera_pairs, d->sms);
+    grow(d->schur, d->schur_capacity, Q.L.bytes, "GPU BA");
+    char* b = d->schur;
+    auto at = [&](size_t off) { return reinterpret_cast<uint32_t*>(b + off); };
+    sq.C = C;
+    sq.M = M;
+    sq.nchunks = nchunks;
+    sq.bwords = (C + 31) / 32;
+    sq.seg = Q.seg;
+    sq.max_pairs = uint32_t(npairs);
+    sq.max_blocks = uint32_t(camera_pairs);
+    sq.obs_camera = p.obs_camera;
+    sq.obs_point = p.obs_point;
+    sq.point_start = p.point_start;
+    sq.camera_obs = p.camera_obs;
+    sq.active = p.active;
+    sq.chunk_cam = p.chunk_cam;
+    sq.chunk_beg = p.chunk_beg;
+    sq.cam_chunk = p.cam_chunk;
+    sq.counts = at(Q.counts);
+    sq.bits = at(Q.bits);
+    sq.row_blk = at(Q.row_blk);
+    sq.row_pair = at(Q.row_pair);
+    sq.row_ptr = at(Q.row_ptr);
+    sq.col = at(Q.col);
+    sq.pairs = reinterpret_cast<uint2*>(b + Q.pairs);
+    sq.blk_begin = at(Q.begin);
+    sq.blk_rc = reinterpret_cast<uint2*>(b + Q.rc);
+    sq.blk_dst = reinterpret_cast<uint2*>(b + Q.dst);
+    sq.seg_block = at(Q.seg_block);
+    sq.totals = at(Q.totals);
+    sq.part = reinterpret_cast<double*>(b + Q.part);
+    sq.S = reinterpret_cast<double*>(b + Q.S);
+    sq.A = p.A;
+    launches += tba::schur_launch_structure(sq, s);
+    CUDA_TRY(cudaGetLastError());
+    p.S = sq.S;
+    p.row_ptr = sq.row_ptr;
+    p.col = sq.col;
+    ps.C = C;
+    ps.shared = shared;
+    ps.S = p.S;
+    ps.row_ptr = p.row_ptr;
+    ps.col = p.col;
+    ps.Minv = p.camMinv;
+    ps.scf = p.camScf;
+    ps.x = p.x;
+    ps.r = p.r;
+    ps.z = p.z;
+    ps.p = p.p;
+    ps.share = at(Q.share);
+    ps.uni = at(Q.uni);
+    ps.uni_n = at(Q.uni_n);
+    ps.local = at(Q.local);
+    ps.pbuf = reinterpret_cast<double*>(b + Q.pbuf);
+    ps.state = p.state;
+    ps.active = tba::S_CG_ACTIVE;
+    ps.failed = tba::S_CG_FAILED;
+    ps.converged = tba::S_CG_CONVERGED;
+    ps.rho = tba::S_RHO;
+    ps.r0 = tba::S_R0;
+    ps.r2 = tba::S_R2;
+    ps.inner_r0 = tba::S_INNER_R0;
+    ps.steps = tba::S_CG_SOLVE_STEPS;
+    ps.all_steps = tba::S_CG_STEPS;
+    ps.wait = tba::S_WAIT;
+    ps.focal_diag = tba::S_FOCAL_SFF;
+    ps.focal_inv = tba::S_FOCAL_INV;
+    ps.tol = p.tol;
+    ps.tol_inner = p.tol_inner;
+    ps.alpha_limit = 1e20;
+    ps.zx = reinterpret_cast<tba::Flagged*>(b + Q.zx);
+    ps.slots = reinterpret_cast<tba::Flagged*>(b + Q.slots);
+    pcg_blocks = Q.grid;
+    launches += tba::pcg_launch_plan(ps, pcg_blocks, s);
+    CUDA_TRY(cudaGetLastError());
+  }
   // Mixed form: once an LM iteration's PCG needed the FP64 tail, the rest of the solve solves on the
   // FP64 product (the FP32 product does not reach the tolerance on such a system, and its restarts
   // would only add PCG runs).
@@ -730,6 +943,7 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     tba::launch_point_pass(p, s);
     tba::launch_camera_pass(p, s);
     tba::launch_camera_finish(p, s);
+    if (schur) launches += tba::schur_launch_values(sq, s);
     tba::launch_pcg_init(p, s);
     launches += 4;
     if (it == 0 && (ctl->flags & TBA_FLAG_PRODUCT_ERROR) && read_word(d, p.state, tba::S_CG_ACTIVE) != 0) {
@@ -740,7 +954,8 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
       fp64.F32 = nullptr;
       fp64.factored = 0;
       tba::launch_product(p, s);
-      tba::launch_product_rows(p, own, s);
+      if (schur) CUDA_TRY(cudaMemcpyAsync(own, p.Sp, m * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      else tba::launch_product_rows(p, own, s);
       tba::launch_product(fp64, s);
       tba::launch_product_rows(fp64, ref, s);
       launches += p.factored ? 5 : 6;
@@ -769,6 +984,11 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     // `q` selects the product: the engine's own (FP32 factors in the mixed form), or the FP64
     // product of the mixed form's tail.  Only the engine's own products are timed.
     auto run_pcg = [&](uint32_t budget, const tba::Params& q, bool timed) {
+      if (schur && !host_loop) {
+        CUDA_TRY(tba::launch_pcg(ps, budget, pcg_blocks, s));
+        launches++;
+        return;
+      }
       if (!host_loop && !d->host_pcg_only) {
         if (budget <= done) return;
         PcgLoop& loop = d->pcg_loops[&q == &p ? 0 : 1];
@@ -795,7 +1015,7 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
             tba::launch_product(q, s);
           }
           tba::launch_product_finish(q, s);
-          launches += q.factored ? 4 : 5;
+          launches += schur ? 3 : (q.factored ? 4 : 5);
         }
         CUDA_TRY(cudaGetLastError());
         done += k;
@@ -848,10 +1068,8 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     launches += 4;
     CUDA_TRY(cudaGetLastError());
     lm_done++;
-    CUDA_TRY(cudaMemcpyAsync(d->pinned, p.state, 40 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
+    lm_active = read_word(d, p.state, tba::S_ACTIVE) != 0;
     account_loop();
-    lm_active = d->pinned[tba::S_ACTIVE] != 0;
   }
   tba::launch_pack(p, s);
   launches++;
@@ -903,8 +1121,8 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     report->lm_iterations = lm_done;
     const double* st = output ? output + 12 * size_t(C) + 3 * size_t(P) : io.state;
     report->cg_iterations = st ? uint32_t(st[tba::S_CG_STEPS]) : 0;
-    report->engine = p.factored ? 0 : 1;
-    report->product_blocks = p.factored ? p.prod_blocks : 0;
+    report->engine = schur ? 2 : (p.factored ? 0 : 1);
+    report->product_blocks = p.factored && !schur ? p.prod_blocks : 0;
     report->refinements = uint32_t(refinements);
     report->fp64_iterations = fp64_iterations;
     report->product_error_max = product_error_max;
@@ -1670,6 +1888,7 @@ tba_status tba_device_open(int ordinal, tba_device** out) {
     CUDA_TRY(cudaStreamCreateWithFlags(&d->down, cudaStreamNonBlocking));
     CUDA_TRY(cudaMallocHost(&d->pinned, 64 * sizeof(double)));
     CUDA_TRY(tba::configure_kernels());
+    CUDA_TRY(tba::pcg_configure());
     CUDA_TRY(tba::adj_configure());
     CUDA_TRY(tba::batch_configure());
   } catch (const Fail& f) {
@@ -1692,6 +1911,7 @@ void tba_device_close(tba_device* d) {
   d->adj_loop.release();
   if (d->batch_arena) cudaFree(d->batch_arena);
   if (d->arena) cudaFree(d->arena);
+  if (d->schur) cudaFree(d->schur);
   if (d->pinned) cudaFreeHost(d->pinned);
   if (d->stream) cudaStreamDestroy(d->stream);
   if (d->down) cudaStreamDestroy(d->down);

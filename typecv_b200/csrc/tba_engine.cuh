@@ -54,6 +54,9 @@ enum StateWord : int {
   S_INNER_R0 = 36,         // residual^2 that the current inner PCG run is measured against
   S_LOOP_ITERS = 37,       // PCG-step launches of the current device-side PCG loop
   S_LOOP_LIMIT = 38,       // the launches that loop may make (its iteration budget)
+  S_FOCAL_SFF = 39,        // the focal diagonal of the reduced system
+  S_WAIT = 40,             // a wait of the persistent PCG ran out of polls
+  S_READ = 48,             // words a state read copies to the host
   S_WORDS = 64
 };
 
@@ -71,6 +74,7 @@ __host__ __device__ inline size_t product_sums_bytes(uint32_t C, size_t word) { 
 constexpr int kPointThreads = 256;  // threads of the task kernels
 constexpr int kCameraThreads = 128;
 constexpr int kCameraPartials = 60;  // U 21 | b_c 6 | H_cf 6 | (W V^-1 W^T) 21 | W V^-1 b_p 6
+constexpr int kCameraPartialsExplicit = 66;  // the same | W V^-1 g_p 6 (the reduced focal column)
 constexpr int kScalarPartials = 4;   // H_ff obs | b_f obs | focal diag point terms | focal rhs point terms
 
 struct Params {
@@ -105,7 +109,7 @@ struct Params {
   double* rlim;        // C radial limits
   uint32_t* cm_point;  // M, camera-major
   double* cm_pixel;    // 2M, camera-major
-  double* pblk;        // 12P: V^-1 (6), b_p (3), padding
+  double* pblk;        // 12P: V^-1 (6), b_p (3), padding; explicit system: N (6), b_p (3), g_p (3)
   float* pblk32;       // 6P: V^-1 in FP32 for the FP32 product (mixed form), or null
   double* y;           // 4P: y_p of the current Schur product
   double* chunk_prod;  // 8 per camera chunk: sum W_i y (6), focal share
@@ -115,6 +119,14 @@ struct Params {
   float* F32;          // the same factors in FP32 (mixed precision), or null
   uint32_t Mpad;       // stride of a factor component
   uint32_t factored;   // 1: one-pass product over stored factors; 0: two-pass recompute
+  // The explicit reduced system (tba_schur.cuh), in place of the stored factors: the observations'
+  // records, the rows of S and the reduced focal column.
+  uint32_t schur;
+  double* A;                // 18 per observation
+  double* S;                // 36 per block
+  const uint32_t* row_ptr;  // C + 1
+  const uint32_t* col;
+  double* camScf;           // 6C: H_cf - sum W V^-1 g_p
   uint32_t refine;     // 1: this launch evaluates the FP64 product S x of the refinement
   uint32_t prod_blocks;  // grid of the one-pass product
   double* pw;          // 6C: the PCG direction of each camera in world axes (R^T omega, R^T v)

@@ -168,13 +168,54 @@ __global__ void k_finish_metrics(Params P) {
 
 // One observation's contributions to its point block: V (6 unique), b_p (3), the focal cross sum
 // w J_p^T jf (3) and an invalid flag; and its share of the focal diagonal and right-hand side.
-template <bool SHARED>
+//
+// EXPLICIT keeps what the observation's record A_i = W_i N_p needs once the point's N is known (the
+// record's columns are q x h and h with h = du B_0k + dv B_1k, B = w J_p N).
+struct ObsRecord {
+  double q[3], du[3], dv[3], wj[2][3];
+  bool on, dir;  // of a variable camera; of a bearing (no translation rows)
+};
+
+__device__ inline void record_of(const ObsRecord& o, const double n[6], double* out) {
+  double B[2][3];
+  for (int row = 0; row < 2; row++) root_t(n, o.wj[row], B[row]);
+  for (int k = 0; k < 3; k++) {
+    double h[3];
+    for (int j = 0; j < 3; j++) h[j] = o.du[j] * B[0][k] + o.dv[j] * B[1][k];
+    out[6 * k] = o.on ? o.q[1] * h[2] - o.q[2] * h[1] : 0.0;
+    out[6 * k + 1] = o.on ? o.q[2] * h[0] - o.q[0] * h[2] : 0.0;
+    out[6 * k + 2] = o.on ? o.q[0] * h[1] - o.q[1] * h[0] : 0.0;
+    for (int j = 0; j < 3; j++) out[6 * k + 3 + j] = o.on && !o.dir ? h[j] : 0.0;
+  }
+}
+
+// Copies a warp's `n` records between shared memory (18 words a lane) and their consecutive places.
+__device__ inline void store_records(const double* stage, double* A, uint32_t o0, uint32_t n, int lane) {
+  __syncwarp();
+  const double2* s = reinterpret_cast<const double2*>(stage);
+  double2* d = reinterpret_cast<double2*>(A + 18 * size_t(o0));
+  for (uint32_t k = lane; k < 9 * n; k += 32) d[k] = s[k];
+  __syncwarp();
+}
+__device__ inline void load_records(double* stage, const double* A, uint32_t o0, uint32_t n, int lane) {
+  __syncwarp();
+  const double2* s = reinterpret_cast<const double2*>(A + 18 * size_t(o0));
+  double2* d = reinterpret_cast<double2*>(stage);
+#pragma unroll
+  for (uint32_t j = 0; j < 9; j++)
+    if (32 * j + lane < 9 * n) d[32 * j + lane] = __ldg(s + 32 * j + lane);
+  __syncwarp();
+}
+
+template <bool SHARED, bool EXPLICIT>
 __device__ inline void point_obs(const Params& P, uint32_t i, uint32_t pt, double fscale, double (&v)[13],
-                                 double& hff, double& bf) {
+                                 double& hff, double& bf, ObsRecord& rec) {
   double pose[12];
   Geo g;
-  if (!observe(P, i, P.obs_camera[i], pt, fscale, pose, g)) {
+  const uint32_t cam = P.obs_camera[i];
+  if (!observe(P, i, cam, pt, fscale, pose, g)) {
     v[12] = 1;
+    rec.on = false;
     return;
   }
   double jp[2][3];
@@ -182,7 +223,7 @@ __device__ inline void point_obs(const Params& P, uint32_t i, uint32_t pt, doubl
     jp[0][c] = g.du[0] * pose[c] + g.du[1] * pose[3 + c] + g.du[2] * pose[6 + c];
     jp[1][c] = g.dv[0] * pose[c] + g.dv[1] * pose[3 + c] + g.dv[2] * pose[6 + c];
   }
-  if (P.factored) {
+  if (!EXPLICIT && P.factored) {
     // The world-axis factors of the products: q~ = R^T q, R^T du, R^T dv, w, jf.
     double f[kFactors];
     for (int c = 0; c < 3; c++) {
@@ -203,6 +244,17 @@ __device__ inline void point_obs(const Params& P, uint32_t i, uint32_t pt, doubl
   double wjp[2][3];
   for (int row = 0; row < 2; row++)
     for (int j = 0; j < 3; j++) wjp[row][j] = g.w * jp[row][j];
+  if (EXPLICIT) {
+    rec.on = P.active[cam] != 0;
+    rec.dir = directional(P, pt);
+    for (int j = 0; j < 3; j++) {
+      rec.q[j] = g.q[j];
+      rec.du[j] = g.du[j];
+      rec.dv[j] = g.dv[j];
+      rec.wj[0][j] = wjp[0][j];
+      rec.wj[1][j] = wjp[1][j];
+    }
+  }
   v[0] = wjp[0][0] * jp[0][0] + wjp[1][0] * jp[1][0];
   v[1] = wjp[0][0] * jp[0][1] + wjp[1][0] * jp[1][1];
   v[2] = wjp[0][0] * jp[0][2] + wjp[1][0] * jp[1][2];
@@ -219,6 +271,33 @@ __device__ inline void point_obs(const Params& P, uint32_t i, uint32_t pt, doubl
 
 // The point block of `pt` from its summed contributions: damping, equilibrated inverse,
 // right-hand side, and the point's share of the focal diagonal and right-hand side.
+// EXPLICIT: N (zero when the block failed) in `n`, and the point's N, b_p and g_p in its record.
+template <bool SHARED>
+__device__ inline void point_root(const Params& P, uint32_t pt, const double (&v)[13], double lambda, double& diag_pt,
+                                  double& rhs_pt, double (&n)[6]) {
+  double V[9] = {v[0], v[1], v[2], v[1], v[3], v[4], v[2], v[4], v[5]};
+  for (int j = 0; j < 3; j++) V[j * 4] += lambda * fmax(V[j * 4], 1e-10);
+  double2* blk = reinterpret_cast<double2*>(P.pblk + 12 * size_t(pt));
+  if (v[12] != 0 || !inverse_root3_spd(V, n)) {
+    P.state[S_POINT_FAILED] = 1;
+    for (int k = 0; k < 6; k++) n[k] = 0;
+    for (int k = 0; k < 6; k++) blk[k] = make_double2(0, 0);
+    return;
+  }
+  for (int k = 0; k < 3; k++) blk[k] = make_double2(n[2 * k], n[2 * k + 1]);
+  blk[3] = make_double2(v[6], v[7]);
+  blk[4] = make_double2(v[8], v[9]);
+  blk[5] = make_double2(v[10], v[11]);
+  if (SHARED) {
+    const double g[3] = {v[9], v[10], v[11]}, b[3] = {v[6], v[7], v[8]};
+    double ng[3], nb[3];
+    root_t(n, g, ng);
+    root_t(n, b, nb);
+    diag_pt += ng[0] * ng[0] + ng[1] * ng[1] + ng[2] * ng[2];
+    rhs_pt += ng[0] * nb[0] + ng[1] * nb[1] + ng[2] * nb[2];
+  }
+}
+
 template <bool SHARED>
 __device__ inline void point_finish(const Params& P, uint32_t pt, const double (&v)[13], double lambda,
                                     double& diag_pt, double& rhs_pt) {
@@ -252,43 +331,73 @@ __device__ inline void point_finish(const Params& P, uint32_t pt, const double (
   }
 }
 
-template <bool SHARED>
+template <bool SHARED, bool EXPLICIT>
 __global__ void __launch_bounds__(kPointThreads, TBA_POINT_MIN_BLOCKS) k_point_pass(Params P) {
   __shared__ double red[kScalarPartials * (kPointThreads / 32)];
+  __shared__ double2 stage_all[EXPLICIT ? kPointThreads * 9 : 1];
   if (P.state[S_ACTIVE] == 0) return;
   const double lambda = P.state[S_LAMBDA], fscale = focal_scale(P, P.state[S_LOG_FOCAL]);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  double* stage = reinterpret_cast<double*>(stage_all) + (EXPLICIT ? warp * 32 * 18 : 0);
   double sc[kScalarPartials] = {0, 0, 0, 0};  // hff, bf, diag_pt, rhs_pt (lane-local)
   uint32_t tb, te;
   block_tasks(P, tb, te);
   for (uint32_t t = tb + warp; t < te; t += nwarps) {
     const uint32_t p0 = P.tasks[t], p1 = P.tasks[t + 1];
     const uint32_t o0 = P.point_start[p0], n = P.point_start[p1] - o0;
+    ObsRecord rec;
+    rec.on = false;
     if (n <= uint32_t(kTaskObs)) {
       double v[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
       int seg = -1 - lane;
       uint32_t pt = 0;
-      if (uint32_t(lane) < n) {
+      const bool valid = uint32_t(lane) < n;
+      if (valid) {
         pt = P.obs_point[o0 + lane];
         seg = int(pt);
-        point_obs<SHARED>(P, o0 + lane, pt, fscale, v, sc[0], sc[1]);
+        point_obs<SHARED, EXPLICIT>(P, o0 + lane, pt, fscale, v, sc[0], sc[1], rec);
       }
       const Runs runs = lane_runs(seg, lane);
       run_scan(v, runs);
-      if (uint32_t(lane) < n && run_tail(runs, lane))
+      const bool tail = valid && run_tail(runs, lane);
+      if (EXPLICIT) {
+        double root[6] = {0, 0, 0, 0, 0, 0};
+        if (tail) point_root<SHARED>(P, pt, v, lambda, sc[2], sc[3], root);
+        const unsigned tails = __ballot_sync(kFull, tail);
+        const int src = valid ? __ffs(tails & (kFull << lane)) - 1 : lane;
+        for (int k = 0; k < 6; k++) root[k] = __shfl_sync(kFull, root[k], src);
+        if (valid) record_of(rec, root, stage + 18 * lane);
+        store_records(stage, P.A, o0, n, lane);
+      } else if (tail) {
         point_finish<SHARED>(P, pt, v, lambda, sc[2], sc[3]);
+      }
     } else {
       const uint32_t pt = P.obs_point[o0];
       double v[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
       for (uint32_t base = 0; base < n; base += kTaskObs) {
         if (base + lane < n) {
           double u[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-          point_obs<SHARED>(P, o0 + base + lane, pt, fscale, u, sc[0], sc[1]);
+          point_obs<SHARED, EXPLICIT>(P, o0 + base + lane, pt, fscale, u, sc[0], sc[1], rec);
           for (int k = 0; k < 13; k++) v[k] += u[k];
         }
       }
       warp_allsum(v);
-      if (lane == 0) point_finish<SHARED>(P, pt, v, lambda, sc[2], sc[3]);
+      if (EXPLICIT) {
+        double root[6] = {0, 0, 0, 0, 0, 0};
+        if (lane == 0) point_root<SHARED>(P, pt, v, lambda, sc[2], sc[3], root);
+        for (int k = 0; k < 6; k++) root[k] = __shfl_sync(kFull, root[k], 0);
+        for (uint32_t base = 0; base < n; base += kTaskObs) {
+          const uint32_t m = min(uint32_t(kTaskObs), n - base);
+          if (uint32_t(lane) < m) {
+            double u[13], skip0 = 0, skip1 = 0;
+            point_obs<SHARED, EXPLICIT>(P, o0 + base + lane, pt, fscale, u, skip0, skip1, rec);
+            record_of(rec, root, stage + 18 * lane);
+          }
+          store_records(stage, P.A, o0 + base, m, lane);
+        }
+      } else if (lane == 0) {
+        point_finish<SHARED>(P, pt, v, lambda, sc[2], sc[3]);
+      }
     }
   }
   block_sum(sc, red);
@@ -306,8 +415,10 @@ __device__ inline void camera_rows(const Geo& g, bool dir, double jc[2][6]) {
     for (int c = 3; c < 6; c++) jc[0][c] = jc[1][c] = 0;
 }
 
+template <bool EXPLICIT>
 __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camera_pass(Params P) {
-  __shared__ double red[kCameraPartials * (kCameraThreads / 32)];
+  constexpr int kParts = EXPLICIT ? kCameraPartialsExplicit : kCameraPartials, kSecond = kParts - 33;
+  __shared__ double red[kParts * (kCameraThreads / 32)];
   if (P.state[S_ACTIVE] == 0) return;
   const uint32_t ch = blockIdx.x, c = P.chunk_cam[ch];
   if (P.active[c] == 0) return;
@@ -339,13 +450,13 @@ __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camer
     for (int j = 0; j < 33; j++) {
       double s = a[j];
       for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(kFull, s, d);
-      if (lane == 0) red[warp * kCameraPartials + j] = s;
+      if (lane == 0) red[warp * kParts + j] = s;
     }
   }
-  // Pass 2: W V^-1 W^T (lower triangle) and W V^-1 b_p.
+  // Pass 2: W V^-1 W^T (lower triangle) and W V^-1 b_p (explicit system: from A = W N, and W V^-1 g_p).
   {
-    double b[27];
-    for (int j = 0; j < 27; j++) b[j] = 0;
+    double b[kSecond];
+    for (int j = 0; j < kSecond; j++) b[j] = 0;
     for (uint32_t kk = k0 + threadIdx.x; kk < k1; kk += blockDim.x) {
       const uint32_t pt = P.cm_point[kk];
       const double2 uv = reinterpret_cast<const double2*>(P.cm_pixel)[kk];
@@ -364,6 +475,19 @@ __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camer
         for (int l = 0; l < 3; l++) Wc[j][l] = jc[0][j] * jp[0][l] + jc[1][j] * jp[1][l];
       double vb[6], bb[3];
       load6(P.pblk + 12 * size_t(pt), vb);
+      if (EXPLICIT) {
+        double tail[6], nb[3], ng[3], A[6][3];
+        load6(P.pblk + 12 * size_t(pt) + 6, tail);
+        root_t(vb, tail, nb);
+        root_t(vb, tail + 3, ng);
+        for (int j = 0; j < 6; j++) {
+          root_t(vb, Wc[j], A[j]);
+          for (int l = 0; l <= j; l++) b[sym6(j, l)] += A[j][0] * A[l][0] + A[j][1] * A[l][1] + A[j][2] * A[l][2];
+          b[21 + j] += A[j][0] * nb[0] + A[j][1] * nb[1] + A[j][2] * nb[2];
+          b[kSecond - 6 + j] += A[j][0] * ng[0] + A[j][1] * ng[1] + A[j][2] * ng[2];
+        }
+        continue;
+      }
       bb[0] = P.pblk[12 * size_t(pt) + 6];
       bb[1] = P.pblk[12 * size_t(pt) + 7];
       bb[2] = P.pblk[12 * size_t(pt) + 8];
@@ -375,61 +499,89 @@ __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camer
         b[21 + j] += t0 * bb[0] + t1 * bb[1] + t2 * bb[2];
       }
     }
-    for (int j = 0; j < 27; j++) {
+    for (int j = 0; j < kSecond; j++) {
       double s = b[j];
       for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(kFull, s, d);
-      if (lane == 0) red[warp * kCameraPartials + 33 + j] = s;
+      if (lane == 0) red[warp * kParts + 33 + j] = s;
     }
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < kCameraPartials; j += blockDim.x) {
+  for (int j = threadIdx.x; j < kParts; j += blockDim.x) {
     double s = 0;
-    for (int w = 0; w < nwarps; w++) s += red[w * kCameraPartials + j];
-    P.chunk_part[size_t(kCameraPartials) * ch + j] = s;
+    for (int w = 0; w < nwarps; w++) s += red[w * kParts + j];
+    P.chunk_part[size_t(kParts) * ch + j] = s;
   }
 }
 
-__global__ void k_camera_finish(Params P) {
+// One camera per warp: its chunks' partial sums (a value a lane), the damped block and right-hand side,
+// and the inverse of the preconditioner block.  The lanes hold the Cholesky factor alike and solve one
+// column of the inverse each (one thread per camera spent 42 us on 7 cameras and 70 us on 200).
+constexpr int kFinishThreads = 128;
+
+template <bool EXPLICIT>
+__global__ void __launch_bounds__(kFinishThreads) k_camera_finish(Params P) {
+  constexpr int kParts = EXPLICIT ? kCameraPartialsExplicit : kCameraPartials;
+  __shared__ double sums[kFinishThreads / 32][kParts], inverse[kFinishThreads / 32][36];
   if (P.state[S_ACTIVE] == 0) return;
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * (kFinishThreads / 32) + warp;
   if (c >= P.C) return;
   double* U = P.camU + 21 * size_t(c);
   double* Minv = P.camMinv + 36 * size_t(c);
-  double* rhs = P.camRhs + 6 * size_t(c);
-  double* hcf = P.camHcf + 6 * size_t(c);
+  double* diagonal = nullptr;  // the camera's diagonal block in the explicit system
+  if (EXPLICIT) {
+    const uint32_t b0 = P.row_ptr[c];
+    uint32_t lo = 0, hi = P.row_ptr[c + 1] - b0 - 1;  // the row holds camera c
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (P.col[b0 + mid] < c) lo = mid + 1;
+      else hi = mid;
+    }
+    diagonal = P.S + 36 * size_t(b0 + lo);
+  }
   if (P.active[c] == 0) {
-    for (int j = 0; j < 21; j++) U[j] = 0;
-    for (int j = 0; j < 36; j++) Minv[j] = 0;
-    for (int j = 0; j < 6; j++) {
-      U[sym6(j, j)] = 1;
-      Minv[j * 7] = 1;
-      rhs[j] = 0;
-      hcf[j] = 0;
+    for (int j = lane; j < 36; j += 32) {
+      const double v = j % 7 == 0 ? 1 : 0;
+      Minv[j] = v;
+      if (EXPLICIT) diagonal[j] = v;
+    }
+    if (lane < 6) {
+      for (int k = 0; k <= lane; k++) U[sym6(lane, k)] = k == lane ? 1 : 0;
+      P.camRhs[6 * size_t(c) + lane] = 0;
+      P.camHcf[6 * size_t(c) + lane] = 0;
+      if (EXPLICIT) P.camScf[6 * size_t(c) + lane] = 0;
     }
     return;
   }
-  double a[kCameraPartials];
-  for (int j = 0; j < kCameraPartials; j++) a[j] = 0;
-  for (uint32_t ch = P.cam_chunk[c]; ch < P.cam_chunk[c + 1]; ch++)
-    for (int j = 0; j < kCameraPartials; j++) a[j] += P.chunk_part[size_t(kCameraPartials) * ch + j];
-  const double lambda = P.state[S_LAMBDA];
-  for (int j = 0; j < 6; j++) a[sym6(j, j)] += lambda * fmax(a[sym6(j, j)], 1e-10);
+  double* a = sums[warp];
+  for (int j = lane; j < kParts; j += 32) {
+    double s = 0;
+#pragma unroll 4
+    for (uint32_t ch = P.cam_chunk[c]; ch < P.cam_chunk[c + 1]; ch++) s += P.chunk_part[size_t(kParts) * ch + j];
+    a[j] = s;
+  }
+  __syncwarp();
+  if (lane < 6) {
+    const double d = a[sym6(lane, lane)];
+    a[sym6(lane, lane)] = d + P.state[S_LAMBDA] * fmax(d, 1e-10);
+    P.camRhs[6 * size_t(c) + lane] = a[21 + lane] - a[54 + lane];
+    P.camHcf[6 * size_t(c) + lane] = a[27 + lane];
+    if (EXPLICIT) P.camScf[6 * size_t(c) + lane] = a[27 + lane] - a[kParts - 6 + lane];
+  }
+  __syncwarp();
   double S[21];
-  for (int j = 0; j < 21; j++) {
-    U[j] = a[j];
-    S[j] = a[j] - a[33 + j];
-  }
-  for (int j = 0; j < 6; j++) {
-    rhs[j] = a[21 + j] - a[54 + j];
-    hcf[j] = a[27 + j];
-  }
-  double inv[36];
-  if (inverse6_spd(S, inv)) {
-    for (int j = 0; j < 36; j++) Minv[j] = inv[j];
-  } else {
-    for (int j = 0; j < 36; j++) Minv[j] = 0;
-    Minv[0] = -1;
-  }
+#pragma unroll
+  for (int j = 0; j < 21; j++) S[j] = a[j] - a[33 + j];
+  if (lane < 21) U[lane] = a[lane];
+  if (EXPLICIT)
+    for (int j = lane; j < 36; j += 32) diagonal[j] = a[sym6(j / 6, j % 6)] - a[33 + sym6(j / 6, j % 6)];
+  double col[6];
+  const bool ok = inverse6_column(S, lane < 6 ? lane : 0, col);
+  if (lane < 6)
+    for (int i = 0; i < 6; i++) inverse[warp][6 * i + lane] = col[i];
+  __syncwarp();
+  for (int j = lane; j < 36; j += 32)
+    Minv[j] = ok ? (inverse[warp][j] + inverse[warp][j % 6 * 6 + j / 6]) * 0.5 : (j == 0 ? -1.0 : 0.0);
 }
 
 // ---- K9/K21: damped focal scalars and the PCG start --------------------------------------------
@@ -460,6 +612,7 @@ __global__ void __launch_bounds__(1024) k_pcg_init(Params P) {
       diag += st[S_LAMBDA] * fmax(diag, 1e-10);
       st[S_FOCAL_DIAG] = diag;
       const double sff = diag - v[2];
+      st[S_FOCAL_SFF] = sff;
       st[S_FOCAL_INV] = sff > 0 ? 1 / sff : -1;
       st[S_FOCAL_RHS] = -v[1] - v[3];
     }
@@ -524,6 +677,14 @@ __device__ inline void schur_point_finish(const Params& P, uint32_t pt, const do
   double vb[6];
   load6(P.pblk + 12 * size_t(pt), vb);
   double2* y = reinterpret_cast<double2*>(P.y + 4 * size_t(pt));
+  if (P.schur) {
+    double t[3], v[3];
+    root_t(vb, s, t);
+    root_n(vb, t, v);
+    y[0] = make_double2(v[0], v[1]);
+    y[1] = make_double2(v[2], 0);
+    return;
+  }
   y[0] = make_double2(vb[0] * s[0] + vb[1] * s[1] + vb[2] * s[2], vb[1] * s[0] + vb[3] * s[1] + vb[4] * s[2]);
   y[1] = make_double2(vb[2] * s[0] + vb[4] * s[1] + vb[5] * s[2], 0);
 }
@@ -953,6 +1114,69 @@ __global__ void __launch_bounds__(256) k_product_columns(Params P) {
   if (SHARED) {
     const double pf = P.p[n];
     const double spf = st[S_FOCAL_DIAG] * pf + t[1] + __ldcg(P.Sp + n);
+    P.Sp[n] = spf;
+    den += pf * spf;
+  }
+  *P.ticket = 0;
+  const double alpha = st[S_RHO] / den;
+  if (!(den > 0) || !(fabs(alpha) < 1e20)) {
+    st[S_CG_ACTIVE] = 0;
+    st[S_CG_FAILED] = 1;
+    return;
+  }
+  st[S_ALPHA] = alpha;
+}
+
+// The product of the explicit system, one camera row per warp, for PCG steps launched one by one (the
+// persistent PCG of tba_pcg.cu does the same inside its launch); the last block adds the focal row
+// and forms alpha, as k_product_columns.
+template <bool SHARED>
+__global__ void __launch_bounds__(256) k_schur_rows(Params P) {
+  __shared__ double red[2 * 8];
+  if (P.state[S_CG_ACTIVE] == 0) return;
+  const uint32_t n = 6 * P.C, c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  double v[2] = {0, 0};
+  if (c < P.C) {
+    const uint32_t b0 = P.row_ptr[c], w = 6 * (P.row_ptr[c + 1] - b0);
+    const double* row = P.S + 36 * size_t(b0);
+    double acc[6] = {0, 0, 0, 0, 0, 0};
+    for (uint32_t j = lane; j < w; j += 32) {
+      const uint32_t b = j / 6;
+      const double x = P.p[6 * P.col[b0 + b] + (j - 6 * b)];
+      for (int a = 0; a < 6; a++) acc[a] += row[6 * size_t(j) + a] * x;
+    }
+    warp_allsum(acc);
+    if (lane < 6) {
+      double sp = acc[0];
+      for (int a = 1; a < 6; a++)
+        if (lane == a) sp = acc[a];
+      const uint32_t j = 6 * c + lane;
+      if (SHARED) {
+        sp += P.camScf[j] * P.p[n];
+        v[1] = P.camScf[j] * P.p[j];
+      }
+      P.Sp[j] = sp;
+      v[0] = P.p[j] * sp;
+    }
+  }
+  block_sum(v, red);
+  if (threadIdx.x == 0) {
+    P.blk_part[4 * blockIdx.x] = v[0];
+    P.blk_part[4 * blockIdx.x + 1] = v[1];
+  }
+  if (!last_block(P.ticket)) return;
+  double t[2] = {0, 0};
+  for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+    t[0] += __ldcg(P.blk_part + 4 * b);
+    t[1] += __ldcg(P.blk_part + 4 * b + 1);
+  }
+  block_sum(t, red);
+  if (threadIdx.x != 0) return;
+  double* st = P.state;
+  double den = t[0];
+  if (SHARED) {
+    const double pf = P.p[n], spf = st[S_FOCAL_SFF] * pf + t[1];
     P.Sp[n] = spf;
     den += pf * spf;
   }
@@ -1411,15 +1635,27 @@ __device__ inline void update_wt(const Params& P, uint32_t i, uint32_t c, uint32
 
 // The candidate point: X + V^-1 (b_p - sum_i W_i^T x), then the bearing or similarity
 // normalisation of the gauge.
-__device__ inline void candidate_point(const Params& P, uint32_t pt, const double s[3], double X[3]) {
+// (EXPLICIT: s = sum_i A_i^T x, so X + N (N^T (b_p - g_p x_f) - s).)
+template <bool EXPLICIT>
+__device__ inline void candidate_point(const Params& P, uint32_t pt, const double s[3], double xf, double X[3]) {
   double vb[6];
   load6(P.pblk + 12 * size_t(pt), vb);
-  const double* bb = P.pblk + 12 * size_t(pt) + 6;
-  const double r0 = bb[0] - s[0], r1 = bb[1] - s[1], r2 = bb[2] - s[2];
   const double* X0 = P.points + 3 * size_t(pt);
-  X[0] = X0[0] + (vb[0] * r0 + vb[1] * r1 + vb[2] * r2);
-  X[1] = X0[1] + (vb[1] * r0 + vb[3] * r1 + vb[4] * r2);
-  X[2] = X0[2] + (vb[2] * r0 + vb[4] * r1 + vb[5] * r2);
+  if (EXPLICIT) {
+    double tail[6], t[3], d[3];
+    load6(P.pblk + 12 * size_t(pt) + 6, tail);
+    for (int k = 0; k < 3; k++) tail[k] -= tail[3 + k] * xf;
+    root_t(vb, tail, t);
+    for (int k = 0; k < 3; k++) t[k] -= s[k];
+    root_n(vb, t, d);
+    for (int k = 0; k < 3; k++) X[k] = X0[k] + d[k];
+  } else {
+    const double* bb = P.pblk + 12 * size_t(pt) + 6;
+    const double r0 = bb[0] - s[0], r1 = bb[1] - s[1], r2 = bb[2] - s[2];
+    X[0] = X0[0] + (vb[0] * r0 + vb[1] * r1 + vb[2] * r2);
+    X[1] = X0[1] + (vb[1] * r0 + vb[3] * r1 + vb[4] * r2);
+    X[2] = X0[2] + (vb[2] * r0 + vb[4] * r1 + vb[5] * r2);
+  }
   const double* st = P.state;
   if (directional(P, pt)) {
     const double norm = sqrt(X[0] * X[0] + X[1] * X[1] + X[2] * X[2]);
@@ -1448,14 +1684,26 @@ __device__ inline void candidate_obs(const Params& P, uint32_t i, uint32_t pt, c
   sq += os;
 }
 
-template <bool SHARED>
+// A_i^T x of one observation, from its record.
+__device__ inline void record_wt(const double* rec, const double* x, double t[3]) {
+  double xc[6];
+  load6(x, xc);
+  for (int k = 0; k < 3; k++) {
+    t[k] = 0;
+    for (int j = 0; j < 6; j++) t[k] += rec[6 * k + j] * xc[j];
+  }
+}
+
+template <bool SHARED, bool EXPLICIT>
 __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_points(Params P) {
   __shared__ double red[2 * (kPointThreads / 32)];
+  __shared__ double2 stage_all[EXPLICIT ? kPointThreads * 9 : 1];
   const double* st = P.state;
   if (st[S_ACTIVE] == 0 || st[S_CG_FAILED] != 0 || st[S_TRIAL_VALID] == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const double fscale = focal_scale(P, st[S_LOG_FOCAL]), fscale_trial = focal_scale(P, st[S_LOG_FOCAL_TRIAL]);
   const double xf = SHARED ? P.x[P.m - 1] : 0.0;
+  double* stage = reinterpret_cast<double*>(stage_all) + (EXPLICIT ? warp * 32 * 18 : 0);
   double cs[2] = {0, 0};
   uint32_t tb, te;
   block_tasks(P, tb, te);
@@ -1468,16 +1716,18 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_
       double s[3] = {0, 0, 0};
       int seg = -1 - lane;
       uint32_t pt = 0;
+      if (EXPLICIT) load_records(stage, P.A, o0, n, lane);
       if (valid) {
         pt = P.obs_point[i];
         seg = int(pt);
-        update_wt(P, i, P.obs_camera[i], pt, fscale, xf, SHARED, s);
+        if (EXPLICIT) record_wt(stage + 18 * lane, P.x + 6 * size_t(P.obs_camera[i]), s);
+        else update_wt(P, i, P.obs_camera[i], pt, fscale, xf, SHARED, s);
       }
       const Runs runs = lane_runs(seg, lane);
       run_scan(s, runs);
       const bool tail = valid && run_tail(runs, lane);
       double X[3] = {0, 0, 0};
-      if (tail) candidate_point(P, pt, s, X);
+      if (tail) candidate_point<EXPLICIT>(P, pt, s, xf, X);
       const unsigned tails = __ballot_sync(kFull, tail);
       const int src = valid ? __ffs(tails & (kFull << lane)) - 1 : lane;
       for (int j = 0; j < 3; j++) X[j] = __shfl_sync(kFull, X[j], src);
@@ -1489,14 +1739,15 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_
         if (base + lane < n) {
           const uint32_t i = o0 + base + lane;
           double u[3];
-          update_wt(P, i, P.obs_camera[i], pt, fscale, xf, SHARED, u);
+          if (EXPLICIT) record_wt(P.A + 18 * size_t(i), P.x + 6 * size_t(P.obs_camera[i]), u);
+          else update_wt(P, i, P.obs_camera[i], pt, fscale, xf, SHARED, u);
           s[0] += u[0];
           s[1] += u[1];
           s[2] += u[2];
         }
       warp_allsum(s);
       double X[3] = {0, 0, 0};
-      if (lane == 0) candidate_point(P, pt, s, X);
+      if (lane == 0) candidate_point<EXPLICIT>(P, pt, s, xf, X);
       for (int j = 0; j < 3; j++) X[j] = __shfl_sync(kFull, X[j], 0);
       for (uint32_t base = 0; base < n; base += kTaskObs)
         if (base + lane < n) candidate_obs(P, o0 + base + lane, pt, X, fscale_trial, cs[0], cs[1]);
@@ -1576,7 +1827,7 @@ __global__ void k_pack(Params P) {
 
 uint32_t product_finish_blocks(const Params& p) {
   const uint32_t a = (6 * p.C + kReduceThreads - 1) / kReduceThreads, b = (p.m + kUpdateRows - 1) / kUpdateRows;
-  const uint32_t c = (p.m + kColumnRows - 1) / kColumnRows;
+  const uint32_t c = (p.m + kColumnRows - 1) / kColumnRows;  // (covers the C / 8 blocks of k_schur_rows)
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 
@@ -1665,13 +1916,31 @@ void launch_initialize(const Params& p, cudaStream_t s) {
 void launch_cost(const Params& p, cudaStream_t s) { k_cost<<<p.task_blocks, kPointThreads, 0, s>>>(p); }
 void launch_finish_metrics(const Params& p, cudaStream_t s) { k_finish_metrics<<<1, 1024, 0, s>>>(p); }
 void launch_point_pass(const Params& p, cudaStream_t s) {
-  if (p.shared) k_point_pass<true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
-  else k_point_pass<false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  if (p.schur) {
+    if (p.shared) k_point_pass<true, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    else k_point_pass<false, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  } else if (p.shared) {
+    k_point_pass<true, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  } else {
+    k_point_pass<false, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  }
 }
-void launch_camera_pass(const Params& p, cudaStream_t s) { k_camera_pass<<<p.nchunks, kCameraThreads, 0, s>>>(p); }
-void launch_camera_finish(const Params& p, cudaStream_t s) { k_camera_finish<<<(p.C + 127) / 128, 128, 0, s>>>(p); }
+void launch_camera_pass(const Params& p, cudaStream_t s) {
+  if (p.schur) k_camera_pass<true><<<p.nchunks, kCameraThreads, 0, s>>>(p);
+  else k_camera_pass<false><<<p.nchunks, kCameraThreads, 0, s>>>(p);
+}
+void launch_camera_finish(const Params& p, cudaStream_t s) {
+  constexpr uint32_t per = kFinishThreads / 32;
+  if (p.schur) k_camera_finish<true><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
+  else k_camera_finish<false><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
+}
 void launch_pcg_init(const Params& p, cudaStream_t s) { k_pcg_init<<<1, 1024, 0, s>>>(p); }
 void launch_product(const Params& p, cudaStream_t s) {
+  if (p.schur && p.factored) {
+    if (p.shared) k_schur_rows<true><<<(p.C + 7) / 8, 256, 0, s>>>(p);
+    else k_schur_rows<false><<<(p.C + 7) / 8, 256, 0, s>>>(p);
+    return;
+  }
   if (p.factored) {
     Params q = p;
     void* args[] = {&q};
@@ -1687,7 +1956,9 @@ void launch_product(const Params& p, cudaStream_t s) {
   }
 }
 void launch_product_finish(const Params& p, cudaStream_t s) {
-  if (p.factored) {
+  if (p.schur) {
+    // (the product's last block formed alpha)
+  } else if (p.factored) {
     if (p.shared) k_product_columns<true><<<(p.m + kColumnRows - 1) / kColumnRows, 256, 0, s>>>(p);
     else k_product_columns<false><<<(p.m + kColumnRows - 1) / kColumnRows, 256, 0, s>>>(p);
   } else {
@@ -1724,8 +1995,14 @@ void launch_product_rows(const Params& p, double* out, cudaStream_t s) {
 }
 void launch_update_cameras(const Params& p, cudaStream_t s) { k_update_cameras<<<1, 256, 0, s>>>(p); }
 void launch_update_points(const Params& p, cudaStream_t s) {
-  if (p.shared) k_update_points<true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
-  else k_update_points<false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  if (p.schur) {
+    if (p.shared) k_update_points<true, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    else k_update_points<false, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  } else if (p.shared) {
+    k_update_points<true, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  } else {
+    k_update_points<false, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+  }
 }
 void launch_accept(const Params& p, cudaStream_t s) { k_accept<<<1, 256, 0, s>>>(p); }
 void launch_commit(const Params& p, cudaStream_t s) {

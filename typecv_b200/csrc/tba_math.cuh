@@ -101,6 +101,40 @@ __host__ __device__ inline bool inverse3_spd(const double a[9], double out[6]) {
   return true;
 }
 
+// The upper triangular N with a^-1 = N N^T for a 3x3 SPD block `a` (row-major), from the same
+// equilibrated Cholesky factor and pivot floors as inverse3_spd: N = D L^-T.  Output: 00, 01, 02, 11,
+// 12, 22.
+__host__ __device__ inline bool inverse_root3_spd(const double a[9], double n[6]) {
+  if (!(fmin(a[0], fmin(a[4], a[8])) > 0)) return false;
+  const double d0 = 1 / sqrt(a[0]), d1 = 1 / sqrt(a[4]), d2 = 1 / sqrt(a[8]);
+  const double l10 = a[3] * d0 * d1, l20 = a[6] * d0 * d2;
+  const double pivot1 = 1 - l10 * l10;
+  if (!(pivot1 > 1e-14)) return false;
+  const double l11 = sqrt(pivot1), l21 = (a[7] * d1 * d2 - l20 * l10) / l11;
+  const double pivot2 = 1 - l20 * l20 - l21 * l21;
+  if (!(pivot2 > 1e-14)) return false;
+  const double i11 = 1 / l11, i22 = 1 / sqrt(pivot2);
+  n[0] = d0;
+  n[1] = -d0 * l10 * i11;
+  n[2] = d0 * (l10 * l21 * i11 - l20) * i22;
+  n[3] = d1 * i11;
+  n[4] = -d1 * l21 * i11 * i22;
+  n[5] = d2 * i22;
+  return true;
+}
+
+// N^T s and N s.
+__host__ __device__ inline void root_t(const double n[6], const double s[3], double out[3]) {
+  out[0] = n[0] * s[0];
+  out[1] = n[1] * s[0] + n[3] * s[1];
+  out[2] = n[2] * s[0] + n[4] * s[1] + n[5] * s[2];
+}
+__host__ __device__ inline void root_n(const double n[6], const double s[3], double out[3]) {
+  out[0] = n[0] * s[0] + n[1] * s[1] + n[2] * s[2];
+  out[1] = n[3] * s[1] + n[4] * s[2];
+  out[2] = n[5] * s[2];
+}
+
 // solve3: x = a^-1 b by the equilibrated Cholesky factorisation of the SPD block `a` (row-major),
 // with the same pivot floors as inverse3_spd; false when `a` is not safely positive definite.
 __host__ __device__ inline bool solve3_spd(const double a[9], const double b[3], double x[3]) {
@@ -124,6 +158,51 @@ __host__ __device__ inline bool solve3_spd(const double a[9], const double b[3],
 // Index of entry (i, j) of a symmetric 6x6 block stored as its lower triangle, row by row.
 __host__ __device__ constexpr int sym6(int i, int j) {
   return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
+}
+
+// Column `column` of the inverse that inverse6_spd forms, before its symmetrisation; every index of
+// the factor is known at compile time, so it stays in registers.
+__device__ inline bool inverse6_column(const double (&s)[21], int column, double (&out)[6]) {
+  double L[21], scale[6], inv[6];
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    ok = ok && s[sym6(i, i)] > 0;
+    scale[i] = 1 / sqrt(s[sym6(i, i)]);
+  }
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+#pragma unroll
+    for (int j = 0; j <= i; j++) {
+      double value = s[sym6(i, j)] * scale[i] * scale[j];
+#pragma unroll
+      for (int k = 0; k < j; k++) value -= L[sym6(i, k)] * L[sym6(j, k)];
+      if (i == j) {
+        ok = ok && value > 1e-14;
+        L[sym6(i, i)] = sqrt(value);
+        inv[i] = 1 / L[sym6(i, i)];
+      } else {
+        L[sym6(i, j)] = value * inv[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    double t = i == column ? scale[i] : 0.0;
+#pragma unroll
+    for (int j = 0; j < i; j++) t -= L[sym6(i, j)] * out[j];
+    out[i] = t * inv[i];
+  }
+#pragma unroll
+  for (int i = 5; i >= 0; i--) {
+    double t = out[i];
+#pragma unroll
+    for (int j = i + 1; j < 6; j++) t -= L[sym6(j, i)] * out[j];
+    out[i] = t * inv[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 6; i++) out[i] *= scale[i];
+  return ok;
 }
 
 // solve6 on the six unit vectors: the equilibrated Cholesky inverse of a 6x6 SPD block given by

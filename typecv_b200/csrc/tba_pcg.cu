@@ -1,0 +1,390 @@
+// The persistent PCG (tba_pcg.cuh), sm_100a, FP64.
+//
+// Each block owns a run of cameras (about the same number of 6x6 blocks of S each) and keeps in shared
+// memory, as far as they fit, its rows of S, the direction p of the cameras its rows touch, and its
+// shares of x, r and S p.  A step is
+//   p = z + beta p of the block's columns, S p of its rows, p . S p          -> sum over the grid, alpha
+//   x += alpha p, r -= alpha S p, z = M^-1 r of its own cameras, r.r, z.r    -> sum over the grid, beta
+// and only z and four partial sums a block cross between blocks, as values that carry their step's
+// number (Flagged): no barrier, no fence, and the L1 keeps what the step only reads.  Every block adds
+// the partial sums in the same order, so all take the same decisions.  A block can publish a step's z
+// only once every block has published the sums that follow its use of the last z, so one buffer does.
+// What bounds a step is the two exchanges through the L2 (about 0.7 us each) with many blocks, and the
+// block's own chain of reductions with one.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "tba_pcg.cuh"
+#include "tba_warp.cuh"
+
+namespace tba {
+namespace {
+
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr uint32_t kSmemBytes = 208 * 1024;
+
+__device__ __forceinline__ void publish(Flagged* p, double v, uint64_t step) {
+  asm volatile(
+      "{\n .reg .b128 w;\n mov.b128 w, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], w;\n}" ::"l"(p),
+      "l"(__double_as_longlong(v)), "l"(step)
+      : "memory");
+}
+
+__device__ __forceinline__ Flagged peek(const Flagged* p) {
+  uint64_t v, s;
+  asm volatile("{\n .reg .b128 w;\n ld.relaxed.gpu.global.b128 w, [%2];\n mov.b128 {%0, %1}, w;\n}"
+               : "=l"(v), "=l"(s)
+               : "l"(p)
+               : "memory");
+  return Flagged{__longlong_as_double(v), s};
+}
+
+// The value of `step`; false when it did not come within the poll limit.
+__device__ __forceinline__ bool await(const Flagged* p, uint64_t step, double& v) {
+  for (uint32_t k = 0; k < kPcgWaitPolls; k++) {
+    const Flagged f = peek(p);
+    if (f.step == step) {
+      v = f.value;
+      return true;
+    }
+  }
+  return false;
+}
+
+struct Shared {
+  double red[2][kWarps][2];
+  double part[kWarps][6];
+  double sum[2];
+  int gave_up;
+};
+
+// Adds v over the grid; every thread returns with the sums (false: a wait gave up).  `which` is the
+// step's first or second reduction.
+__device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], uint64_t step, int which) {
+  warp_allsum(v);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) {
+    sh.red[which][warp][0] = v[0];
+    sh.red[which][warp][1] = v[1];
+  }
+  __syncthreads();
+  if (gridDim.x == 1) {
+    v[0] = v[1] = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+      v[0] += sh.red[which][w][0];
+      v[1] += sh.red[which][w][1];
+    }
+    return true;
+  }
+  if (warp == 0) {
+    double t[2] = {lane < kWarps ? sh.red[which][lane][0] : 0.0, lane < kWarps ? sh.red[which][lane][1] : 0.0};
+    warp_allsum(t);
+    Flagged* slots = A.slots + 2 * size_t(which);
+    if (lane < 2) publish(slots + 4 * size_t(blockIdx.x) + lane, lane == 0 ? t[0] : t[1], step);
+    bool ok = sh.gave_up == 0;
+    t[0] = t[1] = 0;
+    for (uint32_t b = lane; b < gridDim.x && ok; b += 32) {
+      double s0 = 0, s1 = 0;
+      ok = await(slots + 4 * size_t(b), step, s0) && await(slots + 4 * size_t(b) + 1, step, s1);
+      t[0] += s0;
+      t[1] += s1;
+    }
+    warp_allsum(t);
+    ok = __all_sync(kFull, ok);
+    if (lane == 0) {
+      sh.sum[0] = t[0];
+      sh.sum[1] = t[1];
+      if (!ok) sh.gave_up = 1;
+    }
+  }
+  __syncthreads();
+  v[0] = sh.sum[0];
+  v[1] = sh.sum[1];
+  return sh.gave_up == 0;
+}
+
+// Shares of about the same number of blocks of S; the distinct cameras of a share's columns.
+__global__ void __launch_bounds__(256) k_pcg_plan(PcgSystem A) {
+  extern __shared__ uint32_t place[];  // C: 1 for a camera that occurs, then its place
+  __shared__ uint32_t range[2], warp_sum[8];
+  if (threadIdx.x < 2) {
+    const uint64_t target = uint64_t(A.row_ptr[A.C]) * (blockIdx.x + threadIdx.x) / gridDim.x;
+    uint32_t lo = 0, hi = A.C;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (A.row_ptr[mid] < target) lo = mid + 1;
+      else hi = mid;
+    }
+    range[threadIdx.x] = lo;
+    A.share[blockIdx.x + threadIdx.x] = lo;
+  }
+  for (uint32_t c = threadIdx.x; c < A.C; c += blockDim.x) place[c] = 0;
+  __syncthreads();
+  const uint32_t k0 = A.row_ptr[range[0]], k1 = A.row_ptr[range[1]];
+  for (uint32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) place[A.col[k]] = 1;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t base = 0;
+  for (uint32_t c0 = 0; c0 < A.C; c0 += blockDim.x) {
+    const uint32_t c = c0 + threadIdx.x;
+    const bool on = c < A.C && place[c] != 0;
+    const unsigned mask = __ballot_sync(kFull, on);
+    if (lane == 0) warp_sum[warp] = __popc(mask);
+    __syncthreads();
+    uint32_t at = base;
+    for (int w = 0; w < 8; w++) {
+      if (w < warp) at += warp_sum[w];
+      base += warp_sum[w];
+    }
+    at += __popc(mask & ((1u << lane) - 1u));
+    if (on) {
+      A.uni[size_t(blockIdx.x) * A.C + at] = c;
+      place[c] = at;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) A.uni_n[blockIdx.x] = base;
+  for (uint32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) A.local[k] = place[A.col[k]];
+}
+
+template <bool SHARED>
+__global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit) {
+  extern __shared__ __align__(16) double pcg_smem[];
+  __shared__ Shared sh;
+  double* st = A.state;
+  if (st[A.active] == 0 || limit == 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool alone = gridDim.x == 1;
+  const uint32_t c0 = A.share[blockIdx.x], c1 = A.share[blockIdx.x + 1], nr = c1 - c0, rows = 6 * nr, first = 6 * c0,
+                 n = 6 * A.C;
+  const uint32_t* uni = A.uni + size_t(blockIdx.x) * A.C;
+  const uint32_t cols = 6 * A.uni_n[blockIdx.x];
+  const uint32_t k0 = A.row_ptr[c0], blocks = A.row_ptr[c1] - k0;
+  // Shared memory, as far as it goes: the direction, the own vectors, the own rows of S, their columns'
+  // places and the own preconditioner blocks.
+  uint32_t used = 0;
+  auto take = [&](size_t words, double* global) {
+    if ((used + words) * sizeof(double) > kSmemBytes) return global;
+    double* p = pcg_smem + used;
+    used += uint32_t((words + 1) & ~size_t(1));
+    return p;
+  };
+  double* pl = take(cols, A.pbuf + size_t(blockIdx.x) * n);
+  double* own = take(4 * size_t(rows), nullptr);  // x, r, S p, z
+  const bool keep = own != nullptr;
+  double* xs = keep ? own : A.x + first;
+  double* rs = keep ? own + rows : A.r + first;
+  double* ss = keep ? own + 2 * size_t(rows) : A.p + first;  // p's place is free once it is loaded
+  double* zs = keep ? own + 3 * size_t(rows) : A.z + first;
+  const double* S = A.S + 36 * size_t(k0);
+  if (double* to = take(36 * size_t(blocks), nullptr)) {
+    const double2* from = reinterpret_cast<const double2*>(S);
+    for (uint32_t k = threadIdx.x; k < 18 * blocks; k += kThreads) reinterpret_cast<double2*>(to)[k] = from[k];
+    S = to;
+  }
+  const uint32_t* local = A.local + k0;
+  if (double* to = take((size_t(blocks) + 1) / 2, nullptr)) {
+    uint32_t* words = reinterpret_cast<uint32_t*>(to);
+    for (uint32_t k = threadIdx.x; k < blocks; k += kThreads) words[k] = local[k];
+    local = words;
+  }
+  const double* Minv = A.Minv + 36 * size_t(c0);
+  if (double* to = take(36 * size_t(nr), nullptr)) {
+    for (uint32_t k = threadIdx.x; k < 36 * nr; k += kThreads) to[k] = Minv[k];
+    Minv = to;
+  }
+  // The first step's direction is z + 0 p.
+  for (uint32_t j = threadIdx.x; j < cols; j += kThreads) pl[j] = 0;
+  if (keep)
+    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
+      xs[i] = A.x[first + i];
+      rs[i] = A.r[first + i];
+      zs[i] = A.z[first + i];
+    }
+  double xf = 0, rf = 0, zf = 0, pf = 0, sff = 0, finv = 0;  // the focal unknown, alike in every block
+  if (SHARED) {
+    xf = A.x[n];
+    rf = A.r[n];
+    zf = A.z[n];
+    sff = st[A.focal_diag];
+    finv = st[A.focal_inv];
+  }
+  double rho = st[A.rho], beta = 0, r2 = st[A.r2];
+  const double bound = fmax(A.tol * A.tol * st[A.r0], A.inner_r0 >= 0 ? A.tol_inner * A.tol_inner * st[A.inner_r0] : 0.0);
+  // A warp per camera row, or several warps on a row's columns; a lane sums one of the six rows over
+  // every fifth column.
+  const uint32_t splits = nr == 0 || nr >= uint32_t(kWarps) ? 1 : kWarps / nr;
+  const uint32_t lane_row = lane % 6, lane_col = lane / 6;
+  bool active = true, failed = false, converged = false, ok = true;
+  uint32_t it = 0;
+  if (threadIdx.x == 0) sh.gave_up = 0;
+  __syncthreads();
+  // Index of own scalar row i in pl (a row's own camera is among its columns).
+  auto place_of = [&](uint32_t i) {
+    const uint32_t c = c0 + i / 6;
+    uint32_t lo = 0, hi = cols / 6 - 1;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (uni[mid] < c) lo = mid + 1;
+      else hi = mid;
+    }
+    return 6 * lo + i % 6;
+  };
+  const uint32_t my_place = threadIdx.x < rows ? place_of(threadIdx.x) : 0;
+  while (active && it < limit) {
+    const uint64_t step = it + 1;
+    for (uint32_t j = threadIdx.x; j < cols; j += kThreads) {
+      const uint32_t b = j / 6, g = 6 * uni[b] + (j - 6 * b);
+      double zv = 0;
+      if (alone) zv = zs[g];
+      else if (it == 0) zv = A.z[g];
+      else if (*(volatile int*)&sh.gave_up != 0 || !await(A.zx + g, it, zv)) *(volatile int*)&sh.gave_up = 1;
+      pl[j] = zv + beta * pl[j];
+    }
+    __syncthreads();
+    for (uint32_t item = warp; item < nr * splits; item += kWarps) {
+      const uint32_t row = item / splits, part = item - row * splits;
+      const uint32_t b0 = A.row_ptr[c0 + row] - k0, w = 6 * (A.row_ptr[c0 + row + 1] - k0 - b0);
+      const uint32_t lo = w * part / splits, hi = w * (part + 1) / splits;
+      const double* Sr = S + 36 * size_t(b0);
+      double acc = 0;
+      if (lane < 30) {
+#pragma unroll 4
+        for (uint32_t j = lo + lane_col; j < hi; j += 5) {
+          const uint32_t b = j / 6;
+          acc += Sr[6 * size_t(j) + lane_row] * pl[6 * local[b0 + b] + (j - 6 * b)];
+        }
+      }
+      const double far = __shfl_down_sync(kFull, acc, 24);
+      acc += __shfl_down_sync(kFull, acc, 12);
+      acc += __shfl_down_sync(kFull, acc, 6);
+      if (lane < 6) {
+        double* out = splits == 1 ? ss + 6 * row : sh.part[item];
+        out[lane] = acc + far;
+      }
+    }
+    __syncthreads();
+    if (SHARED) pf = zf + beta * pf;
+    double v[2] = {0, 0};  // p . S p over the own camera rows, the focal row's camera share
+    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
+      double sp = 0;
+      if (splits == 1) {
+        sp = ss[i];
+      } else {
+        for (uint32_t k = 0; k < splits; k++) sp += sh.part[i / 6 * splits + k][i % 6];
+      }
+      const double pv = pl[i == threadIdx.x ? my_place : place_of(i)];
+      if (SHARED) {
+        const double f = A.scf[first + i];
+        sp += f * pf;
+        v[1] += f * pv;
+      }
+      ss[i] = sp;
+      v[0] += pv * sp;
+    }
+    if (!(ok = grid_sum(A, sh, v, step, 0))) break;
+    const double spf = SHARED ? sff * pf + v[1] : 0.0, den = SHARED ? v[0] + pf * spf : v[0], alpha = rho / den;
+    if (!(den > 0) || !(fabs(alpha) < A.alpha_limit)) {
+      active = false;
+      failed = true;
+      break;
+    }
+    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
+      xs[i] += alpha * pl[i == threadIdx.x ? my_place : place_of(i)];
+      rs[i] -= alpha * ss[i];
+    }
+    __syncthreads();
+    v[0] = v[1] = 0;  // r . r, z . r
+    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
+      const double* Mi = Minv + 6 * size_t(i);
+      const double* rc = rs + i - i % 6;
+      const double rr = rs[i];
+      const double zz = Mi[0] * rc[0] + Mi[1] * rc[1] + Mi[2] * rc[2] + Mi[3] * rc[3] + Mi[4] * rc[4] + Mi[5] * rc[5];
+      if (alone) zs[i] = zz;
+      else publish(A.zx + first + i, zz, step);
+      v[0] += rr * rr;
+      v[1] += zz * rr;
+    }
+    if (!(ok = grid_sum(A, sh, v, step, 1))) break;
+    it++;
+    r2 = v[0];
+    double next = v[1];
+    if (SHARED) {
+      xf += alpha * pf;
+      rf -= alpha * spf;
+      zf = finv * rf;
+      r2 += rf * rf;
+      next += rf * zf;
+    }
+    if (r2 <= bound) {
+      active = false;
+      converged = true;
+    } else if (!(next > 0)) {
+      active = false;
+      failed = true;
+    } else {
+      beta = next / rho;
+      rho = next;
+    }
+  }
+  if (keep)
+    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
+      A.x[first + i] = xs[i];
+      A.r[first + i] = rs[i];
+    }
+  if (threadIdx.x != 0 || (blockIdx.x != 0 && ok)) return;
+  if (!ok) {
+    st[A.wait] = 1;
+    st[A.failed] = 1;
+    st[A.active] = 0;
+    return;
+  }
+  if (SHARED) {
+    A.x[n] = xf;
+    A.r[n] = rf;
+  }
+  st[A.steps] += it;
+  if (A.all_steps >= 0) st[A.all_steps] += it;
+  st[A.r2] = r2;
+  st[A.rho] = rho;
+  if (failed) st[A.failed] = 1;
+  if (converged && A.converged >= 0) st[A.converged] = 1;
+  if (!active) st[A.active] = 0;
+}
+
+}  // namespace
+
+cudaError_t pcg_configure() {
+  cudaError_t e = cudaFuncSetAttribute(k_pcg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_pcg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
+  return e;
+}
+
+uint32_t pcg_grid(uint64_t blocks, uint32_t C, int sms) {
+  const uint64_t bytes = 288 * blocks;
+  if (bytes + (5 * 6 + 36) * 8 * uint64_t(C) <= kSmemBytes) return 1;  // all in one block: nothing to exchange
+  const uint64_t share = 48 * 1024;
+  return uint32_t(std::min<uint64_t>(std::min<uint64_t>((bytes + share - 1) / share, C), uint64_t(std::max(1, sms))));
+}
+
+uint32_t pcg_launch_plan(const PcgSystem& a, uint32_t grid, cudaStream_t s) {
+  k_pcg_plan<<<grid, 256, size_t(a.C) * sizeof(uint32_t), s>>>(a);
+  return 1;
+}
+
+cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaStream_t s) {
+  const void* f = a.shared ? reinterpret_cast<const void*>(k_pcg<true>) : reinterpret_cast<const void*>(k_pcg<false>);
+  PcgSystem q = a;
+  void* args[] = {&q, &limit};
+  if (grid == 1) return cudaLaunchKernel(f, dim3(1), dim3(kThreads), args, kSmemBytes, s);
+  // No step of an earlier run may be taken for one of this run's.
+  cudaError_t e = cudaMemsetAsync(a.zx, 0, 6 * size_t(a.C) * sizeof(Flagged), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(a.slots, 0, 4 * size_t(grid) * sizeof(Flagged), s);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kThreads), args, kSmemBytes, s);
+}
+
+}  // namespace tba

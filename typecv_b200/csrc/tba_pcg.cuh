@@ -1,0 +1,51 @@
+// The PCG on an explicit reduced camera system (tba_schur.cuh) as one persistent launch.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace tba {
+
+constexpr uint32_t kPcgWaitPolls = 1u << 21;  // polls of one word before a wait gives up (about a second)
+
+// A double and the step it belongs to, written and read as one 16-byte word: a reader that finds the
+// step it waits for has the value, with no fence on either side.
+struct alignas(16) Flagged {
+  double value;
+  uint64_t step;
+};
+
+// The system, its vectors and the words of the solver's state that the PCG reads and writes.
+struct PcgSystem {
+  uint32_t C, shared;  // cameras; a focal unknown after the 6C camera unknowns
+  const double* S;     // 6x6 blocks by columns: entry (row a, column b) of block k at 36 k + 6 b + a
+  const uint32_t* row_ptr;  // C + 1 first blocks of the rows
+  const uint32_t* col;      // camera of each block
+  // Per block of the launch (pcg_launch_plan): its first camera, its distinct columns' cameras and, per
+  // block of S, the place of its camera among them.
+  uint32_t* share;     // grid + 1
+  uint32_t* uni;       // grid x C
+  uint32_t* uni_n;     // grid
+  uint32_t* local;     // per block of S
+  const double* Minv;  // 36C block-Jacobi preconditioner
+  const double* scf;   // 6C focal column (with the focal unknown)
+  double *x, *r, *z, *p;  // 6C (+ 1); x and r are updated, z and p hold the start (p = z or a restart's)
+  double* pbuf;           // grid x 6C: a block's direction when it does not fit shared memory
+  double* state;
+  int active, failed, converged, rho, r0, r2, inner_r0, steps, all_steps, wait;  // words; -1: not kept
+  int focal_diag, focal_inv;
+  double tol, tol_inner, alpha_limit;
+  Flagged* zx;         // 6C: z between blocks
+  Flagged* slots;      // 4 per block: its partial sums of the step's two reductions
+};
+
+cudaError_t pcg_configure();
+// Blocks of a run on a system of at most `blocks` 6x6 blocks.
+uint32_t pcg_grid(uint64_t blocks, uint32_t C, int sms);
+// The blocks' shares and columns, once per structure.
+uint32_t pcg_launch_plan(const PcgSystem& a, uint32_t grid, cudaStream_t s);
+// Up to `limit` PCG steps from the vectors and state as k_pcg_init (or a restart) left them.
+cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaStream_t s);
+
+}  // namespace tba
