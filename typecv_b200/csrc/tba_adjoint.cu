@@ -7,6 +7,8 @@
 //                    preconditioner and the reduced right-hand side (plus the gauge term)
 //   k_adj_prod_*     the Schur product S p = U p - sum_i W_i V^-1 sum_j W_j^T p, two passes over
 //                    the stored cross blocks
+//   k_adj_records    explicit reduced system: the cross blocks W_i turned into records W_i N_p in place
+//   k_adj_rows       explicit reduced system: S p, one camera row per warp
 //   k_adj_vec        one PCG step on the camera vectors (one block)
 //   k_adj_back       point back-substitution
 //   k_adj_vjp        per observation: ybar_i = W~_i J_i lambda_i, and the intrinsics' shares
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(256) k_adj_points(AdjParams A) {
     }
     gsq[0] += g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
     double M9[9] = {V[0], V[1], V[2], V[1], V[3], V[4], V[2], V[4], V[5]};
-    double inv[6];
+    double inv[6], root[6] = {0, 0, 0, 0, 0, 0};
     double* vi = A.Vinv + 6 * size_t(pt);
     bool ok = inverse3_spd(M9, inv);
     if (!ok) {
@@ -273,11 +275,54 @@ __global__ void __launch_bounds__(256) k_adj_points(AdjParams A) {
       for (int j = 0; j < 6; j++) vi[j] = 0;
     } else {
       for (int j = 0; j < 6; j++) vi[j] = inv[j];
+      if (A.schur) inverse_root3_spd(M9, root);  // (the same pivots as the inverse)
     }
+    if (A.schur)
+      for (int j = 0; j < 6; j++) A.root[6 * size_t(pt) + j] = root[j];
     for (int j = 0; j < 3; j++) A.bp[3 * size_t(pt) + j] = A.rhs_mode ? A.cot[6 * size_t(A.C) + 3 * size_t(pt) + j] : -g[j];
   }
   adj_block_sum(gsq, red);
   if (threadIdx.x == 0) atomicAdd(A.state + A_GNORM, gsq[0]);
+}
+
+// One observation per lane through shared memory, so that the 144-byte blocks move as whole lines.
+__global__ void __launch_bounds__(128) k_adj_records(AdjParams A) {
+  __shared__ double2 stage_all[128 * 9];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* stage = reinterpret_cast<double*>(stage_all + warp * 32 * 9);
+  const uint32_t step = gridDim.x * blockDim.x;
+  for (uint32_t o0 = blockIdx.x * blockDim.x + 32 * warp; o0 < A.M; o0 += step) {
+    const uint32_t n = min(32u, A.M - o0);
+    double2* g = reinterpret_cast<double2*>(A.Hcp + 18 * size_t(o0));
+    double2* s = reinterpret_cast<double2*>(stage);
+    for (uint32_t k = lane; k < 9 * n; k += 32) s[k] = g[k];
+    __syncwarp();
+    if (uint32_t(lane) < n) {
+      double W[18], N[6];
+      for (int j = 0; j < 18; j++) W[j] = stage[18 * lane + j];
+      load6(A.root + 6 * size_t(A.obs_point[o0 + lane]), N);
+      for (int a = 0; a < 6; a++) {
+        double row[3];
+        root_t(N, W + 3 * a, row);
+        for (int k = 0; k < 3; k++) stage[18 * lane + 6 * k + a] = row[k];
+      }
+    }
+    __syncwarp();
+    for (uint32_t k = lane; k < 9 * n; k += 32) g[k] = s[k];
+    __syncwarp();
+  }
+}
+
+// The diagonal block of camera c in the explicit system.
+__device__ inline double* adj_diagonal(const AdjParams& A, uint32_t c) {
+  const uint32_t b0 = A.row_ptr[c];
+  uint32_t lo = 0, hi = A.row_ptr[c + 1] - b0 - 1;  // the row holds camera c
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) / 2;
+    if (A.col[b0 + mid] < c) lo = mid + 1;
+    else hi = mid;
+  }
+  return A.S + 36 * size_t(b0 + lo);
 }
 
 // The unit gradient of the anchor-to-scale-camera baseline with respect to the scale camera's
@@ -307,6 +352,10 @@ __global__ void __launch_bounds__(128) k_adj_cameras(AdjParams A) {
         Minv[7 * j] = 1;
         bc[j] = 0;
       }
+      if (A.schur) {
+        double* block = adj_diagonal(A, c);
+        for (int j = 0; j < 36; j++) block[j] = Minv[j];
+      }
     }
     return;
   }
@@ -319,6 +368,15 @@ __global__ void __launch_bounds__(128) k_adj_cameras(AdjParams A) {
     const double* W = A.Hcp + 18 * size_t(i);
     const double* vi = A.Vinv + 6 * size_t(pt);
     const double* b = A.bp + 3 * size_t(pt);
+    if (A.schur) {
+      double nb[3];
+      root_t(A.root + 6 * size_t(pt), b, nb);
+      for (int a = 0; a < 6; a++) {
+        for (int bb = 0; bb <= a; bb++) s[27 + sym6(a, bb)] += W[a] * W[bb] + W[6 + a] * W[6 + bb] + W[12 + a] * W[12 + bb];
+        s[48 + a] += W[a] * nb[0] + W[6 + a] * nb[1] + W[12 + a] * nb[2];
+      }
+      continue;
+    }
     for (int a = 0; a < 6; a++) {
       const double t0 = W[3 * a] * vi[0] + W[3 * a + 1] * vi[1] + W[3 * a + 2] * vi[2];
       const double t1 = W[3 * a] * vi[1] + W[3 * a + 1] * vi[3] + W[3 * a + 2] * vi[4];
@@ -339,6 +397,10 @@ __global__ void __launch_bounds__(128) k_adj_cameras(AdjParams A) {
   }
   double S[21];
   for (int j = 0; j < 21; j++) S[j] = U[j] - s[27 + j];
+  if (A.schur) {
+    double* block = adj_diagonal(A, c);
+    for (int j = 0; j < 36; j++) block[j] = S[sym6(j / 6, j % 6)];
+  }
   double inv[36];
   if (inverse6_spd(S, inv)) {
     for (int j = 0; j < 36; j++) Minv[j] = inv[j];
@@ -574,6 +636,25 @@ __global__ void __launch_bounds__(32 * kAdjColumnWarps) k_adj_columns(AdjParams 
   A.Sp[j] = up + (A.active[c] != 0 ? sum : 0.0);
 }
 
+// S p of the explicit system, one camera row per warp.
+__global__ void __launch_bounds__(256) k_adj_rows(AdjParams A) {
+  if (A.state[A_ACTIVE] == 0) return;
+  const uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (c >= A.C) return;
+  const uint32_t lane = threadIdx.x & 31, b0 = A.row_ptr[c], w = 6 * (A.row_ptr[c + 1] - b0);
+  const double* row = A.S + 36 * size_t(b0);
+  double acc = 0;
+  if (lane < 30)
+    for (uint32_t j = lane / 6; j < w; j += 5) {
+      const uint32_t b = j / 6;
+      acc += row[6 * size_t(j) + lane % 6] * A.p[6 * A.col[b0 + b] + (j - 6 * b)];
+    }
+  const double far = __shfl_down_sync(kFull, acc, 24);
+  acc += __shfl_down_sync(kFull, acc, 12);
+  acc += __shfl_down_sync(kFull, acc, 6);
+  if (lane < 6) A.Sp[6 * size_t(c) + lane] = acc + far;
+}
+
 __global__ void __launch_bounds__(1024) k_adj_vec(AdjParams A) {
   __shared__ double red[64];
   double* st = A.state;
@@ -639,17 +720,30 @@ __global__ void k_adj_loop_next(AdjParams A) {
 
 __global__ void __launch_bounds__(256) k_adj_back(AdjParams A) {
   for (uint32_t pt = blockIdx.x * blockDim.x + threadIdx.x; pt < A.P; pt += gridDim.x * blockDim.x) {
-    double t[3] = {A.bp[3 * size_t(pt)], A.bp[3 * size_t(pt) + 1], A.bp[3 * size_t(pt) + 2]};
+    double t[3] = {A.bp[3 * size_t(pt)], A.bp[3 * size_t(pt) + 1], A.bp[3 * size_t(pt) + 2]}, sub[3] = {0, 0, 0};
     for (uint32_t i = A.point_start[pt]; i < A.point_start[pt + 1]; i++) {
       const uint32_t c = A.obs_camera[i];
       if (A.active[c] == 0) continue;
       const double* W = A.Hcp + 18 * size_t(i);
       const double* xc = A.x + 6 * size_t(c);
+      if (A.schur) {
+        for (int k = 0; k < 3; k++)
+          for (int a = 0; a < 6; a++) sub[k] += W[6 * k + a] * xc[a];
+        continue;
+      }
       for (int a = 0; a < 6; a++) {
         t[0] -= W[3 * a] * xc[a];
         t[1] -= W[3 * a + 1] * xc[a];
         t[2] -= W[3 * a + 2] * xc[a];
       }
+    }
+    if (A.schur) {  // V^-1 (b - sum W^T x) = N (N^T b - sum A^T x)
+      const double* N = A.root + 6 * size_t(pt);
+      double nb[3];
+      root_t(N, t, nb);
+      for (int k = 0; k < 3; k++) nb[k] -= sub[k];
+      root_n(N, nb, A.lp + 3 * size_t(pt));
+      continue;
     }
     const double* vi = A.Vinv + 6 * size_t(pt);
     double* l = A.lp + 3 * size_t(pt);
@@ -881,8 +975,9 @@ uint32_t adj_launch_reset(const AdjParams& a, cudaStream_t s) {
 uint32_t adj_launch_assemble(const AdjParams& a, cudaStream_t s) {
   k_adj_obs<<<grid_for(a.M, 128), 128, 0, s>>>(a);
   k_adj_points<<<grid_for(a.P, 256), 256, 0, s>>>(a);
+  if (a.schur) k_adj_records<<<grid_for(a.M, 128), 128, 0, s>>>(a);
   k_adj_cameras<<<a.C, 128, 0, s>>>(a);
-  return 3;
+  return a.schur ? 4 : 3;
 }
 
 uint32_t adj_launch_pcg_init(const AdjParams& a, cudaStream_t s) {
@@ -918,6 +1013,13 @@ cudaError_t adj_configure() {
 }
 
 uint32_t adj_launch_pcg_step(const AdjParams& a, cudaStream_t s, cudaEvent_t before, cudaEvent_t after) {
+  if (a.schur) {
+    if (before) cudaEventRecord(before, s);
+    k_adj_rows<<<(a.C + 7) / 8, 256, 0, s>>>(a);
+    if (after) cudaEventRecord(after, s);
+    k_adj_vec<<<1, 1024, 0, s>>>(a);
+    return 2;
+  }
   if (a.prod_blocks) {
     if (before) cudaEventRecord(before, s);
     k_adj_product<<<a.prod_blocks, kAdjProductThreads, adj_product_smem(a.C), s>>>(a);

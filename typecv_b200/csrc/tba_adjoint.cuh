@@ -35,6 +35,7 @@ enum AdjWord : int {
   A_BASELINE = 14, A_ORIGIN = 15, A_SCALE = 18, A_INVALID = 19, A_COST = 20, A_POINT_SINGULAR = 21,
   A_LOOP_ITERS = 22,  // PCG steps of the current device-side PCG loop
   A_LOOP_LIMIT = 23,  // the steps that loop may take
+  A_WAIT = 24,        // a wait of the persistent PCG ran out of polls
   A_WORDS = 32
 };
 
@@ -88,6 +89,13 @@ struct AdjParams {
   uint32_t prod_blocks;      // 0: the two-pass product
   uint32_t prod_copies;      // copies of the camera sums in a block's shared memory (warp w adds to w % copies)
   double* part;              // prod_blocks x 6C
+  // The explicit reduced system (tba_schur.cuh): each observation's cross block becomes its record
+  // A_i = W_i N_p in place (by columns), and S holds the system's blocks.
+  uint32_t schur;
+  double* root;             // 6P: N with V^-1 = N N^T
+  double* S;
+  const uint32_t* row_ptr;
+  const uint32_t* col;
   // The condition of the CUDA graph's while node that runs the PCG steps on the device (set by
   // k_adj_loop_next inside the loop's body graph; unused outside it).  The step kernels read
   // neither `mu` nor `rhs_mode`.
@@ -103,7 +111,7 @@ cudaError_t adj_configure();  // the one-pass product's shared-memory limit
 
 uint32_t adj_launch_init(const AdjParams& a, cudaStream_t s);        // gauge origin and baseline
 uint32_t adj_launch_reset(const AdjParams& a, cudaStream_t s);       // zero the per-solve sums and flags
-uint32_t adj_launch_assemble(const AdjParams& a, cudaStream_t s);    // per observation, points, cameras
+uint32_t adj_launch_assemble(const AdjParams& a, cudaStream_t s);    // per observation, points (records), cameras
 uint32_t adj_launch_pcg_init(const AdjParams& a, cudaStream_t s);
 // Product + vector step; with events, the one-pass product's launch is bracketed by them.
 uint32_t adj_launch_pcg_step(const AdjParams& a, cudaStream_t s, cudaEvent_t before = nullptr,

@@ -375,12 +375,13 @@ uint64_t count_pairs(const uint32_t* ps, uint32_t P) {
 uint64_t schur_block_bound(uint64_t C, uint64_t pairs) { return std::min(C * C, 2 * pairs + C); }
 
 // Whether a solve forms the reduced system explicitly: its values cost about 0.04 ns a pair of
-// observations of one point, once per LM iteration, and a PCG step then a pass over the blocks (here a
-// quarter of their bound, at 5 TB/s) and two grid barriers, against a pass over every observation (0.03
-// ns each) and five launches; compared over 16 PCG steps.
-bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t max_cg) {
-  if (pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
-  const double steps = std::min<uint32_t>(max_cg, 16);
+// observations of one point, once per linear solve, and a PCG step then a pass over the blocks (here a
+// quarter of their bound, at 5 TB/s) and two exchanges, against a pass over every observation (0.03
+// ns each) and five launches; compared over `steps` PCG steps (16 for an LM iteration, 64 for the
+// adjoint's tighter solves, at most the budget).
+bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t budget, uint32_t expected) {
+  if (6 * C + 1 > tba::product_max_unknowns() || pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
+  const double steps = std::min(budget, expected);
   const double blocks = double(schur_block_bound(C, pairs)) / 4;
   return 4e-5 * double(pairs) + steps * (5 + 288e-6 / 5 * blocks) < steps * (14 + 3e-5 * double(M));
 }
@@ -391,8 +392,11 @@ struct SchurLayout {
   Layout L;
   size_t counts, bits, row_blk, row_pair, row_ptr, col, pairs, begin, rc, dst, seg_block, totals, part, S;
   size_t share, uni, uni_n, local, pbuf, zx, slots;  // the persistent PCG's
-  uint32_t seg = 0, grid = 1;
-  SchurLayout(uint32_t C, uint64_t npairs, uint32_t nchunks, uint64_t blocks, uint64_t camera_pairs, int sms) {
+  uint32_t C, nchunks, seg = 0, grid = 1;
+  uint64_t npairs, camera_pairs;
+  SchurLayout(uint32_t C, uint64_t npairs, uint32_t nchunks, int sms)
+      : C(C), nchunks(nchunks), npairs(npairs), camera_pairs(std::min<uint64_t>(npairs, uint64_t(C) * (C + 1) / 2)) {
+    const uint64_t blocks = schur_block_bound(C, npairs);
     // Pairs per warp of the block sums: a few warps' worth of segments on every SM.
     seg = tba::kPairSegMin;
     while (seg < tba::kPairSegMax && npairs / seg > uint64_t(64) * uint64_t(sms)) seg *= 2;
@@ -421,7 +425,67 @@ struct SchurLayout {
     part = L.take<double>(72 * segs);
     S = L.take<double>(36 * blocks);
   }
+  // The parts of the structure's and the PCG's parameters that lie in this memory.
+  void bind(char* base, tba::SchurParams& q, tba::PcgSystem& a) const {
+    auto u32 = [&](size_t off) { return reinterpret_cast<uint32_t*>(base + off); };
+    auto u2 = [&](size_t off) { return reinterpret_cast<uint2*>(base + off); };
+    auto f64 = [&](size_t off) { return reinterpret_cast<double*>(base + off); };
+    q.C = a.C = C;
+    q.nchunks = nchunks;
+    q.bwords = (C + 31) / 32;
+    q.seg = seg;
+    q.max_pairs = uint32_t(npairs);
+    q.max_blocks = uint32_t(camera_pairs);
+    q.counts = u32(counts);
+    q.bits = u32(bits);
+    q.row_blk = u32(row_blk);
+    q.row_pair = u32(row_pair);
+    q.row_ptr = u32(row_ptr);
+    q.col = u32(col);
+    q.pairs = u2(pairs);
+    q.blk_begin = u32(begin);
+    q.blk_rc = u2(rc);
+    q.blk_dst = u2(dst);
+    q.seg_block = u32(seg_block);
+    q.totals = u32(totals);
+    q.part = f64(part);
+    q.S = f64(S);
+    a.S = q.S;
+    a.row_ptr = q.row_ptr;
+    a.col = q.col;
+    a.share = u32(share);
+    a.uni = u32(uni);
+    a.uni_n = u32(uni_n);
+    a.local = u32(local);
+    a.pbuf = f64(pbuf);
+    a.zx = reinterpret_cast<tba::Flagged*>(base + zx);
+    a.slots = reinterpret_cast<tba::Flagged*>(base + slots);
+  }
 };
+
+// The device's free memory, with the explicit system's buffer given back when `need` takes it.
+size_t free_memory(tba_device* d, size_t need) {
+  size_t free_bytes = 0, total_bytes = 0;
+  CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (need > free_bytes && d->schur) {
+    CUDA_TRY(cudaFree(d->schur));
+    d->schur = nullptr;
+    d->schur_capacity = 0;
+    CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+  }
+  return free_bytes;
+}
+
+// Whether the workspace and an explicit system's memory of these sizes fit the device, with what the
+// handle holds given back where it has to grow.
+bool memory_for(tba_device* d, size_t workspace, size_t schur) {
+  if (d->capacity >= workspace && d->schur_capacity >= schur) return true;
+  size_t free_bytes = 0, total_bytes = 0;
+  CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+  const size_t held = (d->capacity < workspace ? d->capacity : 0) + (d->schur_capacity < schur ? d->schur_capacity : 0);
+  const size_t need = (d->capacity < workspace ? workspace : 0) + (d->schur_capacity < schur ? schur : 0);
+  return need <= free_bytes + held;
+}
 
 // Grows a device buffer kept by the handle to `bytes` (its old contents are dropped).
 void grow(char*& buffer, size_t& capacity, size_t bytes, const char* what) {
@@ -437,6 +501,19 @@ void grow(char*& buffer, size_t& capacity, size_t bytes, const char* what) {
                                      std::to_string(free_bytes) + " bytes"};
   CUDA_TRY(cudaMalloc(&buffer, bytes));
   capacity = bytes;
+}
+
+// The handle's buffers for a call that needs these sizes.  A workspace that has to grow may need the
+// memory of an explicit system that this call does not use.
+void make_room(tba_device* d, size_t workspace, size_t schur, const char* what) {
+  const bool both = d->capacity < workspace && d->schur_capacity < schur;
+  if (d->schur && (both || (d->capacity < workspace && schur == 0))) {
+    CUDA_TRY(cudaFree(d->schur));
+    d->schur = nullptr;
+    d->schur_capacity = 0;
+  }
+  grow(d->arena, d->capacity, workspace, what);
+  grow(d->schur, d->schur_capacity, schur, what);
 }
 
 // Makes `loop` a graph of one while node whose body `capture(handle, stream)` records (returning its
@@ -613,7 +690,7 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   // The explicit reduced system takes the place of the product over stored factors where it costs less
   // and fits the device; it is FP64, so a mixed request then needs no refinement.
   const uint64_t npairs = io.plan ? io.plan->pairs : count_pairs(index + 2 * size_t(M), P);
-  bool schur = p.factored && prefer_schur(C, M, npairs, ctl->max_cg);
+  bool schur = p.factored && prefer_schur(C, M, npairs, ctl->max_cg, 16);
   bool mixed = false;
   size_t factor_bytes = 0, factor32_bytes = 0;
   uint32_t max_prod_blocks = 1;
@@ -673,23 +750,12 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   lay_out();
   if (schur) {
     // What the explicit system would add: when it does not fit, the product over stored factors.
-    const uint64_t bound = schur_block_bound(C, npairs), camera_pairs = std::min<uint64_t>(npairs, uint64_t(C) * (C + 1) / 2);
-    const size_t more = SchurLayout(C, npairs, uint32_t(max_chunks), bound, camera_pairs, d->sms).L.bytes;
-    if (d->capacity < L.bytes || d->schur_capacity < more) {
-      size_t free_bytes = 0, total_bytes = 0;
-      CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
-      if (L.bytes + more > free_bytes + d->capacity + d->schur_capacity) {
-        schur = false;
-        lay_out();
-      }
+    if (!memory_for(d, L.bytes, SchurLayout(C, npairs, uint32_t(max_chunks), d->sms).L.bytes)) {
+      schur = false;
+      lay_out();
     }
   }
-  if (d->capacity < L.bytes && d->schur && !schur) {  // the workspace may need the explicit system's memory
-    CUDA_TRY(cudaFree(d->schur));
-    d->schur = nullptr;
-    d->schur_capacity = 0;
-  }
-  grow(d->arena, d->capacity, L.bytes, "GPU BA");
+  make_room(d, L.bytes, 0, "GPU BA");
   char* a = d->arena;
   auto D = [&](size_t off) { return reinterpret_cast<double*>(a + off); };
   auto U32 = [&](size_t off) { return reinterpret_cast<uint32_t*>(a + off); };
@@ -835,20 +901,9 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   tba::PcgSystem ps{};
   uint32_t pcg_blocks = 0;
   if (schur) {
-    // The structure of S.  Where the bound on its blocks is far above what scenes have (a local
-    // covisibility), the counted structure sizes the blocks.
-    uint64_t blocks = schur_block_bound(C, npairs), camera_pairs = std::min<uint64_t>(npairs, uint64_t(C) * (C + 1) / 2);
-    const SchurLayout Q(C, npairs, nchunks, blocks, camera_pairs, d->sms);
+    const SchurLayout Q(C, npairs, nchunks, d->sms);
     grow(d->schur, d->schur_capacity, Q.L.bytes, "GPU BA");
-    char* b = d->schur;
-    auto at = [&](size_t off) { return reinterpret_cast<uint32_t*>(b + off); };
-    sq.C = C;
-    sq.M = M;
-    sq.nchunks = nchunks;
-    sq.bwords = (C + 31) / 32;
-    sq.seg = Q.seg;
-    sq.max_pairs = uint32_t(npairs);
-    sq.max_blocks = uint32_t(camera_pairs);
+    Q.bind(d->schur, sq, ps);
     sq.obs_camera = p.obs_camera;
     sq.obs_point = p.obs_point;
     sq.point_start = p.point_start;
@@ -857,42 +912,19 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     sq.chunk_cam = p.chunk_cam;
     sq.chunk_beg = p.chunk_beg;
     sq.cam_chunk = p.cam_chunk;
-    sq.counts = at(Q.counts);
-    sq.bits = at(Q.bits);
-    sq.row_blk = at(Q.row_blk);
-    sq.row_pair = at(Q.row_pair);
-    sq.row_ptr = at(Q.row_ptr);
-    sq.col = at(Q.col);
-    sq.pairs = reinterpret_cast<uint2*>(b + Q.pairs);
-    sq.blk_begin = at(Q.begin);
-    sq.blk_rc = reinterpret_cast<uint2*>(b + Q.rc);
-    sq.blk_dst = reinterpret_cast<uint2*>(b + Q.dst);
-    sq.seg_block = at(Q.seg_block);
-    sq.totals = at(Q.totals);
-    sq.part = reinterpret_cast<double*>(b + Q.part);
-    sq.S = reinterpret_cast<double*>(b + Q.S);
     sq.A = p.A;
     launches += tba::schur_launch_structure(sq, s);
     CUDA_TRY(cudaGetLastError());
     p.S = sq.S;
     p.row_ptr = sq.row_ptr;
     p.col = sq.col;
-    ps.C = C;
     ps.shared = shared;
-    ps.S = p.S;
-    ps.row_ptr = p.row_ptr;
-    ps.col = p.col;
     ps.Minv = p.camMinv;
     ps.scf = p.camScf;
     ps.x = p.x;
     ps.r = p.r;
     ps.z = p.z;
     ps.p = p.p;
-    ps.share = at(Q.share);
-    ps.uni = at(Q.uni);
-    ps.uni_n = at(Q.uni_n);
-    ps.local = at(Q.local);
-    ps.pbuf = reinterpret_cast<double*>(b + Q.pbuf);
     ps.state = p.state;
     ps.active = tba::S_CG_ACTIVE;
     ps.failed = tba::S_CG_FAILED;
@@ -909,8 +941,6 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     ps.tol = p.tol;
     ps.tol_inner = p.tol_inner;
     ps.alpha_limit = 1e20;
-    ps.zx = reinterpret_cast<tba::Flagged*>(b + Q.zx);
-    ps.slots = reinterpret_cast<tba::Flagged*>(b + Q.slots);
     pcg_blocks = Q.grid;
     launches += tba::pcg_launch_plan(ps, pcg_blocks, s);
     CUDA_TRY(cudaGetLastError());
@@ -1252,8 +1282,7 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
     if (d->batch_arena) CUDA_TRY(cudaFree(d->batch_arena));
     d->batch_arena = nullptr;
     d->batch_capacity = 0;
-    size_t free_bytes = 0, total_bytes = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+    const size_t free_bytes = free_memory(d, L.bytes);
     if (L.bytes > free_bytes)
       throw Fail{TBA_ERROR_BUDGET, "GPU BA batch needs " + std::to_string(L.bytes) +
                                        " bytes of device memory, more than the working budget of " +
@@ -1530,6 +1559,13 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
                                                                  (A.ntasks + 7) / 8))
                       : 0;
   A.prod_copies = tba::adj_product_copies(C);
+  // The explicit reduced system in place of the product over the cross blocks, where it costs less and
+  // fits the device.
+  const uint64_t npairs = count_pairs(index + 2 * size_t(M), P);
+  bool schur = prefer_schur(C, M, npairs, vc->max_cg, 64);
+  Chunks chunks;
+  if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, M, d->sms);
+  const uint32_t nchunks = uint32_t(chunks.cam.size());
   Layout L;
   const size_t o_poses = L.take<double>(12 * size_t(C)), o_points = L.take<double>(3 * size_t(P)),
                o_cams = L.take<double>(6 * size_t(C)), o_pixels = L.take<double>(2 * size_t(M)),
@@ -1545,19 +1581,12 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
                o_state = L.take<double>(tba::A_WORDS), o_tposes = L.take<double>(12 * size_t(C)),
                o_tpoints = L.take<double>(3 * size_t(P)), o_tobs = L.take<uint32_t>(task_obs.size()),
                o_part = L.take<double>(size_t(A.prod_blocks) * 6 * C);
-  if (d->capacity < L.bytes) {
-    if (d->arena) CUDA_TRY(cudaFree(d->arena));
-    d->arena = nullptr;
-    d->capacity = 0;
-    size_t free_bytes = 0, total_bytes = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
-    if (L.bytes > free_bytes)
-      throw Fail{TBA_ERROR_BUDGET, "GPU BA adjoint needs " + std::to_string(L.bytes) +
-                                       " bytes of device memory, more than the working budget of " +
-                                       std::to_string(free_bytes) + " bytes"};
-    CUDA_TRY(cudaMalloc(&d->arena, L.bytes));
-    d->capacity = L.bytes;
-  }
+  const size_t product_only = L.bytes;
+  const size_t o_root = L.take<double>(schur ? 6 * size_t(P) : 0), o_ccam = L.take<uint32_t>(nchunks),
+               o_cbeg = L.take<uint32_t>(nchunks + 1), o_cfirst = L.take<uint32_t>(schur ? C + 1 : 0);
+  const SchurLayout Q(schur ? C : 0, schur ? npairs : 0, nchunks, d->sms);
+  if (schur && !memory_for(d, L.bytes, Q.L.bytes)) schur = false;
+  make_room(d, schur ? L.bytes : product_only, schur ? Q.L.bytes : 0, "GPU BA adjoint");
   char* a = d->arena;
   auto D = [&](size_t off) { return reinterpret_cast<double*>(a + off); };
   A.poses = D(o_poses);
@@ -1597,6 +1626,43 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
   A.task_obs = reinterpret_cast<const uint32_t*>(a + o_tobs);
   A.part = D(o_part);
   A.mu = 0;
+  tba::SchurParams sq{};
+  tba::PcgSystem ps{};
+  if (schur) {
+    Q.bind(d->schur, sq, ps);
+    sq.M = M;
+    sq.obs_camera = A.obs_camera;
+    sq.obs_point = A.obs_point;
+    sq.point_start = A.point_start;
+    sq.camera_obs = A.camera_obs;
+    sq.active = A.active;
+    sq.chunk_cam = reinterpret_cast<const uint32_t*>(a + o_ccam);
+    sq.chunk_beg = reinterpret_cast<const uint32_t*>(a + o_cbeg);
+    sq.cam_chunk = reinterpret_cast<const uint32_t*>(a + o_cfirst);
+    sq.A = A.Hcp;
+    A.schur = 1;
+    A.root = D(o_root);
+    A.S = sq.S;
+    A.row_ptr = sq.row_ptr;
+    A.col = sq.col;
+    A.prod_blocks = 0;
+    ps.Minv = A.Minv;
+    ps.x = A.x;
+    ps.r = A.r;
+    ps.z = A.z;
+    ps.p = A.p;
+    ps.state = A.state;
+    ps.active = tba::A_ACTIVE;
+    ps.failed = tba::A_FAILED;
+    ps.converged = ps.inner_r0 = ps.all_steps = -1;
+    ps.rho = tba::A_RHO;
+    ps.r0 = tba::A_R0;
+    ps.r2 = tba::A_R2;
+    ps.steps = tba::A_STEPS;
+    ps.wait = tba::A_WAIT;
+    ps.tol = A.tol;
+    ps.alpha_limit = 1e30;
+  }
 
   cudaStream_t s = d->stream;
   cudaEvent_t e0 = event(d, 0), e1 = event(d, 1);
@@ -1611,12 +1677,20 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
   up(dindex, index, sizeof(uint32_t) * (3 * size_t(M) + P + 2 * size_t(C) + 2));
   up(const_cast<uint32_t*>(A.task_obs), task_obs.data(), sizeof(uint32_t) * task_obs.size());
   uint32_t launches = 0;
+  if (schur) {
+    up(const_cast<uint32_t*>(sq.chunk_cam), chunks.cam.data(), sizeof(uint32_t) * chunks.cam.size());
+    up(const_cast<uint32_t*>(sq.chunk_beg), chunks.beg.data(), sizeof(uint32_t) * chunks.beg.size());
+    up(const_cast<uint32_t*>(sq.cam_chunk), chunks.cam_first.data(), sizeof(uint32_t) * chunks.cam_first.size());
+    launches += tba::schur_launch_structure(sq, s);
+    launches += tba::pcg_launch_plan(ps, Q.grid, s);
+  }
   launches += tba::adj_launch_init(A, s);
   CUDA_TRY(cudaGetLastError());
 
   auto read_state = [&]() {
     CUDA_TRY(cudaMemcpyAsync(d->pinned, A.state, tba::A_WORDS * sizeof(double), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
+    if (d->pinned[tba::A_WAIT] != 0) throw Fail{TBA_ERROR_CUDA, "GPU BA adjoint: a wait between the PCG's blocks ran out"};
   };
   uint32_t cg_total = 0, failed = 0, point_failures = 0;
   const bool time_products = (vc->flags & TBA_VJP_FLAG_TIME_PRODUCTS) != 0;
@@ -1629,11 +1703,20 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
     A.rhs_mode = mode;
     if (!cotangent_ready) launches += tba::adj_launch_reset(A, s);
     launches += tba::adj_launch_assemble(A, s);
+    if (schur) launches += tba::schur_launch_values(sq, s);
     launches += tba::adj_launch_pcg_init(A, s);
     CUDA_TRY(cudaGetLastError());
     uint32_t done = 0;
-    const bool timed = time_products && A.prod_blocks;
-    const bool on_device = !timed && vc->max_cg > 0 && !d->host_pcg_only &&
+    const bool timed = time_products && (A.prod_blocks || schur);
+    // One persistent launch where the system spreads over several blocks.  A small one keeps a launch per
+    // product and vector step, as the report's launch count has it.
+    const bool persistent = schur && Q.grid > 1 && !timed;
+    if (persistent) {
+      CUDA_TRY(tba::launch_pcg(ps, vc->max_cg, Q.grid, s));
+      launches++;
+      done = vc->max_cg;
+    }
+    const bool on_device = !persistent && !timed && vc->max_cg > 0 && !d->host_pcg_only &&
                            device_loop_ready(d, d->adj_loop, build_adjoint_loop(d->adj_loop, A, s));
     if (on_device) {
       // One launch of the device-side PCG loop, which stops on the device.
@@ -1778,8 +1861,7 @@ void evaluate_observations(tba_device* d, const tba_observation_control* oc, con
     if (d->arena) CUDA_TRY(cudaFree(d->arena));
     d->arena = nullptr;
     d->capacity = 0;
-    size_t free_bytes = 0, total_bytes = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+    const size_t free_bytes = free_memory(d, L.bytes);
     if (L.bytes > free_bytes)
       throw Fail{TBA_ERROR_BUDGET, "GPU observation evaluation exceeds budget"};
     CUDA_TRY(cudaMalloc(&d->arena, L.bytes));
@@ -2280,8 +2362,7 @@ tba_status tba_linearize_inverse_depth(tba_device* d, uint32_t count, const doub
       if (d->arena) CUDA_TRY(cudaFree(d->arena));
       d->arena = nullptr;
       d->capacity = 0;
-      size_t free_bytes = 0, total_bytes = 0;
-      CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+      const size_t free_bytes = free_memory(d, L.bytes);
       if (L.bytes > free_bytes) throw Fail{TBA_ERROR_BUDGET, "Inverse-depth measurement budget cannot fit the observations"};
       CUDA_TRY(cudaMalloc(&d->arena, L.bytes));
       d->capacity = L.bytes;
