@@ -72,6 +72,9 @@ struct tba_device {
   size_t batch_capacity = 0;
   cudaGraphExec_t batch_graph = nullptr;
   std::vector<char> batch_key;
+  // One LM iteration of a batch on the grid kernels.
+  cudaGraphExec_t window_graph = nullptr;
+  std::vector<char> window_key;
   std::map<std::string, int> tuned;
   // The grid engine's device-side PCG loops (the solve's own product and the mixed form's FP64
   // tail) and the adjoint's.
@@ -331,10 +334,14 @@ struct Chunks {
   std::vector<uint32_t> cam, beg, cam_first;
 };
 
-// Chunks of each camera's observation list, sized so that the camera pass has a few blocks per SM.
-Chunks build_chunks(const uint32_t* cs, uint32_t C, uint32_t M, int sms) {
-  uint32_t size = M / std::max(1, 8 * sms);
-  size = std::min<uint32_t>(2048, std::max<uint32_t>(128, (size + 127) / 128 * 128));
+// Chunks of each camera's observation list, sized so that the camera pass has a few blocks per SM over
+// M observations in all.
+uint32_t chunk_size(uint64_t M, int sms) {
+  const uint64_t size = M / uint64_t(std::max(1, 8 * sms));
+  return uint32_t(std::min<uint64_t>(2048, std::max<uint64_t>(128, (size + 127) / 128 * 128)));
+}
+
+Chunks build_chunks(const uint32_t* cs, uint32_t C, uint32_t size) {
   Chunks ch;
   for (uint32_t c = 0; c < C; c++) {
     ch.cam_first.push_back(uint32_t(ch.cam.size()));
@@ -630,10 +637,51 @@ HostPlan make_plan(const tba_control* ctl, const uint32_t* index, int sms) {
   plan.tasks = build_tasks(ps, P);
   plan.task_obs.resize(plan.tasks.size());
   for (size_t t = 0; t < plan.tasks.size(); t++) plan.task_obs[t] = ps[plan.tasks[t]];
-  plan.chunks = build_chunks(cs, C, M, sms);
+  plan.chunks = build_chunks(cs, C, chunk_size(M, sms));
   for (uint32_t c = 0; c < C; c++) plan.fixed += active[c] == 0;
   plan.pairs = count_pairs(ps, P);
   return plan;
+}
+
+// The explicit system's structure, values and PCG of one problem, from the problem's parameters; the
+// problem takes the system's blocks.
+void bind_problem(tba::Params& p, tba::SchurParams& q, tba::PcgSystem& a) {
+  q.M = p.M;
+  q.obs_camera = p.obs_camera;
+  q.obs_point = p.obs_point;
+  q.point_start = p.point_start;
+  q.camera_obs = p.camera_obs;
+  q.active = p.active;
+  q.chunk_cam = p.chunk_cam;
+  q.chunk_beg = p.chunk_beg;
+  q.cam_chunk = p.cam_chunk;
+  q.A = p.A;
+  p.S = q.S;
+  p.row_ptr = q.row_ptr;
+  p.col = q.col;
+  a.shared = p.shared;
+  a.Minv = p.camMinv;
+  a.scf = p.camScf;
+  a.x = p.x;
+  a.r = p.r;
+  a.z = p.z;
+  a.p = p.p;
+  a.state = p.state;
+  a.active = tba::S_CG_ACTIVE;
+  a.failed = tba::S_CG_FAILED;
+  a.converged = tba::S_CG_CONVERGED;
+  a.rho = tba::S_RHO;
+  a.r0 = tba::S_R0;
+  a.r2 = tba::S_R2;
+  a.inner_r0 = tba::S_INNER_R0;
+  a.steps = tba::S_CG_SOLVE_STEPS;
+  a.all_steps = tba::S_CG_STEPS;
+  a.wait = tba::S_WAIT;
+  a.focal_diag = tba::S_FOCAL_SFF;
+  a.focal_inv = tba::S_FOCAL_INV;
+  a.tol = p.tol;
+  a.tol_inner = p.tol_inner;
+  a.alpha_limit = 1e20;
 }
 
 // Where a solve reads its problem and where it leaves the solution.  With `device_source` the
@@ -904,43 +952,8 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     const SchurLayout Q(C, npairs, nchunks, d->sms);
     grow(d->schur, d->schur_capacity, Q.L.bytes, "GPU BA");
     Q.bind(d->schur, sq, ps);
-    sq.obs_camera = p.obs_camera;
-    sq.obs_point = p.obs_point;
-    sq.point_start = p.point_start;
-    sq.camera_obs = p.camera_obs;
-    sq.active = p.active;
-    sq.chunk_cam = p.chunk_cam;
-    sq.chunk_beg = p.chunk_beg;
-    sq.cam_chunk = p.cam_chunk;
-    sq.A = p.A;
+    bind_problem(p, sq, ps);
     launches += tba::schur_launch_structure(sq, s);
-    CUDA_TRY(cudaGetLastError());
-    p.S = sq.S;
-    p.row_ptr = sq.row_ptr;
-    p.col = sq.col;
-    ps.shared = shared;
-    ps.Minv = p.camMinv;
-    ps.scf = p.camScf;
-    ps.x = p.x;
-    ps.r = p.r;
-    ps.z = p.z;
-    ps.p = p.p;
-    ps.state = p.state;
-    ps.active = tba::S_CG_ACTIVE;
-    ps.failed = tba::S_CG_FAILED;
-    ps.converged = tba::S_CG_CONVERGED;
-    ps.rho = tba::S_RHO;
-    ps.r0 = tba::S_R0;
-    ps.r2 = tba::S_R2;
-    ps.inner_r0 = tba::S_INNER_R0;
-    ps.steps = tba::S_CG_SOLVE_STEPS;
-    ps.all_steps = tba::S_CG_STEPS;
-    ps.wait = tba::S_WAIT;
-    ps.focal_diag = tba::S_FOCAL_SFF;
-    ps.focal_inv = tba::S_FOCAL_INV;
-    ps.tol = p.tol;
-    ps.tol_inner = p.tol_inner;
-    ps.alpha_limit = 1e20;
     pcg_blocks = Q.grid;
     launches += tba::pcg_launch_plan(ps, pcg_blocks, s);
     CUDA_TRY(cudaGetLastError());
@@ -1183,6 +1196,324 @@ tba_control batch_problem_control(const tba_batch_control* bc, const tba_batch_p
   return c;
 }
 
+// One problem of a batch as the host schedules it.
+struct WindowPlan {
+  std::vector<uint32_t> tasks;
+  Chunks chunks;
+  uint64_t pairs = 0;
+};
+
+struct BatchReport {
+  int shape = 0;
+  uint32_t threads = 0, blocks = 0, launches = 0;
+  bool replayed = false, mixed = false;
+};
+
+// The batch on the grid kernels: every kernel of an LM iteration runs over all problems at once (its
+// blocks a list of (problem, block)), with each problem's reduced system explicit and its PCG in one
+// block; the iteration is a CUDA graph, replayed while the batch's lists keep their places.  The scene's
+// poses and points are updated in place.  False (nothing launched) when the workspace does not fit.
+bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_problem* probs, uint32_t count,
+                   const std::vector<WindowPlan>& plans, const std::vector<uint32_t>& order, const double* scene,
+                   size_t scene_len, const uint32_t* index, size_t index_len, size_t output_len, cudaEvent_t uploaded,
+                   cudaEvent_t begun, BatchReport& rep, double*& dout_of, uint64_t& h2d) {
+  const bool shared = bc->shared_focal != 0;
+  Layout L;
+  const size_t o_scene = L.take<double>(scene_len), o_index = L.take<uint32_t>(index_len), o_out = L.take<double>(output_len);
+  // The plans' arrays, then the lists of blocks, in one upload.
+  std::vector<uint32_t> flat;
+  struct Place {
+    size_t tasks, obs, cam, beg, first;
+  };
+  std::vector<Place> places(count);
+  uint64_t tasks_total = 0;
+  for (uint32_t k = 0; k < count; k++) tasks_total += plans[k].tasks.size() - 1;
+  // Tasks per warp of the task kernels: a few waves of blocks over the batch, up to eight.
+  const uint32_t per_warp = uint32_t(std::min<uint64_t>(8, std::max<uint64_t>(1, tasks_total / (8 * 8 * uint64_t(d->sms)))));
+  std::vector<uint2> lists[12];  // one, task, chunk, finish, setup, commit, pack | camera, pairs, ends, sums
+  std::vector<SchurLayout> systems;
+  systems.reserve(count);
+  uint32_t Cmax = 2;
+  for (uint32_t k = 0; k < count; k++) {
+    const tba_batch_problem& q = probs[k];
+    const WindowPlan& w = plans[k];
+    Place& at = places[k];
+    const uint32_t* ps = index + q.index_offset + 2 * size_t(q.observations);
+    at.tasks = flat.size();
+    flat.insert(flat.end(), w.tasks.begin(), w.tasks.end());
+    at.obs = flat.size();
+    for (uint32_t t : w.tasks) flat.push_back(ps[t]);
+    at.cam = flat.size();
+    flat.insert(flat.end(), w.chunks.cam.begin(), w.chunks.cam.end());
+    at.beg = flat.size();
+    flat.insert(flat.end(), w.chunks.beg.begin(), w.chunks.beg.end());
+    at.first = flat.size();
+    flat.insert(flat.end(), w.chunks.cam_first.begin(), w.chunks.cam_first.end());
+    systems.emplace_back(q.cameras, w.pairs, uint32_t(w.chunks.cam.size()), d->sms);
+    Cmax = std::max(Cmax, q.cameras);
+  }
+  auto task_blocks = [&](uint32_t k) {
+    return std::max<uint32_t>(1, uint32_t((plans[k].tasks.size() - 1 + 8 * per_warp - 1) / (8 * per_warp)));
+  };
+  for (uint32_t k : order) {  // largest problems first
+    const tba_batch_problem& q = probs[k];
+    const SchurLayout& y = systems[k];
+    const uint32_t C = q.cameras, P = q.points, M = q.observations;
+    const uint64_t n[11] = {1,
+                            task_blocks(k),
+                            plans[k].chunks.cam.size(),
+                            (C + 3) / 4,
+                            (std::max(M, C) + 255) / 256,
+                            (std::max(12 * C, 3 * P) + 255) / 256,
+                            (12 * uint64_t(C) + 3 * uint64_t(P) + 27 + 255) / 256,
+                            C,
+                            (y.camera_pairs + 255) / 256,
+                            (y.camera_pairs + 7) / 8,
+                            ((y.npairs + y.seg - 1) / y.seg + 7) / 8};
+    for (int j = 0; j < 11; j++)
+      for (uint32_t b = 0; b < n[j]; b++) lists[j].push_back(make_uint2(k, b));
+  }
+  const size_t o_flat = L.take<uint32_t>(flat.size());
+  size_t o_list[11];
+  for (int j = 0; j < 11; j++) o_list[j] = L.take<uint2>(lists[j].size());
+  const size_t o_params = L.take<tba::Params>(count), o_schur = L.take<tba::SchurParams>(count),
+               o_pcg = L.take<tba::PcgSystem>(count), o_active = L.take<uint32_t>(1);
+  // The bit matrices together (zeroed at once), then each problem's workspace.
+  size_t bit_words = 0;
+  for (uint32_t k = 0; k < count; k++) bit_words += size_t(probs[k].cameras) * ((probs[k].cameras + 31) / 32);
+  const size_t o_bits = L.take<uint32_t>(bit_words);
+  struct Work {
+    size_t tposes, tpoints, rlim, cmp, cmx, pblk, A, pw, xw, U, Minv, rhs, hcf, scf, chunk, vec, scal, cost, ticket, state, system;
+  };
+  std::vector<Work> works(count);
+  for (uint32_t k = 0; k < count; k++) {
+    const size_t C = probs[k].cameras, P = probs[k].points, M = probs[k].observations, m = 6 * C + (shared ? 1 : 0);
+    Work& w = works[k];
+    w.tposes = L.take<double>(12 * C);
+    w.tpoints = L.take<double>(3 * P);
+    w.rlim = L.take<double>(C);
+    w.cmp = L.take<uint32_t>(M);
+    w.cmx = L.take<double>(2 * M);
+    w.pblk = L.take<double>(12 * P);
+    w.A = L.take<double>(18 * M);
+    w.pw = L.take<double>(6 * C);
+    w.xw = L.take<double>(6 * C);
+    w.U = L.take<double>(21 * C);
+    w.Minv = L.take<double>(36 * C);
+    w.rhs = L.take<double>(6 * C);
+    w.hcf = L.take<double>(6 * C);
+    w.scf = L.take<double>(6 * C);
+    w.chunk = L.take<double>(size_t(tba::kCameraPartialsExplicit) * plans[k].chunks.cam.size());
+    w.vec = L.take<double>(5 * m);
+    w.scal = L.take<double>(size_t(tba::kScalarPartials) * task_blocks(k));
+    w.cost = L.take<double>(4 * size_t(task_blocks(k)));
+    w.ticket = L.take<uint32_t>(8);
+    w.state = L.take<double>(tba::S_WORDS);
+    w.system = L.take<char>(systems[k].L.bytes);
+  }
+  if (d->batch_capacity < L.bytes) {
+    if (L.bytes > free_memory(d, L.bytes) + d->batch_capacity) return false;
+    if (d->batch_graph) {
+      cudaGraphExecDestroy(d->batch_graph);
+      d->batch_graph = nullptr;
+      d->batch_key.clear();
+    }
+    grow(d->batch_arena, d->batch_capacity, L.bytes, "GPU BA batch");
+  }
+  char* a = d->batch_arena;
+  auto f64 = [&](size_t off) { return reinterpret_cast<double*>(a + off); };
+  auto u32 = [&](size_t off) { return reinterpret_cast<uint32_t*>(a + off); };
+  std::vector<tba::Params> params(count);
+  std::vector<tba::SchurParams> schur(count);
+  std::vector<tba::PcgSystem> pcg(count);
+  size_t bits = 0;
+  for (uint32_t k = 0; k < count; k++) {
+    const tba_batch_problem& q = probs[k];
+    const Work& w = works[k];
+    const Place& at = places[k];
+    const size_t C = q.cameras, P = q.points, M = q.observations;
+    tba::Params& p = params[k];
+    tba::SchurParams& y = schur[k];
+    tba::PcgSystem& c = pcg[k];
+    p = tba::Params{};
+    p.C = q.cameras;
+    p.P = q.points;
+    p.M = q.observations;
+    p.m = 6 * q.cameras + (shared ? 1 : 0);
+    p.anchor = q.anchor;
+    p.scale_view = q.scale_view;
+    p.shared = shared;
+    p.huber = bc->huber;
+    p.tol = p.tol_inner = bc->cg_tolerance;
+    p.stall = bc->stall_tolerance;
+    const uint32_t* act = index + q.index_offset + 3 * M + P + C + 2;
+    uint32_t fixed = 0;
+    for (size_t j = 0; j < C; j++) fixed += act[j] == 0;
+    p.normalize_scale = fixed == 1;
+    p.poses = f64(o_scene) + q.scene_offset;
+    p.points = p.poses + 12 * C;
+    p.cams = p.points + 3 * P;
+    p.pixels = p.cams + 6 * C;
+    p.tposes = f64(w.tposes);
+    p.tpoints = f64(w.tpoints);
+    const uint32_t* x = u32(o_index) + q.index_offset;
+    p.obs_camera = x;
+    p.obs_point = x + M;
+    p.point_start = x + 2 * M;
+    p.camera_start = p.point_start + P + 1;
+    p.camera_obs = p.camera_start + C + 1;
+    p.active = p.camera_obs + M;
+    p.tasks = u32(o_flat) + at.tasks;
+    p.task_obs = u32(o_flat) + at.obs;
+    p.ntasks = uint32_t(plans[k].tasks.size() - 1);
+    p.chunk_cam = u32(o_flat) + at.cam;
+    p.chunk_beg = u32(o_flat) + at.beg;
+    p.cam_chunk = u32(o_flat) + at.first;
+    p.nchunks = uint32_t(plans[k].chunks.cam.size());
+    p.task_blocks = task_blocks(k);
+    p.rlim = f64(w.rlim);
+    p.cm_point = u32(w.cmp);
+    p.cm_pixel = f64(w.cmx);
+    p.pblk = f64(w.pblk);
+    p.Mpad = uint32_t((M + 31) / 32 * 32);
+    p.factored = p.schur = 1;
+    p.A = f64(w.A);
+    p.camScf = f64(w.scf);
+    p.pw = f64(w.pw);
+    p.xw = f64(w.xw);
+    p.camU = f64(w.U);
+    p.camMinv = f64(w.Minv);
+    p.camRhs = f64(w.rhs);
+    p.camHcf = f64(w.hcf);
+    p.chunk_part = f64(w.chunk);
+    p.x = f64(w.vec);
+    p.r = p.x + p.m;
+    p.p = p.r + p.m;
+    p.Sp = p.p + p.m;
+    p.z = p.Sp + p.m;
+    p.scal_part = f64(w.scal);
+    p.cost_part = f64(w.cost);
+    p.ticket = u32(w.ticket);
+    p.state = f64(w.state);
+    p.output = f64(o_out) + q.output_offset;
+    y = tba::SchurParams{};
+    c = tba::PcgSystem{};
+    systems[k].bind(a + w.system, y, c);
+    y.bits = u32(o_bits) + bits;
+    bits += size_t(C) * y.bwords;
+    bind_problem(p, y, c);
+  }
+  cudaStream_t s = d->stream;
+  auto up = [&](size_t off, const void* src, size_t bytes) {
+    if (bytes) CUDA_TRY(cudaMemcpyAsync(a + off, src, bytes, cudaMemcpyHostToDevice, s));
+    h2d += bytes;
+  };
+  CUDA_TRY(cudaEventRecord(begun, s));
+  up(o_scene, scene, scene_len * sizeof(double));
+  up(o_index, index, index_len * sizeof(uint32_t));
+  up(o_flat, flat.data(), flat.size() * sizeof(uint32_t));
+  for (int j = 0; j < 11; j++) up(o_list[j], lists[j].data(), lists[j].size() * sizeof(uint2));
+  up(o_params, params.data(), count * sizeof(tba::Params));
+  up(o_schur, schur.data(), count * sizeof(tba::SchurParams));
+  up(o_pcg, pcg.data(), count * sizeof(tba::PcgSystem));
+  CUDA_TRY(cudaEventRecord(uploaded, s));
+
+  struct Key {
+    tba::ManyLists many;
+    tba::SchurLists schur;
+    tba::PcgMany pcg;
+    uint32_t count, limit;
+  } key;
+  std::memset(&key, 0, sizeof key);
+  auto list = [&](auto& to, int j) {
+    to.work = reinterpret_cast<const uint2*>(a + o_list[j]);
+    to.blocks = uint32_t(lists[j].size());
+  };
+  key.many.params = reinterpret_cast<const tba::Params*>(a + o_params);
+  key.many.active = u32(o_active);
+  key.many.count = count;
+  key.many.shared = shared;
+  list(key.many.one, 0);
+  list(key.many.task, 1);
+  list(key.many.chunk, 2);
+  list(key.many.finish, 3);
+  list(key.many.setup, 4);
+  list(key.many.commit, 5);
+  list(key.many.pack, 6);
+  key.schur.params = reinterpret_cast<const tba::SchurParams*>(a + o_schur);
+  key.schur.max_cameras = Cmax;
+  list(key.schur.one, 0);
+  list(key.schur.chunk, 2);
+  list(key.schur.camera, 7);
+  list(key.schur.pairs, 8);
+  list(key.schur.ends, 9);
+  list(key.schur.sums, 10);
+  key.pcg.systems = reinterpret_cast<const tba::PcgSystem*>(a + o_pcg);
+  key.pcg.work = key.many.one.work;
+  key.count = count;
+  key.limit = bc->max_cg;
+  CUDA_TRY(cudaMemsetAsync(a + o_bits, 0, bit_words * sizeof(uint32_t), s));
+  uint32_t launches = tba::launch_many_begin(key.many, s);
+  launches += tba::schur_launch_many_structure(key.schur, s);
+  launches += tba::pcg_launch_many_plan(key.pcg, count, Cmax, s);
+  CUDA_TRY(cudaGetLastError());
+  uint32_t per_iteration = 0;
+  auto iteration = [&]() {
+    per_iteration = tba::launch_many_linearize(key.many, s);
+    per_iteration += tba::schur_launch_many_values(key.schur, s);
+    per_iteration += tba::launch_many_pcg_init(key.many, s);
+    const cudaError_t e = tba::launch_many_pcg(key.pcg, count, shared, bc->max_cg, s);
+    per_iteration += 1 + tba::launch_many_update(key.many, s);
+    return e;
+  };
+  const char* bytes = reinterpret_cast<const char*>(&key);
+  rep.replayed = d->window_graph && d->window_key.size() == sizeof key && std::memcmp(d->window_key.data(), bytes, sizeof key) == 0;
+  if (!rep.replayed) {
+    if (d->window_graph) {
+      CUDA_TRY(cudaGraphExecDestroy(d->window_graph));
+      d->window_graph = nullptr;
+    }
+    cudaGraph_t graph = nullptr;
+    CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t e1 = iteration();
+    const cudaError_t e2 = cudaGetLastError(), e3 = cudaStreamEndCapture(s, &graph);
+    CUDA_TRY(e1);
+    CUDA_TRY(e2);
+    CUDA_TRY(e3);
+    const cudaError_t e4 = cudaGraphInstantiate(&d->window_graph, graph, 0);
+    cudaGraphDestroy(graph);
+    if (e4 != cudaSuccess) d->window_graph = nullptr;
+    CUDA_TRY(e4);
+    d->window_key.assign(bytes, bytes + sizeof key);
+  } else {
+    per_iteration = 3 + 2 + 1 + 1 + 5;
+  }
+  // Iterations are issued one ahead of the last one known to have left active problems.
+  uint32_t* active = reinterpret_cast<uint32_t*>(d->pinned);
+  *active = 1;
+  cudaEvent_t done[2] = {event(d, 6), event(d, 7)};
+  for (uint32_t it = 0; it < bc->iterations; it++) {
+    if (it >= 2) {
+      CUDA_TRY(cudaEventSynchronize(done[it & 1]));
+      if (*reinterpret_cast<volatile uint32_t*>(active) == 0) break;
+    }
+    CUDA_TRY(cudaGraphLaunch(d->window_graph, s));
+    launches += per_iteration;
+    CUDA_TRY(cudaMemcpyAsync(active, key.many.active, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaEventRecord(done[it & 1], s));
+  }
+  launches += tba::launch_many_pack(key.many, s);
+  CUDA_TRY(cudaGetLastError());
+  // The host arrays above stay until their copies are done.
+  CUDA_TRY(cudaEventSynchronize(uploaded));
+  rep.shape = tba::kBatchGridShape;
+  rep.threads = tba::kBatchGridThreads;
+  rep.blocks = key.many.task.blocks;
+  rep.launches = launches;
+  dout_of = f64(o_out);
+  return true;
+}
+
 void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_problem* probs, uint32_t count,
                  const double* scene, size_t scene_len, const uint32_t* index, size_t index_len, double* output,
                  size_t output_len, tba_batch_report* report) {
@@ -1194,7 +1525,11 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   std::vector<uint64_t> task_first(count), task_count(count);
   // Each problem is checked and scheduled on its own; the problems are spread over host threads and
   // the failure reported is the one of the first failing problem, as a loop in order would report.
-  std::vector<std::vector<uint32_t>> problem_tasks(count);
+  std::vector<WindowPlan> plans(count);
+  const bool auto_shape = bc->schedule == 0, grid_forced = bc->schedule == uint32_t(tba::kBatchGridShape) + 1;
+  uint64_t M_all = 0;
+  for (uint32_t k = 0; k < count; k++) M_all += probs[k].observations;
+  const uint32_t chunk = std::min<uint32_t>(1024, chunk_size(M_all, d->sms));
   std::mutex fail_mu;
   uint32_t fail_at = UINT32_MAX;
   Fail first_fail{TBA_OK, ""};
@@ -1218,7 +1553,12 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
           argument("Invalid GPU BA batch: a result record lies outside the output array");
         check_index(&c, index + q.index_offset);
         check_scene(&c, scene + q.scene_offset, tba_scene_size(&c));
-        problem_tasks[k] = build_tasks(index + q.index_offset + 2 * size_t(q.observations), q.points);
+        const uint32_t* ps = index + q.index_offset + 2 * size_t(q.observations);
+        plans[k].tasks = build_tasks(ps, q.points);
+        if (auto_shape || grid_forced) {
+          plans[k].chunks = build_chunks(ps + q.points + 1, q.cameras, chunk);
+          plans[k].pairs = count_pairs(ps, q.points);
+        }
       } catch (const Fail& f) {
         std::lock_guard<std::mutex> lock(fail_mu);
         if (k < fail_at) {
@@ -1231,7 +1571,7 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   });
   if (fail_at != UINT32_MAX) throw first_fail;
   for (uint32_t k = 0; k < count; k++) {
-    const std::vector<uint32_t>& t = problem_tasks[k];
+    const std::vector<uint32_t>& t = plans[k].tasks;
     task_first[k] = tasks.size();
     task_count[k] = t.size() - 1;
     tasks.insert(tasks.end(), t.begin(), t.end());
@@ -1253,6 +1593,79 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
     return uint64_t(probs[a].observations) * probs[a].cameras > uint64_t(probs[b].observations) * probs[b].cameras;
   });
+
+  cudaStream_t s = d->stream;
+  cudaEvent_t e0 = event(d, 0), e1 = event(d, 1), e2 = event(d, 2), e3 = event(d, 3);
+  uint64_t h2d = 0;
+  double tune_ms = 0;
+  BatchReport ran;
+  // Download of the result records, merged into contiguous runs, and the report.
+  auto finish = [&](const double* dout) {
+    CUDA_TRY(cudaEventRecord(e2, s));
+    uint64_t d2h = 0;
+    for (uint32_t j = 0; j < count;) {
+      const tba_batch_problem& q0 = probs[by_out[j]];
+      const size_t begin = q0.output_offset;
+      tba_control c0 = batch_problem_control(bc, q0);
+      size_t end = begin + tba_output_size(&c0);
+      uint32_t k = j + 1;
+      while (k < count && probs[by_out[k]].output_offset == end) {
+        const tba_control ck = batch_problem_control(bc, probs[by_out[k]]);
+        end += tba_output_size(&ck);
+        k++;
+      }
+      CUDA_TRY(cudaMemcpyAsync(output + begin, dout + begin, (end - begin) * sizeof(double), cudaMemcpyDeviceToHost, s));
+      d2h += (end - begin) * sizeof(double);
+      j = k;
+    }
+    CUDA_TRY(cudaEventRecord(e3, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (report) {
+      std::memset(report, 0, sizeof *report);
+      float ms = 0;
+      CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+      report->upload_ms = ms;
+      CUDA_TRY(cudaEventElapsedTime(&ms, e1, e2));
+      report->solve_ms = ms;
+      CUDA_TRY(cudaEventElapsedTime(&ms, e2, e3));
+      report->download_ms = ms;
+      report->tune_ms = tune_ms;
+      report->h2d_bytes = h2d;
+      report->d2h_bytes = d2h;
+      for (uint32_t k = 0; k < count; k++) {
+        const tba_batch_problem& q = probs[k];
+        const double* st = output + q.output_offset + 12 * size_t(q.cameras) + 3 * size_t(q.points);
+        report->lm_iterations += uint64_t(st[tba::S_ACCEPTED] + st[tba::S_REJECTED]);
+        report->cg_iterations += uint64_t(st[tba::S_CG_STEPS]);
+      }
+      report->problems = count;
+      report->schedule = uint32_t(ran.shape);
+      report->threads = ran.threads;
+      report->blocks = ran.blocks;
+      report->graph_replayed = ran.replayed ? 1 : 0;
+      report->kernel_launches = ran.launches;
+      report->form = ran.mixed ? TBA_PRECISION_MIXED : TBA_PRECISION_FP64;
+      report->wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - wall0).count();
+    }
+  };
+  // The grid kernels unless another shape is asked for.  They form each reduced system, at a cost that
+  // grows with the pairs of observations of a point; beyond tracks of about 64 that is more than the
+  // block solver's passes over the observations, and they need the memory for them.
+  if (auto_shape || grid_forced) {
+    uint64_t pairs = 0;
+    bool fits = true;
+    for (uint32_t k = 0; k < count; k++) {
+      pairs += plans[k].pairs;
+      fits = fits && plans[k].pairs < 0x7fffffffull;
+    }
+    double* dout = nullptr;
+    if (fits && (grid_forced || pairs <= 32 * M_all) &&
+        batch_on_grid(d, bc, probs, count, plans, order, scene, scene_len, index, index_len, output_len, e1, e0, ran, dout, h2d)) {
+      finish(dout);
+      return;
+    }
+    if (grid_forced) throw Fail{TBA_ERROR_BUDGET, "GPU BA batch needs more device memory than the working budget"};
+  }
 
   // Device layout: the caller's arrays as they are, then the schedule and the workspace.
   Layout L;
@@ -1346,9 +1759,6 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   args.stall = bc->stall_tolerance;
   const size_t smem = tba::batch_smem_bytes(Cmax);
 
-  cudaStream_t s = d->stream;
-  cudaEvent_t e0 = event(d, 0), e1 = event(d, 1), e2 = event(d, 2), e3 = event(d, 3);
-  uint64_t h2d = 0;
   auto up = [&](size_t off, const void* src, size_t bytes) {
     if (bytes) CUDA_TRY(cudaMemcpyAsync(a + off, src, bytes, cudaMemcpyHostToDevice, s));
     h2d += bytes;
@@ -1383,7 +1793,6 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   // device copy of the results).  A mixed request tries the FP64 form too and keeps it when it is
   // faster: on small windows the FP32 product saves less than the FP64 refinement of each PCG
   // solution costs.  The result is the FP64 form's, which the mixed form only approximates.
-  double tune_ms = 0;
   int shape = -1;
   bool run_mixed = mixed;
   if (bc->schedule > 0) {
@@ -1481,53 +1890,13 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
     d->batch_key = key;
   }
   CUDA_TRY(cudaGraphLaunch(d->batch_graph, s));
-  CUDA_TRY(cudaEventRecord(e2, s));
-  // Download the result records, merged into contiguous runs.
-  uint64_t d2h = 0;
-  for (uint32_t j = 0; j < count;) {
-    const tba_batch_problem& q0 = probs[by_out[j]];
-    const size_t begin = q0.output_offset;
-    tba_control c0 = batch_problem_control(bc, q0);
-    size_t end = begin + tba_output_size(&c0);
-    uint32_t k = j + 1;
-    while (k < count && probs[by_out[k]].output_offset == end) {
-      const tba_control ck = batch_problem_control(bc, probs[by_out[k]]);
-      end += tba_output_size(&ck);
-      k++;
-    }
-    CUDA_TRY(cudaMemcpyAsync(output + begin, dout + begin, (end - begin) * sizeof(double), cudaMemcpyDeviceToHost, s));
-    d2h += (end - begin) * sizeof(double);
-    j = k;
-  }
-  CUDA_TRY(cudaEventRecord(e3, s));
-  CUDA_TRY(cudaStreamSynchronize(s));
-  if (report) {
-    std::memset(report, 0, sizeof *report);
-    float ms = 0;
-    CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
-    report->upload_ms = ms;
-    CUDA_TRY(cudaEventElapsedTime(&ms, e1, e2));
-    report->solve_ms = ms;
-    CUDA_TRY(cudaEventElapsedTime(&ms, e2, e3));
-    report->download_ms = ms;
-    report->tune_ms = tune_ms;
-    report->h2d_bytes = h2d;
-    report->d2h_bytes = d2h;
-    for (uint32_t k = 0; k < count; k++) {
-      const tba_batch_problem& q = probs[k];
-      const double* st = output + q.output_offset + 12 * size_t(q.cameras) + 3 * size_t(q.points);
-      report->lm_iterations += uint64_t(st[tba::S_ACCEPTED] + st[tba::S_REJECTED]);
-      report->cg_iterations += uint64_t(st[tba::S_CG_STEPS]);
-    }
-    report->problems = count;
-    report->schedule = uint32_t(shape);
-    report->threads = uint32_t(tba::batch_shape(shape).threads);
-    report->blocks = uint32_t(blocks);
-    report->graph_replayed = replayed ? 1 : 0;
-    report->kernel_launches = 2;
-    report->form = run_mixed ? TBA_PRECISION_MIXED : TBA_PRECISION_FP64;
-    report->wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - wall0).count();
-  }
+  ran.shape = shape;
+  ran.threads = uint32_t(tba::batch_shape(shape).threads);
+  ran.blocks = uint32_t(blocks);
+  ran.launches = 2;
+  ran.replayed = replayed;
+  ran.mixed = run_mixed;
+  finish(dout);
 }
 
 // ---- the adjoint ---------------------------------------------------------------------------------
@@ -1564,7 +1933,7 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
   const uint64_t npairs = count_pairs(index + 2 * size_t(M), P);
   bool schur = prefer_schur(C, M, npairs, vc->max_cg, 64);
   Chunks chunks;
-  if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, M, d->sms);
+  if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, chunk_size(M, d->sms));
   const uint32_t nchunks = uint32_t(chunks.cam.size());
   Layout L;
   const size_t o_poses = L.take<double>(12 * size_t(C)), o_points = L.take<double>(3 * size_t(P)),
@@ -1989,6 +2358,7 @@ void tba_device_close(tba_device* d) {
   if (d->down) cudaStreamSynchronize(d->down);
   for (cudaEvent_t e : d->events) cudaEventDestroy(e);
   if (d->batch_graph) cudaGraphExecDestroy(d->batch_graph);
+  if (d->window_graph) cudaGraphExecDestroy(d->window_graph);
   for (PcgLoop& loop : d->pcg_loops) loop.release();
   d->adj_loop.release();
   if (d->batch_arena) cudaFree(d->batch_arena);
@@ -2037,11 +2407,11 @@ tba_status tba_bundle_adjust(tba_device* d, const tba_control* control, const do
 }
 
 uint32_t tba_batch_max_cameras(void) { return tba::batch_max_cameras(); }
-uint32_t tba_batch_shapes(void) { return uint32_t(tba::kBatchShapes); }
+uint32_t tba_batch_shapes(void) { return uint32_t(tba::kBatchShapes) + 1; }
 
 tba_status tba_batch_shape(uint32_t k, uint32_t* threads, uint32_t* min_blocks) {
-  if (k >= uint32_t(tba::kBatchShapes)) return TBA_ERROR_ARGUMENT;
-  const tba::BatchShape s = tba::batch_shape(int(k));
+  if (k > uint32_t(tba::kBatchGridShape)) return TBA_ERROR_ARGUMENT;
+  const tba::BatchShape s = k == uint32_t(tba::kBatchGridShape) ? tba::BatchShape{tba::kBatchGridThreads, 2} : tba::batch_shape(int(k));
   if (threads) *threads = uint32_t(s.threads);
   if (min_blocks) *min_blocks = uint32_t(s.min_blocks);
   return TBA_OK;

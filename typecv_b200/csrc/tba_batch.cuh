@@ -52,6 +52,10 @@ struct BatchShape {
   int threads, min_blocks;
 };
 constexpr int kBatchShapes = 4;
+// One more shape, not a launch of the block solver: every problem solved side by side by the grid
+// engine's kernels on explicit reduced systems (FP64).
+constexpr int kBatchGridShape = kBatchShapes;
+constexpr int kBatchGridThreads = 256;
 BatchShape batch_shape(int k);
 size_t batch_smem_bytes(uint32_t Cmax);
 // The largest camera count whose shared-memory layout fits one block.

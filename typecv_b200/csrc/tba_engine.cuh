@@ -155,6 +155,31 @@ struct Params {
   cudaGraphConditionalHandle pcg_loop;
 };
 
+// A batch of problems solved side by side by the same kernels: every problem's parameters in device
+// memory, and a kernel's blocks as a list of (problem, block of that problem).
+struct Many {
+  const Params* params;
+  const uint2* work;
+};
+struct ManyLists {
+  const Params* params;
+  uint32_t* active;  // receives whether problems are still active (0: none) after an LM iteration
+  uint32_t count, shared;
+  struct List {
+    const uint2* work;
+    uint32_t blocks;
+    Many of(const ManyLists& b) const { return Many{b.params, work}; }
+  };
+  // A block per: problem; share of the tasks; camera chunk; four cameras; 256 observations or cameras;
+  // 256 candidate values; 256 result values.
+  List one, task, chunk, finish, setup, commit, pack;
+};
+uint32_t launch_many_begin(const ManyLists& b, cudaStream_t s);
+uint32_t launch_many_linearize(const ManyLists& b, cudaStream_t s);
+uint32_t launch_many_pcg_init(const ManyLists& b, cudaStream_t s);
+uint32_t launch_many_update(const ManyLists& b, cudaStream_t s);
+uint32_t launch_many_pack(const ManyLists& b, cudaStream_t s);
+
 // Launches (tba_kernels.cu), each on stream `s`; grids come from `p`.
 void launch_initialize(const Params& p, cudaStream_t s);
 void launch_cost(const Params& p, cudaStream_t s);

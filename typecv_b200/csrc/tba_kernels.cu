@@ -51,6 +51,30 @@
 namespace tba {
 namespace {
 
+// Where a block's problem and its place in that problem's grid come from: a solve's parameters are the
+// kernel's argument and the grid is the problem's; a batch (Many) has a list of (problem, block) and
+// copies the problem's parameters to shared memory.
+template <class W>
+struct Slot {};
+template <>
+struct Slot<Many> {
+  Params p;
+};
+__device__ inline const Params& block_problem(const Params& P, Slot<Params>&, uint32_t& bid) {
+  bid = blockIdx.x;
+  return P;
+}
+__device__ inline const Params& block_problem(const Many& W, Slot<Many>& slot, uint32_t& bid) {
+  const uint2 w = W.work[blockIdx.x];
+  static_assert(sizeof(Params) % 8 == 0, "copied as 8-byte words");
+  const uint64_t* from = reinterpret_cast<const uint64_t*>(W.params + w.x);
+  uint64_t* to = reinterpret_cast<uint64_t*>(&slot.p);
+  for (uint32_t k = threadIdx.x; k < sizeof(Params) / 8; k += blockDim.x) to[k] = from[k];
+  __syncthreads();
+  bid = w.y;
+  return slot.p;
+}
+
 // The camera record with the accepted (or candidate) focal scale applied.
 __device__ inline Camera camera_at(const Params& P, uint32_t c, double fscale) {
   const double2* k = reinterpret_cast<const double2*>(P.cams + 6 * size_t(c));
@@ -61,9 +85,9 @@ __device__ inline Camera camera_at(const Params& P, uint32_t c, double fscale) {
 __device__ inline double focal_scale(const Params& P, double log_scale) { return P.shared ? exp(log_scale) : 1.0; }
 
 // The tasks [begin, end) of this block: a contiguous share of the task list.
-__device__ inline void block_tasks(const Params& P, uint32_t& begin, uint32_t& end) {
-  begin = uint32_t(uint64_t(P.ntasks) * blockIdx.x / gridDim.x);
-  end = uint32_t(uint64_t(P.ntasks) * (blockIdx.x + 1) / gridDim.x);
+__device__ inline void block_tasks(const Params& P, uint32_t bid, uint32_t grid, uint32_t& begin, uint32_t& end) {
+  begin = uint32_t(uint64_t(P.ntasks) * bid / grid);
+  end = uint32_t(uint64_t(P.ntasks) * (bid + 1) / grid);
 }
 
 __device__ inline bool directional(const Params& P, uint32_t pt) { return pt >= P.P - P.D; }
@@ -91,7 +115,12 @@ __device__ inline bool last_block(uint32_t* ticket) {
 
 // ---- K1: initializeBundle, and the per-solve set-up -----------------------------------------------
 
-__global__ void k_initialize(Params P) {
+template <class W>
+__global__ void k_initialize(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
+  if (threadIdx.x != 0) return;
   double* st = P.state;
   for (int j = 0; j < S_WORDS; j++) st[j] = 0;
   st[S_LAMBDA] = 1e-3;
@@ -115,8 +144,12 @@ __global__ void k_initialize(Params P) {
 }
 
 // Per-camera radial limits; the camera-major copies of each observation's point and pixel.
-__global__ void k_setup(Params P) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+template <class W>
+__global__ void k_setup(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
+  const uint32_t k = bid * blockDim.x + threadIdx.x;
   if (k < P.C) P.rlim[k] = radial_limit(P.cams[6 * size_t(k) + 4], P.cams[6 * size_t(k) + 5]);
   if (k < P.M) {
     const uint32_t i = P.camera_obs[k];
@@ -127,11 +160,15 @@ __global__ void k_setup(Params P) {
 
 // ---- K3/K4: the linearised cost of the scene ---------------------------------------------------
 
-__global__ void __launch_bounds__(kPointThreads) k_cost(Params P) {
+template <class W>
+__global__ void __launch_bounds__(kPointThreads) k_cost(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ double red[3 * (kPointThreads / 32)];
   double v[3] = {0, 0, 0};  // cost, squared error, invalid projections
   const double fscale = focal_scale(P, P.state[S_LOG_FOCAL]);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.M; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = bid * blockDim.x + threadIdx.x; i < P.M; i += P.task_blocks * blockDim.x) {
     double pose[12];
     Geo g;
     if (!observe(P, i, P.obs_camera[i], P.obs_point[i], fscale, pose, g)) {
@@ -143,10 +180,14 @@ __global__ void __launch_bounds__(kPointThreads) k_cost(Params P) {
   }
   block_sum(v, red);
   if (threadIdx.x == 0)
-    for (int n = 0; n < 3; n++) P.cost_part[4 * blockIdx.x + n] = v[n];
+    for (int n = 0; n < 3; n++) P.cost_part[4 * bid + n] = v[n];
 }
 
-__global__ void k_finish_metrics(Params P) {
+template <class W>
+__global__ void k_finish_metrics(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ double red[3 * 32];
   double* st = P.state;
   double v[3] = {0, 0, 0};
@@ -331,8 +372,11 @@ __device__ inline void point_finish(const Params& P, uint32_t pt, const double (
   }
 }
 
-template <bool SHARED, bool EXPLICIT>
-__global__ void __launch_bounds__(kPointThreads, TBA_POINT_MIN_BLOCKS) k_point_pass(Params P) {
+template <bool SHARED, bool EXPLICIT, class W>
+__global__ void __launch_bounds__(kPointThreads, TBA_POINT_MIN_BLOCKS) k_point_pass(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ double red[kScalarPartials * (kPointThreads / 32)];
   __shared__ double2 stage_all[EXPLICIT ? kPointThreads * 9 : 1];
   if (P.state[S_ACTIVE] == 0) return;
@@ -341,7 +385,7 @@ __global__ void __launch_bounds__(kPointThreads, TBA_POINT_MIN_BLOCKS) k_point_p
   double* stage = reinterpret_cast<double*>(stage_all) + (EXPLICIT ? warp * 32 * 18 : 0);
   double sc[kScalarPartials] = {0, 0, 0, 0};  // hff, bf, diag_pt, rhs_pt (lane-local)
   uint32_t tb, te;
-  block_tasks(P, tb, te);
+  block_tasks(P, bid, P.task_blocks, tb, te);
   for (uint32_t t = tb + warp; t < te; t += nwarps) {
     const uint32_t p0 = P.tasks[t], p1 = P.tasks[t + 1];
     const uint32_t o0 = P.point_start[p0], n = P.point_start[p1] - o0;
@@ -402,7 +446,7 @@ __global__ void __launch_bounds__(kPointThreads, TBA_POINT_MIN_BLOCKS) k_point_p
   }
   block_sum(sc, red);
   if (threadIdx.x == 0)
-    for (int k = 0; k < kScalarPartials; k++) P.scal_part[kScalarPartials * blockIdx.x + k] = sc[k];
+    for (int k = 0; k < kScalarPartials; k++) P.scal_part[kScalarPartials * bid + k] = sc[k];
 }
 
 // ---- K6/K8/K21: camera blocks ------------------------------------------------------------------
@@ -415,12 +459,15 @@ __device__ inline void camera_rows(const Geo& g, bool dir, double jc[2][6]) {
     for (int c = 3; c < 6; c++) jc[0][c] = jc[1][c] = 0;
 }
 
-template <bool EXPLICIT>
-__global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camera_pass(Params P) {
+template <bool EXPLICIT, class W>
+__global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camera_pass(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   constexpr int kParts = EXPLICIT ? kCameraPartialsExplicit : kCameraPartials, kSecond = kParts - 33;
   __shared__ double red[kParts * (kCameraThreads / 32)];
   if (P.state[S_ACTIVE] == 0) return;
-  const uint32_t ch = blockIdx.x, c = P.chunk_cam[ch];
+  const uint32_t ch = bid, c = P.chunk_cam[ch];
   if (P.active[c] == 0) return;
   const uint32_t k0 = P.chunk_beg[ch], k1 = P.chunk_beg[ch + 1];
   double pose[12];
@@ -518,13 +565,16 @@ __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camer
 // column of the inverse each (one thread per camera spent 42 us on 7 cameras and 70 us on 200).
 constexpr int kFinishThreads = 128;
 
-template <bool EXPLICIT>
-__global__ void __launch_bounds__(kFinishThreads) k_camera_finish(Params P) {
+template <bool EXPLICIT, class W>
+__global__ void __launch_bounds__(kFinishThreads) k_camera_finish(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   constexpr int kParts = EXPLICIT ? kCameraPartialsExplicit : kCameraPartials;
   __shared__ double sums[kFinishThreads / 32][kParts], inverse[kFinishThreads / 32][36];
   if (P.state[S_ACTIVE] == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t c = blockIdx.x * (kFinishThreads / 32) + warp;
+  const uint32_t c = bid * (kFinishThreads / 32) + warp;
   if (c >= P.C) return;
   double* U = P.camU + 21 * size_t(c);
   double* Minv = P.camMinv + 36 * size_t(c);
@@ -594,7 +644,11 @@ __device__ inline double precondition(const Params& P, uint32_t i) {
   return Mi[0] * rc[0] + Mi[1] * rc[1] + Mi[2] * rc[2] + Mi[3] * rc[3] + Mi[4] * rc[4] + Mi[5] * rc[5];
 }
 
-__global__ void __launch_bounds__(1024) k_pcg_init(Params P) {
+template <class W>
+__global__ void __launch_bounds__(1024) k_pcg_init(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ double red[4 * 32];
   __shared__ int fail;
   double* st = P.state;
@@ -701,7 +755,7 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_schur_p
   const double pf = SHARED ? P.p[P.m - 1] : 0.0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   uint32_t tb, te;
-  block_tasks(P, tb, te);
+  block_tasks(P, blockIdx.x, gridDim.x, tb, te);
   for (uint32_t t = tb + warp; t < te; t += nwarps) {
     const uint32_t p0 = P.tasks[t], p1 = P.tasks[t + 1];
     const uint32_t o0 = P.point_start[p0], n = P.point_start[p1] - o0;
@@ -903,7 +957,7 @@ __global__ void __launch_bounds__(STAGED ? (sizeof(T) == 4 ? kStagedThreadsF32 :
   const double pf = SHARED ? P.p[m - 1] : 0.0;
   double ef = 0;
   uint32_t tb, te;
-  block_tasks(P, tb, te);
+  block_tasks(P, blockIdx.x, gridDim.x, tb, te);
   uint32_t t = tb + warp;
   uint32_t o_next = t < te ? P.task_obs[t] : 0, e_next = t < te ? P.task_obs[t + 1] : 0;
   for (; t < te; t += nwarps) {
@@ -1525,7 +1579,11 @@ __global__ void __launch_bounds__(kUpdateThreads) k_refine(Params P) {
 
 // ---- K14/K15/K16: the candidate cameras, the focal scale and the gauge --------------------------
 
-__global__ void __launch_bounds__(256) k_update_cameras(Params P) {
+template <class W>
+__global__ void __launch_bounds__(256) k_update_cameras(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ int ok;
   double* st = P.state;
   if (threadIdx.x == 0) st[S_TRIAL_VALID] = 0;
@@ -1694,8 +1752,11 @@ __device__ inline void record_wt(const double* rec, const double* x, double t[3]
   }
 }
 
-template <bool SHARED, bool EXPLICIT>
-__global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_points(Params P) {
+template <bool SHARED, bool EXPLICIT, class W>
+__global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_points(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ double red[2 * (kPointThreads / 32)];
   __shared__ double2 stage_all[EXPLICIT ? kPointThreads * 9 : 1];
   const double* st = P.state;
@@ -1706,7 +1767,7 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_
   double* stage = reinterpret_cast<double*>(stage_all) + (EXPLICIT ? warp * 32 * 18 : 0);
   double cs[2] = {0, 0};
   uint32_t tb, te;
-  block_tasks(P, tb, te);
+  block_tasks(P, bid, P.task_blocks, tb, te);
   for (uint32_t t = tb + warp; t < te; t += nwarps) {
     const uint32_t p0 = P.tasks[t], p1 = P.tasks[t + 1];
     const uint32_t o0 = P.point_start[p0], n = P.point_start[p1] - o0;
@@ -1755,14 +1816,18 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_
   }
   block_sum(cs, red);
   if (threadIdx.x == 0) {
-    P.cost_part[4 * blockIdx.x] = cs[0];
-    P.cost_part[4 * blockIdx.x + 1] = cs[1];
+    P.cost_part[4 * bid] = cs[0];
+    P.cost_part[4 * bid + 1] = cs[1];
   }
 }
 
 // ---- K18/K19: acceptance and commit ------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) k_accept(Params P) {
+template <class W>
+__global__ void __launch_bounds__(256) k_accept(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   __shared__ double red[2 * 8];
   double* st = P.state;
   double v[2] = {0, 0};
@@ -1794,10 +1859,22 @@ __global__ void __launch_bounds__(256) k_accept(Params P) {
   st[S_POINT_FAILED] = 0;
 }
 
-__global__ void k_commit(Params P) {
+// How many problems of a batch are still active.
+__global__ void __launch_bounds__(256) k_many_active(const Params* params, uint32_t count, uint32_t* active) {
+  uint32_t n = 0;
+  for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) n += params[k].state[S_ACTIVE] != 0;
+  n = __syncthreads_count(n != 0);
+  if (threadIdx.x == 0) *active = n;
+}
+
+template <class W>
+__global__ void k_commit(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
   const double* st = P.state;
   if (st[S_COMMIT] == 0) return;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = bid * blockDim.x + threadIdx.x;
   if (i < 12 * P.C) P.poses[i] = P.tposes[i];
   if (i < 3 * P.P) P.points[i] = P.tpoints[i];
   if (i == 0 && P.shared) P.state[S_LOG_FOCAL] = st[S_LOG_FOCAL_TRIAL];
@@ -1805,8 +1882,12 @@ __global__ void k_commit(Params P) {
 
 // ---- K20: packBundleResult ----------------------------------------------------------------------
 
-__global__ void k_pack(Params P) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+template <class W>
+__global__ void k_pack(W w) {
+  __shared__ Slot<W> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
+  const uint32_t i = bid * blockDim.x + threadIdx.x;
   const uint32_t np = 12 * P.C, total = np + 3 * P.P;
   if (i < np) P.output[i] = P.poses[i];
   else if (i < total) P.output[i] = P.points[i - np];
@@ -1917,22 +1998,22 @@ void launch_cost(const Params& p, cudaStream_t s) { k_cost<<<p.task_blocks, kPoi
 void launch_finish_metrics(const Params& p, cudaStream_t s) { k_finish_metrics<<<1, 1024, 0, s>>>(p); }
 void launch_point_pass(const Params& p, cudaStream_t s) {
   if (p.schur) {
-    if (p.shared) k_point_pass<true, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
-    else k_point_pass<false, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    if (p.shared) k_point_pass<true, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    else k_point_pass<false, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   } else if (p.shared) {
-    k_point_pass<true, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    k_point_pass<true, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   } else {
-    k_point_pass<false, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    k_point_pass<false, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   }
 }
 void launch_camera_pass(const Params& p, cudaStream_t s) {
-  if (p.schur) k_camera_pass<true><<<p.nchunks, kCameraThreads, 0, s>>>(p);
-  else k_camera_pass<false><<<p.nchunks, kCameraThreads, 0, s>>>(p);
+  if (p.schur) k_camera_pass<true, Params><<<p.nchunks, kCameraThreads, 0, s>>>(p);
+  else k_camera_pass<false, Params><<<p.nchunks, kCameraThreads, 0, s>>>(p);
 }
 void launch_camera_finish(const Params& p, cudaStream_t s) {
   constexpr uint32_t per = kFinishThreads / 32;
-  if (p.schur) k_camera_finish<true><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
-  else k_camera_finish<false><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
+  if (p.schur) k_camera_finish<true, Params><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
+  else k_camera_finish<false, Params><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
 }
 void launch_pcg_init(const Params& p, cudaStream_t s) { k_pcg_init<<<1, 1024, 0, s>>>(p); }
 void launch_product(const Params& p, cudaStream_t s) {
@@ -1996,15 +2077,47 @@ void launch_product_rows(const Params& p, double* out, cudaStream_t s) {
 void launch_update_cameras(const Params& p, cudaStream_t s) { k_update_cameras<<<1, 256, 0, s>>>(p); }
 void launch_update_points(const Params& p, cudaStream_t s) {
   if (p.schur) {
-    if (p.shared) k_update_points<true, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
-    else k_update_points<false, true><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    if (p.shared) k_update_points<true, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    else k_update_points<false, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   } else if (p.shared) {
-    k_update_points<true, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    k_update_points<true, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   } else {
-    k_update_points<false, false><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    k_update_points<false, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   }
 }
 void launch_accept(const Params& p, cudaStream_t s) { k_accept<<<1, 256, 0, s>>>(p); }
+// The kernels of one LM iteration up to the PCG, and after it, over a batch's lists of blocks.
+uint32_t launch_many_begin(const ManyLists& b, cudaStream_t s) {
+  k_initialize<Many><<<b.one.blocks, 32, 0, s>>>(b.one.of(b));
+  k_setup<Many><<<b.setup.blocks, 256, 0, s>>>(b.setup.of(b));
+  k_cost<Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
+  k_finish_metrics<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
+  return 4;
+}
+uint32_t launch_many_linearize(const ManyLists& b, cudaStream_t s) {
+  if (b.shared) k_point_pass<true, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
+  else k_point_pass<false, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
+  k_camera_pass<true, Many><<<b.chunk.blocks, kCameraThreads, 0, s>>>(b.chunk.of(b));
+  k_camera_finish<true, Many><<<b.finish.blocks, kFinishThreads, 0, s>>>(b.finish.of(b));
+  return 3;
+}
+uint32_t launch_many_pcg_init(const ManyLists& b, cudaStream_t s) {
+  k_pcg_init<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
+  return 1;
+}
+uint32_t launch_many_update(const ManyLists& b, cudaStream_t s) {
+  k_update_cameras<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
+  if (b.shared) k_update_points<true, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
+  else k_update_points<false, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
+  k_accept<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
+  k_commit<Many><<<b.commit.blocks, 256, 0, s>>>(b.commit.of(b));
+  k_many_active<<<1, 256, 0, s>>>(b.params, b.count, b.active);
+  return 5;
+}
+uint32_t launch_many_pack(const ManyLists& b, cudaStream_t s) {
+  k_pack<Many><<<b.pack.blocks, 256, 0, s>>>(b.pack.of(b));
+  return 1;
+}
 void launch_commit(const Params& p, cudaStream_t s) {
   const uint32_t n = (12 * p.C > 3 * p.P ? 12 * p.C : 3 * p.P);
   k_commit<<<(n + 255) / 256, 256, 0, s>>>(p);

@@ -52,6 +52,30 @@ __device__ __forceinline__ bool await(const Flagged* p, uint64_t step, double& v
   return false;
 }
 
+// A block's system and its place in that system's grid: the kernel's argument, or a batch's list (one
+// block a system).
+template <class W>
+struct PcgSlot {};
+template <>
+struct PcgSlot<PcgMany> {
+  PcgSystem a;
+};
+__device__ inline const PcgSystem& block_system(const PcgSystem& A, PcgSlot<PcgSystem>&, uint32_t& bid, uint32_t& grid) {
+  bid = blockIdx.x;
+  grid = gridDim.x;
+  return A;
+}
+__device__ inline const PcgSystem& block_system(const PcgMany& W, PcgSlot<PcgMany>& slot, uint32_t& bid, uint32_t& grid) {
+  static_assert(sizeof(PcgSystem) % 8 == 0, "copied as 8-byte words");
+  const uint64_t* from = reinterpret_cast<const uint64_t*>(W.systems + W.work[blockIdx.x].x);
+  uint64_t* to = reinterpret_cast<uint64_t*>(&slot.a);
+  for (uint32_t k = threadIdx.x; k < sizeof(PcgSystem) / 8; k += blockDim.x) to[k] = from[k];
+  __syncthreads();
+  bid = 0;
+  grid = 1;
+  return slot.a;
+}
+
 struct Shared {
   double red[2][kWarps][2];
   double part[kWarps][6];
@@ -61,7 +85,8 @@ struct Shared {
 
 // Adds v over the grid; every thread returns with the sums (false: a wait gave up).  `which` is the
 // step's first or second reduction.
-__device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], uint64_t step, int which) {
+__device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], uint64_t step, int which, uint32_t bid,
+                                uint32_t grid) {
   warp_allsum(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) {
@@ -69,7 +94,7 @@ __device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], 
     sh.red[which][warp][1] = v[1];
   }
   __syncthreads();
-  if (gridDim.x == 1) {
+  if (grid == 1) {
     v[0] = v[1] = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; w++) {
@@ -82,10 +107,10 @@ __device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], 
     double t[2] = {lane < kWarps ? sh.red[which][lane][0] : 0.0, lane < kWarps ? sh.red[which][lane][1] : 0.0};
     warp_allsum(t);
     Flagged* slots = A.slots + 2 * size_t(which);
-    if (lane < 2) publish(slots + 4 * size_t(blockIdx.x) + lane, lane == 0 ? t[0] : t[1], step);
+    if (lane < 2) publish(slots + 4 * size_t(bid) + lane, lane == 0 ? t[0] : t[1], step);
     bool ok = sh.gave_up == 0;
     t[0] = t[1] = 0;
-    for (uint32_t b = lane; b < gridDim.x && ok; b += 32) {
+    for (uint32_t b = lane; b < grid && ok; b += 32) {
       double s0 = 0, s1 = 0;
       ok = await(slots + 4 * size_t(b), step, s0) && await(slots + 4 * size_t(b) + 1, step, s1);
       t[0] += s0;
@@ -106,11 +131,15 @@ __device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], 
 }
 
 // Shares of about the same number of blocks of S; the distinct cameras of a share's columns.
-__global__ void __launch_bounds__(256) k_pcg_plan(PcgSystem A) {
+template <class W>
+__global__ void __launch_bounds__(256) k_pcg_plan(W w) {
+  __shared__ PcgSlot<W> slot;
+  uint32_t bid, grid;
+  const PcgSystem& A = block_system(w, slot, bid, grid);
   extern __shared__ uint32_t place[];  // C: 1 for a camera that occurs, then its place
   __shared__ uint32_t range[2], warp_sum[8];
   if (threadIdx.x < 2) {
-    const uint64_t target = uint64_t(A.row_ptr[A.C]) * (blockIdx.x + threadIdx.x) / gridDim.x;
+    const uint64_t target = uint64_t(A.row_ptr[A.C]) * (bid + threadIdx.x) / grid;
     uint32_t lo = 0, hi = A.C;
     while (lo < hi) {
       const uint32_t mid = (lo + hi) / 2;
@@ -118,7 +147,7 @@ __global__ void __launch_bounds__(256) k_pcg_plan(PcgSystem A) {
       else hi = mid;
     }
     range[threadIdx.x] = lo;
-    A.share[blockIdx.x + threadIdx.x] = lo;
+    A.share[bid + threadIdx.x] = lo;
   }
   for (uint32_t c = threadIdx.x; c < A.C; c += blockDim.x) place[c] = 0;
   __syncthreads();
@@ -140,27 +169,30 @@ __global__ void __launch_bounds__(256) k_pcg_plan(PcgSystem A) {
     }
     at += __popc(mask & ((1u << lane) - 1u));
     if (on) {
-      A.uni[size_t(blockIdx.x) * A.C + at] = c;
+      A.uni[size_t(bid) * A.C + at] = c;
       place[c] = at;
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) A.uni_n[blockIdx.x] = base;
+  if (threadIdx.x == 0) A.uni_n[bid] = base;
   for (uint32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) A.local[k] = place[A.col[k]];
 }
 
-template <bool SHARED>
-__global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit) {
+template <bool SHARED, class W>
+__global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   extern __shared__ __align__(16) double pcg_smem[];
   __shared__ Shared sh;
+  __shared__ PcgSlot<W> slot;
+  uint32_t bid, grid;
+  const PcgSystem& A = block_system(system, slot, bid, grid);
   double* st = A.state;
   if (st[A.active] == 0 || limit == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool alone = gridDim.x == 1;
-  const uint32_t c0 = A.share[blockIdx.x], c1 = A.share[blockIdx.x + 1], nr = c1 - c0, rows = 6 * nr, first = 6 * c0,
+  const bool alone = grid == 1;
+  const uint32_t c0 = A.share[bid], c1 = A.share[bid + 1], nr = c1 - c0, rows = 6 * nr, first = 6 * c0,
                  n = 6 * A.C;
-  const uint32_t* uni = A.uni + size_t(blockIdx.x) * A.C;
-  const uint32_t cols = 6 * A.uni_n[blockIdx.x];
+  const uint32_t* uni = A.uni + size_t(bid) * A.C;
+  const uint32_t cols = 6 * A.uni_n[bid];
   const uint32_t k0 = A.row_ptr[c0], blocks = A.row_ptr[c1] - k0;
   // Shared memory, as far as it goes: the direction, the own vectors, the own rows of S, their columns'
   // places and the own preconditioner blocks.
@@ -171,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit
     used += uint32_t((words + 1) & ~size_t(1));
     return p;
   };
-  double* pl = take(cols, A.pbuf + size_t(blockIdx.x) * n);
+  double* pl = take(cols, A.pbuf + size_t(bid) * n);
   double* own = take(4 * size_t(rows), nullptr);  // x, r, S p, z
   const bool keep = own != nullptr;
   double* xs = keep ? own : A.x + first;
@@ -284,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit
       ss[i] = sp;
       v[0] += pv * sp;
     }
-    if (!(ok = grid_sum(A, sh, v, step, 0))) break;
+    if (!(ok = grid_sum(A, sh, v, step, 0, bid, grid))) break;
     const double spf = SHARED ? sff * pf + v[1] : 0.0, den = SHARED ? v[0] + pf * spf : v[0], alpha = rho / den;
     if (!(den > 0) || !(fabs(alpha) < A.alpha_limit)) {
       active = false;
@@ -307,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit
       v[0] += rr * rr;
       v[1] += zz * rr;
     }
-    if (!(ok = grid_sum(A, sh, v, step, 1))) break;
+    if (!(ok = grid_sum(A, sh, v, step, 1, bid, grid))) break;
     it++;
     r2 = v[0];
     double next = v[1];
@@ -334,7 +366,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit
       A.x[first + i] = xs[i];
       A.r[first + i] = rs[i];
     }
-  if (threadIdx.x != 0 || (blockIdx.x != 0 && ok)) return;
+  if (threadIdx.x != 0 || (bid != 0 && ok)) return;
   if (!ok) {
     st[A.wait] = 1;
     st[A.failed] = 1;
@@ -357,10 +389,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(PcgSystem A, uint32_t limit
 }  // namespace
 
 cudaError_t pcg_configure() {
-  cudaError_t e = cudaFuncSetAttribute(k_pcg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_pcg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
-  return e;
+  const void* kernels[] = {
+      reinterpret_cast<const void*>(k_pcg<false, PcgSystem>), reinterpret_cast<const void*>(k_pcg<true, PcgSystem>),
+      reinterpret_cast<const void*>(k_pcg<false, PcgMany>), reinterpret_cast<const void*>(k_pcg<true, PcgMany>)};
+  for (const void* f : kernels) {
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 uint32_t pcg_grid(uint64_t blocks, uint32_t C, int sms) {
@@ -371,12 +407,13 @@ uint32_t pcg_grid(uint64_t blocks, uint32_t C, int sms) {
 }
 
 uint32_t pcg_launch_plan(const PcgSystem& a, uint32_t grid, cudaStream_t s) {
-  k_pcg_plan<<<grid, 256, size_t(a.C) * sizeof(uint32_t), s>>>(a);
+  k_pcg_plan<PcgSystem><<<grid, 256, size_t(a.C) * sizeof(uint32_t), s>>>(a);
   return 1;
 }
 
 cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaStream_t s) {
-  const void* f = a.shared ? reinterpret_cast<const void*>(k_pcg<true>) : reinterpret_cast<const void*>(k_pcg<false>);
+  const void* f = a.shared ? reinterpret_cast<const void*>(k_pcg<true, PcgSystem>)
+                           : reinterpret_cast<const void*>(k_pcg<false, PcgSystem>);
   PcgSystem q = a;
   void* args[] = {&q, &limit};
   if (grid == 1) return cudaLaunchKernel(f, dim3(1), dim3(kThreads), args, kSmemBytes, s);
@@ -385,6 +422,18 @@ cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaSt
   if (e == cudaSuccess) e = cudaMemsetAsync(a.slots, 0, 4 * size_t(grid) * sizeof(Flagged), s);
   if (e != cudaSuccess) return e;
   return cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kThreads), args, kSmemBytes, s);
+}
+
+uint32_t pcg_launch_many_plan(const PcgMany& b, uint32_t count, uint32_t max_cameras, cudaStream_t s) {
+  k_pcg_plan<PcgMany><<<count, 256, size_t(max_cameras) * sizeof(uint32_t), s>>>(b);
+  return 1;
+}
+
+cudaError_t launch_many_pcg(const PcgMany& b, uint32_t count, bool shared, uint32_t limit, cudaStream_t s) {
+  const void* f = shared ? reinterpret_cast<const void*>(k_pcg<true, PcgMany>) : reinterpret_cast<const void*>(k_pcg<false, PcgMany>);
+  PcgMany q = b;
+  void* args[] = {&q, &limit};
+  return cudaLaunchKernel(f, dim3(count), dim3(kThreads), args, kSmemBytes, s);
 }
 
 }  // namespace tba

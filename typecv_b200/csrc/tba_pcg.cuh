@@ -48,4 +48,12 @@ uint32_t pcg_launch_plan(const PcgSystem& a, uint32_t grid, cudaStream_t s);
 // Up to `limit` PCG steps from the vectors and state as k_pcg_init (or a restart) left them.
 cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaStream_t s);
 
+// The systems of a batch, one block each (list: problem of each block).
+struct PcgMany {
+  const PcgSystem* systems;
+  const uint2* work;
+};
+uint32_t pcg_launch_many_plan(const PcgMany& b, uint32_t count, uint32_t max_cameras, cudaStream_t s);
+cudaError_t launch_many_pcg(const PcgMany& b, uint32_t count, bool shared, uint32_t limit, cudaStream_t s);
+
 }  // namespace tba

@@ -19,6 +19,28 @@ namespace {
 
 constexpr int kPairThreads = 256;
 
+// A block's problem and its place in that problem's grid: the kernel's argument, or a batch's list.
+template <class W>
+struct SchurSlot {};
+template <>
+struct SchurSlot<SchurMany> {
+  SchurParams p;
+};
+__device__ inline const SchurParams& block_problem(const SchurParams& Q, SchurSlot<SchurParams>&, uint32_t& bid) {
+  bid = blockIdx.x;
+  return Q;
+}
+__device__ inline const SchurParams& block_problem(const SchurMany& W, SchurSlot<SchurMany>& slot, uint32_t& bid) {
+  const uint2 w = W.work[blockIdx.x];
+  static_assert(sizeof(SchurParams) % 8 == 0, "copied as 8-byte words");
+  const uint64_t* from = reinterpret_cast<const uint64_t*>(W.params + w.x);
+  uint64_t* to = reinterpret_cast<uint64_t*>(&slot.p);
+  for (uint32_t k = threadIdx.x; k < sizeof(SchurParams) / 8; k += blockDim.x) to[k] = from[k];
+  __syncthreads();
+  bid = w.y;
+  return slot.p;
+}
+
 // Calls f(camera of j, j) for every pair (i, j) that the observation at position k of the
 // camera-major list contributes to its camera's row: later variable cameras of the same point, and a
 // later observation of the same camera (a point seen twice by one camera).
@@ -32,9 +54,13 @@ __device__ inline void row_pairs(const SchurParams& Q, uint32_t k, uint32_t c, F
   }
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pairs_count(SchurParams Q) {
+template <class W>
+__global__ void __launch_bounds__(kPairThreads) k_pairs_count(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
   extern __shared__ uint32_t hist[];
-  const uint32_t ch = blockIdx.x, c = Q.chunk_cam[ch];
+  const uint32_t ch = bid, c = Q.chunk_cam[ch];
   if (Q.active[c] == 0) return;
   for (uint32_t d = c + threadIdx.x; d < Q.C; d += blockDim.x) hist[d] = 0;
   __syncthreads();
@@ -52,9 +78,13 @@ __device__ inline uint32_t row_count(const SchurParams& Q, uint32_t c, uint32_t 
   return n;
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pairs_rows(SchurParams Q) {
+template <class W>
+__global__ void __launch_bounds__(kPairThreads) k_pairs_rows(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
   __shared__ uint32_t sum[2];
-  const uint32_t c = blockIdx.x;
+  const uint32_t c = bid;
   if (threadIdx.x < 2) sum[threadIdx.x] = 0;
   if (threadIdx.x == 0) atomicOr(Q.bits + size_t(c) * Q.bwords + c / 32, 1u << (c % 32));
   __syncthreads();
@@ -112,7 +142,11 @@ __device__ inline void block_scan(uint32_t (&v)[N], uint32_t (&total)[N], uint32
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(1024) k_pairs_scan(SchurParams Q) {
+template <class W>
+__global__ void __launch_bounds__(1024) k_pairs_scan(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
   __shared__ uint32_t warp_sum[32][3];
   uint32_t base[3] = {0, 0, 0};
   for (uint32_t c0 = 0; c0 < Q.C; c0 += blockDim.x) {
@@ -139,9 +173,13 @@ __global__ void __launch_bounds__(1024) k_pairs_scan(SchurParams Q) {
   }
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pairs_place(SchurParams Q) {
+template <class W>
+__global__ void __launch_bounds__(kPairThreads) k_pairs_place(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
   __shared__ uint32_t warp_sum[kPairThreads / 32][2];
-  const uint32_t c = blockIdx.x;
+  const uint32_t c = bid;
   // The cameras of the row's blocks, in order.
   uint32_t at = Q.row_ptr[c];
   for (uint32_t w0 = 0; w0 < Q.bwords; w0 += blockDim.x) {
@@ -184,8 +222,12 @@ __device__ inline uint32_t block_of(const SchurParams& Q, uint32_t c, uint32_t d
   return n + __popc(row[d / 32] & ((1u << (d % 32)) - 1u));
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pairs_blocks(SchurParams Q) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+template <class W>
+__global__ void __launch_bounds__(kPairThreads) k_pairs_blocks(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
+  const uint32_t b = bid * blockDim.x + threadIdx.x;
   if (b >= Q.totals[0]) return;
   const uint2 rc = Q.blk_rc[b];
   Q.blk_dst[b] = make_uint2(block_of(Q, rc.x, rc.y), block_of(Q, rc.y, rc.x));
@@ -193,9 +235,13 @@ __global__ void __launch_bounds__(kPairThreads) k_pairs_blocks(SchurParams Q) {
   for (uint32_t s = (begin + Q.seg - 1) / Q.seg; s * Q.seg < end; s++) Q.seg_block[s] = b;
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pairs_fill(SchurParams Q) {
+template <class W>
+__global__ void __launch_bounds__(kPairThreads) k_pairs_fill(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
   extern __shared__ uint32_t cursor[];
-  const uint32_t ch = blockIdx.x, c = Q.chunk_cam[ch];
+  const uint32_t ch = bid, c = Q.chunk_cam[ch];
   if (Q.active[c] == 0) return;
   for (uint32_t d = c + threadIdx.x; d < Q.C; d += blockDim.x) cursor[d] = Q.counts[size_t(ch) * Q.C + d];
   __syncthreads();
@@ -231,8 +277,12 @@ __device__ inline void store_entry(const SchurParams& Q, uint32_t b, uint32_t r,
 // matrix instruction's inner dimension (four pairs are three instructions); a lane loads its own
 // element of each record from global memory, so a record is read as whole 48-byte columns.  The
 // segment's pairs come 32 at a time, one a lane, so that a record's loads wait for one load only.
-__global__ void __launch_bounds__(256) k_block_sums(SchurParams Q) {
-  const uint32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+template <class W>
+__global__ void __launch_bounds__(256) k_block_sums(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
+  const uint32_t s = bid * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t npairs = Q.totals[1];
   const uint32_t lo = s * Q.seg;
   if (lo >= npairs) return;
@@ -289,8 +339,12 @@ __global__ void __launch_bounds__(256) k_block_sums(SchurParams Q) {
   }
 }
 
-__global__ void __launch_bounds__(256) k_block_ends(SchurParams Q) {
-  const uint32_t b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+template <class W>
+__global__ void __launch_bounds__(256) k_block_ends(W w) {
+  __shared__ SchurSlot<W> slot;
+  uint32_t bid;
+  const SchurParams& Q = block_problem(w, slot, bid);
+  const uint32_t b = bid * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= Q.totals[0]) return;
   const uint32_t begin = Q.blk_begin[b], end = Q.blk_begin[b + 1], s0 = begin / Q.seg, s1 = (end - 1) / Q.seg;
   if (s0 == s1) return;
@@ -321,6 +375,23 @@ uint32_t schur_launch_values(const SchurParams& q, cudaStream_t s) {
   const uint32_t segs = (q.max_pairs + q.seg - 1) / q.seg;
   k_block_sums<<<(segs + 7) / 8, 256, 0, s>>>(q);
   k_block_ends<<<(q.max_blocks + 7) / 8, 256, 0, s>>>(q);
+  return 2;
+}
+
+uint32_t schur_launch_many_structure(const SchurLists& b, cudaStream_t s) {
+  const size_t smem = size_t(b.max_cameras) * sizeof(uint32_t);
+  k_pairs_count<SchurMany><<<b.chunk.blocks, kPairThreads, smem, s>>>(b.chunk.of(b));
+  k_pairs_rows<SchurMany><<<b.camera.blocks, kPairThreads, 0, s>>>(b.camera.of(b));
+  k_pairs_scan<SchurMany><<<b.one.blocks, 1024, 0, s>>>(b.one.of(b));
+  k_pairs_place<SchurMany><<<b.camera.blocks, kPairThreads, 0, s>>>(b.camera.of(b));
+  k_pairs_blocks<SchurMany><<<b.pairs.blocks, kPairThreads, 0, s>>>(b.pairs.of(b));
+  k_pairs_fill<SchurMany><<<b.chunk.blocks, kPairThreads, smem, s>>>(b.chunk.of(b));
+  return 6;
+}
+
+uint32_t schur_launch_many_values(const SchurLists& b, cudaStream_t s) {
+  k_block_sums<SchurMany><<<b.sums.blocks, 256, 0, s>>>(b.sums.of(b));
+  k_block_ends<SchurMany><<<b.ends.blocks, 256, 0, s>>>(b.ends.of(b));
   return 2;
 }
 

@@ -56,6 +56,25 @@ struct SchurParams {
   double* S;     // 36 per block, by columns (entry (row a, column b) at 6 b + a)
 };
 
+// The same over a batch: every problem's parameters in device memory, and lists of (problem, block).
+struct SchurMany {
+  const SchurParams* params;
+  const uint2* work;
+};
+struct SchurLists {
+  const SchurParams* params;
+  uint32_t max_cameras;
+  struct List {
+    const uint2* work;
+    uint32_t blocks;
+    SchurMany of(const SchurLists& b) const { return SchurMany{b.params, work}; }
+  };
+  // A block per: problem; camera chunk; camera; 256 camera pairs; eight camera pairs; eight segments.
+  List one, chunk, camera, pairs, ends, sums;
+};
+uint32_t schur_launch_many_structure(const SchurLists& b, cudaStream_t s);  // (bits zeroed by the caller)
+uint32_t schur_launch_many_values(const SchurLists& b, cudaStream_t s);
+
 // Structure of S (indices already checked), on stream s; returns the kernels launched.
 uint32_t schur_launch_structure(const SchurParams& q, cudaStream_t s);
 // The off-diagonal blocks of S from the records; returns the kernels launched.
