@@ -426,7 +426,7 @@ struct SchurLayout {
     uni = L.take<uint32_t>(size_t(grid) * C);
     uni_n = L.take<uint32_t>(grid);
     local = L.take<uint32_t>(blocks);
-    pbuf = L.take<double>(size_t(grid) * 6 * C);
+    pbuf = L.take<double>(size_t(grid) * 12 * C);
     zx = L.take<tba::Flagged>(6 * size_t(C));
     slots = L.take<tba::Flagged>(4 * size_t(grid));
     part = L.take<double>(72 * segs);

@@ -40,14 +40,23 @@ __device__ __forceinline__ Flagged peek(const Flagged* p) {
   return Flagged{__longlong_as_double(v), s};
 }
 
-// The value of `step`; false when it did not come within the poll limit.
-__device__ __forceinline__ bool await(const Flagged* p, uint64_t step, double& v) {
+// The values of `step` at N places, looked for together (a place beyond `n` is left out); false when
+// they did not come within the poll limit.
+template <int N>
+__device__ __forceinline__ bool await(const Flagged* const (&p)[N], int n, uint64_t step, double (&v)[N]) {
   for (uint32_t k = 0; k < kPcgWaitPolls; k++) {
-    const Flagged f = peek(p);
-    if (f.step == step) {
-      v = f.value;
-      return true;
-    }
+    Flagged f[N];
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j < n) f[j] = peek(p[j]);
+    bool all = true;
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      if (j < n) {
+        all = all && f[j].step == step;
+        v[j] = f[j].value;
+      }
+    if (all) return true;
   }
   return false;
 }
@@ -83,46 +92,64 @@ struct Shared {
   int gave_up;
 };
 
-// Adds v over the grid; every thread returns with the sums (false: a wait gave up).  `which` is the
-// step's first or second reduction.
-__device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], uint64_t step, int which, uint32_t bid,
-                                uint32_t grid) {
-  warp_allsum(v);
+constexpr int kSlotsEach = 5;  // partial sums of 32 x 5 blocks in one round of a warp (148 SMs)
+
+// Adds v, which only the first `warps` warps have, over the grid; every thread returns with the sums
+// (false: a wait gave up).  `which` is the step's first or second reduction.  While the first warp
+// waits for the other blocks' sums, the others run `meanwhile`.
+template <class F>
+__device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], uint64_t step, int which, int warps,
+                                uint32_t bid, uint32_t grid, F meanwhile) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-    sh.red[which][warp][0] = v[0];
-    sh.red[which][warp][1] = v[1];
+  if (warp < warps) {
+    warp_allsum(v);
+    if (lane == 0) {
+      sh.red[which][warp][0] = v[0];
+      sh.red[which][warp][1] = v[1];
+    }
   }
   __syncthreads();
   if (grid == 1) {
     v[0] = v[1] = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++) {
+    for (int w = 0; w < warps; w++) {
       v[0] += sh.red[which][w][0];
       v[1] += sh.red[which][w][1];
     }
     return true;
   }
   if (warp == 0) {
-    double t[2] = {lane < kWarps ? sh.red[which][lane][0] : 0.0, lane < kWarps ? sh.red[which][lane][1] : 0.0};
-    warp_allsum(t);
+    double t[2] = {lane < warps ? sh.red[which][lane][0] : 0.0, lane < warps ? sh.red[which][lane][1] : 0.0};
+    if (warps > 1) warp_allsum(t);
     Flagged* slots = A.slots + 2 * size_t(which);
+    t[1] = __shfl_sync(kFull, t[1], 0);  // lane 1 publishes the second sum
     if (lane < 2) publish(slots + 4 * size_t(bid) + lane, lane == 0 ? t[0] : t[1], step);
-    bool ok = sh.gave_up == 0;
-    t[0] = t[1] = 0;
-    for (uint32_t b = lane; b < grid && ok; b += 32) {
-      double s0 = 0, s1 = 0;
-      ok = await(slots + 4 * size_t(b), step, s0) && await(slots + 4 * size_t(b) + 1, step, s1);
-      t[0] += s0;
-      t[1] += s1;
+    bool ok = *(volatile int*)&sh.gave_up == 0;
+    double s[2] = {0, 0};
+    for (uint32_t base = 0; base < grid && ok; base += 32 * kSlotsEach) {
+      const Flagged* at[2 * kSlotsEach];
+      double got[2 * kSlotsEach];
+      int n = 0;
+#pragma unroll
+      for (int j = 0; j < kSlotsEach; j++) {
+        const uint32_t b = base + 32 * j + lane;
+        at[2 * j] = slots + 4 * size_t(b);
+        at[2 * j + 1] = slots + 4 * size_t(b) + 1;
+        if (b < grid) n = 2 * j + 2;
+      }
+      ok = await(at, n, step, got);
+#pragma unroll
+      for (int j = 0; j < 2 * kSlotsEach; j++)
+        if (j < n) s[j & 1] += got[j];
     }
-    warp_allsum(t);
+    warp_allsum(s);
     ok = __all_sync(kFull, ok);
     if (lane == 0) {
-      sh.sum[0] = t[0];
-      sh.sum[1] = t[1];
+      sh.sum[0] = s[0];
+      sh.sum[1] = s[1];
       if (!ok) sh.gave_up = 1;
     }
+  } else {
+    meanwhile();
   }
   __syncthreads();
   v[0] = sh.sum[0];
@@ -189,13 +216,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   if (st[A.active] == 0 || limit == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool alone = grid == 1;
-  const uint32_t c0 = A.share[bid], c1 = A.share[bid + 1], nr = c1 - c0, rows = 6 * nr, first = 6 * c0,
-                 n = 6 * A.C;
+  const uint32_t c0 = A.share[bid], c1 = A.share[bid + 1], nr = c1 - c0, rows = 6 * nr, first = 6 * c0, n = 6 * A.C;
   const uint32_t* uni = A.uni + size_t(bid) * A.C;
   const uint32_t cols = 6 * A.uni_n[bid];
   const uint32_t k0 = A.row_ptr[c0], blocks = A.row_ptr[c1] - k0;
-  // Shared memory, as far as it goes: the direction, the own vectors, the own rows of S, their columns'
-  // places and the own preconditioner blocks.
+  // Shared memory, as far as it goes: the direction and the columns' z, the own vectors, the rows' first
+  // blocks, the own rows of S, their columns' places and the own preconditioner blocks.
   uint32_t used = 0;
   auto take = [&](size_t words, double* global) {
     if ((used + words) * sizeof(double) > kSmemBytes) return global;
@@ -203,13 +229,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
     used += uint32_t((words + 1) & ~size_t(1));
     return p;
   };
-  double* pl = take(cols, A.pbuf + size_t(bid) * n);
+  double* pl = take(cols, A.pbuf + 2 * size_t(bid) * n);
+  double* zl = alone ? nullptr : take(cols, A.pbuf + (2 * size_t(bid) + 1) * n);  // the columns' z of the next step
   double* own = take(4 * size_t(rows), nullptr);  // x, r, S p, z
   const bool keep = own != nullptr;
   double* xs = keep ? own : A.x + first;
   double* rs = keep ? own + rows : A.r + first;
-  double* ss = keep ? own + 2 * size_t(rows) : A.p + first;  // p's place is free once it is loaded
+  double* ss = keep ? own + 2 * size_t(rows) : A.p + first;  // p's place: the first direction is z
   double* zs = keep ? own + 3 * size_t(rows) : A.z + first;
+  const uint32_t* row_ptr = A.row_ptr + c0;
+  if (double* to = take((size_t(nr) + 2) / 2, nullptr)) {
+    uint32_t* words = reinterpret_cast<uint32_t*>(to);
+    for (uint32_t k = threadIdx.x; k <= nr; k += kThreads) words[k] = row_ptr[k];
+    row_ptr = words;
+  }
   const double* S = A.S + 36 * size_t(k0);
   if (double* to = take(36 * size_t(blocks), nullptr)) {
     const double2* from = reinterpret_cast<const double2*>(S);
@@ -227,8 +260,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
     for (uint32_t k = threadIdx.x; k < 36 * nr; k += kThreads) to[k] = Minv[k];
     Minv = to;
   }
-  // The first step's direction is z + 0 p.
-  for (uint32_t j = threadIdx.x; j < cols; j += kThreads) pl[j] = 0;
+  for (uint32_t j = threadIdx.x; j < cols; j += kThreads) {
+    const uint32_t b = j / 6;
+    pl[j] = 0;  // (beta is zero in the first step)
+    if (!alone) zl[j] = A.z[6 * uni[b] + (j - 6 * b)];
+  }
   if (keep)
     for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
       xs[i] = A.x[first + i];
@@ -245,10 +281,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   }
   double rho = st[A.rho], beta = 0, r2 = st[A.r2];
   const double bound = fmax(A.tol * A.tol * st[A.r0], A.inner_r0 >= 0 ? A.tol_inner * A.tol_inner * st[A.inner_r0] : 0.0);
-  // A warp per camera row, or several warps on a row's columns; a lane sums one of the six rows over
-  // every fifth column.
+  // A warp per camera row, or several warps on a row's blocks; a lane sums one of the six rows over every
+  // fifth block.  The first `owners` warps hold the own rows' scalars.
   const uint32_t splits = nr == 0 || nr >= uint32_t(kWarps) ? 1 : kWarps / nr;
-  const uint32_t lane_row = lane % 6, lane_col = lane / 6;
+  const int owners = int(min(uint32_t(kWarps), (rows + 31) / 32));
+  const uint32_t lane_row = lane % 6, lane_block = lane / 6;
   bool active = true, failed = false, converged = false, ok = true;
   uint32_t it = 0;
   if (threadIdx.x == 0) sh.gave_up = 0;
@@ -265,36 +302,32 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
     return 6 * lo + i % 6;
   };
   const uint32_t my_place = threadIdx.x < rows ? place_of(threadIdx.x) : 0;
+  const uint32_t my_part = threadIdx.x / 6 * splits, my_row = threadIdx.x % 6;
+  const double* const znext = alone ? zs : zl;
   while (active && it < limit) {
     const uint64_t step = it + 1;
-    for (uint32_t j = threadIdx.x; j < cols; j += kThreads) {
-      const uint32_t b = j / 6, g = 6 * uni[b] + (j - 6 * b);
-      double zv = 0;
-      if (alone) zv = zs[g];
-      else if (it == 0) zv = A.z[g];
-      else if (*(volatile int*)&sh.gave_up != 0 || !await(A.zx + g, it, zv)) *(volatile int*)&sh.gave_up = 1;
-      pl[j] = zv + beta * pl[j];
-    }
+    for (uint32_t j = threadIdx.x; j < cols; j += kThreads) pl[j] = znext[j] + beta * pl[j];
     __syncthreads();
     for (uint32_t item = warp; item < nr * splits; item += kWarps) {
-      const uint32_t row = item / splits, part = item - row * splits;
-      const uint32_t b0 = A.row_ptr[c0 + row] - k0, w = 6 * (A.row_ptr[c0 + row + 1] - k0 - b0);
-      const uint32_t lo = w * part / splits, hi = w * (part + 1) / splits;
-      const double* Sr = S + 36 * size_t(b0);
-      double acc = 0;
+      const uint32_t row = splits == 1 ? item : item / splits, part = item - row * splits;
+      const uint32_t b0 = row_ptr[row] - k0, nb = row_ptr[row + 1] - k0 - b0;
+      const uint32_t lo = b0 + nb * part / splits, hi = b0 + nb * (part + 1) / splits;
+      double acc[3] = {0, 0, 0};  // independent sums: one chain of dependent FMAs a lane was half of a step
       if (lane < 30) {
-#pragma unroll 4
-        for (uint32_t j = lo + lane_col; j < hi; j += 5) {
-          const uint32_t b = j / 6;
-          acc += Sr[6 * size_t(j) + lane_row] * pl[6 * local[b0 + b] + (j - 6 * b)];
+#pragma unroll 2
+        for (uint32_t b = lo + lane_block; b < hi; b += 5) {
+          const double* Sb = S + 36 * size_t(b) + lane_row;
+          const double* pb = pl + 6 * local[b];
+#pragma unroll
+          for (int k = 0; k < 6; k++) acc[k % 3] += Sb[6 * k] * pb[k];
         }
       }
-      const double far = __shfl_down_sync(kFull, acc, 24);
-      acc += __shfl_down_sync(kFull, acc, 12);
-      acc += __shfl_down_sync(kFull, acc, 6);
+      acc[0] += acc[1] + acc[2];
+      const double far = __shfl_down_sync(kFull, acc[0], 24), near = __shfl_down_sync(kFull, acc[0], 6),
+                   mid = __shfl_down_sync(kFull, acc[0], 12), mid2 = __shfl_down_sync(kFull, acc[0], 18);
       if (lane < 6) {
         double* out = splits == 1 ? ss + 6 * row : sh.part[item];
-        out[lane] = acc + far;
+        out[lane] = (acc[0] + near) + (mid + mid2) + far;
       }
     }
     __syncthreads();
@@ -304,8 +337,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
       double sp = 0;
       if (splits == 1) {
         sp = ss[i];
-      } else {
-        for (uint32_t k = 0; k < splits; k++) sp += sh.part[i / 6 * splits + k][i % 6];
+      } else {  // (several warps a row: at most 15 rows of cameras, one scalar row a thread)
+        for (uint32_t k = 0; k < splits; k++) sp += sh.part[my_part + k][my_row];
       }
       const double pv = pl[i == threadIdx.x ? my_place : place_of(i)];
       if (SHARED) {
@@ -316,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
       ss[i] = sp;
       v[0] += pv * sp;
     }
-    if (!(ok = grid_sum(A, sh, v, step, 0, bid, grid))) break;
+    if (!(ok = grid_sum(A, sh, v, step, 0, owners, bid, grid, [] {}))) break;
     const double spf = SHARED ? sff * pf + v[1] : 0.0, den = SHARED ? v[0] + pf * spf : v[0], alpha = rho / den;
     if (!(den > 0) || !(fabs(alpha) < A.alpha_limit)) {
       active = false;
@@ -333,13 +366,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
       const double* Mi = Minv + 6 * size_t(i);
       const double* rc = rs + i - i % 6;
       const double rr = rs[i];
-      const double zz = Mi[0] * rc[0] + Mi[1] * rc[1] + Mi[2] * rc[2] + Mi[3] * rc[3] + Mi[4] * rc[4] + Mi[5] * rc[5];
+      const double zz = (Mi[0] * rc[0] + Mi[1] * rc[1]) + (Mi[2] * rc[2] + Mi[3] * rc[3]) + (Mi[4] * rc[4] + Mi[5] * rc[5]);
       if (alone) zs[i] = zz;
       else publish(A.zx + first + i, zz, step);
       v[0] += rr * rr;
       v[1] += zz * rr;
     }
-    if (!(ok = grid_sum(A, sh, v, step, 1, bid, grid))) break;
+    // The columns' new z, while the first warp waits for the sums.
+    auto fetch = [&] {
+      for (uint32_t j = threadIdx.x - 32; j < cols; j += 2 * (kThreads - 32)) {
+        const uint32_t j1 = j + (kThreads - 32), b = j / 6, b1 = j1 / 6;
+        const Flagged* at[2] = {A.zx + 6 * uni[b] + (j - 6 * b), nullptr};
+        if (j1 < cols) at[1] = A.zx + 6 * uni[b1] + (j1 - 6 * b1);
+        double got[2];
+        if (*(volatile int*)&sh.gave_up != 0 || !await(at, j1 < cols ? 2 : 1, step, got)) {
+          *(volatile int*)&sh.gave_up = 1;
+          break;
+        }
+        zl[j] = got[0];
+        if (j1 < cols) zl[j1] = got[1];
+      }
+    };
+    if (!(ok = grid_sum(A, sh, v, step, 1, owners, bid, grid, fetch))) break;
     it++;
     r2 = v[0];
     double next = v[1];

@@ -31,7 +31,7 @@ struct PcgSystem {
   const double* Minv;  // 36C block-Jacobi preconditioner
   const double* scf;   // 6C focal column (with the focal unknown)
   double *x, *r, *z, *p;  // 6C (+ 1); x and r are updated, z and p hold the start (p = z or a restart's)
-  double* pbuf;           // grid x 6C: a block's direction when it does not fit shared memory
+  double* pbuf;           // grid x 2 x 6C: a block's direction and its columns' z when they do not fit shared memory
   double* state;
   int active, failed, converged, rho, r0, r2, inner_r0, steps, all_steps, wait;  // words; -1: not kept
   int focal_diag, focal_inv;
