@@ -1211,8 +1211,7 @@ struct BatchReport {
 
 // The batch on the grid kernels: every kernel of an LM iteration runs over all problems at once (its
 // blocks a list of (problem, block)), with each problem's reduced system explicit and its PCG in one
-// block; the iteration is a CUDA graph, replayed while the batch's lists keep their places.  The scene's
-// poses and points are updated in place.  False (nothing launched) when the workspace does not fit.
+// block; the iteration is a CUDA graph, replayed while the batch's lists keep their places.  False (nothing launched) when the workspace does not fit.
 bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_problem* probs, uint32_t count,
                    const std::vector<WindowPlan>& plans, const std::vector<uint32_t>& order, const double* scene,
                    size_t scene_len, const uint32_t* index, size_t index_len, size_t output_len, cudaEvent_t uploaded,
@@ -1283,12 +1282,16 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   for (uint32_t k = 0; k < count; k++) bit_words += size_t(probs[k].cameras) * ((probs[k].cameras + 31) / 32);
   const size_t o_bits = L.take<uint32_t>(bit_words);
   struct Work {
-    size_t tposes, tpoints, rlim, cmp, cmx, pblk, A, pw, xw, U, Minv, rhs, hcf, scf, chunk, vec, scal, cost, ticket, state, system;
+    size_t poses, points, cams, pixels, tposes, tpoints, rlim, cmp, cmx, pblk, A, pw, xw, U, Minv, rhs, hcf, scf, chunk, vec, scal, cost, ticket, state, system;
   };
   std::vector<Work> works(count);
   for (uint32_t k = 0; k < count; k++) {
     const size_t C = probs[k].cameras, P = probs[k].points, M = probs[k].observations, m = 6 * C + (shared ? 1 : 0);
     Work& w = works[k];
+    w.poses = L.take<double>(12 * C);
+    w.points = L.take<double>(3 * P);
+    w.cams = L.take<double>(6 * C);
+    w.pixels = L.take<double>(2 * M);
     w.tposes = L.take<double>(12 * C);
     w.tpoints = L.take<double>(3 * P);
     w.rlim = L.take<double>(C);
@@ -1350,10 +1353,11 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
     uint32_t fixed = 0;
     for (size_t j = 0; j < C; j++) fixed += act[j] == 0;
     p.normalize_scale = fixed == 1;
-    p.poses = f64(o_scene) + q.scene_offset;
-    p.points = p.poses + 12 * C;
-    p.cams = p.points + 3 * P;
-    p.pixels = p.cams + 6 * C;
+    p.packed = f64(o_scene) + q.scene_offset;
+    p.poses = f64(w.poses);
+    p.points = f64(w.points);
+    p.cams = f64(w.cams);
+    p.pixels = f64(w.pixels);
     p.tposes = f64(w.tposes);
     p.tpoints = f64(w.tpoints);
     const uint32_t* x = u32(o_index) + q.index_offset;

@@ -89,6 +89,7 @@ struct Params {
   const double* pixels;  // 2M
   double* tposes;   // 12C
   double* tpoints;  // 3P
+  const double* packed;  // a batch's problem as the caller packed it (any 8-byte place), or null
   // index sections
   const uint32_t* obs_camera;
   const uint32_t* obs_point;

@@ -113,6 +113,23 @@ __device__ inline bool last_block(uint32_t* ticket) {
   return last;
 }
 
+// A batch's problems lie one after another in the caller's arrays, at places that 16-byte loads cannot
+// take; their scene sections are copied to places of their own (which the solve then updates).
+__global__ void __launch_bounds__(256) k_unpack(Many w) {
+  __shared__ Slot<Many> slot;
+  uint32_t bid;
+  const Params& P = block_problem(w, slot, bid);
+  const uint32_t blocks = ((P.M > P.C ? P.M : P.C) + 255) / 256;
+  const uint32_t np = 12 * P.C, nx = np + 3 * P.P, nk = nx + 6 * P.C, n = nk + 2 * P.M;
+  for (uint32_t i = bid * blockDim.x + threadIdx.x; i < n; i += blocks * blockDim.x) {
+    const double v = P.packed[i];
+    if (i < np) P.poses[i] = v;
+    else if (i < nx) P.points[i - np] = v;
+    else if (i < nk) const_cast<double*>(P.cams)[i - nx] = v;
+    else const_cast<double*>(P.pixels)[i - nk] = v;
+  }
+}
+
 // ---- K1: initializeBundle, and the per-solve set-up -----------------------------------------------
 
 template <class W>
@@ -2088,11 +2105,12 @@ void launch_update_points(const Params& p, cudaStream_t s) {
 void launch_accept(const Params& p, cudaStream_t s) { k_accept<<<1, 256, 0, s>>>(p); }
 // The kernels of one LM iteration up to the PCG, and after it, over a batch's lists of blocks.
 uint32_t launch_many_begin(const ManyLists& b, cudaStream_t s) {
+  k_unpack<<<b.setup.blocks, 256, 0, s>>>(b.setup.of(b));
   k_initialize<Many><<<b.one.blocks, 32, 0, s>>>(b.one.of(b));
   k_setup<Many><<<b.setup.blocks, 256, 0, s>>>(b.setup.of(b));
   k_cost<Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
   k_finish_metrics<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
-  return 4;
+  return 5;
 }
 uint32_t launch_many_linearize(const ManyLists& b, cudaStream_t s) {
   if (b.shared) k_point_pass<true, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
