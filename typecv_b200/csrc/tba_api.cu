@@ -357,11 +357,15 @@ Chunks build_chunks(const uint32_t* cs, uint32_t C, uint32_t size) {
   return ch;
 }
 
+void check_waits(const double* words) {
+  if (words[tba::S_WAIT] != 0) throw Fail{TBA_ERROR_CUDA, "GPU BA: a wait between the PCG's blocks ran out"};
+}
+
 // Reads the state words into the pinned buffer; returns word `word`.
 double read_word(tba_device* d, const double* state, int word) {
   CUDA_TRY(cudaMemcpyAsync(d->pinned, state, tba::S_READ * sizeof(double), cudaMemcpyDeviceToHost, d->stream));
   CUDA_TRY(cudaStreamSynchronize(d->stream));
-  if (d->pinned[tba::S_WAIT] != 0) throw Fail{TBA_ERROR_CUDA, "GPU BA: a wait between the PCG's blocks ran out"};
+  check_waits(d->pinned);
   return d->pinned[word];
 }
 
@@ -643,6 +647,12 @@ HostPlan make_plan(const tba_control* ctl, const uint32_t* index, int sms) {
   return plan;
 }
 
+// Blocks of the acceptance: each adds the task blocks' costs again, so there are few of them, each with
+// a few thousand values of the candidate to copy.
+uint32_t commit_grid(uint32_t C, uint32_t P) {
+  return uint32_t(std::min<uint64_t>(592, std::max<uint64_t>(1, (std::max<uint64_t>(12ull * C, 3ull * P) + 2047) / 2048)));
+}
+
 // The explicit system's structure, values and PCG of one problem, from the problem's parameters; the
 // problem takes the system's blocks.
 void bind_problem(tba::Params& p, tba::SchurParams& q, tba::PcgSystem& a) {
@@ -656,6 +666,7 @@ void bind_problem(tba::Params& p, tba::SchurParams& q, tba::PcgSystem& a) {
   q.chunk_beg = p.chunk_beg;
   q.cam_chunk = p.cam_chunk;
   q.A = p.A;
+  q.go = p.state + tba::S_ACTIVE;
   p.S = q.S;
   p.row_ptr = q.row_ptr;
   p.col = q.col;
@@ -682,6 +693,16 @@ void bind_problem(tba::Params& p, tba::SchurParams& q, tba::PcgSystem& a) {
   a.tol = p.tol;
   a.tol_inner = p.tol_inner;
   a.alpha_limit = 1e20;
+  a.rhs = p.camRhs;
+  a.scal_part = p.scal_part;
+  a.scal_blocks = p.task_blocks;
+  a.solving = tba::S_ACTIVE;
+  a.block_failed = tba::S_POINT_FAILED;
+  a.lambda = tba::S_LAMBDA;
+  a.focal_full = tba::S_FOCAL_DIAG;
+  a.focal_rhs = tba::S_FOCAL_RHS;
+  a.clear_from = tba::S_RHO;
+  a.clear_to = 25;
 }
 
 // Where a solve reads its problem and where it leaves the solution.  With `device_source` the
@@ -909,6 +930,7 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   p.ntasks = ntasks;
   p.nchunks = nchunks;
   p.task_blocks = std::max<uint32_t>(1, std::min<uint32_t>(max_task_blocks, (ntasks + 7) / 8));
+  p.commit_blocks = commit_grid(C, P);
   p.prod_blocks = std::max<uint32_t>(1, std::min<uint32_t>(max_prod_blocks, (ntasks + 15) / 16));
   CUDA_TRY(cudaEventRecord(e_up, s));
   if (io.checks) {
@@ -967,7 +989,13 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   std::vector<std::pair<size_t, size_t>> product_events;
   std::vector<std::pair<size_t, uint32_t>> product_spans;  // (first event pair, real steps) per LM iteration
   const bool time_products = (ctl->flags & TBA_FLAG_TIME_PRODUCTS) != 0;
+  const bool diagnose = (ctl->flags & TBA_FLAG_PRODUCT_ERROR) != 0;
   const bool host_loop = time_products || (ctl->flags & TBA_FLAG_HOST_PCG_LOOP) != 0;
+  // With the explicit system nothing in an iteration needs the host, so iterations are issued one ahead
+  // of the last state read.
+  const bool ahead = schur && !host_loop && !diagnose;
+  cudaEvent_t read_done[2] = {event(d, ev), event(d, ev + 1)};
+  ev += 2;
   // Kernels per step of the device-side PCG loop launched last, while its step count is unread.
   uint32_t loop_kernels = 0;
   tba::launch_initialize(p, s);
@@ -987,9 +1015,12 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     tba::launch_camera_pass(p, s);
     tba::launch_camera_finish(p, s);
     if (schur) launches += tba::schur_launch_values(sq, s);
-    tba::launch_pcg_init(p, s);
-    launches += 4;
-    if (it == 0 && (ctl->flags & TBA_FLAG_PRODUCT_ERROR) && read_word(d, p.state, tba::S_CG_ACTIVE) != 0) {
+    launches += 3;
+    if (!schur || host_loop || diagnose) {  // (the persistent PCG starts itself)
+      tba::launch_pcg_init(p, s);
+      launches++;
+    }
+    if (it == 0 && diagnose && read_word(d, p.state, tba::S_CG_ACTIVE) != 0) {
       // The solve's own product and the FP64 two-pass product on the first PCG direction.
       double* own = D(o_diag);
       double* ref = own + m;
@@ -1028,7 +1059,9 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     // product of the mixed form's tail.  Only the engine's own products are timed.
     auto run_pcg = [&](uint32_t budget, const tba::Params& q, bool timed) {
       if (schur && !host_loop) {
-        CUDA_TRY(tba::launch_pcg(ps, budget, pcg_blocks, s));
+        tba::PcgSystem a = ps;
+        if (diagnose) a.rhs = nullptr;  // k_pcg_init has run
+        CUDA_TRY(tba::launch_pcg(a, budget, pcg_blocks, s));
         launches++;
         return;
       }
@@ -1107,12 +1140,29 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     tba::launch_update_cameras(p, s);
     tba::launch_update_points(p, s);
     tba::launch_accept(p, s);
-    tba::launch_commit(p, s);
-    launches += 4;
+    launches += 3;
     CUDA_TRY(cudaGetLastError());
     lm_done++;
+    if (ahead) {
+      // The state goes to the host while the next iteration, a no-op should this one have ended the solve,
+      // is issued.
+      double* words = d->pinned + tba::S_READ * (it & 1);
+      CUDA_TRY(cudaMemcpyAsync(words, p.state, tba::S_READ * sizeof(double), cudaMemcpyDeviceToHost, s));
+      CUDA_TRY(cudaEventRecord(read_done[it & 1], s));
+      if (it > 0) {
+        CUDA_TRY(cudaEventSynchronize(read_done[(it - 1) & 1]));
+        check_waits(d->pinned + tba::S_READ * ((it - 1) & 1));
+        lm_active = d->pinned[tba::S_READ * ((it - 1) & 1) + tba::S_ACTIVE] != 0;
+      }
+      continue;
+    }
     lm_active = read_word(d, p.state, tba::S_ACTIVE) != 0;
     account_loop();
+  }
+  if (ahead) {
+    // Iterations that ran: the accepted and rejected steps.
+    if (read_word(d, p.state, tba::S_ACCEPTED) >= 0)
+      lm_done = uint32_t(d->pinned[tba::S_ACCEPTED] + d->pinned[tba::S_REJECTED]);
   }
   tba::launch_pack(p, s);
   launches++;
@@ -1263,7 +1313,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
                             plans[k].chunks.cam.size(),
                             (C + 3) / 4,
                             (std::max(M, C) + 255) / 256,
-                            (std::max(12 * C, 3 * P) + 255) / 256,
+                            commit_grid(C, P),
                             (12 * uint64_t(C) + 3 * uint64_t(P) + 27 + 255) / 256,
                             C,
                             (y.camera_pairs + 255) / 256,
@@ -1375,6 +1425,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
     p.cam_chunk = u32(o_flat) + at.first;
     p.nchunks = uint32_t(plans[k].chunks.cam.size());
     p.task_blocks = task_blocks(k);
+    p.commit_blocks = commit_grid(q.cameras, q.points);
     p.rlim = f64(w.rlim);
     p.cm_point = u32(w.cmp);
     p.cm_pixel = f64(w.cmx);
@@ -1465,7 +1516,6 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   auto iteration = [&]() {
     per_iteration = tba::launch_many_linearize(key.many, s);
     per_iteration += tba::schur_launch_many_values(key.schur, s);
-    per_iteration += tba::launch_many_pcg_init(key.many, s);
     const cudaError_t e = tba::launch_many_pcg(key.pcg, count, shared, bc->max_cg, s);
     per_iteration += 1 + tba::launch_many_update(key.many, s);
     return e;
@@ -1490,7 +1540,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
     CUDA_TRY(e4);
     d->window_key.assign(bytes, bytes + sizeof key);
   } else {
-    per_iteration = 3 + 2 + 1 + 1 + 5;
+    per_iteration = 3 + 2 + 1 + 4;
   }
   // Iterations are issued one ahead of the last one known to have left active problems.
   uint32_t* active = reinterpret_cast<uint32_t*>(d->pinned);
@@ -2341,7 +2391,7 @@ tba_status tba_device_open(int ordinal, tba_device** out) {
     d->sms = prop.multiProcessorCount;
     CUDA_TRY(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking));
     CUDA_TRY(cudaStreamCreateWithFlags(&d->down, cudaStreamNonBlocking));
-    CUDA_TRY(cudaMallocHost(&d->pinned, 64 * sizeof(double)));
+    CUDA_TRY(cudaMallocHost(&d->pinned, 128 * sizeof(double)));
     CUDA_TRY(tba::configure_kernels());
     CUDA_TRY(tba::pcg_configure());
     CUDA_TRY(tba::adj_configure());

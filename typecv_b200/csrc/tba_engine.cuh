@@ -46,7 +46,7 @@ enum StateWord : int {
   S_FOCAL_DIAG = 28,       // damped H_ff
   S_FOCAL_INV = 29,        // 1 / S_ff (preconditioner), -1 when not positive
   S_FOCAL_RHS = 30,        // reduced focal right-hand side
-  S_POINT_FAILED = 31,     // a point block failed this LM iteration
+  S_POINT_FAILED = 31,     // a point block (or a preconditioner block) failed this LM iteration
   S_ALPHA = 32,            // step length of the current PCG iteration
   S_BETA = 33,             // direction update of the current PCG iteration
   S_REFINE = 34,           // an FP64 refinement of the PCG solution is under way
@@ -106,6 +106,7 @@ struct Params {
   const uint32_t* cam_chunk;    // C + 1 first chunk of each camera
   uint32_t nchunks;
   uint32_t task_blocks;  // grid of the task kernels (point pass, Schur points, update, cost)
+  uint32_t commit_blocks;  // grid of the acceptance (which copies an accepted candidate)
   // linearisation
   double* rlim;        // C radial limits
   uint32_t* cm_point;  // M, camera-major
@@ -172,12 +173,11 @@ struct ManyLists {
     Many of(const ManyLists& b) const { return Many{b.params, work}; }
   };
   // A block per: problem; share of the tasks; camera chunk; four cameras; 256 observations or cameras;
-  // 256 candidate values; 256 result values.
+  // share of the acceptance; 256 result values.
   List one, task, chunk, finish, setup, commit, pack;
 };
 uint32_t launch_many_begin(const ManyLists& b, cudaStream_t s);
 uint32_t launch_many_linearize(const ManyLists& b, cudaStream_t s);
-uint32_t launch_many_pcg_init(const ManyLists& b, cudaStream_t s);
 uint32_t launch_many_update(const ManyLists& b, cudaStream_t s);
 uint32_t launch_many_pack(const ManyLists& b, cudaStream_t s);
 
@@ -206,7 +206,6 @@ void launch_product_rows(const Params& p, double* out, cudaStream_t s);
 void launch_update_cameras(const Params& p, cudaStream_t s);
 void launch_update_points(const Params& p, cudaStream_t s);
 void launch_accept(const Params& p, cudaStream_t s);
-void launch_commit(const Params& p, cudaStream_t s);
 void launch_pack(const Params& p, cudaStream_t s);
 // Blocks of the widest PCG-step kernel (sizes blk_part).
 uint32_t product_finish_blocks(const Params& p);

@@ -21,7 +21,7 @@
 //                         normalizeBundleCandidate (cameras) (K14/K15/K16)
 // k_update_points         updateBundleCandidate (points) + normalizeBundleCandidate (points) +
 //                         bundleCandidatePartials (K14/K16/K17)
-// k_accept/k_commit       acceptBundleCandidate + commitBundleCandidate (K18/K19)
+// k_accept                acceptBundleCandidate + commitBundleCandidate (K18/K19)
 // k_pack                  packBundleResult (K20)
 //
 // No kernel stores the Schur cross blocks W_i = w J_c^T J_p (21 words per observation).  The
@@ -649,6 +649,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_camera_finish(W w) {
   __syncwarp();
   for (int j = lane; j < 36; j += 32)
     Minv[j] = ok ? (inverse[warp][j] + inverse[warp][j % 6 * 6 + j / 6]) * 0.5 : (j == 0 ? -1.0 : 0.0);
+  if (!ok && lane == 0) P.state[S_POINT_FAILED] = 1;  // (the solve fails as with a point block)
 }
 
 // ---- K9/K21: damped focal scalars and the PCG start --------------------------------------------
@@ -661,18 +662,15 @@ __device__ inline double precondition(const Params& P, uint32_t i) {
   return Mi[0] * rc[0] + Mi[1] * rc[1] + Mi[2] * rc[2] + Mi[3] * rc[3] + Mi[4] * rc[4] + Mi[5] * rc[5];
 }
 
-template <class W>
-__global__ void __launch_bounds__(1024) k_pcg_init(W w) {
-  __shared__ Slot<W> slot;
-  uint32_t bid;
-  const Params& P = block_problem(w, slot, bid);
+__global__ void __launch_bounds__(1024) k_pcg_init(Params P) {
   __shared__ double red[4 * 32];
   __shared__ int fail;
   double* st = P.state;
+  if (st[S_ACTIVE] == 0) return;
+  __syncthreads();
   if (threadIdx.x == 0)
     for (int j = S_RHO; j <= 25; j++) st[j] = 0;
   __syncthreads();
-  if (st[S_ACTIVE] == 0) return;
   if (P.shared) {
     double v[4] = {0, 0, 0, 0};
     for (uint32_t b = threadIdx.x; b < P.task_blocks; b += blockDim.x)
@@ -1603,9 +1601,10 @@ __global__ void __launch_bounds__(256) k_update_cameras(W w) {
   const Params& P = block_problem(w, slot, bid);
   __shared__ int ok;
   double* st = P.state;
+  if (st[S_ACTIVE] == 0) return;
   if (threadIdx.x == 0) st[S_TRIAL_VALID] = 0;
   __syncthreads();
-  if (st[S_ACTIVE] == 0 || st[S_CG_FAILED] != 0) return;
+  if (st[S_CG_FAILED] != 0) return;
   const uint32_t C = P.C;
   if (threadIdx.x == 0) {
     ok = 1;
@@ -1840,13 +1839,18 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_
 
 // ---- K18/K19: acceptance and commit ------------------------------------------------------------
 
+// Every block adds the candidate's cost over the task blocks in the same order and takes the same
+// decision, copies its share of an accepted candidate, and the block that ends last writes the state
+// (the others have read it by then).  An iteration past the end of a solve changes nothing.
 template <class W>
 __global__ void __launch_bounds__(256) k_accept(W w) {
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
-  __shared__ double red[2 * 8];
+  __shared__ double red[2 * 8], sums[2];
+  __shared__ bool last;
   double* st = P.state;
+  if (st[S_ACTIVE] == 0) return;
   double v[2] = {0, 0};
   const bool valid = st[S_TRIAL_VALID] != 0;
   if (valid)
@@ -1855,16 +1859,30 @@ __global__ void __launch_bounds__(256) k_accept(W w) {
       v[1] += P.cost_part[4 * b + 1];
     }
   block_sum(v, red);
-  if (threadIdx.x != 0) return;
-  st[S_COMMIT] = 0;
-  if (st[S_ACTIVE] == 0) return;
-  const double cost = v[0], squares = v[1];
-  if (valid && cost < st[S_COST]) {
-    const double change = st[S_COST] - cost;
+  if (threadIdx.x == 0) {
+    sums[0] = v[0];
+    sums[1] = v[1];
+  }
+  __syncthreads();
+  const double cost = sums[0], squares = sums[1], before = st[S_COST];
+  const bool commit = valid && cost < before;
+  if (commit) {
+    const uint32_t step = P.commit_blocks * blockDim.x, first = bid * blockDim.x + threadIdx.x;
+    for (uint32_t i = first; i < 12 * P.C; i += step) P.poses[i] = P.tposes[i];
+    for (uint32_t i = first; i < 3 * P.P; i += step) P.points[i] = P.tpoints[i];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(P.ticket + 3, 1u) == P.commit_blocks - 1;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  P.ticket[3] = 0;
+  st[S_COMMIT] = commit ? 1 : 0;
+  if (commit) {
+    const double change = before - cost;
     st[S_COST] = cost;
     st[S_SSE] = squares;
     st[S_ACCEPTED] += 1;
-    st[S_COMMIT] = 1;
+    if (P.shared) st[S_LOG_FOCAL] = st[S_LOG_FOCAL_TRIAL];
     st[S_LAMBDA] = fmax(1e-10, st[S_LAMBDA] / 3);
     if (change < fmax(P.stall, 1e-9) * fmax(1.0, cost)) st[S_ACTIVE] = 0;
   } else {
@@ -1882,19 +1900,6 @@ __global__ void __launch_bounds__(256) k_many_active(const Params* params, uint3
   for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) n += params[k].state[S_ACTIVE] != 0;
   n = __syncthreads_count(n != 0);
   if (threadIdx.x == 0) *active = n;
-}
-
-template <class W>
-__global__ void k_commit(W w) {
-  __shared__ Slot<W> slot;
-  uint32_t bid;
-  const Params& P = block_problem(w, slot, bid);
-  const double* st = P.state;
-  if (st[S_COMMIT] == 0) return;
-  const uint32_t i = bid * blockDim.x + threadIdx.x;
-  if (i < 12 * P.C) P.poses[i] = P.tposes[i];
-  if (i < 3 * P.P) P.points[i] = P.tpoints[i];
-  if (i == 0 && P.shared) P.state[S_LOG_FOCAL] = st[S_LOG_FOCAL_TRIAL];
 }
 
 // ---- K20: packBundleResult ----------------------------------------------------------------------
@@ -2102,7 +2107,7 @@ void launch_update_points(const Params& p, cudaStream_t s) {
     k_update_points<false, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   }
 }
-void launch_accept(const Params& p, cudaStream_t s) { k_accept<<<1, 256, 0, s>>>(p); }
+void launch_accept(const Params& p, cudaStream_t s) { k_accept<<<p.commit_blocks, 256, 0, s>>>(p); }
 // The kernels of one LM iteration up to the PCG, and after it, over a batch's lists of blocks.
 uint32_t launch_many_begin(const ManyLists& b, cudaStream_t s) {
   k_unpack<<<b.setup.blocks, 256, 0, s>>>(b.setup.of(b));
@@ -2119,26 +2124,17 @@ uint32_t launch_many_linearize(const ManyLists& b, cudaStream_t s) {
   k_camera_finish<true, Many><<<b.finish.blocks, kFinishThreads, 0, s>>>(b.finish.of(b));
   return 3;
 }
-uint32_t launch_many_pcg_init(const ManyLists& b, cudaStream_t s) {
-  k_pcg_init<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
-  return 1;
-}
 uint32_t launch_many_update(const ManyLists& b, cudaStream_t s) {
   k_update_cameras<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
   if (b.shared) k_update_points<true, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
   else k_update_points<false, true, Many><<<b.task.blocks, kPointThreads, 0, s>>>(b.task.of(b));
-  k_accept<Many><<<b.one.blocks, 256, 0, s>>>(b.one.of(b));
-  k_commit<Many><<<b.commit.blocks, 256, 0, s>>>(b.commit.of(b));
+  k_accept<Many><<<b.commit.blocks, 256, 0, s>>>(b.commit.of(b));
   k_many_active<<<1, 256, 0, s>>>(b.params, b.count, b.active);
-  return 5;
+  return 4;
 }
 uint32_t launch_many_pack(const ManyLists& b, cudaStream_t s) {
   k_pack<Many><<<b.pack.blocks, 256, 0, s>>>(b.pack.of(b));
   return 1;
-}
-void launch_commit(const Params& p, cudaStream_t s) {
-  const uint32_t n = (12 * p.C > 3 * p.P ? 12 * p.C : 3 * p.P);
-  k_commit<<<(n + 255) / 256, 256, 0, s>>>(p);
 }
 void launch_pack(const Params& p, cudaStream_t s) {
   const uint32_t n = 12 * p.C + 3 * p.P + 27;

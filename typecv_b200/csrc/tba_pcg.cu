@@ -8,7 +8,8 @@
 // and only z and four partial sums a block cross between blocks, as values that carry their step's
 // number (Flagged): no barrier, no fence, and the L1 keeps what the step only reads.  Every block adds
 // the partial sums in the same order, so all take the same decisions.  A block can publish a step's z
-// only once every block has published the sums that follow its use of the last z, so one buffer does.
+// only once every block has published the sums that follow its use of the last z, and a reduction's
+// sums only after the other reduction (the start counts as a second one), so one buffer of each does.
 // What bounds a step is the two exchanges through the L2 (about 0.7 us each) with many blocks, and the
 // block's own chain of reductions with one.
 #include <cuda_runtime.h>
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   uint32_t bid, grid;
   const PcgSystem& A = block_system(system, slot, bid, grid);
   double* st = A.state;
-  if (st[A.active] == 0 || limit == 0) return;
+  if (st[A.rhs ? A.solving : A.active] == 0 || limit == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool alone = grid == 1;
   const uint32_t c0 = A.share[bid], c1 = A.share[bid + 1], nr = c1 - c0, rows = 6 * nr, first = 6 * c0, n = 6 * A.C;
@@ -260,27 +261,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
     for (uint32_t k = threadIdx.x; k < 36 * nr; k += kThreads) to[k] = Minv[k];
     Minv = to;
   }
+  const bool starting = A.rhs != nullptr;
   for (uint32_t j = threadIdx.x; j < cols; j += kThreads) {
     const uint32_t b = j / 6;
     pl[j] = 0;  // (beta is zero in the first step)
-    if (!alone) zl[j] = A.z[6 * uni[b] + (j - 6 * b)];
+    if (!alone && !starting) zl[j] = A.z[6 * uni[b] + (j - 6 * b)];
   }
-  if (keep)
+  if (keep || starting)
     for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
-      xs[i] = A.x[first + i];
-      rs[i] = A.r[first + i];
-      zs[i] = A.z[first + i];
+      xs[i] = starting ? 0 : A.x[first + i];
+      rs[i] = starting ? A.rhs[first + i] : A.r[first + i];
+      if (!starting) zs[i] = A.z[first + i];
     }
   double xf = 0, rf = 0, zf = 0, pf = 0, sff = 0, finv = 0;  // the focal unknown, alike in every block
-  if (SHARED) {
+  if (SHARED && !starting) {
     xf = A.x[n];
     rf = A.r[n];
     zf = A.z[n];
     sff = st[A.focal_diag];
     finv = st[A.focal_inv];
   }
-  double rho = st[A.rho], beta = 0, r2 = st[A.r2];
-  const double bound = fmax(A.tol * A.tol * st[A.r0], A.inner_r0 >= 0 ? A.tol_inner * A.tol_inner * st[A.inner_r0] : 0.0);
+  double rho = st[A.rho], beta = 0, r0 = st[A.r0], r2 = st[A.r2];
+  double inner = A.inner_r0 >= 0 ? st[A.inner_r0] : 0.0;
   // A warp per camera row, or several warps on a row's blocks; a lane sums one of the six rows over every
   // fifth block.  The first `owners` warps hold the own rows' scalars.
   const uint32_t splits = nr == 0 || nr >= uint32_t(kWarps) ? 1 : kWarps / nr;
@@ -304,8 +306,91 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   const uint32_t my_place = threadIdx.x < rows ? place_of(threadIdx.x) : 0;
   const uint32_t my_part = threadIdx.x / 6 * splits, my_row = threadIdx.x % 6;
   const double* const znext = alone ? zs : zl;
+  // z = M^-1 r of the own cameras (to the other blocks as the z of `step`); r . r and z . r.
+  auto precondition = [&](uint64_t step, double (&v)[2]) {
+    v[0] = v[1] = 0;
+    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
+      const double* Mi = Minv + 6 * size_t(i);
+      const double* rc = rs + i - i % 6;
+      const double rr = rs[i];
+      const double zz = (Mi[0] * rc[0] + Mi[1] * rc[1]) + (Mi[2] * rc[2] + Mi[3] * rc[3]) + (Mi[4] * rc[4] + Mi[5] * rc[5]);
+      if (alone) zs[i] = zz;
+      else publish(A.zx + first + i, zz, step);
+      v[0] += rr * rr;
+      v[1] += zz * rr;
+    }
+  };
+  // The columns' z of `step`, while the first warp waits for the sums.
+  auto fetch = [&](uint64_t step) {
+    for (uint32_t j = threadIdx.x - 32; j < cols; j += 2 * (kThreads - 32)) {
+      const uint32_t j1 = j + (kThreads - 32), b = j / 6, b1 = j1 / 6;
+      const Flagged* at[2] = {A.zx + 6 * uni[b] + (j - 6 * b), nullptr};
+      if (j1 < cols) at[1] = A.zx + 6 * uni[b1] + (j1 - 6 * b1);
+      double got[2];
+      if (*(volatile int*)&sh.gave_up != 0 || !await(at, j1 < cols ? 2 : 1, step, got)) {
+        *(volatile int*)&sh.gave_up = 1;
+        break;
+      }
+      zl[j] = got[0];
+      if (j1 < cols) zl[j1] = got[1];
+    }
+  };
+  if (starting) {
+    double focal = 0, full = 0;
+    if (SHARED) {
+      // H_ff and b_f with the points' shares, alike in every block.
+      double t[4] = {0, 0, 0, 0};
+      for (uint32_t b = threadIdx.x; b < A.scal_blocks; b += kThreads)
+        for (int k = 0; k < 4; k++) t[k] += A.scal_part[4 * size_t(b) + k];
+      warp_allsum(t);
+      double* to = &sh.part[0][0];  // 16 x 6 values
+      if (lane == 0)
+        for (int k = 0; k < 4; k++) to[4 * warp + k] = t[k];
+      __syncthreads();
+      for (int k = 0; k < 4; k++) t[k] = 0;
+      for (int w = 0; w < kWarps; w++)
+        for (int k = 0; k < 4; k++) t[k] += to[4 * w + k];
+      full = t[0] + st[A.lambda] * fmax(t[0], 1e-10);
+      sff = full - t[2];
+      finv = sff > 0 ? 1 / sff : -1;
+      rf = focal = -t[1] - t[3];
+      zf = finv * rf;
+    }
+    const bool fail = st[A.block_failed] != 0 || (SHARED && !(finv > 0));
+    double v[2] = {0, 0};
+    if (!fail) {
+      precondition(1, v);
+      ok = grid_sum(A, sh, v, 1, 1, owners, bid, grid, [&] { fetch(1); });
+      r0 = r2 = inner = v[0] + rf * rf;
+      rho = v[1] + rf * zf;
+    }
+    active = !fail && ok && r0 > 0 && rho > 0;
+    if (bid == 0 && threadIdx.x == 0 && ok) {
+      for (int k = A.clear_from; k <= A.clear_to; k++) st[k] = 0;
+      if (SHARED) {
+        st[A.focal_full] = full;
+        st[A.focal_diag] = sff;
+        st[A.focal_inv] = finv;
+        st[A.focal_rhs] = focal;
+      }
+      if (!fail) {
+        st[A.rho] = rho;
+        st[A.r0] = st[A.r2] = st[A.inner_r0] = r0;
+      }
+      if (active) st[A.active] = 1;
+      else if (fail || r0 > 1e-24) st[A.failed] = 1;
+    }
+    if (!active && ok) {
+      // (x of a solve that starts at its solution is zero)
+      if (!fail)
+        for (uint32_t i = threadIdx.x; i < rows; i += kThreads) A.x[first + i] = 0;
+      if (SHARED && !fail && bid == 0 && threadIdx.x == 0) A.x[n] = 0;
+      return;
+    }
+  }
+  const double bound = fmax(A.tol * A.tol * r0, A.inner_r0 >= 0 ? A.tol_inner * A.tol_inner * inner : 0.0);
   while (active && it < limit) {
-    const uint64_t step = it + 1;
+    const uint64_t step = it + 2;
     for (uint32_t j = threadIdx.x; j < cols; j += kThreads) pl[j] = znext[j] + beta * pl[j];
     __syncthreads();
     for (uint32_t item = warp; item < nr * splits; item += kWarps) {
@@ -361,33 +446,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
       rs[i] -= alpha * ss[i];
     }
     __syncthreads();
-    v[0] = v[1] = 0;  // r . r, z . r
-    for (uint32_t i = threadIdx.x; i < rows; i += kThreads) {
-      const double* Mi = Minv + 6 * size_t(i);
-      const double* rc = rs + i - i % 6;
-      const double rr = rs[i];
-      const double zz = (Mi[0] * rc[0] + Mi[1] * rc[1]) + (Mi[2] * rc[2] + Mi[3] * rc[3]) + (Mi[4] * rc[4] + Mi[5] * rc[5]);
-      if (alone) zs[i] = zz;
-      else publish(A.zx + first + i, zz, step);
-      v[0] += rr * rr;
-      v[1] += zz * rr;
-    }
-    // The columns' new z, while the first warp waits for the sums.
-    auto fetch = [&] {
-      for (uint32_t j = threadIdx.x - 32; j < cols; j += 2 * (kThreads - 32)) {
-        const uint32_t j1 = j + (kThreads - 32), b = j / 6, b1 = j1 / 6;
-        const Flagged* at[2] = {A.zx + 6 * uni[b] + (j - 6 * b), nullptr};
-        if (j1 < cols) at[1] = A.zx + 6 * uni[b1] + (j1 - 6 * b1);
-        double got[2];
-        if (*(volatile int*)&sh.gave_up != 0 || !await(at, j1 < cols ? 2 : 1, step, got)) {
-          *(volatile int*)&sh.gave_up = 1;
-          break;
-        }
-        zl[j] = got[0];
-        if (j1 < cols) zl[j1] = got[1];
-      }
-    };
-    if (!(ok = grid_sum(A, sh, v, step, 1, owners, bid, grid, fetch))) break;
+    precondition(step, v);
+    if (!(ok = grid_sum(A, sh, v, step, 1, owners, bid, grid, [&] { fetch(step); }))) break;
     it++;
     r2 = v[0];
     double next = v[1];

@@ -35,6 +35,12 @@ struct PcgSystem {
   double* state;
   int active, failed, converged, rho, r0, r2, inner_r0, steps, all_steps, wait;  // words; -1: not kept
   int focal_diag, focal_inv;
+  // With `rhs` (6C) the run starts itself: r = rhs, x = 0, z = M^-1 r, the focal unknown from the task
+  // blocks' partial sums, and the start's words (k_pcg_init does the same for steps launched one by one).
+  const double* rhs;
+  const double* scal_part;  // 4 per task block: H_ff, b_f, and the points' shares of them
+  uint32_t scal_blocks;
+  int solving, block_failed, lambda, focal_full, focal_rhs, clear_from, clear_to;
   double tol, tol_inner, alpha_limit;
   Flagged* zx;         // 6C: z between blocks
   Flagged* slots;      // 4 per block: its partial sums of the step's two reductions

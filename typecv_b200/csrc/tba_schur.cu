@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
+  if (Q.go && *Q.go == 0) return;
   const uint32_t s = bid * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t npairs = Q.totals[1];
   const uint32_t lo = s * Q.seg;
@@ -344,6 +345,7 @@ __global__ void __launch_bounds__(256) k_block_ends(W w) {
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
+  if (Q.go && *Q.go == 0) return;
   const uint32_t b = bid * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= Q.totals[0]) return;
   const uint32_t begin = Q.blk_begin[b], end = Q.blk_begin[b + 1], s0 = begin / Q.seg, s1 = (end - 1) / Q.seg;

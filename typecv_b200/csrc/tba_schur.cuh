@@ -50,7 +50,8 @@ struct SchurParams {
   uint2* blk_dst;       // its blocks in the two rows of S
   uint32_t* seg_block;  // camera pair of each segment's first pair
   uint32_t* totals;     // camera pairs, observation pairs, blocks of S
-  // Values.
+  // Values (nothing is done while *go is zero).
+  const double* go;
   double* A;     // 18 per observation: W_i N_p by columns ([k * 6 + row])
   double* part;  // 2 x 36 per segment: the sums of camera pairs that cross segments
   double* S;     // 36 per block, by columns (entry (row a, column b) at 6 b + a)
