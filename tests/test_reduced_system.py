@@ -32,12 +32,12 @@ def solve(device, C, P, M, s, i, flags=0, **kw):
     return tb.solve_packed(device, tb.make_control(C, P, M, anchor=0, scale_view=1, flags=flags, **kw), s, i)
 
 
-def against_oracle(device, C, P, M, s, i, shared, iterations, engine):
-    kw = dict(iterations=iterations, shared_focal=shared, max_cg=200)
+def against_oracle(device, C, P, M, s, i, shared, iterations, engine, tolerance=1e-6):
+    kw = dict(iterations=iterations, shared_focal=shared, max_cg=200, tolerance=tolerance)
     out, rep = solve(device, C, P, M, s, i, **kw)
     assert rep["engine"] == engine
     ref = ob.gpu_operator_packed({"C": C, "P": P, "M": M, "scene": s, "index": i}, 0, 1, iterations=iterations,
-                                 huber=2.0, max_cg=200, shared=shared)
+                                 huber=2.0, max_cg=200, shared=shared, tolerance=tolerance)
     b = 12 * C + 3 * P
     assert out[b + 10] == ref[b + 10] and out[b + 11] == ref[b + 11]
     assert abs(out[b + 6] - ref[b + 6]) <= COST_REL * ref[b + 6]
@@ -84,10 +84,11 @@ def test_every_camera_fixed_but_one(device):
 
 
 def test_dense_covisibility_keeps_the_product_over_factors(device):
-    # Every one of 120 cameras sees every point: 59 pairs an observation.
+    # Every one of 120 cameras sees every point: 59 pairs an observation.  (At the default PCG tolerance two
+    # solves of this scene that differ in rounding alone stop 1e-7 apart, on the bar itself.)
     sc = S.ring_scene(seed=11, cameras=120, points=1500)
     s, i = sc.packed()
-    against_oracle(device, sc.C, sc.P, sc.M, s, i, True, 2, engine=0)
+    against_oracle(device, sc.C, sc.P, sc.M, s, i, True, 2, engine=0, tolerance=1e-9)
 
 
 @pytest.mark.parametrize("shared", [False, True])
