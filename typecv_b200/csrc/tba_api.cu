@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -309,6 +310,42 @@ void raise_checks(const HostChecks& h, const unsigned long long* keys) {
   if (h.activity) argument(h.activity);
   if (keys[tba::CK_SCENE] != none) argument("GPU BA input exceeds supported coordinate bounds");
   if (h.camera_bounds) argument(h.camera_bounds);
+}
+
+// The adjoint, the observation evaluation and the batch on the grid kernels leave the O(M) checks to the
+// device from this many observations on; below, the kernels' launches and the read cost more than the host's
+// pass over the arrays.  Whole calls, checks on the host and on the device: an evaluation of 2,046
+// observations 134 and 145 us, of 8,190 157 and 135, of 32,772 312 and 185, of 299,873 2,000 and 870; an
+// adjoint 279 and 294, 376 and 362, 695 and 548, 3,300 and 1,840; a batch of two such windows 547 and 580,
+// 653 and 630, 980 and 817 (32,772 each).
+constexpr uint64_t kDeviceCheckMin = 8192;
+
+// The device's part of the checks, on arrays just uploaded, and the first failure of both parts raised;
+// `claims` is M words of scratch, `keys` CK_WORDS words.
+void device_checks(tba_device* d, const HostChecks& h, uint32_t C, uint32_t P, uint32_t M, const uint32_t* index,
+                   const double* const (&sections)[4], uint32_t* claims, unsigned long long* keys) {
+  tba::CheckParams cp{};
+  cp.C = C;
+  cp.P = P;
+  cp.M = M;
+  cp.index = index;
+  const uint64_t len[4] = {12 * uint64_t(C), 3 * uint64_t(P), 6 * uint64_t(C), 2 * uint64_t(M)};
+  uint64_t base = 0;
+  for (int k = 0; k < 4; k++) {
+    cp.seg[k] = sections[k];
+    cp.base[k] = base;
+    cp.len[k] = len[k];
+    base += len[k];
+  }
+  cp.claims = claims;
+  cp.keys = keys;
+  cp.lists = !h.camera_ends && !h.camera_offsets;
+  CUDA_TRY(tba::launch_checks(cp, d->sms, d->stream));
+  CUDA_TRY(cudaMemcpyAsync(d->pinned, keys, tba::CK_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, d->stream));
+  CUDA_TRY(cudaStreamSynchronize(d->stream));
+  unsigned long long found[tba::CK_WORDS];
+  std::memcpy(found, d->pinned, sizeof found);
+  raise_checks(h, found);
 }
 
 // Runs of whole points of at most 32 observations; a longer point is a run of its own.
@@ -938,34 +975,19 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   CUDA_TRY(cudaEventRecord(e_up, s));
   if (io.checks) {
     const auto c0 = std::chrono::steady_clock::now();
-    tba::CheckParams cp{};
-    cp.C = C;
-    cp.P = P;
-    cp.M = M;
-    cp.index = dindex;
-    cp.seg[0] = p.poses;
-    cp.seg[1] = p.points;
-    cp.seg[2] = p.cams;
-    cp.seg[3] = p.pixels;
-    cp.base[0] = 0;
-    cp.len[0] = 12 * uint64_t(C);
-    cp.base[1] = cp.len[0];
-    cp.len[1] = 3 * uint64_t(P);
-    cp.base[2] = cp.base[1] + cp.len[1];
-    cp.len[2] = 6 * uint64_t(C);
-    cp.base[3] = cp.base[2] + cp.len[2];
-    cp.len[3] = 2 * uint64_t(M);
-    cp.claims = p.cm_point;  // scratch until k_setup writes the camera-major point index
-    cp.keys = reinterpret_cast<unsigned long long*>(a + o_keys);
-    cp.lists = !io.checks->camera_ends && !io.checks->camera_offsets;
-    CUDA_TRY(tba::launch_checks(cp, d->sms, s));
-    CUDA_TRY(cudaMemcpyAsync(d->pinned, cp.keys, tba::CK_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    unsigned long long keys[tba::CK_WORDS];
-    std::memcpy(keys, d->pinned, sizeof keys);
-    if (io.check_ms)
-      *io.check_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - c0).count();
-    raise_checks(*io.checks, keys);
+    // (claims: scratch until k_setup writes the camera-major point index)
+    auto spent = [&] {
+      if (io.check_ms)
+        *io.check_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - c0).count();
+    };
+    try {
+      device_checks(d, *io.checks, C, P, M, dindex, {p.poses, p.points, p.cams, p.pixels}, p.cm_point,
+                    reinterpret_cast<unsigned long long*>(a + o_keys));
+    } catch (...) {
+      spent();
+      throw;
+    }
+    spent();
     if (!plannable) throw Fail{TBA_ERROR_INTERNAL, "GPU BA checks passed a problem without a schedule"};
   }
 
@@ -1264,11 +1286,14 @@ struct BatchReport {
 
 // The batch on the grid kernels: every kernel of an LM iteration runs over all problems at once (its
 // blocks a list of (problem, block)), with each problem's reduced system explicit and its PCG in one
-// block; the iteration is a CUDA graph, replayed while the batch's lists keep their places.  False (nothing launched) when the workspace does not fit.
+// block; the iteration is a CUDA graph, replayed while the batch's lists keep their places.  With
+// `whole_check` the device checks the arrays first, and the host's checks give the message.  False
+// (nothing launched) when the workspace does not fit.
 bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_problem* probs, uint32_t count,
                    const std::vector<WindowPlan>& plans, const std::vector<uint32_t>& order, const double* scene,
                    size_t scene_len, const uint32_t* index, size_t index_len, size_t output_len, cudaEvent_t uploaded,
-                   cudaEvent_t begun, BatchReport& rep, double*& dout_of, uint64_t& h2d) {
+                   cudaEvent_t begun, BatchReport& rep, double*& dout_of, uint64_t& h2d,
+                   const std::function<void()>* whole_check) {
   const bool shared = bc->shared_focal != 0;
   Layout L;
   const size_t o_scene = L.take<double>(scene_len), o_index = L.take<uint32_t>(index_len), o_out = L.take<double>(output_len);
@@ -1336,6 +1361,10 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   size_t bit_words = 0;
   for (uint32_t k = 0; k < count; k++) bit_words += size_t(probs[k].cameras) * ((probs[k].cameras + 31) / 32);
   const size_t o_bits = L.take<uint32_t>(bit_words);
+  uint64_t M_all = 0;
+  for (uint32_t k = 0; k < count; k++) M_all += probs[k].observations;
+  const size_t o_claims = L.take<uint32_t>(whole_check ? M_all : 0), o_bad = L.take<uint32_t>(1),
+               o_checks = L.take<tba::CheckProblem>(count);
   struct Work {
     size_t poses, points, cams, pixels, tposes, tpoints, rlim, cmp, cmx, pblk, A, pw, xw, U, Minv, rhs, hcf, scf, chunk, vec, scal, cost, ticket, state, system;
   };
@@ -1476,7 +1505,32 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   up(o_params, params.data(), count * sizeof(tba::Params));
   up(o_schur, schur.data(), count * sizeof(tba::SchurParams));
   up(o_pcg, pcg.data(), count * sizeof(tba::PcgSystem));
+  std::vector<tba::CheckProblem> checks(count);
+  if (whole_check) {
+    uint64_t claims = 0;
+    for (uint32_t k = 0; k < count; k++) {
+      const tba::Params& p = params[k];
+      checks[k] = tba::CheckProblem{p.C, p.P, p.M, (std::max(p.M, p.C) + 255) / 256, p.obs_camera, p.packed, u32(o_claims) + claims};
+      claims += p.M;
+    }
+    up(o_checks, checks.data(), count * sizeof(tba::CheckProblem));
+  }
   CUDA_TRY(cudaEventRecord(uploaded, s));
+  uint32_t launches = 0;
+  if (whole_check) {
+    CUDA_TRY(cudaMemsetAsync(a + o_claims, 0, M_all * sizeof(uint32_t), s));
+    CUDA_TRY(cudaMemsetAsync(a + o_bad, 0, sizeof(uint32_t), s));
+    tba::launch_check_batch(reinterpret_cast<const tba::CheckProblem*>(a + o_checks), reinterpret_cast<const uint2*>(a + o_list[4]),
+                            uint32_t(lists[4].size()), u32(o_bad), s);
+    launches++;
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(d->pinned, a + o_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (*reinterpret_cast<const uint32_t*>(d->pinned) != 0) {
+      (*whole_check)();
+      throw Fail{TBA_ERROR_INTERNAL, "GPU BA batch checks disagree"};
+    }
+  }
 
   struct Key {
     tba::ManyLists many;
@@ -1513,7 +1567,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   key.count = count;
   key.limit = bc->max_cg;
   CUDA_TRY(cudaMemsetAsync(a + o_bits, 0, bit_words * sizeof(uint32_t), s));
-  uint32_t launches = tba::launch_many_begin(key.many, s);
+  launches += tba::launch_many_begin(key.many, s);
   launches += tba::schur_launch_many_structure(key.schur, s);
   launches += tba::pcg_launch_many_plan(key.pcg, count, Cmax, s);
   CUDA_TRY(cudaGetLastError());
@@ -1592,43 +1646,73 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   std::mutex fail_mu;
   uint32_t fail_at = UINT32_MAX;
   Fail first_fail{TBA_OK, ""};
-  parallel_ranges(count, 2, [&](uint64_t b, uint64_t e, unsigned) {
-    for (uint64_t k = b; k < e; k++) {
-      try {
-        const tba_batch_problem& q = probs[k];
-        const tba_control c = batch_problem_control(bc, q);
-        check_control(&c);
-        if (q.reserved != 0) argument("Invalid GPU BA batch: reserved field must be 0");
-        if (q.cameras > max_cams)
-          argument("Batched GPU BA problem has " + std::to_string(q.cameras) +
-                   " cameras; the block solver takes at most " + std::to_string(max_cams));
-        if (uint64_t(3) * q.observations + q.points + 2ull * q.cameras + 2 > 0xffffffffull)
-          argument("GPU BA scene dimensions exceed integer index bounds");
-        if (q.scene_offset > scene_len || scene_len - q.scene_offset < tba_scene_size(&c))
-          argument("Invalid GPU BA batch: a scene lies outside the scene array");
-        if (q.index_offset > index_len || index_len - q.index_offset < tba_index_size(&c))
-          argument("Invalid GPU BA batch: an index lies outside the index array");
-        if (q.output_offset > output_len || output_len - q.output_offset < tba_output_size(&c))
-          argument("Invalid GPU BA batch: a result record lies outside the output array");
-        check_index(&c, index + q.index_offset);
-        check_scene(&c, scene + q.scene_offset, tba_scene_size(&c));
-        const uint32_t* ps = index + q.index_offset + 2 * size_t(q.observations);
-        plans[k].tasks = build_tasks(ps, q.points);
-        if (auto_shape || grid_forced) {
-          plans[k].chunks = build_chunks(ps + q.points + 1, q.cameras, chunk);
-          plans[k].pairs = count_pairs(ps, q.points);
+  // On the grid kernels the O(M) checks run on the device: the host makes the others here, and repeats all
+  // of them, for the message, where one of either kind fails.
+  std::vector<uint8_t> suspect(count, 0);
+  auto check_problems = [&](bool whole) {
+    parallel_ranges(count, 2, [&](uint64_t b, uint64_t e, unsigned) {
+      for (uint64_t k = b; k < e; k++) {
+        try {
+          const tba_batch_problem& q = probs[k];
+          const tba_control c = batch_problem_control(bc, q);
+          check_control(&c);
+          if (q.reserved != 0) argument("Invalid GPU BA batch: reserved field must be 0");
+          if (q.cameras > max_cams)
+            argument("Batched GPU BA problem has " + std::to_string(q.cameras) +
+                     " cameras; the block solver takes at most " + std::to_string(max_cams));
+          if (uint64_t(3) * q.observations + q.points + 2ull * q.cameras + 2 > 0xffffffffull)
+            argument("GPU BA scene dimensions exceed integer index bounds");
+          if (q.scene_offset > scene_len || scene_len - q.scene_offset < tba_scene_size(&c))
+            argument("Invalid GPU BA batch: a scene lies outside the scene array");
+          if (q.index_offset > index_len || index_len - q.index_offset < tba_index_size(&c))
+            argument("Invalid GPU BA batch: an index lies outside the index array");
+          if (q.output_offset > output_len || output_len - q.output_offset < tba_output_size(&c))
+            argument("Invalid GPU BA batch: a result record lies outside the output array");
+          if (whole) {
+            check_index(&c, index + q.index_offset);
+            check_scene(&c, scene + q.scene_offset, tba_scene_size(&c));
+          } else {
+            const HostChecks h = host_checks(&c, index + q.index_offset, scene + q.scene_offset);
+            if (h.point_ends || h.camera_ends || h.camera_offsets || h.activity || h.camera_bounds) {
+              suspect[k] = 1;
+              continue;
+            }
+          }
+          const uint32_t* ps = index + q.index_offset + 2 * size_t(q.observations);
+          plans[k].tasks = build_tasks(ps, q.points);
+          if (auto_shape || grid_forced) {
+            plans[k].chunks = build_chunks(ps + q.points + 1, q.cameras, chunk);
+            plans[k].pairs = count_pairs(ps, q.points);
+          }
+        } catch (const Fail& f) {
+          std::lock_guard<std::mutex> lock(fail_mu);
+          if (k < fail_at) {
+            fail_at = uint32_t(k);
+            first_fail = f;
+          }
+          return;
         }
-      } catch (const Fail& f) {
-        std::lock_guard<std::mutex> lock(fail_mu);
-        if (k < fail_at) {
-          fail_at = uint32_t(k);
-          first_fail = f;
-        }
-        return;
       }
+    });
+    if (fail_at != UINT32_MAX) throw first_fail;
+  };
+  bool checked = false;
+  auto check_whole = [&] {
+    if (!checked) check_problems(true);
+    checked = true;
+  };
+  if ((auto_shape || grid_forced) && M_all >= kDeviceCheckMin) {
+    try {
+      check_problems(false);
+    } catch (const Fail&) {
+      fail_at = UINT32_MAX;
+      check_whole();
+      throw;
     }
-  });
-  if (fail_at != UINT32_MAX) throw first_fail;
+    if (std::find(suspect.begin(), suspect.end(), 1) != suspect.end()) check_whole();
+  } else {
+    check_whole();
+  }
   for (uint32_t k = 0; k < count; k++) {
     const std::vector<uint32_t>& t = plans[k].tasks;
     task_first[k] = tasks.size();
@@ -1643,8 +1727,10 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   for (uint32_t j = 1; j < count; j++) {
     const tba_batch_problem& prev = probs[by_out[j - 1]];
     const tba_control pc = batch_problem_control(bc, prev);
-    if (prev.output_offset + tba_output_size(&pc) > probs[by_out[j]].output_offset)
+    if (prev.output_offset + tba_output_size(&pc) > probs[by_out[j]].output_offset) {
+      check_whole();
       argument("Invalid GPU BA batch: result records overlap");
+    }
   }
   // Largest problems first (longest-processing-time order for the persistent blocks).
   std::vector<uint32_t> order(count);
@@ -1718,11 +1804,14 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
       fits = fits && plans[k].pairs < 0x7fffffffull;
     }
     double* dout = nullptr;
+    const std::function<void()> whole = check_whole;
     if (fits && (grid_forced || pairs <= 32 * M_all) &&
-        batch_on_grid(d, bc, probs, count, plans, order, scene, scene_len, index, index_len, output_len, e1, e0, ran, dout, h2d)) {
+        batch_on_grid(d, bc, probs, count, plans, order, scene, scene_len, index, index_len, output_len, e1, e0, ran, dout, h2d,
+                      checked ? nullptr : static_cast<const std::function<void()>*>(&whole))) {
       finish(dout);
       return;
     }
+    check_whole();
     if (grid_forced) throw Fail{TBA_ERROR_BUDGET, "GPU BA batch needs more device memory than the working budget"};
   }
 
@@ -1960,9 +2049,10 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
 
 // ---- the adjoint ---------------------------------------------------------------------------------
 
-void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, const uint32_t* index,
-               const double* cotangent, double* pixels_bar, double* intrinsics_bar, double* solution,
-               tba_vjp_report* report) {
+// `checks`: the host's part of the checks, whose O(M) part then runs on the device; null when all are done.
+void solve_vjp(tba_device* d, const tba_vjp_control* vc, const HostChecks* checks, const double* scene,
+               const uint32_t* index, const double* cotangent, double* pixels_bar, double* intrinsics_bar,
+               double* solution, tba_vjp_report* report) {
   const auto wall0 = std::chrono::steady_clock::now();
   const uint32_t C = vc->cameras, P = vc->points, M = vc->observations;
   const uint32_t* active = index + 3 * size_t(M) + P + C + 2;
@@ -1992,6 +2082,7 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
   const uint64_t npairs = count_pairs(index + 2 * size_t(M), P);
   bool schur = prefer_schur(C, M, npairs, vc->max_cg, 64);
   Chunks chunks;
+  if (checks && (checks->camera_ends || checks->camera_offsets)) schur = false;  // no chunks; the checks will fail
   if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, chunk_size(M, d->sms));
   const uint32_t nchunks = uint32_t(chunks.cam.size());
   Layout L;
@@ -2104,6 +2195,10 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
   up(const_cast<double*>(A.pixels), scene + 18 * size_t(C) + 3 * size_t(P), 2 * sizeof(double) * M);
   up(dindex, index, sizeof(uint32_t) * (3 * size_t(M) + P + 2 * size_t(C) + 2));
   up(const_cast<uint32_t*>(A.task_obs), task_obs.data(), sizeof(uint32_t) * task_obs.size());
+  // Before any kernel follows the arrays (scratch: the place of the pixels' cotangent).
+  if (checks)
+    device_checks(d, *checks, C, P, M, dindex, {A.poses, A.points, A.cams, A.pixels}, reinterpret_cast<uint32_t*>(A.ybar),
+                  reinterpret_cast<unsigned long long*>(A.ybar + M));
   uint32_t launches = 0;
   if (schur) {
     up(const_cast<uint32_t*>(sq.chunk_cam), chunks.cam.data(), sizeof(uint32_t) * chunks.cam.size());
@@ -2272,9 +2367,11 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const double* scene, co
 
 // ---- observation evaluation ------------------------------------------------------------------------
 
-void evaluate_observations(tba_device* d, const tba_observation_control* oc, const double* cameras,
+// (`check`: false is returned, with nothing evaluated, when the device finds the arrays out of order.)
+bool evaluate_observations(tba_device* d, const tba_observation_control* oc, const double* cameras,
                            const double* points, const double* pixels, const uint32_t* indices,
-                           const uint32_t* offsets, uint32_t* flags, double* summary, tba_observation_report* report) {
+                           const uint32_t* offsets, uint32_t* flags, double* summary, tba_observation_report* report,
+                           bool check) {
   const auto wall0 = std::chrono::steady_clock::now();
   const uint32_t C = oc->cameras, P = oc->points, M = oc->observations;
   const bool guarded = oc->max_relative_depth_std > 0;
@@ -2334,6 +2431,29 @@ void evaluate_observations(tba_device* d, const tba_observation_control* oc, con
     up(o_tasks, tasks.data(), sizeof(uint32_t) * tasks.size());
   }
   CUDA_TRY(cudaEventRecord(e1, s));
+  if (check) {
+    // Whether the arrays are in order, before any kernel follows their indices.
+    tba::ObservationChecks k{};
+    k.C = C;
+    k.P = P;
+    k.M = M;
+    k.indices = p.indices;
+    k.offsets = p.offsets;
+    k.values[0] = p.cameras;
+    k.values[1] = p.points;
+    k.values[2] = p.pixels;
+    k.counts[0] = 18 * uint64_t(C);
+    k.counts[1] = 3 * uint64_t(P);
+    k.counts[2] = 2 * uint64_t(M);
+    k.bad = reinterpret_cast<uint32_t*>(p.summary);  // (written by the evaluation)
+    CUDA_TRY(cudaMemsetAsync(k.bad, 0, sizeof(uint32_t), s));
+    tba::launch_check_observations(k, d->sms, s);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(d->pinned, k.bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    if (*reinterpret_cast<const uint32_t*>(d->pinned) != 0) return false;
+    CUDA_TRY(cudaEventRecord(e1, s));
+  }
   tba::launch_observations(p, s);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaEventRecord(e2, s));
@@ -2353,9 +2473,10 @@ void evaluate_observations(tba_device* d, const tba_observation_control* oc, con
     report->download_ms = ms;
     report->h2d_bytes = h2d;
     report->d2h_bytes = nflags * sizeof(uint32_t) + 2 * sizeof(double);
-    report->kernel_launches = (guarded ? (p.ntasks ? 1u : 0u) : (M ? 1u : 0u)) + (M ? 1u : 0u) + 1u;
+    report->kernel_launches = (guarded ? (p.ntasks ? 1u : 0u) : (M ? 1u : 0u)) + (M ? 1u : 0u) + 1u + (check ? 1u : 0u);
     report->wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - wall0).count();
   }
+  return true;
 }
 
 }  // namespace
@@ -2534,10 +2655,20 @@ tba_status tba_bundle_vjp(tba_device* d, const tba_vjp_control* vc, const double
         if (!std::isfinite(cotangent[i])) argument("Invalid GPU BA adjoint: the cotangent is not finite");
     if (uint64_t(3) * c.observations + c.points + 2ull * c.cameras + 2 > 0xffffffffull)
       argument("GPU BA scene dimensions exceed integer index bounds");
-    check_index(&c, index);
-    check_scene(&c, scene, scene_len);
-    CUDA_TRY(cudaSetDevice(d->ordinal));
-    solve_vjp(d, vc, scene, index, cotangent, pixels_bar, intrinsics_bar, solution, report);
+    const bool on_device = c.observations >= kDeviceCheckMin;
+    auto host_check = [&] {
+      check_index(&c, index);
+      check_scene(&c, scene, scene_len);
+    };
+    if (!on_device) host_check();
+    const HostChecks checks = on_device ? host_checks(&c, index, scene) : HostChecks{};
+    try {
+      CUDA_TRY(cudaSetDevice(d->ordinal));
+      solve_vjp(d, vc, on_device ? &checks : nullptr, scene, index, cotangent, pixels_bar, intrinsics_bar, solution, report);
+    } catch (const Fail& f) {
+      if (on_device && f.status == TBA_ERROR_BUDGET) host_check();  // arrays out of order are reported first
+      throw;
+    }
   } catch (const Fail& f) {
     d->error = f.message;
     return f.status;
@@ -2572,43 +2703,58 @@ tba_status tba_evaluate_observations(tba_device* d, const tba_observation_contro
     if (cameras_len < 18 * C || points_len < 3 * P || pixels_len < 2 * M || indices_len < 2 * M ||
         flags_len < M + (guarded ? P : 0))
       argument("Invalid GPU observation arrays: lengths");
-    FirstFailure ff;
-    parallel_ranges(M, 1u << 18, [&](uint64_t b, uint64_t e, unsigned) {
-      for (uint64_t i = b; i < e; i++)
-        if (indices[2 * i] >= C || indices[2 * i + 1] >= P)
-          return ff.record(i, "Invalid GPU observation indices: a camera or point out of range");
-    });
-    ff.raise();
-    if (guarded) {
-      if (!offsets || offsets_len < P + 1) argument("Invalid GPU observation arrays: track offsets");
-      if (offsets[0] != 0 || offsets[P] != M) argument("Invalid GPU observation arrays: track offsets");
-      FirstFailure tf;
-      parallel_ranges(P, 1u << 16, [&](uint64_t b, uint64_t e, unsigned) {
-        for (uint64_t h = b; h < e; h++) {
-          if (offsets[h + 1] < offsets[h] || offsets[h + 1] > M)
-            return tf.record(h, "Invalid GPU observation arrays: track offsets");
-          for (uint64_t i = offsets[h]; i < offsets[h + 1]; i++)
-            if (indices[2 * i + 1] != h) return tf.record(h, "Invalid GPU observation arrays: track offsets");
-        }
+    // The O(M) checks run on the device after the upload; the host makes them where the device finds the
+    // arrays out of order, for the message a serial scan meets first, and on small calls.
+    auto host_check = [&] {
+      FirstFailure ff;
+      parallel_ranges(M, 1u << 18, [&](uint64_t b, uint64_t e, unsigned) {
+        for (uint64_t i = b; i < e; i++)
+          if (indices[2 * i] >= C || indices[2 * i + 1] >= P)
+            return ff.record(i, "Invalid GPU observation indices: a camera or point out of range");
       });
-      tf.raise();
-    }
-    FirstFailure bf;
-    auto bounded = [&](const double* v, uint64_t n, uint64_t base) {
-      parallel_ranges(n, 1u << 18, [&](uint64_t b, uint64_t e, unsigned) {
-        for (uint64_t i = b; i < e; i++) {
-          const double x = v[i];
-          if (!std::isfinite(x) || std::fabs(x) > 1e9 || (x != 0 && std::fabs(x) < 1e-30))
-            return bf.record(base + i, "Invalid GPU scene coordinate bounds");
-        }
-      });
+      ff.raise();
+      if (guarded) {
+        if (!offsets || offsets_len < P + 1) argument("Invalid GPU observation arrays: track offsets");
+        if (offsets[0] != 0 || offsets[P] != M) argument("Invalid GPU observation arrays: track offsets");
+        FirstFailure tf;
+        parallel_ranges(P, 1u << 16, [&](uint64_t b, uint64_t e, unsigned) {
+          for (uint64_t h = b; h < e; h++) {
+            if (offsets[h + 1] < offsets[h] || offsets[h + 1] > M)
+              return tf.record(h, "Invalid GPU observation arrays: track offsets");
+            for (uint64_t i = offsets[h]; i < offsets[h + 1]; i++)
+              if (indices[2 * i + 1] != h) return tf.record(h, "Invalid GPU observation arrays: track offsets");
+          }
+        });
+        tf.raise();
+      }
+      FirstFailure bf;
+      auto bounded = [&](const double* v, uint64_t n, uint64_t base) {
+        parallel_ranges(n, 1u << 18, [&](uint64_t b, uint64_t e, unsigned) {
+          for (uint64_t i = b; i < e; i++) {
+            const double x = v[i];
+            if (!std::isfinite(x) || std::fabs(x) > 1e9 || (x != 0 && std::fabs(x) < 1e-30))
+              return bf.record(base + i, "Invalid GPU scene coordinate bounds");
+          }
+        });
+      };
+      bounded(cameras, 18 * C, 0);
+      bounded(points, 3 * P, 18 * C);
+      bounded(pixels, 2 * M, 18 * C + 3 * P);
+      bf.raise();
     };
-    bounded(cameras, 18 * C, 0);
-    bounded(points, 3 * P, 18 * C);
-    bounded(pixels, 2 * M, 18 * C + 3 * P);
-    bf.raise();
-    CUDA_TRY(cudaSetDevice(d->ordinal));
-    evaluate_observations(d, oc, cameras, points, pixels, indices, offsets, flags, summary, report);
+    const bool on_device = M >= kDeviceCheckMin && !(guarded && (!offsets || offsets_len < P + 1));
+    if (!on_device) host_check();
+    if (on_device && guarded && (offsets[0] != 0 || offsets[P] != M)) host_check();
+    try {
+      CUDA_TRY(cudaSetDevice(d->ordinal));
+      if (!evaluate_observations(d, oc, cameras, points, pixels, indices, offsets, flags, summary, report, on_device)) {
+        host_check();
+        throw Fail{TBA_ERROR_INTERNAL, "GPU observation checks disagree"};
+      }
+    } catch (const Fail& f) {
+      if (on_device && f.status == TBA_ERROR_BUDGET) host_check();  // arrays out of order are reported first
+      throw;
+    }
   } catch (const Fail& f) {
     d->error = f.message;
     return f.status;

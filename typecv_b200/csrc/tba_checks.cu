@@ -57,7 +57,71 @@ __global__ void __launch_bounds__(256) k_check_scene(const double* x, uint64_t n
   }
 }
 
+__device__ inline bool outside(double v) { return !isfinite(v) || fabs(v) > 1e9 || (v != 0 && fabs(v) < 1e-30); }
+
+// Every check of a problem, strided over its blocks.  The host has checked the camera offsets.
+__global__ void __launch_bounds__(256) k_check_batch(const CheckProblem* problems, const uint2* work, uint32_t* bad) {
+  const uint2 w = work[blockIdx.x];
+  const CheckProblem A = problems[w.x];
+  const uint32_t first = w.y * blockDim.x + threadIdx.x, step = A.blocks * blockDim.x;
+  const uint32_t* obs_camera = A.index;
+  const uint32_t* obs_point = A.index + A.M;
+  const uint32_t* ps = obs_point + A.M;
+  const uint32_t* cs = ps + A.P + 1;
+  const uint32_t* cam_obs = cs + A.C + 1;
+  bool failed = false;
+  for (uint32_t p = first; p < A.P; p += step) {
+    const uint32_t b = ps[p], e = ps[p + 1];
+    if (e > A.M || uint64_t(e) < uint64_t(b) + 2) {
+      failed = true;
+    } else {
+      for (uint32_t i = b; i < e; i++) failed = failed || obs_point[i] != p;
+    }
+  }
+  for (uint32_t i = first; i < A.M; i += step) failed = failed || obs_camera[i] >= A.C;
+  for (uint32_t cam = w.y; cam < A.C; cam += A.blocks)
+    for (uint32_t k = cs[cam] + threadIdx.x; k < cs[cam + 1]; k += blockDim.x) {
+      const uint32_t i = cam_obs[k];
+      if (i >= A.M || obs_camera[i] != cam || atomicAdd(A.claims + i, 1u) != 0) failed = true;
+    }
+  const uint64_t n = 18ull * A.C + 3ull * A.P + 2ull * A.M;
+  for (uint64_t i = first; i < n; i += step) failed = failed || outside(A.scene[i]);
+  if (__syncthreads_or(failed) && threadIdx.x == 0) *bad = 1;
+}
+
+__global__ void __launch_bounds__(256) k_check_observations(ObservationChecks A) {
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  bool failed = false;
+  const uint2* ix = reinterpret_cast<const uint2*>(A.indices);
+  for (uint64_t i = first; i < A.M; i += step) {
+    const uint2 v = ix[i];
+    failed = failed || v.x >= A.C || v.y >= A.P;
+  }
+  if (A.offsets)
+    for (uint64_t h = first; h < A.P; h += step) {
+      const uint32_t b = A.offsets[h], e = A.offsets[h + 1];
+      if (e < b || e > A.M) {
+        failed = true;
+      } else {
+        for (uint32_t i = b; i < e; i++) failed = failed || ix[i].y != h;
+      }
+    }
+  for (int k = 0; k < 3; k++)
+    for (uint64_t i = first; i < A.counts[k]; i += step) failed = failed || outside(A.values[k][i]);
+  if (__syncthreads_or(failed) && threadIdx.x == 0) *A.bad = 1;
+}
+
 }  // namespace
+
+void launch_check_batch(const CheckProblem* problems, const uint2* work, uint32_t blocks, uint32_t* bad, cudaStream_t s) {
+  k_check_batch<<<blocks, 256, 0, s>>>(problems, work, bad);
+}
+
+void launch_check_observations(const ObservationChecks& p, int sms, cudaStream_t s) {
+  const uint64_t most = p.M > p.P ? p.M : p.P;
+  const uint64_t want = (most + 255) / 256, cap = 8ull * uint64_t(sms > 0 ? sms : 1);
+  k_check_observations<<<uint32_t(want < 1 ? 1 : (want < cap ? want : cap)), 256, 0, s>>>(p);
+}
 
 cudaError_t launch_checks(const CheckParams& p, int sms, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(p.keys, 0xff, CK_WORDS * sizeof(unsigned long long), s);

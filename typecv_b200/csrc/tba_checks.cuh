@@ -33,4 +33,26 @@ struct CheckParams {
 // Enqueues the checks on `s` (memsets included).
 cudaError_t launch_checks(const CheckParams& p, int sms, cudaStream_t s);
 
+// The same checks over a batch, whose only answer is whether all passed (the host's checks then find the
+// message): a list of (problem, block of that problem).
+struct CheckProblem {
+  uint32_t C, P, M, blocks;
+  const uint32_t* index;
+  const double* scene;
+  uint32_t* claims;  // M words, zero
+};
+void launch_check_batch(const CheckProblem* problems, const uint2* work, uint32_t blocks, uint32_t* bad, cudaStream_t s);
+
+// The checks of an observation evaluation's arrays: camera and point of every observation, the tracks'
+// offsets (with `offsets`), and the values' bounds.
+struct ObservationChecks {
+  uint32_t C, P, M;
+  const uint32_t* indices;
+  const uint32_t* offsets;  // or null
+  const double* values[3];  // cameras, points, pixels
+  uint64_t counts[3];
+  uint32_t* bad;            // zero before the launch
+};
+void launch_check_observations(const ObservationChecks& p, int sms, cudaStream_t s);
+
 }  // namespace tba
