@@ -3,10 +3,13 @@
 // failure a serial scan in the same order would meet first.
 #include "tba_checks.cuh"
 
+#include "tba_launch.cuh"
+
 namespace tba {
 namespace {
 
 __global__ void __launch_bounds__(256) k_check_points(CheckParams A) {
+  after_previous();
   const uint32_t* ps = A.index + 2 * size_t(A.M);
   const uint32_t* obs_point = A.index + A.M;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < A.P; p += gridDim.x * blockDim.x) {
@@ -28,6 +31,7 @@ __global__ void __launch_bounds__(256) k_check_points(CheckParams A) {
 }
 
 __global__ void __launch_bounds__(256) k_check_cameras(CheckParams A) {
+  after_previous();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < A.M; i += gridDim.x * blockDim.x)
     if (A.index[i] >= A.C) atomicMin(A.keys + CK_CAMERA, (unsigned long long)i);
 }
@@ -35,6 +39,7 @@ __global__ void __launch_bounds__(256) k_check_cameras(CheckParams A) {
 // One block per camera (grid-stride): every entry of the camera's list must be an observation of
 // that camera, claimed once.  The camera offsets were checked on the host (monotone, within M).
 __global__ void __launch_bounds__(256) k_check_lists(CheckParams A) {
+  after_previous();
   const uint32_t* obs_camera = A.index;
   const uint32_t* cs = A.index + 2 * size_t(A.M) + A.P + 1;
   const uint32_t* cam_obs = cs + A.C + 1;
@@ -50,6 +55,7 @@ __global__ void __launch_bounds__(256) k_check_lists(CheckParams A) {
 
 __global__ void __launch_bounds__(256) k_check_scene(const double* x, uint64_t n, uint64_t base,
                                                       unsigned long long* keys) {
+  after_previous();
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
     const double v = x[i];
     if (!isfinite(v) || fabs(v) > 1e9 || (v != 0 && fabs(v) < 1e-30))
@@ -127,17 +133,17 @@ cudaError_t launch_checks(const CheckParams& p, int sms, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(p.keys, 0xff, CK_WORDS * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
   const uint32_t grid = uint32_t(sms > 0 ? sms : 1) * 8;
-  if (p.P) k_check_points<<<grid, 256, 0, s>>>(p);
-  if (p.M) k_check_cameras<<<grid, 256, 0, s>>>(p);
+  if (p.P) launch_dependent(k_check_points, grid, 256, 0, s, p);
+  if (p.M) launch_dependent(k_check_cameras, grid, 256, 0, s, p);
   if (p.lists && p.C) {
     if (p.M) {
       e = cudaMemsetAsync(p.claims, 0, sizeof(uint32_t) * p.M, s);
       if (e != cudaSuccess) return e;
     }
-    k_check_lists<<<p.C < 4u * uint32_t(sms) ? p.C : 4u * uint32_t(sms), 256, 0, s>>>(p);
+    launch_dependent(k_check_lists, p.C < 4u * uint32_t(sms) ? p.C : 4u * uint32_t(sms), 256, 0, s, p);
   }
   for (int k = 0; k < 4; k++)
-    if (p.len[k]) k_check_scene<<<grid, 256, 0, s>>>(p.seg[k], p.len[k], p.base[k], p.keys);
+    if (p.len[k]) launch_dependent(k_check_scene, grid, 256, 0, s, p.seg[k], p.len[k], p.base[k], p.keys);
   return cudaGetLastError();
 }
 

@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "tba_engine.cuh"
+#include "tba_launch.cuh"
 #include "tba_warp.cuh"
 
 // Compile-time tuning: occupancy floors of __launch_bounds__ for the heavy kernels.
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(256) k_unpack(Many w) {
 
 template <class W>
 __global__ void k_initialize(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -163,6 +165,7 @@ __global__ void k_initialize(W w) {
 // Per-camera radial limits; the camera-major copies of each observation's point and pixel.
 template <class W>
 __global__ void k_setup(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -179,6 +182,7 @@ __global__ void k_setup(W w) {
 
 template <class W>
 __global__ void __launch_bounds__(kPointThreads) k_cost(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -202,6 +206,7 @@ __global__ void __launch_bounds__(kPointThreads) k_cost(W w) {
 
 template <class W>
 __global__ void k_finish_metrics(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -391,6 +396,7 @@ __device__ inline void point_finish(const Params& P, uint32_t pt, const double (
 
 template <bool SHARED, bool EXPLICIT, class W>
 __global__ void __launch_bounds__(kPointThreads, TBA_POINT_MIN_BLOCKS) k_point_pass(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -478,6 +484,7 @@ __device__ inline void camera_rows(const Geo& g, bool dir, double jc[2][6]) {
 
 template <bool EXPLICIT, class W>
 __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camera_pass(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -584,6 +591,7 @@ constexpr int kFinishThreads = 128;
 
 template <bool EXPLICIT, class W>
 __global__ void __launch_bounds__(kFinishThreads) k_camera_finish(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -1596,6 +1604,7 @@ __global__ void __launch_bounds__(kUpdateThreads) k_refine(Params P) {
 
 template <class W>
 __global__ void __launch_bounds__(256) k_update_cameras(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -1770,6 +1779,7 @@ __device__ inline void record_wt(const double* rec, const double* x, double t[3]
 
 template <bool SHARED, bool EXPLICIT, class W>
 __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_points(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -1844,6 +1854,7 @@ __global__ void __launch_bounds__(kPointThreads, TBA_SCHUR_MIN_BLOCKS) k_update_
 // (the others have read it by then).  An iteration past the end of a solve changes nothing.
 template <class W>
 __global__ void __launch_bounds__(256) k_accept(W w) {
+  after_previous();
   __shared__ Slot<W> slot;
   uint32_t bid;
   const Params& P = block_problem(w, slot, bid);
@@ -2012,16 +2023,18 @@ int product_blocks_per_sm(const Params& p) {
 }
 
 void launch_initialize(const Params& p, cudaStream_t s) {
-  k_initialize<<<1, 1, 0, s>>>(p);
+  launch_dependent(k_initialize<Params>, 1, 1, 0, s, p);
   const uint32_t n = p.M > p.C ? p.M : p.C;
-  k_setup<<<(n + 255) / 256, 256, 0, s>>>(p);
+  launch_dependent(k_setup<Params>, (n + 255) / 256, 256, 0, s, p);
 }
-void launch_cost(const Params& p, cudaStream_t s) { k_cost<<<p.task_blocks, kPointThreads, 0, s>>>(p); }
-void launch_finish_metrics(const Params& p, cudaStream_t s) { k_finish_metrics<<<1, 1024, 0, s>>>(p); }
+void launch_cost(const Params& p, cudaStream_t s) { launch_dependent(k_cost<Params>, p.task_blocks, kPointThreads, 0, s, p); }
+void launch_finish_metrics(const Params& p, cudaStream_t s) {
+  launch_dependent(k_finish_metrics<Params>, 1, 1024, 0, s, p);
+}
 void launch_point_pass(const Params& p, cudaStream_t s) {
   if (p.schur) {
-    if (p.shared) k_point_pass<true, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
-    else k_point_pass<false, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    if (p.shared) launch_dependent(k_point_pass<true, true, Params>, p.task_blocks, kPointThreads, 0, s, p);
+    else launch_dependent(k_point_pass<false, true, Params>, p.task_blocks, kPointThreads, 0, s, p);
   } else if (p.shared) {
     k_point_pass<true, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   } else {
@@ -2029,12 +2042,12 @@ void launch_point_pass(const Params& p, cudaStream_t s) {
   }
 }
 void launch_camera_pass(const Params& p, cudaStream_t s) {
-  if (p.schur) k_camera_pass<true, Params><<<p.nchunks, kCameraThreads, 0, s>>>(p);
+  if (p.schur) launch_dependent(k_camera_pass<true, Params>, p.nchunks, kCameraThreads, 0, s, p);
   else k_camera_pass<false, Params><<<p.nchunks, kCameraThreads, 0, s>>>(p);
 }
 void launch_camera_finish(const Params& p, cudaStream_t s) {
   constexpr uint32_t per = kFinishThreads / 32;
-  if (p.schur) k_camera_finish<true, Params><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
+  if (p.schur) launch_dependent(k_camera_finish<true, Params>, (p.C + per - 1) / per, kFinishThreads, 0, s, p);
   else k_camera_finish<false, Params><<<(p.C + per - 1) / per, kFinishThreads, 0, s>>>(p);
 }
 void launch_pcg_init(const Params& p, cudaStream_t s) { k_pcg_init<<<1, 1024, 0, s>>>(p); }
@@ -2096,18 +2109,24 @@ void launch_refine(const Params& p, cudaStream_t s) {
 void launch_product_rows(const Params& p, double* out, cudaStream_t s) {
   k_product_rows<<<(p.m + 255) / 256, 256, 0, s>>>(p, p.factored ? 1 : 0, out);
 }
-void launch_update_cameras(const Params& p, cudaStream_t s) { k_update_cameras<<<1, 256, 0, s>>>(p); }
+void launch_update_cameras(const Params& p, cudaStream_t s) {
+  if (p.schur) launch_dependent(k_update_cameras<Params>, 1, 256, 0, s, p);
+  else k_update_cameras<<<1, 256, 0, s>>>(p);
+}
 void launch_update_points(const Params& p, cudaStream_t s) {
   if (p.schur) {
-    if (p.shared) k_update_points<true, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
-    else k_update_points<false, true, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
+    if (p.shared) launch_dependent(k_update_points<true, true, Params>, p.task_blocks, kPointThreads, 0, s, p);
+    else launch_dependent(k_update_points<false, true, Params>, p.task_blocks, kPointThreads, 0, s, p);
   } else if (p.shared) {
     k_update_points<true, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   } else {
     k_update_points<false, false, Params><<<p.task_blocks, kPointThreads, 0, s>>>(p);
   }
 }
-void launch_accept(const Params& p, cudaStream_t s) { k_accept<<<p.commit_blocks, 256, 0, s>>>(p); }
+void launch_accept(const Params& p, cudaStream_t s) {
+  if (p.schur) launch_dependent(k_accept<Params>, p.commit_blocks, 256, 0, s, p);
+  else k_accept<<<p.commit_blocks, 256, 0, s>>>(p);
+}
 // The kernels of one LM iteration up to the PCG, and after it, over a batch's lists of blocks.
 uint32_t launch_many_begin(const ManyLists& b, cudaStream_t s) {
   k_unpack<<<b.setup.blocks, 256, 0, s>>>(b.setup.of(b));

@@ -1,13 +1,16 @@
-// Launches of the LM iteration's kernels, each before the kernel ahead of it in the stream has ended.
+// Launches of a solve's kernels, each before the kernel ahead of it in the stream has ended.
 //
 // An iteration of the explicit system is ten short kernels, each of which needs all of the one before.
 // Launched the ordinary way a kernel's blocks are set up once the last block of the kernel before is gone,
-// about 1.5 us of an idle device per kernel.  Launched with launch_dependent they are set up as soon as the
+// about 2 us of an idle device per kernel.  Launched with launch_dependent they are set up as soon as the
 // kernel before has started all of its own, take room that it leaves free, and wait in after_previous() for
-// its end and its writes.
+// its end and its writes: six iterations on a 7-camera window 880 -> 770 us.  (The batch's
+// kernels are nodes of a graph, where it gained nothing: 24 windows 3.35 ms either way.)
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <cstdint>
 
 namespace tba {
 

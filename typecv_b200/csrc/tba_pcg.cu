@@ -16,6 +16,7 @@
 
 #include <algorithm>
 
+#include "tba_launch.cuh"
 #include "tba_pcg.cuh"
 #include "tba_warp.cuh"
 
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(256) k_pcg_plan(W w) {
 
 template <bool SHARED, class W>
 __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
+  after_previous();
   extern __shared__ __align__(16) double pcg_smem[];
   __shared__ Shared sh;
   __shared__ PcgSlot<W> slot;
@@ -520,16 +522,15 @@ uint32_t pcg_launch_plan(const PcgSystem& a, uint32_t grid, cudaStream_t s) {
 }
 
 cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaStream_t s) {
-  const void* f = a.shared ? reinterpret_cast<const void*>(k_pcg<true, PcgSystem>)
-                           : reinterpret_cast<const void*>(k_pcg<false, PcgSystem>);
-  PcgSystem q = a;
-  void* args[] = {&q, &limit};
-  if (grid == 1) return cudaLaunchKernel(f, dim3(1), dim3(kThreads), args, kSmemBytes, s);
+  const auto f = a.shared ? k_pcg<true, PcgSystem> : k_pcg<false, PcgSystem>;
+  if (grid == 1) return launch_dependent(f, 1, kThreads, kSmemBytes, s, a, limit);
   // No step of an earlier run may be taken for one of this run's.
   cudaError_t e = cudaMemsetAsync(a.zx, 0, 6 * size_t(a.C) * sizeof(Flagged), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(a.slots, 0, 4 * size_t(grid) * sizeof(Flagged), s);
   if (e != cudaSuccess) return e;
-  return cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kThreads), args, kSmemBytes, s);
+  PcgSystem q = a;
+  void* args[] = {&q, &limit};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(f), dim3(grid), dim3(kThreads), args, kSmemBytes, s);
 }
 
 uint32_t pcg_launch_many_plan(const PcgMany& b, uint32_t count, uint32_t max_cameras, cudaStream_t s) {
@@ -538,10 +539,9 @@ uint32_t pcg_launch_many_plan(const PcgMany& b, uint32_t count, uint32_t max_cam
 }
 
 cudaError_t launch_many_pcg(const PcgMany& b, uint32_t count, bool shared, uint32_t limit, cudaStream_t s) {
-  const void* f = shared ? reinterpret_cast<const void*>(k_pcg<true, PcgMany>) : reinterpret_cast<const void*>(k_pcg<false, PcgMany>);
-  PcgMany q = b;
-  void* args[] = {&q, &limit};
-  return cudaLaunchKernel(f, dim3(count), dim3(kThreads), args, kSmemBytes, s);
+  const auto f = shared ? k_pcg<true, PcgMany> : k_pcg<false, PcgMany>;
+  f<<<count, kThreads, kSmemBytes, s>>>(b, limit);
+  return cudaGetLastError();
 }
 
 }  // namespace tba

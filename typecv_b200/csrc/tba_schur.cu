@@ -11,6 +11,7 @@
 //   k_block_ends    camera pairs that cross segments: their partial sums in segment order
 #include <cuda_runtime.h>
 
+#include "tba_launch.cuh"
 #include "tba_schur.cuh"
 #include "tba_warp.cuh"
 
@@ -56,6 +57,7 @@ __device__ inline void row_pairs(const SchurParams& Q, uint32_t k, uint32_t c, F
 
 template <class W>
 __global__ void __launch_bounds__(kPairThreads) k_pairs_count(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -80,6 +82,7 @@ __device__ inline uint32_t row_count(const SchurParams& Q, uint32_t c, uint32_t 
 
 template <class W>
 __global__ void __launch_bounds__(kPairThreads) k_pairs_rows(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -144,6 +147,7 @@ __device__ inline void block_scan(uint32_t (&v)[N], uint32_t (&total)[N], uint32
 
 template <class W>
 __global__ void __launch_bounds__(1024) k_pairs_scan(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(1024) k_pairs_scan(W w) {
 
 template <class W>
 __global__ void __launch_bounds__(kPairThreads) k_pairs_place(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -224,6 +229,7 @@ __device__ inline uint32_t block_of(const SchurParams& Q, uint32_t c, uint32_t d
 
 template <class W>
 __global__ void __launch_bounds__(kPairThreads) k_pairs_blocks(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -237,6 +243,7 @@ __global__ void __launch_bounds__(kPairThreads) k_pairs_blocks(W w) {
 
 template <class W>
 __global__ void __launch_bounds__(kPairThreads) k_pairs_fill(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -279,6 +286,7 @@ __device__ inline void store_entry(const SchurParams& Q, uint32_t b, uint32_t r,
 // segment's pairs come 32 at a time, one a lane, so that a record's loads wait for one load only.
 template <class W>
 __global__ void __launch_bounds__(256) k_block_sums(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -300,7 +308,7 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
   double d0 = 0, d1 = 0;
   for (uint32_t base = lo; base < hi; base += 32) {
     const uint32_t n = min(32u, hi - base);
-    const uint2 mine = uint32_t(lane) < n ? __ldg(Q.pairs + base + lane) : make_uint2(0, 0);
+    const uint2 mine = uint32_t(lane) < n ? Q.pairs[base + lane] : make_uint2(0, 0);
     for (uint32_t p = base; p < base + n;) {
       const uint32_t e = min(stop, base + n);
 #pragma unroll 4
@@ -312,8 +320,8 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
           const uint32_t i = __shfl_sync(kFull, mine.x, k - base), j = __shfl_sync(kFull, mine.y, k - base);
           a[t] = c[t] = 0;
           if (r < 6 && k < e) {
-            a[t] = __ldg(Q.A + 18 * size_t(i) + word[t]);
-            c[t] = __ldg(Q.A + 18 * size_t(j) + word[t]);
+            a[t] = Q.A[18 * size_t(i) + word[t]];
+            c[t] = Q.A[18 * size_t(j) + word[t]];
           }
         }
 #pragma unroll
@@ -342,6 +350,7 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
 
 template <class W>
 __global__ void __launch_bounds__(256) k_block_ends(W w) {
+  after_previous();
   __shared__ SchurSlot<W> slot;
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
@@ -350,12 +359,20 @@ __global__ void __launch_bounds__(256) k_block_ends(W w) {
   if (b >= Q.totals[0]) return;
   const uint32_t begin = Q.blk_begin[b], end = Q.blk_begin[b + 1], s0 = begin / Q.seg, s1 = (end - 1) / Q.seg;
   if (s0 == s1) return;
-  for (uint32_t e = threadIdx.x & 31; e < 36; e += 32) {
-    double v = Q.part[36 * (2 * size_t(s0) + 1) + e];
-#pragma unroll 8
-    for (uint32_t s = s0 + 1; s <= s1; s++) v += __ldg(Q.part + 36 * 2 * size_t(s) + e);
-    store_entry(Q, b, e / 6, e % 6, v);
+  // An entry a lane, and the last four with the first lanes' (together: their loads wait once).
+  const uint32_t e = threadIdx.x & 31;
+  const double* part = Q.part + 36 * (2 * size_t(s0) + 1) + e;
+  const bool two = e < 4;
+  double v = part[0], u = two ? part[32] : 0.0;
+  part -= 36;
+#pragma unroll 4
+  for (uint32_t s = s0 + 1; s <= s1; s++) {
+    part += 72;
+    v += part[0];
+    if (two) u += part[32];
   }
+  store_entry(Q, b, e / 6, e % 6, v);
+  if (two) store_entry(Q, b, 5, e + 2, u);
 }
 
 }  // namespace
@@ -363,20 +380,20 @@ __global__ void __launch_bounds__(256) k_block_ends(W w) {
 uint32_t schur_launch_structure(const SchurParams& q, cudaStream_t s) {
   const size_t smem = size_t(q.C) * sizeof(uint32_t);
   cudaMemsetAsync(q.bits, 0, size_t(q.C) * q.bwords * sizeof(uint32_t), s);
-  k_pairs_count<<<q.nchunks, kPairThreads, smem, s>>>(q);
-  k_pairs_rows<<<q.C, kPairThreads, 0, s>>>(q);
-  k_pairs_scan<<<1, 1024, 0, s>>>(q);
-  k_pairs_place<<<q.C, kPairThreads, 0, s>>>(q);
-  if (q.max_blocks) k_pairs_blocks<<<(q.max_blocks + kPairThreads - 1) / kPairThreads, kPairThreads, 0, s>>>(q);
-  k_pairs_fill<<<q.nchunks, kPairThreads, smem, s>>>(q);
+  launch_dependent(k_pairs_count<SchurParams>, q.nchunks, kPairThreads, smem, s, q);
+  launch_dependent(k_pairs_rows<SchurParams>, q.C, kPairThreads, 0, s, q);
+  launch_dependent(k_pairs_scan<SchurParams>, 1, 1024, 0, s, q);
+  launch_dependent(k_pairs_place<SchurParams>, q.C, kPairThreads, 0, s, q);
+  if (q.max_blocks) launch_dependent(k_pairs_blocks<SchurParams>, (q.max_blocks + kPairThreads - 1) / kPairThreads, kPairThreads, 0, s, q);
+  launch_dependent(k_pairs_fill<SchurParams>, q.nchunks, kPairThreads, smem, s, q);
   return q.max_blocks ? 6 : 5;
 }
 
 uint32_t schur_launch_values(const SchurParams& q, cudaStream_t s) {
   if (!q.max_pairs) return 0;
   const uint32_t segs = (q.max_pairs + q.seg - 1) / q.seg;
-  k_block_sums<<<(segs + 7) / 8, 256, 0, s>>>(q);
-  k_block_ends<<<(q.max_blocks + 7) / 8, 256, 0, s>>>(q);
+  launch_dependent(k_block_sums<SchurParams>, (segs + 7) / 8, 256, 0, s, q);
+  launch_dependent(k_block_ends<SchurParams>, (q.max_blocks + 7) / 8, 256, 0, s, q);
   return 2;
 }
 
