@@ -1307,7 +1307,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   for (uint32_t k = 0; k < count; k++) tasks_total += plans[k].tasks.size() - 1;
   // Tasks per warp of the task kernels: a few waves of blocks over the batch, up to eight.
   const uint32_t per_warp = uint32_t(std::min<uint64_t>(8, std::max<uint64_t>(1, tasks_total / (8 * 8 * uint64_t(d->sms)))));
-  std::vector<uint2> lists[12];  // one, task, chunk, finish, setup, commit, pack | camera, pairs, ends, sums
+  std::vector<uint2> lists[10];  // one, task, chunk, finish, setup, commit, pack | camera, pairs, sums
   std::vector<SchurLayout> systems;
   systems.reserve(count);
   uint32_t Cmax = 2;
@@ -1338,7 +1338,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
     const tba_batch_problem& q = probs[k];
     const SchurLayout& y = systems[k];
     const uint32_t C = q.cameras, P = q.points, M = q.observations;
-    const uint64_t n[11] = {1,
+    const uint64_t n[10] = {1,
                             task_blocks(k),
                             plans[k].chunks.cam.size(),
                             (C + 3) / 4,
@@ -1347,14 +1347,13 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
                             (12 * uint64_t(C) + 3 * uint64_t(P) + 27 + 255) / 256,
                             C,
                             (y.camera_pairs + 255) / 256,
-                            (y.camera_pairs + 7) / 8,
                             ((y.npairs + y.seg - 1) / y.seg + 7) / 8};
-    for (int j = 0; j < 11; j++)
+    for (int j = 0; j < 10; j++)
       for (uint32_t b = 0; b < n[j]; b++) lists[j].push_back(make_uint2(k, b));
   }
   const size_t o_flat = L.take<uint32_t>(flat.size());
-  size_t o_list[11];
-  for (int j = 0; j < 11; j++) o_list[j] = L.take<uint2>(lists[j].size());
+  size_t o_list[10];
+  for (int j = 0; j < 10; j++) o_list[j] = L.take<uint2>(lists[j].size());
   const size_t o_params = L.take<tba::Params>(count), o_schur = L.take<tba::SchurParams>(count),
                o_pcg = L.take<tba::PcgSystem>(count), o_active = L.take<uint32_t>(1);
   // The bit matrices together (zeroed at once), then each problem's workspace.
@@ -1501,7 +1500,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   up(o_scene, scene, scene_len * sizeof(double));
   up(o_index, index, index_len * sizeof(uint32_t));
   up(o_flat, flat.data(), flat.size() * sizeof(uint32_t));
-  for (int j = 0; j < 11; j++) up(o_list[j], lists[j].data(), lists[j].size() * sizeof(uint2));
+  for (int j = 0; j < 10; j++) up(o_list[j], lists[j].data(), lists[j].size() * sizeof(uint2));
   up(o_params, params.data(), count * sizeof(tba::Params));
   up(o_schur, schur.data(), count * sizeof(tba::SchurParams));
   up(o_pcg, pcg.data(), count * sizeof(tba::PcgSystem));
@@ -1560,8 +1559,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   list(key.schur.chunk, 2);
   list(key.schur.camera, 7);
   list(key.schur.pairs, 8);
-  list(key.schur.ends, 9);
-  list(key.schur.sums, 10);
+  list(key.schur.sums, 9);
   key.pcg.systems = reinterpret_cast<const tba::PcgSystem*>(a + o_pcg);
   key.pcg.work = key.many.one.work;
   key.count = count;

@@ -305,10 +305,12 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
     word[t] = uint32_t(4 * t + q) % 3 * 6 + r;
   }
   uint32_t b = Q.seg_block[s], begin = Q.blk_begin[b], stop = Q.blk_begin[b + 1];
+  const double* const A = Q.A;
+  const uint2* const pairs = Q.pairs;
   double d0 = 0, d1 = 0;
   for (uint32_t base = lo; base < hi; base += 32) {
     const uint32_t n = min(32u, hi - base);
-    const uint2 mine = uint32_t(lane) < n ? Q.pairs[base + lane] : make_uint2(0, 0);
+    const uint2 mine = uint32_t(lane) < n ? pairs[base + lane] : make_uint2(0, 0);
     for (uint32_t p = base; p < base + n;) {
       const uint32_t e = min(stop, base + n);
 #pragma unroll 4
@@ -320,8 +322,8 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
           const uint32_t i = __shfl_sync(kFull, mine.x, k - base), j = __shfl_sync(kFull, mine.y, k - base);
           a[t] = c[t] = 0;
           if (r < 6 && k < e) {
-            a[t] = Q.A[18 * size_t(i) + word[t]];
-            c[t] = Q.A[18 * size_t(j) + word[t]];
+            a[t] = A[18 * size_t(i) + word[t]];
+            c[t] = A[18 * size_t(j) + word[t]];
           }
         }
 #pragma unroll
@@ -355,10 +357,12 @@ __global__ void __launch_bounds__(256) k_block_ends(W w) {
   uint32_t bid;
   const SchurParams& Q = block_problem(w, slot, bid);
   if (Q.go && *Q.go == 0) return;
-  const uint32_t b = bid * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (b >= Q.totals[0]) return;
-  const uint32_t begin = Q.blk_begin[b], end = Q.blk_begin[b + 1], s0 = begin / Q.seg, s1 = (end - 1) / Q.seg;
-  if (s0 == s1) return;
+  const uint32_t s = bid * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint64_t lo = uint64_t(s) * Q.seg;
+  if (s == 0 || lo >= Q.totals[1]) return;
+  const uint32_t b = Q.seg_block[s], begin = Q.blk_begin[b], end = Q.blk_begin[b + 1];
+  const uint32_t s0 = begin / Q.seg, s1 = (end - 1) / Q.seg;
+  if (begin >= lo || s0 != s - 1) return;
   // An entry a lane, and the last four with the first lanes' (together: their loads wait once).
   const uint32_t e = threadIdx.x & 31;
   const double* part = Q.part + 36 * (2 * size_t(s0) + 1) + e;
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(256) k_block_ends(W w) {
   double v = part[0], u = two ? part[32] : 0.0;
   part -= 36;
 #pragma unroll 4
-  for (uint32_t s = s0 + 1; s <= s1; s++) {
+  for (uint32_t k = s0 + 1; k <= s1; k++) {
     part += 72;
     v += part[0];
     if (two) u += part[32];
@@ -393,7 +397,7 @@ uint32_t schur_launch_values(const SchurParams& q, cudaStream_t s) {
   if (!q.max_pairs) return 0;
   const uint32_t segs = (q.max_pairs + q.seg - 1) / q.seg;
   launch_dependent(k_block_sums<SchurParams>, (segs + 7) / 8, 256, 0, s, q);
-  launch_dependent(k_block_ends<SchurParams>, (q.max_blocks + 7) / 8, 256, 0, s, q);
+  launch_dependent(k_block_ends<SchurParams>, (segs + 7) / 8, 256, 0, s, q);
   return 2;
 }
 
@@ -410,7 +414,7 @@ uint32_t schur_launch_many_structure(const SchurLists& b, cudaStream_t s) {
 
 uint32_t schur_launch_many_values(const SchurLists& b, cudaStream_t s) {
   k_block_sums<SchurMany><<<b.sums.blocks, 256, 0, s>>>(b.sums.of(b));
-  k_block_ends<SchurMany><<<b.ends.blocks, 256, 0, s>>>(b.ends.of(b));
+  k_block_ends<SchurMany><<<b.sums.blocks, 256, 0, s>>>(b.sums.of(b));
   return 2;
 }
 

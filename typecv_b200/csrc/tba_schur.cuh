@@ -70,8 +70,8 @@ struct SchurLists {
     uint32_t blocks;
     SchurMany of(const SchurLists& b) const { return SchurMany{b.params, work}; }
   };
-  // A block per: problem; camera chunk; camera; 256 camera pairs; eight camera pairs; eight segments.
-  List one, chunk, camera, pairs, ends, sums;
+  // A block per: problem; camera chunk; camera; 256 camera pairs; eight segments.
+  List one, chunk, camera, pairs, sums;
 };
 uint32_t schur_launch_many_structure(const SchurLists& b, cudaStream_t s);  // (bits zeroed by the caller)
 uint32_t schur_launch_many_values(const SchurLists& b, cudaStream_t s);
