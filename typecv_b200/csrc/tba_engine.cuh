@@ -111,7 +111,7 @@ struct Params {
   double* rlim;        // C radial limits
   uint32_t* cm_point;  // M, camera-major
   double* cm_pixel;    // 2M, camera-major
-  double* pblk;        // 12P: V^-1 (6), b_p (3), padding; explicit system: N (6), b_p (3), g_p (3)
+  double* pblk;        // 12P: V^-1 (6), b_p (3), padding; explicit system: N (6), (N^T b_p, N^T g_p) a column
   float* pblk32;       // 6P: V^-1 in FP32 for the FP32 product (mixed form), or null
   double* y;           // 4P: y_p of the current Schur product
   double* chunk_prod;  // 8 per camera chunk: sum W_i y (6), focal share
