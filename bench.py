@@ -98,6 +98,23 @@ def product_bytes(scene, shared, prod_blocks, factor_bytes=8):
             + 2 * factor_bytes * m * prod_blocks)
 
 
+def system_bytes(scene):
+    """Algorithmic bytes of one launch of k_schur_rows, S p on the explicit reduced camera system: a 6x6
+    block and its camera for every ordered pair of variable cameras that share a point (and every
+    camera's own), and the vectors p, S p and the focal column."""
+    import numpy as np
+    cov = np.zeros((scene.C, scene.C), dtype=bool)
+    for k in range(1, scene.M):
+        same = scene.obs_point[k:] == scene.obs_point[:-k]
+        if not same.any():
+            break
+        cov[scene.obs_camera[:-k][same], scene.obs_camera[k:][same]] = True
+    cov |= cov.T
+    np.fill_diagonal(cov, True)
+    cov[scene.anchor] = cov[:, scene.anchor] = False
+    return int(cov.sum()) * (36 * 8 + 4) + 3 * 8 * 6 * scene.C
+
+
 def two_pass_bytes(scene, shared):
     """The two-pass Schur product's algorithmic bytes (W read twice, y written and read)."""
     s = 8
@@ -440,6 +457,14 @@ def roofline(scene, reports, precision):
     prod_ms = sum(r["product_ms"] for r in reports)
     prod_n = sum(r["product_launches"] for r in reports)
     blocks = reports[-1].get("product_blocks", 0) or 1
+    if reports[-1].get("engine") == 2:  # the product is a pass over the explicit reduced system
+        nbytes = system_bytes(scene)
+        t_launch = prod_ms / max(prod_n, 1) / 1000
+        achieved = nbytes / t_launch / 1e9 if prod_n else None
+        return {"bound": "hbm", "kernel": "k_schur_rows (S p on the explicit reduced camera system, launched step by step)",
+                "achieved": achieved, "peak": pk["hbm_gbs"], "peak_kind": pk_kind, "unit": "GB/s",
+                "frac": achieved / pk["hbm_gbs"] if achieved else None, "traffic": None, "algorithmic_bytes": nbytes,
+                "launch_ms": 1000 * t_launch, "launches": prod_n, "product_blocks": 0}
     bytes_launch = product_bytes(scene, True, blocks, 4 if precision == "mixed" else 8)
     t_launch = prod_ms / max(prod_n, 1) / 1000
     achieved = bytes_launch / t_launch / 1e9 if prod_n else None

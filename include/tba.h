@@ -51,15 +51,17 @@ typedef enum {
  * product over the FP64 factors); when that residual is above the tolerance the PCG restarts from
  * it on the FP32 product, at most twice, and then finishes on the FP64 product, each restart with
  * an iteration budget of its own.  Once an LM iteration needed that FP64 finish, the call's later
- * iterations solve on the FP64 product alone (tba_report.fp64_iterations).  It has no reference
- * counterpart. */
+ * iterations solve on the FP64 product alone (tba_report.fp64_iterations).  Where the reduced
+ * camera system is formed explicitly (tba_report.engine 2) there is no product over factors to hold
+ * in FP32, and a mixed request runs in FP64 throughout.  It has no reference counterpart. */
 typedef enum { TBA_PRECISION_FP64 = 0, TBA_PRECISION_MIXED = 1 } tba_precision;
 
 /* TBA_FLAG_TIME_PRODUCTS: bracket every Schur product with CUDA events and report their total
  * device time in tba_report.product_ms (a few microseconds of host work per PCG iteration).
- * Without it each PCG run is one launch of a CUDA graph that repeats the PCG step on the device
- * until the PCG stops (or, where the driver cannot build conditional graph nodes, from the host);
- * with it the host launches the steps in chunks, with the same results. */
+ * Without it each PCG run is one launch that ends on the device: a persistent kernel on the explicit
+ * reduced system, else a CUDA graph that repeats the PCG step until the PCG stops (or, where the
+ * driver cannot build conditional graph nodes, steps from the host); with it the host launches the
+ * steps in chunks, with the same results. */
 #define TBA_FLAG_TIME_PRODUCTS 1u
 /* TBA_FLAG_PRODUCT_ERROR: once, on the first PCG direction of the first LM iteration, evaluate S p
  * with the solve's own Schur product and with the FP64 two-pass product (Jacobians recomputed from
@@ -67,8 +69,8 @@ typedef enum { TBA_PRECISION_FP64 = 0, TBA_PRECISION_MIXED = 1 } tba_precision;
  * the mixed form: the FP32 product's error).  Diagnostics only: two more products per call. */
 #define TBA_FLAG_PRODUCT_ERROR 2u
 /* TBA_FLAG_HOST_PCG_LOOP: launch the PCG steps from the host in chunks, as with
- * TBA_FLAG_TIME_PRODUCTS but without the events, instead of the device-side graph loop (for
- * profilers and tools that do not follow the kernels of conditional graph nodes).  Same results. */
+ * TBA_FLAG_TIME_PRODUCTS but without the events, instead of the device-side loop (for profilers and
+ * tools that do not follow the kernels of conditional graph nodes).  Same results. */
 #define TBA_FLAG_HOST_PCG_LOOP 4u
 
 /*
@@ -110,8 +112,9 @@ typedef struct {
   uint32_t product_launches; /* Schur products timed in product_ms */
   uint32_t engine;         /* 0: grid engine, one-pass product over stored factors;
                               1: grid engine, two-pass recompute product (camera systems beyond
-                                 on-chip memory) */
-  uint32_t product_blocks; /* blocks of the one-pass product (each writes one partial row) */
+                                 on-chip memory);
+                              2: grid engine, the reduced camera system formed explicitly */
+  uint32_t product_blocks; /* blocks of the one-pass product (each writes one partial row); engine 2: 0 */
   uint32_t refinements;    /* mixed form: PCG restarts from the FP64 residual */
   uint32_t fp64_iterations; /* mixed form: LM iterations solved on the FP64 product alone, after an
                               earlier iteration of the call needed the FP64 tail */
@@ -218,8 +221,9 @@ tba_status tba_scene_cost_noalloc(const tba_control* control, const double* scen
                                   void* stream, char* message, size_t message_len);
 
 /*
- * Batched local-window bundle adjustment: many independent problems in one persistent launch
- * (captured in a CUDA graph and replayed while the batch keeps its shape).  No counterpart in the
+ * Batched local-window bundle adjustment: many independent problems side by side, every kernel of an
+ * LM iteration over all of them (the iteration captured in a CUDA graph and replayed while the batch
+ * keeps its shape), or one persistent launch whose blocks take whole problems.  No counterpart in the
  * reference, whose mapper runs one `bundleAdjustGpu` call per local window
  * (src/sfm/mapper/mapper.ts:859-925 over the windows of src/sfm/bundle/local-bundle.ts:17-208);
  * each problem here gets exactly the result record of tba_bundle_adjust on the same arrays and
@@ -241,8 +245,10 @@ typedef struct {
 } tba_batch_problem;
 
 /* Options shared by every problem of a batch (tba_control's meaning).  `schedule` picks the
- * launch shape: 0 lets the autotuner choose (timed trial launches the first time a batch shape is
- * seen on the handle, cached afterwards), k >= 1 forces shape k - 1 of tba_batch_shape. */
+ * launch shape: k >= 1 forces shape k - 1 of tba_batch_shape (the last is the kernels over all
+ * problems at once, which run in FP64); 0 takes that last shape where its memory fits and the tracks
+ * are no longer than about 64 observations, and else lets the autotuner choose among the persistent
+ * ones (timed trial launches the first time a batch shape is seen on the handle, cached afterwards). */
 typedef struct {
   uint32_t iterations;
   uint32_t max_cg;
@@ -256,7 +262,7 @@ typedef struct {
 } tba_batch_control;
 
 typedef struct {
-  double solve_ms;     /* device time of the persistent launch (CUDA events) */
+  double solve_ms;     /* device time of the solve (CUDA events) */
   double upload_ms;    /* device time of the host-to-device copies */
   double download_ms;  /* device time of the device-to-host copy */
   double wall_ms;      /* host wall time of the call */
@@ -268,11 +274,11 @@ typedef struct {
   uint32_t problems;
   uint32_t schedule;      /* the launch shape used (0-based) */
   uint32_t threads;       /* threads per block of that shape */
-  uint32_t blocks;        /* persistent blocks launched */
+  uint32_t blocks;        /* persistent blocks launched; the last shape: blocks of its point kernels */
   uint32_t graph_replayed; /* 1: the launch replayed a cached CUDA graph */
   uint32_t kernel_launches;
-  uint32_t form;           /* the tba_precision that ran: a mixed request runs the FP64 form when the
-                              autotuner (schedule 0) timed it faster for this batch shape */
+  uint32_t form;           /* the tba_precision that ran: a mixed request runs the FP64 form on the last
+                              shape, and when the autotuner (schedule 0) timed it faster */
 } tba_batch_report;
 
 /* The largest camera count of one batched problem, and the number of launch shapes. */
@@ -343,7 +349,8 @@ typedef struct {
                                    products that ran PCG steps (CUDA events), else 0 */
   uint32_t product_launches;    /* the products timed in product_ms */
   uint32_t product_blocks;      /* blocks of the one-pass product (each writes one partial row); 0:
-                                   the two-pass product (camera systems beyond shared memory) */
+                                   the explicit reduced system, or the two-pass product (camera systems
+                                   beyond shared memory) */
 } tba_vjp_report;
 
 /* TBA_VJP_FLAG_TIME_PRODUCTS: bracket every one-pass Schur product of the vjp's linear solves with

@@ -502,6 +502,7 @@ struct SchurLayout {
     q.part = f64(part);
     q.S = f64(S);
     a.S = q.S;
+    a.max_blocks = uint32_t(std::min<uint64_t>(schur_block_bound(C, npairs), UINT32_MAX));
     a.row_ptr = q.row_ptr;
     a.col = q.col;
     a.share = u32(share);

@@ -7,13 +7,16 @@
 //     cameraObservations, cameraActive), plus camera-major copies of each observation's point and
 //     pixel so that camera passes stream instead of gathering;
 //   * per point, a 12-word record: the inverse of the damped point block V_p (6, symmetric), its
-//     right-hand side b_p (3) and padding; and y_p = V_p^-1 W^T p of the current product (4);
+//     right-hand side b_p (3) and padding; and y_p = V_p^-1 W^T p of the current product (4).  With the
+//     explicit reduced system: N_p of V_p^-1 = N_p N_p^T (6), N_p^T b_p and N_p^T g_p (6);
 //   * per camera, the damped block U_c (21, lower triangle), the block-Jacobi preconditioner
 //     (S_cc)^-1 (36), the reduced right-hand side (6), the camera/focal coupling H_cf (6) and the
 //     radial limit of its lens model;
 //   * the PCG vectors x, r, p, Sp, z of length m = 6C (+1 with the shared focal);
 //   * the LM/PCG state words of the reference (bundle-shared.ts:362-386) plus the focal scalars.
-// Nothing per observation is stored beyond the inputs: the Jacobian factors are recomputed.
+// Per observation the point pass stores 12 Jacobian factors for the products or, with the explicit
+// reduced system (tba_schur.cuh), the 18 words of A_i = W_i N_p that the system is formed from; the
+// two-pass form stores nothing and recomputes.
 //
 // Work decomposition: observation-parallel "warp tasks" — runs of whole points of at most 32
 // observations, one observation per lane, reduced per point with warp-shuffle segmented scans;

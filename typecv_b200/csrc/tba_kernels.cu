@@ -6,9 +6,11 @@
 // k_cost/k_finish_metrics bundleMetricPartials + finishBundleMetrics (K3/K4)
 // k_point_pass            linearizeBundle + bundlePointBlocks + bundleFocalObservations +
 //                         bundleFocalPoints (K2/K5/K21)
-// k_camera_pass/_finish   bundleCameraRows + bundleFocalCameraRows + invertBundleCameraColumns +
-//                         finalizeBundleCameraInverse (K6/K8/K21)
-// k_pcg_init              dampBundleFocal + initializeBundleCg (K9/K21)
+// k_camera_pass/_finish,  bundleCameraRows + bundleFocalCameraRows + invertBundleCameraColumns +
+// k_camera_blocks         finalizeBundleCameraInverse (K6/K8/K21); _blocks for the explicit system
+// k_pcg_init              dampBundleFocal + initializeBundleCg (K9/K21); the persistent PCG of the
+//                         explicit system (tba_pcg.cu) does this itself
+// k_schur_rows            S p on the explicit reduced system, where the PCG's steps are launched one by one
 // k_product_f             bundleSchurPoint + bundleSchurCamera (K10/K11) in one pass over the
 //                         stored world-axis Jacobian factors, camera sums in shared memory
 // k_product_columns       the fixed-order sum of the product blocks' partial rows
@@ -24,10 +26,11 @@
 // k_accept                acceptBundleCandidate + commitBundleCandidate (K18/K19)
 // k_pack                  packBundleResult (K20)
 //
-// No kernel stores the Schur cross blocks W_i = w J_c^T J_p (21 words per observation).  The
-// point pass stores 12 world-axis Jacobian factors per observation instead (q~ = R^T q, R^T du,
-// R^T dv, w, jf; FP64, and an FP32 copy in the mixed form), from which every product is a few dozen FMAs;
-// the camera passes recompute the factors from the pose, the camera, the point and the pixel.
+// Where the reduced system is formed explicitly (EXPLICIT, Params.schur) the point pass stores the record
+// A_i = W_i N_p of each observation (18 words).  Elsewhere it stores 12 world-axis Jacobian factors
+// (q~ = R^T q, R^T du, R^T dv, w, jf; FP64, and an FP32 copy in the mixed form), from which every product is
+// a few dozen FMAs.  The camera passes recompute the Jacobians from the pose, the camera, the point and the
+// pixel.
 // Every reduction runs in a fixed order (fixed grids, fixed trees, fixed chunking), except the
 // shared-memory camera sums of k_product_f, whose FP64 atomic adds commute only up to rounding.
 #include <cuda_runtime.h>

@@ -207,7 +207,10 @@ __global__ void __launch_bounds__(256) k_pcg_plan(W w) {
   for (uint32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) A.local[k] = place[A.col[k]];
 }
 
-template <bool SHARED, class W>
+// WIDE: for systems whose shares lie in global memory, 16-byte loads of S with two rows a lane (25 -> 19 us a
+// step at 1,500 cameras, S in the L2).  From shared memory a row a lane is the faster one (a step at 7
+// cameras 2.6 and 3.2 us, at 61 cameras 6.2 and 7.3): its step is the instructions' latency, not the loads.
+template <bool SHARED, class W, bool WIDE = false>
 __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   after_previous();
   extern __shared__ __align__(16) double pcg_smem[];
@@ -246,12 +249,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
     for (uint32_t k = threadIdx.x; k <= nr; k += kThreads) words[k] = row_ptr[k];
     row_ptr = words;
   }
+  // A block of S takes 38 words in shared memory, so that a warp's reads of five blocks fall on different
+  // banks (36 where only they fit).
   const double* S = A.S + 36 * size_t(k0);
-  if (double* to = take(36 * size_t(blocks), nullptr)) {
+  const size_t rest = (size_t(blocks) + 1) / 2 + 36 * size_t(nr) + 4;  // the places and preconditioner blocks
+  const uint32_t stride = (used + 38 * size_t(blocks) + rest) * sizeof(double) <= kSmemBytes ? 38 : 36;
+  double* const staged = take(stride * size_t(blocks), nullptr);
+  if (staged) {
     const double2* from = reinterpret_cast<const double2*>(S);
-    for (uint32_t k = threadIdx.x; k < 18 * blocks; k += kThreads) reinterpret_cast<double2*>(to)[k] = from[k];
-    S = to;
+    for (uint32_t k = threadIdx.x; k < 18 * blocks; k += kThreads) {
+      const uint32_t b = k / 18;
+      reinterpret_cast<double2*>(staged)[stride / 2 * b + (k - 18 * b)] = from[k];
+    }
+    S = staged;
   }
+  const uint32_t block_words = staged ? stride : 36;
   const uint32_t* local = A.local + k0;
   if (double* to = take((size_t(blocks) + 1) / 2, nullptr)) {
     uint32_t* words = reinterpret_cast<uint32_t*>(to);
@@ -286,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   double rho = st[A.rho], beta = 0, r0 = st[A.r0], r2 = st[A.r2];
   double inner = A.inner_r0 >= 0 ? st[A.inner_r0] : 0.0;
   // A warp per camera row, or several warps on a row's blocks; a lane sums one of the six rows over every
-  // fifth block.  The first `owners` warps hold the own rows' scalars.
+  // fifth block (WIDE: two rows over every tenth).  The first `owners` warps hold the own rows' scalars.
   const uint32_t splits = nr == 0 || nr >= uint32_t(kWarps) ? 1 : kWarps / nr;
   const int owners = int(min(uint32_t(kWarps), (rows + 31) / 32));
   const uint32_t lane_row = lane % 6, lane_block = lane / 6;
@@ -399,22 +411,54 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
       const uint32_t row = splits == 1 ? item : item / splits, part = item - row * splits;
       const uint32_t b0 = row_ptr[row] - k0, nb = row_ptr[row + 1] - k0 - b0;
       const uint32_t lo = b0 + nb * part / splits, hi = b0 + nb * (part + 1) / splits;
-      double acc[3] = {0, 0, 0};  // independent sums: one chain of dependent FMAs a lane was half of a step
-      if (lane < 30) {
+      double* const out = splits == 1 ? ss + 6 * row : sh.part[item];
+      if constexpr (WIDE) {
+        double acc[2][2] = {{0, 0}, {0, 0}};
+        const uint32_t pair = 2 * (lane % 3);
+        if (lane < 30) {
 #pragma unroll 2
-        for (uint32_t b = lo + lane_block; b < hi; b += 5) {
-          const double* Sb = S + 36 * size_t(b) + lane_row;
-          const double* pb = pl + 6 * local[b];
+          for (uint32_t b = lo + lane / 3; b < hi; b += 10) {
+            const double2* Sb = reinterpret_cast<const double2*>(S + block_words * size_t(b) + pair);
+            const double2* pb = reinterpret_cast<const double2*>(pl + 6 * local[b]);
 #pragma unroll
-          for (int k = 0; k < 6; k++) acc[k % 3] += Sb[6 * k] * pb[k];
+            for (int k = 0; k < 3; k++) {
+              const double2 pv = pb[k], s0 = Sb[6 * k], s1 = Sb[6 * k + 3];
+              acc[0][0] += s0.x * pv.x;
+              acc[0][1] += s0.y * pv.x;
+              acc[1][0] += s1.x * pv.y;
+              acc[1][1] += s1.y * pv.y;
+            }
+          }
         }
-      }
-      acc[0] += acc[1] + acc[2];
-      const double far = __shfl_down_sync(kFull, acc[0], 24), near = __shfl_down_sync(kFull, acc[0], 6),
-                   mid = __shfl_down_sync(kFull, acc[0], 12), mid2 = __shfl_down_sync(kFull, acc[0], 18);
-      if (lane < 6) {
-        double* out = splits == 1 ? ss + 6 * row : sh.part[item];
-        out[lane] = (acc[0] + near) + (mid + mid2) + far;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          double a = acc[0][j] + acc[1][j];
+          a += __shfl_down_sync(kFull, a, 15);
+          const double b1 = __shfl_down_sync(kFull, a, 3), b2 = __shfl_down_sync(kFull, a, 6),
+                       b3 = __shfl_down_sync(kFull, a, 9), b4 = __shfl_down_sync(kFull, a, 12);
+          if (lane < 3) out[pair + j] = (a + b1) + (b2 + b3) + b4;
+        }
+      } else {
+        double acc[3] = {0, 0, 0};  // independent sums: one chain of dependent FMAs a lane was half of a step
+        if (lane < 30) {
+#pragma unroll 2
+          for (uint32_t b = lo + lane_block; b < hi; b += 5) {
+            const double* Sb = S + block_words * size_t(b) + lane_row;
+            const double2* pb = reinterpret_cast<const double2*>(pl + 6 * local[b]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+              const double2 pv = pb[k];
+              acc[2 * k % 3] += Sb[12 * k] * pv.x;
+              acc[(2 * k + 1) % 3] += Sb[12 * k + 6] * pv.y;
+            }
+          }
+        }
+        acc[0] += acc[1] + acc[2];
+        const double far = __shfl_down_sync(kFull, acc[0], 24), near = __shfl_down_sync(kFull, acc[0], 6),
+                     mid = __shfl_down_sync(kFull, acc[0], 12), mid2 = __shfl_down_sync(kFull, acc[0], 18);
+        if (lane < 6) {
+          out[lane] = (acc[0] + near) + (mid + mid2) + far;
+        }
       }
     }
     __syncthreads();
@@ -501,6 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
 cudaError_t pcg_configure() {
   const void* kernels[] = {
       reinterpret_cast<const void*>(k_pcg<false, PcgSystem>), reinterpret_cast<const void*>(k_pcg<true, PcgSystem>),
+      reinterpret_cast<const void*>(k_pcg<false, PcgSystem, true>), reinterpret_cast<const void*>(k_pcg<true, PcgSystem, true>),
       reinterpret_cast<const void*>(k_pcg<false, PcgMany>), reinterpret_cast<const void*>(k_pcg<true, PcgMany>)};
   for (const void* f : kernels) {
     const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes));
@@ -522,7 +567,10 @@ uint32_t pcg_launch_plan(const PcgSystem& a, uint32_t grid, cudaStream_t s) {
 }
 
 cudaError_t launch_pcg(const PcgSystem& a, uint32_t limit, uint32_t grid, cudaStream_t s) {
-  const auto f = a.shared ? k_pcg<true, PcgSystem> : k_pcg<false, PcgSystem>;
+  auto f = a.shared ? k_pcg<true, PcgSystem> : k_pcg<false, PcgSystem>;
+  // Where the shares cannot all lie in shared memory.
+  if (288 * uint64_t(a.max_blocks) > uint64_t(grid) * kSmemBytes)
+    f = a.shared ? k_pcg<true, PcgSystem, true> : k_pcg<false, PcgSystem, true>;
   if (grid == 1) return launch_dependent(f, 1, kThreads, kSmemBytes, s, a, limit);
   // No step of an earlier run may be taken for one of this run's.
   cudaError_t e = cudaMemsetAsync(a.zx, 0, 6 * size_t(a.C) * sizeof(Flagged), s);

@@ -40,6 +40,7 @@ struct PcgSystem {
   const double* rhs;
   const double* scal_part;  // 4 per task block: H_ff, b_f, and the points' shares of them
   uint32_t scal_blocks;
+  uint32_t max_blocks;      // 6x6 blocks of S at most
   int solving, block_failed, lambda, focal_full, focal_rhs, clear_from, clear_to;
   double tol, tol_inner, alpha_limit;
   Flagged* zx;         // 6C: z between blocks
