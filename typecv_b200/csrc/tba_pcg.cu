@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(256) k_pcg_plan(W w) {
   for (uint32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) A.local[k] = place[A.col[k]];
 }
 
-// WIDE: for systems whose shares lie in global memory, 16-byte loads of S with two rows a lane (25 -> 19 us a
-// step at 1,500 cameras, S in the L2).  From shared memory a row a lane is the faster one (a step at 7
-// cameras 2.6 and 3.2 us, at 61 cameras 6.2 and 7.3): its step is the instructions' latency, not the loads.
+// WIDE: for systems whose shares lie in global memory, 16-byte loads of S with two rows a lane: 25 -> 22 us a
+// step at 1,500 cameras with the focal unknown, S in the L2.  From shared memory a row a lane is the faster
+// one (a step at 7 cameras 2.6 and 3.5 us, at 61 cameras 5.8 and 7.0): its step is the instructions' latency.
 template <bool SHARED, class W, bool WIDE = false>
 __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
   after_previous();
