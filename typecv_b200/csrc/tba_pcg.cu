@@ -10,8 +10,9 @@
 // the partial sums in the same order, so all take the same decisions.  A block can publish a step's z
 // only once every block has published the sums that follow its use of the last z, and a reduction's
 // sums only after the other reduction (the start counts as a second one), so one buffer of each does.
-// What bounds a step is the two exchanges through the L2 (about 0.7 us each) with many blocks, and the
-// block's own chain of reductions with one.
+// What bounds a step is the two exchanges through the L2 (1.6 us each between 22 blocks, 2.0 to 2.7 between
+// 148, with the wait for the slowest block), and the block's own chain of reductions, divisions and barriers
+// (2.6 us at 7 cameras in one block).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -283,7 +283,9 @@ __device__ inline void store_entry(const SchurParams& Q, uint32_t b, uint32_t r,
 // One segment of pairs per warp.  The columns of the pairs' records follow one another along the
 // matrix instruction's inner dimension (four pairs are three instructions); a lane loads its own
 // element of each record from global memory, so a record is read as whole 48-byte columns.  The
-// segment's pairs come 32 at a time, one a lane, so that a record's loads wait for one load only.
+// segment's pairs come 32 at a time, one a lane, so that a record's loads wait for one load only.  Bound by
+// the L1: a record of 144 bytes is two lines, and a load's lanes touch four (1.18 ms for 30M pairs, half of
+// the L1's wavefronts on average and three quarters on the busiest SM; DRAM at a fifth).
 template <class W>
 __global__ void __launch_bounds__(256) k_block_sums(W w) {
   after_previous();
@@ -350,6 +352,8 @@ __global__ void __launch_bounds__(256) k_block_sums(W w) {
   }
 }
 
+// A warp per segment boundary: the camera pair that crosses it, taken at the first of the boundaries it
+// crosses.  (A warp per possible camera pair, nearly all with nothing to do: 88 us at 1,500 cameras; 20.)
 template <class W>
 __global__ void __launch_bounds__(256) k_block_ends(W w) {
   after_previous();
