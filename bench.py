@@ -761,6 +761,14 @@ def run_adjoint(args, world, rank, local):
                             "frac": achieved / pk["hbm_gbs"], "traffic": None, "algorithmic_bytes": nbytes,
                             "launch_ms": 1000 * t_launch, "launches": rep_t["product_launches"],
                             "product_blocks": blocks}
+    elif rep_t.get("product_launches", 0):  # S p on the explicit reduced system, launched step by step
+        nbytes = system_bytes(clean)
+        t_launch = rep_t["product_ms"] / rep_t["product_launches"] / 1000
+        achieved = nbytes / t_launch / 1e9
+        line["roofline"] = {"bound": "hbm", "kernel": "k_adj_rows (S p on the explicit reduced camera system)",
+                            "achieved": achieved, "peak": pk["hbm_gbs"], "peak_kind": pk_kind, "unit": "GB/s",
+                            "frac": achieved / pk["hbm_gbs"], "traffic": None, "algorithmic_bytes": nbytes,
+                            "launch_ms": 1000 * t_launch, "launches": rep_t["product_launches"], "product_blocks": 0}
     line["cpu_baseline"] = {"value": 1.0 / dense_s, "unit": "vjp/s", "cores": os.cpu_count() or 1, "kind": "port",
                             "sample": f"one vjp of the 10-camera / 500-point subproblem ({small.M} observations) by "
                                       f"the dense FP64 reference gradient (oracle/adjoint_dense.py, numpy with its BLAS threads: Hessian by "
