@@ -63,6 +63,15 @@ def test_explicit_system_matches_the_oracle(device, scene, shared):
     against_oracle(device, sc.C, sc.P, sc.M, s, i, shared, 5, engine=2)
 
 
+@pytest.mark.parametrize("shared", [False, True])
+def test_a_system_read_from_global_memory(device, shared):
+    # Over 36 MB of S, 240 KB a block: the PCG's blocks cannot hold their shares, and read them 16 bytes at a
+    # time.  (Fewer points would not be worth the system's steps.)
+    sc = S.sphere_scene(seed=12, cameras=1301, points=180001)
+    s, i = sc.packed()
+    against_oracle(device, sc.C, sc.P, sc.M, s, i, shared, 4, engine=2, tolerance=1e-9)
+
+
 def test_a_camera_that_sees_a_point_twice(device):
     sc = S.arc_scene(seed=9, cameras=9, points=257)
     rng = np.random.default_rng(1)
