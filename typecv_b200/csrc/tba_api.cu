@@ -423,15 +423,19 @@ uint64_t count_pairs(const uint32_t* ps, uint32_t P) {
 uint64_t schur_block_bound(uint64_t C, uint64_t pairs) { return std::min(C * C, 2 * pairs + C); }
 
 // Whether a solve forms the reduced system explicitly: its values cost about 0.04 ns a pair of
-// observations of one point, once per linear solve, and a PCG step then a pass over the blocks (here a
-// quarter of their bound, at 5 TB/s) and two exchanges, against a pass over every observation (0.03
-// ns each) and five launches; compared over `steps` PCG steps (16 for an LM iteration, 64 for the
-// adjoint's tighter solves, at most the budget).
+// observations of one point, once per linear solve, and a PCG step then a pass over the blocks (a sixth of
+// their bound where cameras share points with their neighbours, at 8 TB/s from the L2) and two exchanges,
+// against a pass over every observation (0.033 ns each) and five launches in a graph loop; compared over
+// `steps` PCG steps (16 for an LM iteration, 64 for the adjoint's tighter solves, at most the budget).
+// Six iterations on the product and on the system, ms: 331 cameras / 18,137 observations 7.7 and 2.8; 701 /
+// 123,088 6.3 and 2.6; 1,301 / 61,318 8.5 and 5.2, / 369,365 8.0 and 5.1, / 1,106,971 12.7 and 7.1; 2,501 /
+// 246,549 7.8 and 6.2, / 1,230,585 18.8 and 10.0; every camera seeing every point: 120 / 180,000 4.3 and 3.8,
+// 200 / 600,000 6.0 and 14.1.
 bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t budget, uint32_t expected) {
   if (6 * C + 1 > tba::product_max_unknowns() || pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
   const double steps = std::min(budget, expected);
-  const double blocks = double(schur_block_bound(C, pairs)) / 4;
-  return 4e-5 * double(pairs) + steps * (5 + 288e-6 / 5 * blocks) < steps * (14 + 3e-5 * double(M));
+  const double blocks = double(schur_block_bound(C, pairs)) / 6;
+  return 4e-5 * double(pairs) + steps * (8 + 288e-6 / 8 * blocks) < steps * (24 + 3.3e-5 * double(M));
 }
 
 // Device memory of a solve's explicit system beside the workspace: structure, segment sums, blocks.
