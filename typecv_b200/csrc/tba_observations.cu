@@ -133,6 +133,10 @@ __global__ void __launch_bounds__(256, 2) k_obs_tracks(ObsParams A) {
   for (uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < A.ntasks; t += warps) {
     const uint32_t h0 = A.tasks[t], h1 = A.tasks[t + 1];
     const uint32_t o0 = A.offsets[h0], n = A.offsets[h1] - o0;
+    if (n == 0) {  // (the last of such runs lies behind the last observation: nothing to look at)
+      for (uint32_t h = h0 + uint32_t(lane); h < h1; h += 32) A.flags[A.M + h] = 0;
+      continue;
+    }
     if (n <= 32) {
       // The task's tracks: a head bit at each non-empty track's first observation.
       unsigned heads = 0;
