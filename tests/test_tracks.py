@@ -60,3 +60,34 @@ def test_empty_tracks_take_no_part(device, tracks):
     want = OO.evaluate_cpp(q)
     assert np.array_equal(flags, want["flags"]) and np.all(flags[q["count"]:][np.array(tracks) == 0] == 0)
     assert summary[1] == want["summary"][1] > 0 and abs(summary[0] - want["summary"][0]) <= 1e-12 * want["summary"][0]
+
+
+def test_the_checks_of_a_long_track_cost_less_than_its_evaluation(device):
+    q = evaluation(50, [200_000, 200_000])
+    spent = []
+    for _ in range(5):
+        status, said, _, _, rep = evaluate(device, q)
+        assert status == _lib.TBA_OK, said
+        spent.append((rep.wall_ms - rep.evaluate_ms, rep.evaluate_ms))
+    copies_and_checks, kernels = min(spent)
+    assert copies_and_checks < 0.5 * kernels, spent
+
+
+# Empty tracks, tracks of one, of a warp and of more, and long ones: a foreign observation at either end of a
+# track or inside it, offsets that move a track's end, and indices just out of range.
+@pytest.mark.parametrize("where,at,value,message", [
+    (None, 0, 0, ""), ("indices", 1, 2, "offsets"), ("indices", 2 * 8000 + 1, 3, "offsets"),
+    ("indices", 2 * 8999 + 1, 4, "offsets"), ("indices", -1, 3, "offsets"), ("indices", 1, 0, "offsets"),
+    ("offsets", 6, 8999, "offsets"), ("offsets", 6, 9001, "offsets"), ("offsets", 3, 0, "offsets"),
+    ("offsets", 4, 10_290, "offsets"), ("indices", 2 * 8000, 50, "out of range"), ("indices", -1, 8, "out of range")])
+def test_track_checks_at_the_edges(device, where, at, value, message):
+    q = evaluation(50, [0, 1, 0, 33, 257, 8709, 1289, 0])
+    assert (q["count"], q["P"]) == (10_289, 8) and q["offsets"][6] == 9000
+    if where:
+        q[where][at] = value
+        status, said, _, _, _ = evaluate(device, q)
+        assert status == _lib.TBA_ERROR_ARGUMENT and message in said
+        return
+    status, said, flags, _, _ = evaluate(device, q)
+    assert status == _lib.TBA_OK, said
+    assert np.array_equal(flags, OO.evaluate_cpp(q)["flags"])

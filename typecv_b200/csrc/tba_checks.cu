@@ -99,18 +99,18 @@ __global__ void __launch_bounds__(256) k_check_observations(ObservationChecks A)
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   bool failed = false;
   const uint2* ix = reinterpret_cast<const uint2*>(A.indices);
+  // An observation lies in the track of its point: with offsets that never decrease and cover the
+  // observations, that is every track's observations being its point's.  (A thread a track took 12 ms for two
+  // tracks of 200,000 observations, each load waiting for the one before; this is one pass.)
   for (uint64_t i = first; i < A.M; i += step) {
     const uint2 v = ix[i];
-    failed = failed || v.x >= A.C || v.y >= A.P;
+    if (v.x >= A.C || v.y >= A.P) failed = true;
+    else if (A.offsets) failed = failed || i < A.offsets[v.y] || i >= A.offsets[v.y + 1];
   }
   if (A.offsets)
     for (uint64_t h = first; h < A.P; h += step) {
       const uint32_t b = A.offsets[h], e = A.offsets[h + 1];
-      if (e < b || e > A.M) {
-        failed = true;
-      } else {
-        for (uint32_t i = b; i < e; i++) failed = failed || ix[i].y != h;
-      }
+      failed = failed || e < b || e > A.M;
     }
   for (int k = 0; k < 3; k++)
     for (uint64_t i = first; i < A.counts[k]; i += step) failed = failed || outside(A.values[k][i]);
