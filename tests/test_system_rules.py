@@ -1,12 +1,11 @@
 """Which form a call solves on, and what the explicit reduced system may cost a call that gains nothing by
-it: the rule's two sides, a call without iterations, long tracks under the device's checks, and a device
-whose memory is taken."""
+it: the rule's two sides, a call without iterations, and a device whose memory is taken."""
 import numpy as np
 import pytest
 
 import typecv_b200 as tb
-from typecv_b200 import _lib
 from typecv_b200 import synthetic as S
+from typecv_b200.resident import ResidentScene
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +31,37 @@ def test_a_call_without_iterations_forms_no_system(device, shared):
     after, more = solve(device, sc, iterations=1, shared_focal=shared)
     base = 12 * sc.C + 3 * sc.P
     assert more["engine"] == 2 and out[base + 6] == out[base + 8] == after[base + 8]
+
+
+class Taken:
+    """Device memory taken until at most `left` bytes are free."""
+
+    def __init__(self, left):
+        import torch
+        self.torch, self.parts = torch, []
+        while torch.cuda.mem_get_info()[0] - left > 4 << 20:
+            size = torch.cuda.mem_get_info()[0] - left
+            self.parts.append(torch.empty(size // (2 << 20) * (2 << 20), dtype=torch.uint8, device="cuda"))
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.parts.clear()
+        self.torch.cuda.empty_cache()
+
+
+def test_a_resident_scene_takes_the_room_of_the_last_solves_system():
+    kept = S.sphere_scene(seed=14, cameras=801, points=30_001)  # over 180 MB of S beside a small scene
+    large = S.helix_scene(seed=15, cameras=60, points=60_001)   # 14 MB
+    with tb.ShadeDevice.open(0) as dev:
+        out, rep = solve(dev, kept, iterations=2)
+        assert rep["engine"] == 2
+        ctl = tb.make_control(large.C, large.P, large.M, anchor=0, scale_view=1, iterations=2)
+        s, i = large.packed()
+        with Taken(6 << 20), ResidentScene(dev, ctl, s, i) as scene:
+            poses, points = scene.read()
+            assert np.array_equal(poses, s[:12 * large.C]) and np.array_equal(points, s[12 * large.C:][:3 * large.P])
+        again, rep = solve(dev, kept, iterations=2)
+        base = 12 * kept.C + 3 * kept.P
+        assert rep["engine"] == 2 and abs(again[base + 6] - out[base + 6]) <= 1e-9 * out[base + 6]

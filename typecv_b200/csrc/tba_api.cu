@@ -519,6 +519,8 @@ struct SchurLayout {
   }
 };
 
+constexpr size_t kAllocationGrain = size_t(2) << 20;  // an allocation takes whole pages of the device's memory
+
 // The device's free memory, with the explicit system's buffer given back when `need` takes it.
 size_t free_memory(tba_device* d, size_t need) {
   size_t free_bytes = 0, total_bytes = 0;
@@ -2793,6 +2795,8 @@ tba_status tba_scene_create(tba_device* d, const tba_control* shape, const doubl
     r->plan = new HostPlan(make_plan(shape, index, d->sms));
     std::vector<uint32_t> flat;
     for (const std::vector<uint32_t>* v : static_cast<HostPlan*>(r->plan)->sections()) flat.insert(flat.end(), v->begin(), v->end());
+    // (an explicit system's buffer that the handle keeps from its last solve makes room for the scene)
+    free_memory(d, scene_len * sizeof(double) + (index_len + flat.size()) * sizeof(uint32_t) + 3 * kAllocationGrain);
     CUDA_TRY(cudaMalloc(&r->scene, scene_len * sizeof(double)));
     CUDA_TRY(cudaMalloc(&r->index, index_len * sizeof(uint32_t)));
     CUDA_TRY(cudaMalloc(&r->plan_dev, std::max<size_t>(1, flat.size()) * sizeof(uint32_t)));
