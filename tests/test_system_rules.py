@@ -65,3 +65,25 @@ def test_a_resident_scene_takes_the_room_of_the_last_solves_system():
         again, rep = solve(dev, kept, iterations=2)
         base = 12 * kept.C + 3 * kept.P
         assert rep["engine"] == 2 and abs(again[base + 6] - out[base + 6]) <= 1e-9 * out[base + 6]
+
+
+@pytest.fixture(scope="module")
+def dense_ring():
+    # Every one of 26 cameras sees every point, 12.5 pairs an observation: on the edge of the rule.
+    sc = S.ring_scene(seed=1, cameras=26, points=80_000)
+    assert sc.M == 26 * 80_000
+    return sc, sc.packed()
+
+
+@pytest.mark.parametrize("precision,options,engine", [
+    (0, dict(), 2), (1, dict(), 2),                                          # 22 steps an iteration
+    (0, dict(tolerance=1e-3), 2), (1, dict(tolerance=1e-3), 0),              # 14: the FP32 product's are cheaper
+    (0, dict(tolerance=1e-2), 0), (1, dict(tolerance=1e-2), 0),              # 10
+    (0, dict(max_cg=16), 0), (1, dict(max_cg=16), 2),                        # 14 and, with restarts, 32
+    (0, dict(max_cg=24), 2), (0, dict(max_cg=1), 0), (1, dict(max_cg=1), 0)])
+def test_short_solves_of_long_tracks_keep_the_product(device, dense_ring, precision, options, engine):
+    sc, packed = dense_ring
+    out, rep = solve(device, sc, packed, iterations=1, precision=precision, **options)
+    assert rep["engine"] == engine
+    base = 12 * sc.C + 3 * sc.P
+    assert out[base + 6] <= out[base + 8]

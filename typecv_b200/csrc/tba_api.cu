@@ -422,20 +422,43 @@ uint64_t count_pairs(const uint32_t* ps, uint32_t P) {
 // 6x6 blocks of S at most.
 uint64_t schur_block_bound(uint64_t C, uint64_t pairs) { return std::min(C * C, 2 * pairs + C); }
 
-// Whether a solve forms the reduced system explicitly: its values cost about 0.04 ns a pair of
-// observations of one point, once per linear solve, and a PCG step then a pass over the blocks (a sixth of
-// their bound where cameras share points with their neighbours, at 8 TB/s from the L2) and two exchanges,
-// against a pass over every observation (0.033 ns each) and five launches in a graph loop; compared over
-// `steps` PCG steps (16 for an LM iteration, 64 for the adjoint's tighter solves, at most the budget).
-// Six iterations on the product and on the system, ms: 331 cameras / 18,137 observations 7.7 and 2.8; 701 /
-// 123,088 6.3 and 2.6; 1,301 / 61,318 8.5 and 5.2, / 369,365 8.0 and 5.1, / 1,106,971 12.7 and 7.1; 2,501 /
-// 246,549 7.8 and 6.2, / 1,230,585 18.8 and 10.0; every camera seeing every point: 120 / 180,000 4.3 and 3.8,
-// 200 / 600,000 6.0 and 14.1.
-bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t budget, uint32_t expected) {
+// The PCG steps of a solve to `tolerance` that the choice below counts on, from few: spheres, arcs and rings of
+// 16 to 60 cameras took 8 to 19 steps at 1e-2, 10 to 30 at 1e-3 and 21 to 44 at 1e-6, 200 cameras 22, 36 and 68,
+// 1,500 cameras 60, 66 and 75.
+double expected_steps(uint64_t C, double tolerance) {
+  return (10 + 8 * std::log10(1e-2 / tolerance)) * std::max(1.0, std::sqrt(double(C) / 60));
+}
+
+// Whether a solve forms the reduced system explicitly: its values cost about 0.04 ns a pair of observations of
+// one point, once per linear solve, and a PCG step then a pass over the blocks (a sixth of their bound where
+// cameras share points with their neighbours, at 8 TB/s from the L2) and two exchanges, against a pass over
+// every observation (0.033 ns each) and five launches in a graph loop; compared over `most` PCG steps (16 for an
+// LM iteration, 64 for the adjoint's tighter solves).  Six iterations on the product and on the system, ms:
+// 331 cameras / 18,137 observations 7.7 and 2.8; 701 / 123,088 6.3 and 2.6; 1,301 / 61,318 8.5 and 5.2, /
+// 369,365 8.0 and 5.1, / 1,106,971 12.7 and 7.1; 2,501 / 246,549 7.8 and 6.2, / 1,230,585 18.8 and 10.0; every
+// camera seeing every point: 120 / 180,000 4.3 and 3.8, 200 / 600,000 6.0 and 14.1.
+//
+// A solve that its budget (of which it takes some 0.85) or its tolerance ends after few steps has less to gain.
+// There a pair costs 0.036 ns where the records of a camera's neighbours (about eight times the pairs an
+// observation has) lie in the 126 MB L2 together, else 0.046.  Six iterations again: 26 cameras / 2.1M
+// observations of 12.5 pairs: budget 12 8.4 and 10.5, 16 10.1 and 10.7, 24 14.2 and 11.4; tolerance 1e-2 8.3 and
+// 11.0.  200 cameras / 10M of 12.2 pairs: budget 16 41.8 and 52.8, 24 53.8 and 53.0.  600 cameras / 1.3M of 10.3:
+// budget 8 5.3 and 5.6, 12 6.9 and 5.8.
+//
+// The system is FP64, so a mixed request is also weighed against its own product: 0.022 ns an observation where
+// the first PCG run reaches the tolerance; where the budget ends the runs, their restarts make it 0.036 for each
+// step of the budget.  The 26 cameras: tolerance 1e-2 7.8 and 11.0, 1e-3 9.4 and 11.1, 1e-6 16.9 and 11.3, budget
+// 16 17.0 and 10.7; the 200 cameras: 1e-2 43.3 and 55.5, 2e-3 58.7 and 55.9.
+bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t budget, double most, double expected, bool mixed) {
   if (6 * C + 1 > tba::product_max_unknowns() || pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
-  const double steps = std::min(budget, expected);
-  const double blocks = double(schur_block_bound(C, pairs)) / 6;
-  return 4e-5 * double(pairs) + steps * (8 + 288e-6 / 8 * blocks) < steps * (24 + 3.3e-5 * double(M));
+  const double walk = 288e-6 / 8 * double(schur_block_bound(C, pairs)) / 6;
+  // A step's cost on the product less that on the system, at `k` us an observation.
+  const auto step = [&](double k) { return 16 + k * double(M) - walk; };
+  if (!(4e-5 * double(pairs) < most * step(3.3e-5))) return false;
+  const double reach = 144 * double(M) * std::min(1.0, 8 * double(pairs) / double(M) / double(C));
+  const double form = (reach < 126e6 ? 3.6e-5 : 4.6e-5) * double(pairs);
+  if (mixed) return form < std::min(budget * step(3.6e-5), expected * step(2.2e-5));
+  return form < std::min(0.85 * budget, expected) * step(3.3e-5);
 }
 
 // Device memory of a solve's explicit system beside the workspace: structure, segment sums, blocks.
@@ -803,12 +826,14 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   // its refinement residual, its FP64 tail and the back-substitution.
   p.factored = m <= tba::product_max_unknowns();
   p.Mpad = (M + 31) / 32 * 32;
-  // The explicit reduced system takes the place of the product over stored factors where it costs less
-  // and fits the device; it is FP64, so a mixed request then needs no refinement.
+  // The explicit reduced system takes the place of the product over stored factors where it costs less than
+  // the product of the form asked for and fits the device; it is FP64, so a mixed request then needs no refinement.
   // (Without iterations there is no system to form: its structure alone took 0.03 ms at 7 cameras and 0.35 at
   // 1,500 and 1.8M observations, of calls of 0.21 and 5.9 ms.)
   const uint64_t npairs = ctl->iterations == 0 ? 0 : (io.plan ? io.plan->pairs : count_pairs(index + 2 * size_t(M), P));
-  bool schur = p.factored && ctl->iterations > 0 && prefer_schur(C, M, npairs, ctl->max_cg, 16);
+  bool schur = p.factored && ctl->iterations > 0 &&
+               prefer_schur(C, M, npairs, ctl->max_cg, 16, expected_steps(C, ctl->cg_tolerance),
+                            ctl->precision == TBA_PRECISION_MIXED);
   bool mixed = false;
   size_t factor_bytes = 0, factor32_bytes = 0;
   uint32_t max_prod_blocks = 1;
@@ -2087,7 +2112,7 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const HostChecks* check
   // The explicit reduced system in place of the product over the cross blocks, where it costs less and
   // fits the device.
   const uint64_t npairs = count_pairs(index + 2 * size_t(M), P);
-  bool schur = prefer_schur(C, M, npairs, vc->max_cg, 64);
+  bool schur = prefer_schur(C, M, npairs, vc->max_cg, 64, vc->max_cg, false);
   Chunks chunks;
   if (checks && (checks->camera_ends || checks->camera_offsets)) schur = false;  // no chunks; the checks will fail
   if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, chunk_size(M, d->sms));
