@@ -66,7 +66,9 @@ typedef enum { TBA_PRECISION_FP64 = 0, TBA_PRECISION_MIXED = 1 } tba_precision;
 /* TBA_FLAG_PRODUCT_ERROR: once, on the first PCG direction of the first LM iteration, evaluate S p
  * with the solve's own Schur product and with the FP64 two-pass product (Jacobians recomputed from
  * the poses, points and pixels), and report their difference in tba_report.product_error_* (for
- * the mixed form: the FP32 product's error).  Diagnostics only: two more products per call. */
+ * the mixed form: the FP32 product's error; a mixed request with this flag runs the mixed form also
+ * where it would otherwise run in FP64 on the explicit reduced system).  Diagnostics only: two more
+ * products per call. */
 #define TBA_FLAG_PRODUCT_ERROR 2u
 /* TBA_FLAG_HOST_PCG_LOOP: launch the PCG steps from the host in chunks, as with
  * TBA_FLAG_TIME_PRODUCTS but without the events, instead of the device-side loop (for profilers and

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import typecv_b200 as tb
+from typecv_b200 import _lib
 from typecv_b200 import synthetic as S
 from typecv_b200.resident import ResidentScene
 
@@ -87,3 +88,18 @@ def test_short_solves_of_long_tracks_keep_the_product(device, dense_ring, precis
     assert rep["engine"] == engine
     base = 12 * sc.C + 3 * sc.P
     assert out[base + 6] <= out[base + 8]
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_the_product_error_of_a_mixed_request_is_the_fp32_products(device, shared):
+    # FP32 rounds the factors at 6e-8; averaged over a camera's thousands of observations that leaves more than
+    # 1e-11 of S p (FP64's product leaves less than 1e-12 there).
+    sc = S.ring_scene(seed=11)
+    kw = dict(iterations=2, shared_focal=shared, tolerance=1e-8, max_cg=200)
+    _, fp64 = solve(device, sc, flags=_lib.TBA_FLAG_PRODUCT_ERROR, precision=0, **kw)
+    out, mixed = solve(device, sc, flags=_lib.TBA_FLAG_PRODUCT_ERROR, precision=1, **kw)
+    assert fp64["engine"] == 2 and fp64["product_error_norm"] < 1e-12
+    assert mixed["engine"] == 0 and 1e-11 < mixed["product_error_norm"] < 1e-5
+    plain, rep = solve(device, sc, precision=1, **kw)
+    base = 12 * sc.C + 3 * sc.P
+    assert rep["engine"] == 2 and abs(out[base + 6] - plain[base + 6]) <= 1e-6 * plain[base + 6]

@@ -831,7 +831,9 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   // (Without iterations there is no system to form: its structure alone took 0.03 ms at 7 cameras and 0.35 at
   // 1,500 and 1.8M observations, of calls of 0.21 and 5.9 ms.)
   const uint64_t npairs = ctl->iterations == 0 ? 0 : (io.plan ? io.plan->pairs : count_pairs(index + 2 * size_t(M), P));
-  bool schur = p.factored && ctl->iterations > 0 &&
+  // (The product's error asked of a mixed request is the FP32 product's.)
+  const bool keep_product = ctl->precision == TBA_PRECISION_MIXED && (ctl->flags & TBA_FLAG_PRODUCT_ERROR) != 0;
+  bool schur = p.factored && ctl->iterations > 0 && !keep_product &&
                prefer_schur(C, M, npairs, ctl->max_cg, 16, expected_steps(C, ctl->cg_tolerance),
                             ctl->precision == TBA_PRECISION_MIXED);
   bool mixed = false;
