@@ -424,10 +424,12 @@ tba_status tba_linearize_inverse_depth(tba_device* device, uint32_t count, const
                                        tba_observation_report* report);
 
 /*
- * Polls of each main-loop tile wait of tba_linearize_inverse_depth on this handle (default
- * TBA_WAIT_LIMIT_DEFAULT).  No counterpart in the reference: it lets a test make the waits run out
- * (0 polls gives up at once) to exercise the failure path; the drain of the loads in flight after
- * such a failure always keeps the full bound.
+ * Polls of each bounded wait on this handle (default TBA_WAIT_LIMIT_DEFAULT): the main-loop tile waits
+ * of tba_linearize_inverse_depth, and the waits between the blocks of a PCG on the explicit reduced
+ * system (half the default at most), which end a call with TBA_ERROR_CUDA ("a wait between the PCG's
+ * blocks ran out") when they run out and leave the handle usable.  No counterpart in the reference: it
+ * lets a test make the waits run out (0 polls gives up at once) to exercise the failure path; the
+ * drain of the loads in flight after a tile wait's failure always keeps the full bound.
  */
 #define TBA_WAIT_LIMIT_DEFAULT 4194304u
 tba_status tba_device_set_wait_limit(tba_device* device, uint32_t polls);

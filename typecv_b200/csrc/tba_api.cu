@@ -65,8 +65,10 @@ struct tba_device {
   size_t schur_capacity = 0;
   double* pinned = nullptr;  // small host buffer for flag reads
   std::vector<cudaEvent_t> events;
-  // Polls of each main-loop wait of the inverse-depth linearisation (tba_device_set_wait_limit).
+  // Polls of each main-loop wait of the inverse-depth linearisation and, up to its own bound, of each wait
+  // between the blocks of a PCG (tba_device_set_wait_limit).
   uint32_t wait_limit = tba::kIdWaitPolls;
+  uint32_t pcg_polls() const { return std::min(wait_limit, tba::kPcgWaitPolls); }
   // Batched solves: their own workspace, the cached graph of the last launch and its key, and
   // the autotuner's choices by batch shape.
   char* batch_arena = nullptr;
@@ -1036,6 +1038,7 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
     grow(d->schur, d->schur_capacity, Q.L.bytes, "GPU BA");
     Q.bind(d->schur, sq, ps);
     bind_problem(p, sq, ps);
+    ps.polls = d->pcg_polls();
     launches += tba::schur_launch_structure(sq, s);
     pcg_blocks = Q.grid;
     launches += tba::pcg_launch_plan(ps, pcg_blocks, s);
@@ -1525,7 +1528,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
     systems[k].bind(a + w.system, y, c);
     y.bits = u32(o_bits) + bits;
     bits += size_t(C) * y.bwords;
-    bind_problem(p, y, c);
+    bind_problem(p, y, c);  // (one block a problem: nothing waits)
   }
   cudaStream_t s = d->stream;
   auto up = [&](size_t off, const void* src, size_t bytes) {
@@ -2215,6 +2218,7 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const HostChecks* check
     ps.wait = tba::A_WAIT;
     ps.tol = A.tol;
     ps.alpha_limit = 1e30;
+    ps.polls = d->pcg_polls();
   }
 
   cudaStream_t s = d->stream;

@@ -44,10 +44,10 @@ __device__ __forceinline__ Flagged peek(const Flagged* p) {
 }
 
 // The values of `step` at N places, looked for together (a place beyond `n` is left out); false when
-// they did not come within the poll limit.
+// they did not come within `polls` polls.
 template <int N>
-__device__ __forceinline__ bool await(const Flagged* const (&p)[N], int n, uint64_t step, double (&v)[N]) {
-  for (uint32_t k = 0; k < kPcgWaitPolls; k++) {
+__device__ __forceinline__ bool await(const Flagged* const (&p)[N], int n, uint64_t step, uint32_t polls, double (&v)[N]) {
+  for (uint32_t k = 0; k < polls; k++) {
     Flagged f[N];
 #pragma unroll
     for (int j = 0; j < N; j++)
@@ -139,7 +139,7 @@ __device__ inline bool grid_sum(const PcgSystem& A, Shared& sh, double (&v)[2], 
         at[2 * j + 1] = slots + 4 * size_t(b) + 1;
         if (b < grid) n = 2 * j + 2;
       }
-      ok = await(at, n, step, got);
+      ok = await(at, n, step, A.polls, got);
 #pragma unroll
       for (int j = 0; j < 2 * kSlotsEach; j++)
         if (j < n) s[j & 1] += got[j];
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
       const Flagged* at[2] = {A.zx + 6 * uni[b] + (j - 6 * b), nullptr};
       if (j1 < cols) at[1] = A.zx + 6 * uni[b1] + (j1 - 6 * b1);
       double got[2];
-      if (*(volatile int*)&sh.gave_up != 0 || !await(at, j1 < cols ? 2 : 1, step, got)) {
+      if (*(volatile int*)&sh.gave_up != 0 || !await(at, j1 < cols ? 2 : 1, step, A.polls, got)) {
         *(volatile int*)&sh.gave_up = 1;
         break;
       }

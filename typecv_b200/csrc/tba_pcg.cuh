@@ -7,7 +7,7 @@
 
 namespace tba {
 
-constexpr uint32_t kPcgWaitPolls = 1u << 21;  // polls of one word before a wait gives up (about a second)
+constexpr uint32_t kPcgWaitPolls = 1u << 21;  // polls of one wait before it gives up, at most (about a second)
 
 // A double and the step it belongs to, written and read as one 16-byte word: a reader that finds the
 // step it waits for has the value, with no fence on either side.
@@ -42,6 +42,7 @@ struct PcgSystem {
   uint32_t scal_blocks;
   uint32_t max_blocks;      // 6x6 blocks of S at most
   int solving, block_failed, lambda, focal_full, focal_rhs, clear_from, clear_to;
+  uint32_t polls;           // of one wait for other blocks (at most kPcgWaitPolls)
   double tol, tol_inner, alpha_limit;
   Flagged* zx;         // 6C: z between blocks
   Flagged* slots;      // 4 per block: its partial sums of the step's two reductions
