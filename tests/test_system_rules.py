@@ -5,6 +5,8 @@ import pytest
 
 import typecv_b200 as tb
 from typecv_b200 import _lib
+from typecv_b200 import adjoint as AD
+from typecv_b200 import batch as B
 from typecv_b200 import synthetic as S
 from typecv_b200.resident import ResidentScene
 
@@ -103,3 +105,53 @@ def test_the_product_error_of_a_mixed_request_is_the_fp32_products(device, share
     plain, rep = solve(device, sc, precision=1, **kw)
     base = 12 * sc.C + 3 * sc.P
     assert rep["engine"] == 2 and abs(out[base + 6] - plain[base + 6]) <= 1e-6 * plain[base + 6]
+
+
+def test_a_system_that_does_not_fit_leaves_the_product():
+    # 801 cameras: over 180 MB of S beside a workspace of 40 MB, the adjoint's of 100.
+    sc = S.sphere_scene(seed=14, cameras=801, points=30_001, outlier_rate=0.0)
+    s, i = sc.packed()
+    kw = dict(iterations=3, tolerance=1e-9, max_cg=200)
+    n = 12 * sc.C + 3 * sc.P
+    g = np.random.default_rng(3).normal(size=n)
+    g /= np.linalg.norm(g)
+    with tb.ShadeDevice.open(0) as dev:
+        want, rep = solve(dev, sc, (s, i), **kw)
+        assert rep["engine"] == 2
+        at, _ = solve(dev, sc, (s, i), iterations=20, tolerance=1e-10, max_cg=256)
+        there = np.concatenate([at[:n], s[n:]])
+        ybar, kbar, _, rep = AD.bundle_vjp(dev, sc.C, sc.P, sc.M, there, i, g)
+        assert rep["failed"] == 0 and rep["product_blocks"] == 0
+    with tb.ShadeDevice.open(0) as dev, Taken(150 << 20):
+        got, rep = solve(dev, sc, (s, i), **kw)
+        assert rep["engine"] == 0 and abs(got[n + 6] - want[n + 6]) <= 1e-9 * want[n + 6]
+        assert np.max(np.abs(got[:12 * sc.C] - want[:12 * sc.C])) < 1e-7
+        y2, k2, _, rep = AD.bundle_vjp(dev, sc.C, sc.P, sc.M, there, i, g)
+        assert rep["failed"] == 0 and rep["product_blocks"] > 0
+        assert np.linalg.norm(y2 - ybar) <= 1e-8 * np.linalg.norm(ybar)
+        assert np.all(np.abs(k2 - kbar) <= 1e-8 * np.abs(kbar) + 1e-12)
+    with tb.ShadeDevice.open(0) as dev:  # with the memory back, so is the system
+        _, rep = solve(dev, sc, (s, i), **kw)
+        assert rep["engine"] == 2
+
+
+def test_windows_whose_systems_do_not_fit_run_on_the_persistent_launch():
+    # 64 MB with their systems, 30 without.
+    scenes = [S.arc_scene(seed=100 + k, cameras=40, points=4000 + k, track=(8, 10)) for k in range(6)]
+    probs = [B.PackedProblem(sc.C, sc.P, sc.M, *sc.packed(), sc.anchor, sc.scale_view) for sc in scenes]
+    kw = dict(iterations=4, precision="fp64", max_cg=200)
+    with tb.ShadeDevice.open(0) as dev:
+        want, rep = B.batch_adjust(dev, probs, **kw)
+        want = [r.copy() for r in want]
+        assert rep["schedule"] == 4
+        for schedule in (1, 2, 3, 4):  # (the kernels' stacks are allocated once a process)
+            B.batch_adjust(dev, probs, schedule=schedule, **kw)
+    with tb.ShadeDevice.open(0) as dev, Taken(48 << 20):
+        with pytest.raises(tb.RangeError, match="budget"):
+            B.batch_adjust(dev, probs, schedule=5, **kw)
+        got, rep = B.batch_adjust(dev, probs, **kw)
+        assert rep["schedule"] < 4 and rep["tune_ms"] > 0
+        for sc, a, b in zip(scenes, got, want):
+            base = 12 * sc.C + 3 * sc.P
+            assert abs(a[base + 6] - b[base + 6]) <= 1e-9 * b[base + 6]
+            assert np.max(np.abs(a[:12 * sc.C] - b[:12 * sc.C])) < 1e-7
