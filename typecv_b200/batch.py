@@ -1,4 +1,4 @@
-"""Batched local-window bundle adjustment: many independent problems in one persistent launch.
+"""Batched local-window bundle adjustment: many independent problems in one call.
 
 The reference's mapper adjusts its local windows one ``bundleAdjustGpu`` call at a time
 (src/sfm/mapper/mapper.ts:859-925 over the windows planned by src/sfm/bundle/local-bundle.ts:17-208).
@@ -69,7 +69,8 @@ def pack_batch(problems: list[PackedProblem], shared_focal: bool, *, scene: np.n
 
 
 def batch_shapes() -> list[tuple[int, int]]:
-    """The solver's launch shapes: (threads per block, compiled blocks per SM)."""
+    """The solver's launch shapes: (threads per block, compiled blocks per SM).  The last is the kernels over all
+    problems at once, the others one persistent launch."""
     lib = _lib.load()
     out = []
     for k in range(lib.tba_batch_shapes()):
@@ -89,7 +90,9 @@ def batch_adjust(device: ShadeDevice, problems: list[PackedProblem] | PackedBatc
                  schedule: int = 0, output: np.ndarray | None = None):
     """Solve every problem; returns (list of result records, report dict).
 
-    ``schedule`` 0 lets the library's autotuner pick the launch shape; k >= 1 forces shape k - 1.
+    ``schedule`` 0 solves all problems side by side on the last shape, in FP64, where its memory fits and
+    the tracks are no longer than about 64 observations, and else lets the library's autotuner pick a
+    persistent shape; k >= 1 forces shape k - 1 of ``batch_shapes``.
     ``max_cg`` defaults to the reference's default for the largest problem (bundle-host.ts:49-65).
     """
     lib = _lib.load()

@@ -31,8 +31,10 @@
 // (q~ = R^T q, R^T du, R^T dv, w, jf; FP64, and an FP32 copy in the mixed form), from which every product is
 // a few dozen FMAs.  The camera passes recompute the Jacobians from the pose, the camera, the point and the
 // pixel.
-// Every reduction runs in a fixed order (fixed grids, fixed trees, fixed chunking), except the
-// shared-memory camera sums of k_product_f, whose FP64 atomic adds commute only up to rounding.
+// Every reduction here runs in a fixed order (fixed grids, fixed trees, fixed chunking), except the
+// shared-memory camera sums of k_product_f, whose FP64 atomic adds commute only up to rounding.  On the
+// explicit system the block sums (tba_schur.cu) add a camera pair's pairs in an order that changes from
+// call to call, so repeated solves agree to rounding, as they do on k_product_f.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -503,8 +505,7 @@ __device__ inline void camera_rows(const Geo& g, bool dir, double jc[2][6]) {
 }
 
 __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camera_pass(Params P) {
-  constexpr int kParts = kCameraPartials, kSecond = kParts - 33;
-  __shared__ double red[kParts * (kCameraThreads / 32)];
+  __shared__ double red[kCameraPartials * (kCameraThreads / 32)];
   if (P.state[S_ACTIVE] == 0) return;
   const uint32_t ch = blockIdx.x, c = P.chunk_cam[ch];
   if (P.active[c] == 0) return;
@@ -536,13 +537,13 @@ __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camer
     for (int j = 0; j < 33; j++) {
       double s = a[j];
       for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(kFull, s, d);
-      if (lane == 0) red[warp * kParts + j] = s;
+      if (lane == 0) red[warp * kCameraPartials + j] = s;
     }
   }
   // Pass 2: W V^-1 W^T (lower triangle) and W V^-1 b_p.
   {
-    double b[kSecond];
-    for (int j = 0; j < kSecond; j++) b[j] = 0;
+    double b[27];
+    for (int j = 0; j < 27; j++) b[j] = 0;
     for (uint32_t kk = k0 + threadIdx.x; kk < k1; kk += blockDim.x) {
       const uint32_t pt = P.cm_point[kk];
       const double2 uv = reinterpret_cast<const double2*>(P.cm_pixel)[kk];
@@ -572,17 +573,17 @@ __global__ void __launch_bounds__(kCameraThreads, TBA_CAMERA_MIN_BLOCKS) k_camer
         b[21 + j] += t0 * bb[0] + t1 * bb[1] + t2 * bb[2];
       }
     }
-    for (int j = 0; j < kSecond; j++) {
+    for (int j = 0; j < 27; j++) {
       double s = b[j];
       for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(kFull, s, d);
-      if (lane == 0) red[warp * kParts + 33 + j] = s;
+      if (lane == 0) red[warp * kCameraPartials + 33 + j] = s;
     }
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < kParts; j += blockDim.x) {
+  for (int j = threadIdx.x; j < kCameraPartials; j += blockDim.x) {
     double s = 0;
-    for (int w = 0; w < nwarps; w++) s += red[w * kParts + j];
-    P.chunk_part[size_t(kParts) * ch + j] = s;
+    for (int w = 0; w < nwarps; w++) s += red[w * kCameraPartials + j];
+    P.chunk_part[size_t(kCameraPartials) * ch + j] = s;
   }
 }
 

@@ -251,7 +251,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg(W system, uint32_t limit) {
     row_ptr = words;
   }
   // A block of S takes 38 words in shared memory, so that a warp's reads of five blocks fall on different
-  // banks (36 where only they fit).
+  // banks (36 where only they fit).  Eight iterations at 36 and 38 words, ms: 24 cameras 1.44 and 1.42, every
+  // camera seeing every point 1.29 and 1.23, with the focal unknown 1.15 and 1.10; 61 cameras 2.34 and 2.29; a
+  // batch of 24 windows 2.38 and 2.21, with the focal unknown 2.46 and 2.31; 7 and 10 cameras alike.
   const double* S = A.S + 36 * size_t(k0);
   const size_t rest = (size_t(blocks) + 1) / 2 + 36 * size_t(nr) + 4;  // the places and preconditioner blocks
   const uint32_t stride = (used + 38 * size_t(blocks) + rest) * sizeof(double) <= kSmemBytes ? 38 : 36;

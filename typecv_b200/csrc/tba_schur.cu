@@ -6,7 +6,8 @@
 //   k_pairs_place   per camera: its camera pairs with their first pairs, each chunk's positions, and
 //                   the cameras of its blocks of S
 //   k_pairs_blocks  per camera pair: its two blocks of S; the segments that start in it
-//   k_pairs_fill    per camera chunk: its pairs, written at their positions
+//   k_pairs_fill    per camera chunk: its pairs, at their positions (within a chunk's share of a camera
+//                   pair in the order its threads come: an atomic cursor)
 //   k_block_sums    per segment of pairs: sum A_i A_j^T of each camera pair
 //   k_block_ends    camera pairs that cross segments: their partial sums in segment order
 #include <cuda_runtime.h>

@@ -10,7 +10,9 @@
 //     cameras, c(i) < c(j), grouped by camera pair; the camera pairs that occur (a bit matrix), and
 //     the rows of S as runs of 6x6 blocks in camera order
 //   values (per solve): every camera pair's sum of A_i A_j^T on the FP64 matrix instruction, in
-//     equal runs of pairs per warp whose unfinished ends are added afterwards in a fixed order
+//     equal runs of pairs per warp whose unfinished ends are added afterwards in the runs' order.  The
+//     pairs of a camera pair lie in the order in which k_pairs_fill's atomic cursor met them, which
+//     changes from call to call: S repeats to rounding, not bit for bit
 //   PCG: one persistent launch per run (tba_pcg.cu)
 #pragma once
 
