@@ -53,7 +53,8 @@ typedef enum {
  * an iteration budget of its own.  Once an LM iteration needed that FP64 finish, the call's later
  * iterations solve on the FP64 product alone (tba_report.fp64_iterations).  Where the reduced
  * camera system is formed explicitly (tba_report.engine 2) there is no product over factors to hold
- * in FP32, and a mixed request runs in FP64 throughout.  It has no reference counterpart. */
+ * in FP32, and a mixed request runs in FP64 throughout, its one PCG run with those four budgets
+ * together.  It has no reference counterpart. */
 typedef enum { TBA_PRECISION_FP64 = 0, TBA_PRECISION_MIXED = 1 } tba_precision;
 
 /* TBA_FLAG_TIME_PRODUCTS: bracket every Schur product with CUDA events and report their total

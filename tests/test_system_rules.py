@@ -155,3 +155,30 @@ def test_windows_whose_systems_do_not_fit_run_on_the_persistent_launch():
             base = 12 * sc.C + 3 * sc.P
             assert abs(a[base + 6] - b[base + 6]) <= 1e-9 * b[base + 6]
             assert np.max(np.abs(a[:12 * sc.C] - b[:12 * sc.C])) < 1e-7
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_a_mixed_request_keeps_the_budgets_of_its_runs(device, shared):
+    # The mixed form's PCG takes up to four runs of the budget (two in a batch); on the explicit system its one run
+    # takes as many steps.  An FP64 request's solve ends, and fails, with its budget.
+    sc = S.ring_scene(seed=1, cameras=7, points=301)
+    packed = sc.packed()
+    base = 12 * sc.C + 3 * sc.P
+    kw = dict(iterations=1, shared_focal=shared, tolerance=1e-6)
+    free, rep = solve(device, sc, packed, max_cg=200, **kw)
+    steps = rep["cg_iterations"]
+    assert rep["engine"] == 2 and steps >= 10 and free[base + 10] == 1
+    few = steps // 2 + 1
+    out, _ = solve(device, sc, packed, max_cg=few, **kw)
+    assert out[base + 10] == 0 and out[base + 17] == 1
+    for flags in (0, _lib.TBA_FLAG_HOST_PCG_LOOP):
+        out, rep = solve(device, sc, packed, max_cg=few, precision=1, flags=flags, **kw)
+        assert rep["engine"] == 2 and abs(rep["cg_iterations"] - steps) <= 1
+        assert out[base + 10] == 1 and out[base + 17] == 0
+        assert abs(out[base + 6] - free[base + 6]) <= 1e-9 * free[base + 6]
+    out, rep = solve(device, sc, packed, max_cg=steps // 5, precision=1, **kw)
+    assert rep["cg_iterations"] == 4 * (steps // 5) and out[base + 10] == 0 and out[base + 17] == 1
+    window = B.PackedProblem(sc.C, sc.P, sc.M, *packed, sc.anchor, sc.scale_view)
+    for precision, accepted in (("fp64", 0), ("mixed", 1)):
+        recs, _ = B.batch_adjust(device, [window] * 2, max_cg=few, precision=precision, **kw)
+        assert [r[base + 10] for r in recs] == [accepted] * 2 and recs[1][base + 17] == 1 - accepted

@@ -1058,6 +1058,10 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   // With the explicit system nothing in an iteration needs the host, so iterations are issued one ahead
   // of the last state read.
   const bool ahead = schur && !host_loop && !diagnose;
+  // On the explicit system a mixed request's one run has the budgets of the mixed form's runs together, so that
+  // a budget that the form's restarts make do with is enough here too (a run that it ends is a failed solve).
+  constexpr uint32_t kFp32Restarts = 2;
+  const uint32_t pcg_budget = ctl->max_cg * (schur && ctl->precision == TBA_PRECISION_MIXED ? kFp32Restarts + 2 : 1);
   cudaEvent_t read_done[2] = {event(d, ev), event(d, ev + 1)};
   ev += 2;
   // Kernels per step of the device-side PCG loop launched last, while its step count is unread.
@@ -1176,15 +1180,14 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
       loop_kernels = 0;
     };
     if (fp64_only) fp64_iterations++;
-    run_pcg(ctl->max_cg, fp64_only ? tail : p, !fp64_only);
+    run_pcg(pcg_budget, fp64_only ? tail : p, !fp64_only);
     // Mixed form: FP64 iterative refinement.  The true (FP64) residual of the FP32-product solution
     // restarts the PCG from that solution when it is above the tolerance; a restarted run (with an
     // iteration budget of its own) uses the FP32 product again and is checked again.  Only a
     // solution still above the tolerance after kFp32Restarts such runs is finished on the FP64
     // product, which resolves what FP32 factors cannot on badly conditioned systems.
     if (mixed && !fp64_only) {
-      constexpr int kFp32Restarts = 2;
-      for (int round = 0;; round++) {
+      for (uint32_t round = 0;; round++) {
         tba::launch_refine(p, s);
         launches += 4;
         CUDA_TRY(cudaGetLastError());
@@ -1602,7 +1605,8 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   key.pcg.systems = reinterpret_cast<const tba::PcgSystem*>(a + o_pcg);
   key.pcg.work = key.many.one.work;
   key.count = count;
-  key.limit = bc->max_cg;
+  // (a mixed request: the budgets of the mixed form's run and its restart)
+  key.limit = bc->max_cg * (bc->precision == TBA_PRECISION_MIXED ? 2 : 1);
   CUDA_TRY(cudaMemsetAsync(a + o_bits, 0, bit_words * sizeof(uint32_t), s));
   launches += tba::launch_many_begin(key.many, s);
   launches += tba::schur_launch_many_structure(key.schur, s);
@@ -1612,7 +1616,7 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   auto iteration = [&]() {
     per_iteration = tba::launch_many_linearize(key.many, s);
     per_iteration += tba::schur_launch_many_values(key.schur, s);
-    const cudaError_t e = tba::launch_many_pcg(key.pcg, count, shared, bc->max_cg, s);
+    const cudaError_t e = tba::launch_many_pcg(key.pcg, count, shared, key.limit, s);
     per_iteration += 1 + tba::launch_many_update(key.many, s);
     return e;
   };
