@@ -92,6 +92,14 @@ def test_short_solves_of_long_tracks_keep_the_product(device, dense_ring, precis
     assert out[base + 6] <= out[base + 8]
 
 
+@pytest.mark.parametrize("cameras,points,engine", [(300, 50, 2), (400, 30, 2), (600, 30, 0), (600, 10, 0)])
+def test_a_full_system_beyond_the_caches_is_not_formed(device, cameras, points, engine):
+    # Every camera sees every point: S is full, 26, 46 and 104 MB.
+    sc = S.ring_scene(seed=3, cameras=cameras, points=points)
+    _, rep = solve(device, sc, iterations=1)
+    assert sc.M == cameras * points and rep["engine"] == engine
+
+
 @pytest.mark.parametrize("shared", [False, True])
 def test_the_product_error_of_a_mixed_request_is_the_fp32_products(device, shared):
     # FP32 rounds the factors at 6e-8; averaged over a camera's thousands of observations that leaves more than

@@ -410,15 +410,23 @@ double read_word(tba_device* d, const double* state, int word) {
 
 // ---- the explicit reduced camera system ------------------------------------------------------------
 
-// Pairs of observations of one point (all cameras counted as variable).
-uint64_t count_pairs(const uint32_t* ps, uint32_t P) {
+// Pairs of observations of one point (all cameras counted as variable), and the longest track.
+struct Tracks {
+  uint64_t pairs = 0;
+  uint32_t longest = 0;
+};
+
+Tracks count_pairs(const uint32_t* ps, uint32_t P) {
   uint64_t squares = 0, sum = 0;
+  Tracks t;
   for (uint32_t p = 0; p < P; p++) {
-    const uint64_t n = uint32_t(ps[p + 1] - ps[p]);
-    squares += n * n;
+    const uint32_t n = ps[p + 1] - ps[p];
+    squares += uint64_t(n) * n;
     sum += n;
+    t.longest = std::max(t.longest, n);
   }
-  return (squares - sum) / 2;
+  t.pairs = (squares - sum) / 2;
+  return t;
 }
 
 // 6x6 blocks of S at most.
@@ -451,14 +459,24 @@ double expected_steps(uint64_t C, double tolerance) {
 // the first PCG run reaches the tolerance; where the budget ends the runs, their restarts make it 0.036 for each
 // step of the budget.  The 26 cameras: tolerance 1e-2 7.8 and 11.0, 1e-3 9.4 and 11.1, 1e-6 16.9 and 11.3, budget
 // 16 17.0 and 10.7; the 200 cameras: 1e-2 43.3 and 55.5, 2e-3 58.7 and 55.9.
-bool prefer_schur(uint64_t C, uint64_t M, uint64_t pairs, uint32_t budget, double most, double expected, bool mixed) {
+//
+// A track of n cameras makes n^2 blocks of S (each some 0.5 ns to write), which cost a step 0.03 ns each where
+// the PCG's blocks hold them in shared memory, 0.08 from the L2 and 0.14 beyond half of it; on the product its
+// warp takes 0.04 us an observation.  Six iterations, every camera seeing every point: 300 cameras / 50 points
+// 5.8 and 4.0, 400 / 30 6.4 and 4.0, 600 / 30 8.0 and 11.5, 600 / 10 7.6 and 9.9.  (The adjoint's product is
+// slower on these: 600 / 30 6.4 and 4.9 a call; it does not count them.)
+bool prefer_schur(uint64_t C, uint64_t M, Tracks tracks, uint32_t budget, double most, double expected, bool mixed) {
+  const uint64_t pairs = tracks.pairs;
   if (6 * C + 1 > tba::product_max_unknowns() || pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
-  const double walk = 288e-6 / 8 * double(schur_block_bound(C, pairs)) / 6;
+  const double seen = double(std::min<uint64_t>(tracks.longest, C)), dense = seen * seen, bytes = 288 * dense;
+  const double walk = std::max(288e-6 / 8 * double(schur_block_bound(C, pairs)) / 6,
+                               (bytes < 30e6 ? 3e-5 : bytes < 60e6 ? 8e-5 : 1.4e-4) * dense);
   // A step's cost on the product less that on the system, at `k` us an observation.
-  const auto step = [&](double k) { return 16 + k * double(M) - walk; };
-  if (!(4e-5 * double(pairs) < most * step(3.3e-5))) return false;
+  const auto step = [&](double k) { return 16 + std::max(k * double(M), 0.04 * tracks.longest) - walk; };
+  const double write = 5e-4 * dense;
+  if (!(4e-5 * double(pairs) + write < most * step(3.3e-5))) return false;
   const double reach = 144 * double(M) * std::min(1.0, 8 * double(pairs) / double(M) / double(C));
-  const double form = (reach < 126e6 ? 3.6e-5 : 4.6e-5) * double(pairs);
+  const double form = (reach < 126e6 ? 3.6e-5 : 4.6e-5) * double(pairs) + write;
   if (mixed) return form < std::min(budget * step(3.6e-5), expected * step(2.2e-5));
   return form < std::min(0.85 * budget, expected) * step(3.3e-5);
 }
@@ -697,7 +715,7 @@ struct HostPlan {
   std::vector<uint32_t> tasks, task_obs;
   Chunks chunks;
   uint32_t fixed = 0;
-  uint64_t pairs = 0;  // pairs of observations of one point
+  Tracks tracks;
   // The arrays a solve uploads, in the order of a resident scene's device copy.
   std::vector<const std::vector<uint32_t>*> sections() const {
     return {&tasks, &task_obs, &chunks.cam, &chunks.beg, &chunks.cam_first};
@@ -715,7 +733,7 @@ HostPlan make_plan(const tba_control* ctl, const uint32_t* index, int sms) {
   for (size_t t = 0; t < plan.tasks.size(); t++) plan.task_obs[t] = ps[plan.tasks[t]];
   plan.chunks = build_chunks(cs, C, chunk_size(M, sms));
   for (uint32_t c = 0; c < C; c++) plan.fixed += active[c] == 0;
-  plan.pairs = count_pairs(ps, P);
+  plan.tracks = count_pairs(ps, P);
   return plan;
 }
 
@@ -832,11 +850,12 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   // the product of the form asked for and fits the device; it is FP64, so a mixed request then needs no refinement.
   // (Without iterations there is no system to form: its structure alone took 0.03 ms at 7 cameras and 0.35 at
   // 1,500 and 1.8M observations, of calls of 0.21 and 5.9 ms.)
-  const uint64_t npairs = ctl->iterations == 0 ? 0 : (io.plan ? io.plan->pairs : count_pairs(index + 2 * size_t(M), P));
+  const Tracks tracks = ctl->iterations == 0 ? Tracks() : (io.plan ? io.plan->tracks : count_pairs(index + 2 * size_t(M), P));
+  const uint64_t npairs = tracks.pairs;
   // (The product's error asked of a mixed request is the FP32 product's.)
   const bool keep_product = ctl->precision == TBA_PRECISION_MIXED && (ctl->flags & TBA_FLAG_PRODUCT_ERROR) != 0;
   bool schur = p.factored && ctl->iterations > 0 && !keep_product &&
-               prefer_schur(C, M, npairs, ctl->max_cg, 16, expected_steps(C, ctl->cg_tolerance),
+               prefer_schur(C, M, tracks, ctl->max_cg, 16, expected_steps(C, ctl->cg_tolerance),
                             ctl->precision == TBA_PRECISION_MIXED);
   bool mixed = false;
   size_t factor_bytes = 0, factor32_bytes = 0;
@@ -1723,7 +1742,7 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
           plans[k].tasks = build_tasks(ps, q.points);
           if (auto_shape || grid_forced) {
             plans[k].chunks = build_chunks(ps + q.points + 1, q.cameras, chunk);
-            plans[k].pairs = count_pairs(ps, q.points);
+            plans[k].pairs = count_pairs(ps, q.points).pairs;
           }
         } catch (const Fail& f) {
           std::lock_guard<std::mutex> lock(fail_mu);
@@ -2120,8 +2139,8 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const HostChecks* check
   A.prod_copies = tba::adj_product_copies(C);
   // The explicit reduced system in place of the product over the cross blocks, where it costs less and
   // fits the device.
-  const uint64_t npairs = count_pairs(index + 2 * size_t(M), P);
-  bool schur = prefer_schur(C, M, npairs, vc->max_cg, 64, vc->max_cg, false);
+  const uint64_t npairs = count_pairs(index + 2 * size_t(M), P).pairs;
+  bool schur = prefer_schur(C, M, Tracks{npairs, 0}, vc->max_cg, 64, vc->max_cg, false);
   Chunks chunks;
   if (checks && (checks->camera_ends || checks->camera_offsets)) schur = false;  // no chunks; the checks will fail
   if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, chunk_size(M, d->sms));
