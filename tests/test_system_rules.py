@@ -4,10 +4,12 @@ import numpy as np
 import pytest
 
 import typecv_b200 as tb
+from oracle.adjoint_dense import Problem
 from typecv_b200 import _lib
 from typecv_b200 import adjoint as AD
 from typecv_b200 import batch as B
 from typecv_b200 import synthetic as S
+from typecv_b200.bundle import pack_arrays
 from typecv_b200.resident import ResidentScene
 
 pytestmark = pytest.mark.gpu
@@ -190,3 +192,22 @@ def test_a_mixed_request_keeps_the_budgets_of_its_runs(device, shared):
     for precision, accepted in (("fp64", 0), ("mixed", 1)):
         recs, _ = B.batch_adjust(device, [window] * 2, max_cg=few, precision=precision, **kw)
         assert [r[base + 10] for r in recs] == [accepted] * 2 and recs[1][base + 17] == 1 - accepted
+
+
+@pytest.mark.parametrize("fixed,system", [((0,), True), ((0, 1, 3, 4, 5), False), ((0, 1, 2, 3, 4, 5), False)])
+def test_an_adjoint_of_one_variable_camera_forms_no_system(device, fixed, system):
+    sc = S.arc_scene(seed=5, cameras=6, points=203, outlier_rate=0.0)
+    active = np.ones(sc.C, np.uint32)
+    active[list(fixed)] = 0
+    s, i = pack_arrays(sc.truth_poses, sc.points, sc.truth_cameras, sc.obs_camera, sc.obs_point, sc.pixels, active)
+    out, _ = solve(device, sc, (s, i), iterations=20, tolerance=1e-10)
+    n = 12 * sc.C + 3 * sc.P
+    s[:n] = out[:n]
+    g = np.random.default_rng(6).normal(size=n)
+    g /= np.linalg.norm(g)
+    ybar, kbar, sol, rep = AD.bundle_vjp(device, sc.C, sc.P, sc.M, s, i, g, newton_steps=2, want_solution=True)
+    assert rep["failed"] == 0 and (rep["product_blocks"] == 0) == system
+    s[:n] = sol
+    # (differences of 1e-7: the residuals' distances to the Huber threshold are larger)
+    want, _ = Problem(sc.C, sc.P, sc.M, s, i).vjp(g, h=1e-7)
+    assert np.linalg.norm(ybar - want) <= 1e-5 * np.linalg.norm(want)
