@@ -149,8 +149,8 @@ void check_control(const tba_control* c) {
 // threads (serially below `serial_below`).
 template <typename F>
 void parallel_ranges(uint64_t n, uint64_t serial_below, F f) {
-  unsigned threads = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
-  if (n < serial_below || threads == 1) {
+  const unsigned threads = unsigned(std::min<uint64_t>(n, std::min(16u, std::max(1u, std::thread::hardware_concurrency()))));
+  if (n < serial_below || threads <= 1) {
     f(uint64_t(0), n, 0u);
     return;
   }
@@ -1738,6 +1738,7 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
               continue;
             }
           }
+          if (!plans[k].tasks.empty()) continue;  // planned before the whole check
           const uint32_t* ps = index + q.index_offset + 2 * size_t(q.observations);
           plans[k].tasks = build_tasks(ps, q.points);
           if (auto_shape || grid_forced) {
