@@ -102,6 +102,37 @@ def test_a_full_system_beyond_the_caches_is_not_formed(device, cameras, points, 
     assert sc.M == cameras * points and rep["engine"] == engine
 
 
+def scattered(cameras, points, track, seed=1):
+    """Points near the origin, each seen by cameras picked at random from a sphere around it: any two cameras
+    share points."""
+    rng = np.random.default_rng(seed)
+    like = S.sphere_scene(seed=seed, cameras=cameras, points=64, track_mean=20.0)
+    pick = np.sort(np.argsort(rng.random((points, cameras)), axis=1)[:, :track], axis=1)
+    return S.finish("scattered", rng, like.truth_poses, like.truth_cameras, rng.normal(size=(points, 3)), pick.ravel(),
+                    np.repeat(np.arange(points), track), width=1024, height=768)
+
+
+@pytest.mark.parametrize("kind,cameras,points,engine", [
+    ("scattered", 400, 12_000, 2), ("scattered", 900, 30_000, 0), ("scattered", 1500, 30_000, 0), ("sphere", 900, 30_000, 2),
+    ("sphere", 1500, 60_000, 2), ("helix", 1000, 30_000, 2)])
+def test_cameras_that_all_share_points_form_no_large_system(kind, cameras, points, engine):
+    # The same sizes, and systems of 30 to 500 MB where neighbours alone would make 4 to 52.
+    sc = scattered(cameras, points, 5) if kind == "scattered" else \
+        (S.sphere_scene if kind == "sphere" else S.helix_scene)(seed=3, cameras=cameras, points=points)
+    packed = sc.packed()
+    with tb.ShadeDevice.open(0) as dev:
+        out, rep = solve(dev, sc, packed, iterations=2, tolerance=1e-9, max_cg=200)
+        assert rep["engine"] == engine
+        # A resident scene, and the adjoint, take the same side.
+        ctl = tb.make_control(sc.C, sc.P, sc.M, anchor=0, scale_view=1, iterations=2, tolerance=1e-9, max_cg=200)
+        with ResidentScene(dev, ctl, *packed) as scene:
+            kept, _, rep = scene.adjust(output=True)
+        base = 12 * sc.C + 3 * sc.P
+        assert rep["engine"] == engine and abs(kept[base + 6] - out[base + 6]) <= 1e-9 * out[base + 6]
+        _, _, _, rep = AD.bundle_vjp(dev, sc.C, sc.P, sc.M, *packed, np.zeros(base), max_cg=200, tolerance=1e-6)
+        assert (rep["product_blocks"] == 0) == (engine == 2)
+
+
 @pytest.mark.parametrize("shared", [False, True])
 def test_the_product_error_of_a_mixed_request_is_the_fp32_products(device, shared):
     # FP32 rounds the factors at 6e-8; averaged over a camera's thousands of observations that leaves more than

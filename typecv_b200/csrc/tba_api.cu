@@ -410,10 +410,15 @@ double read_word(tba_device* d, const double* state, int word) {
 
 // ---- the explicit reduced camera system ------------------------------------------------------------
 
-// Pairs of observations of one point (all cameras counted as variable), and the longest track.
+// 6x6 blocks of S at most.
+uint64_t schur_block_bound(uint64_t C, uint64_t pairs) { return std::min(C * C, 2 * pairs + C); }
+
+// Pairs of observations of one point (all cameras counted as variable), the longest track, and the blocks of S
+// that its camera pairs spread over (0: not looked for).
 struct Tracks {
   uint64_t pairs = 0;
   uint32_t longest = 0;
+  double spread = 0;
 };
 
 Tracks count_pairs(const uint32_t* ps, uint32_t P) {
@@ -429,8 +434,59 @@ Tracks count_pairs(const uint32_t* ps, uint32_t P) {
   return t;
 }
 
-// 6x6 blocks of S at most.
-uint64_t schur_block_bound(uint64_t C, uint64_t pairs) { return std::min(C * C, 2 * pairs + C); }
+constexpr double kFarSystem = 110e6;  // bytes of S beyond which a step no longer finds it in the L2
+
+// How many blocks of S the camera pairs spread over as if evenly: K of them, one from each of K points all along
+// the list, agree with one another about K^2 / 2D times when they are spread over D.  Where cameras share points
+// with their neighbours D is below 46,000 (spheres of 331 to 4,000 cameras, helices of 1,000 and 3,000), where
+// any camera meets any other it is all pairs: 165,000 at 600 cameras, 950,000 at 4,600.  Taken 256 at a time
+// until they agree often enough to tell; 20 to 60 us, 130 with the arrays out of the caches.  (The arrays are not
+// yet checked.)
+double spread_blocks(uint32_t C, uint32_t P, uint32_t M, const uint32_t* index) {
+  constexpr uint32_t kSamples = 2048, kStep = 256, kPlaces = 4096;
+  const uint32_t* ps = index + 2 * size_t(M);
+  const auto point = [&](uint32_t k) { return uint32_t(uint64_t(P) * (k * 1229 % kSamples) / kSamples); };
+  std::vector<uint64_t> key(kPlaces, UINT64_MAX);
+  std::vector<uint32_t> met(kPlaces, 0);
+  uint32_t one[kStep], two[kStep];
+  uint64_t sampled = 0, agreed = 0, random = 88172645463325252ull;
+  double blocks = 0;
+  for (uint32_t k0 = 0; k0 < kSamples; k0 += kStep) {
+    for (uint32_t k = 0; k < kStep; k++) __builtin_prefetch(ps + point(k0 + k));
+    for (uint32_t k = 0; k < kStep; k++) {
+      const uint32_t p = point(k0 + k), b = ps[p], e = ps[p + 1];
+      one[k] = two[k] = 0;
+      if (e > M || uint64_t(e) < uint64_t(b) + 2) continue;
+      random = random * 6364136223846793005ull + 1442695040888963407ull;
+      const uint32_t n = e - b, i = uint32_t((random >> 33) % n);
+      one[k] = b + i;
+      two[k] = b + (i + 1 + uint32_t((random >> 20) % (n - 1))) % n;
+      __builtin_prefetch(index + one[k]);
+      __builtin_prefetch(index + two[k]);
+    }
+    for (uint32_t k = 0; k < kStep; k++) {
+      const uint32_t c = index[one[k]], d = index[two[k]];
+      if (one[k] == two[k] || c == d) continue;
+      const uint64_t pair = (uint64_t(std::min(c, d)) << 32) | std::max(c, d);
+      uint32_t at = uint32_t((pair * 0x9e3779b97f4a7c15ull) >> 52);
+      while (key[at] != UINT64_MAX && key[at] != pair) at = (at + 1) % kPlaces;
+      key[at] = pair;
+      agreed += met[at]++;
+      sampled++;
+    }
+    blocks = double(sampled) * double(sampled) / double(std::max<uint64_t>(agreed, 1)) + C;
+    if (agreed >= 16 && 288 * blocks < kFarSystem / 2) break;
+  }
+  return blocks;
+}
+
+// The tracks of a problem, as prefer_schur weighs them.
+Tracks survey(uint32_t C, uint32_t P, uint32_t M, const uint32_t* index) {
+  Tracks t = count_pairs(index + 2 * size_t(M), P);
+  if (288.0 * double(schur_block_bound(C, t.pairs)) > kFarSystem)
+    t.spread = std::min(spread_blocks(C, P, M, index), double(schur_block_bound(C, t.pairs)));
+  return t;
+}
 
 // The PCG steps of a solve to `tolerance` that the choice below counts on, from few: spheres, arcs and rings of
 // 16 to 60 cameras took 8 to 19 steps at 1e-2, 10 to 30 at 1e-3 and 21 to 44 at 1e-6, 200 cameras 22, 36 and 68,
@@ -460,17 +516,20 @@ double expected_steps(uint64_t C, double tolerance) {
 // step of the budget.  The 26 cameras: tolerance 1e-2 7.8 and 11.0, 1e-3 9.4 and 11.1, 1e-6 16.9 and 11.3, budget
 // 16 17.0 and 10.7; the 200 cameras: 1e-2 43.3 and 55.5, 2e-3 58.7 and 55.9.
 //
-// A track of n cameras makes n^2 blocks of S (each some 0.5 ns to write), which cost a step 0.03 ns each where
-// the PCG's blocks hold them in shared memory, 0.08 from the L2 and 0.14 beyond half of it; on the product its
-// warp takes 0.04 us an observation.  Six iterations, every camera seeing every point: 300 cameras / 50 points
-// 5.8 and 4.0, 400 / 30 6.4 and 4.0, 600 / 30 8.0 and 11.5, 600 / 10 7.6 and 9.9.  (The adjoint's product is
-// slower on these: 600 / 30 6.4 and 4.9 a call; it does not count them.)
+// A track of n cameras makes n^2 blocks of S (each some 0.5 ns to write), which cost a step 0.04 ns each from
+// shared memory or the L2 and 0.1 beyond; on the product its warp takes 0.04 us an observation.  Six iterations,
+// every camera seeing every point: 300 cameras / 50 points 5.8 and 4.0, 400 / 30 6.4 and 4.0, 540 / 40 7.1 and 6.4,
+// 600 / 30 8.0 and 11.5, 600 / 10 7.6 and 9.9.  (The adjoint's product is slower on these: 600 / 30 6.4 and 4.9 a
+// call; it does not count them.)  Where any camera meets any other S is as large without long tracks: 600 cameras
+// / 100,000 observations of 5 random cameras a point 6.2 and 5.7, 800 / 120,000 7.0 and 12.5, 1,500 / 1.0M 14.8 and
+// 40.3; four iterations on 4,600 / 1.5M 17.4 and 90.7.
 bool prefer_schur(uint64_t C, uint64_t M, Tracks tracks, uint32_t budget, double most, double expected, bool mixed) {
   const uint64_t pairs = tracks.pairs;
   if (6 * C + 1 > tba::product_max_unknowns() || pairs >= 0x7fffffffull || M > 0x0fffffffull) return false;
-  const double seen = double(std::min<uint64_t>(tracks.longest, C)), dense = seen * seen, bytes = 288 * dense;
+  const double seen = double(std::min<uint64_t>(tracks.longest, C)), spread = 288 * tracks.spread > kFarSystem ? tracks.spread : 0,
+               dense = std::max(seen * seen, spread), bytes = 288 * dense;
   const double walk = std::max(288e-6 / 8 * double(schur_block_bound(C, pairs)) / 6,
-                               (bytes < 30e6 ? 3e-5 : bytes < 60e6 ? 8e-5 : 1.4e-4) * dense);
+                               (bytes < 90e6 ? 4e-5 : 1e-4) * dense);
   // A step's cost on the product less that on the system, at `k` us an observation.
   const auto step = [&](double k) { return 16 + std::max(k * double(M), 0.04 * tracks.longest) - walk; };
   const double write = 5e-4 * dense;
@@ -715,7 +774,7 @@ struct HostPlan {
   std::vector<uint32_t> tasks, task_obs;
   Chunks chunks;
   uint32_t fixed = 0;
-  Tracks tracks;
+  Tracks tracks;  // a resident scene's
   // The arrays a solve uploads, in the order of a resident scene's device copy.
   std::vector<const std::vector<uint32_t>*> sections() const {
     return {&tasks, &task_obs, &chunks.cam, &chunks.beg, &chunks.cam_first};
@@ -733,7 +792,6 @@ HostPlan make_plan(const tba_control* ctl, const uint32_t* index, int sms) {
   for (size_t t = 0; t < plan.tasks.size(); t++) plan.task_obs[t] = ps[plan.tasks[t]];
   plan.chunks = build_chunks(cs, C, chunk_size(M, sms));
   for (uint32_t c = 0; c < C; c++) plan.fixed += active[c] == 0;
-  plan.tracks = count_pairs(ps, P);
   return plan;
 }
 
@@ -850,7 +908,7 @@ void solve(tba_device* d, const tba_control* ctl, const double* scene, const uin
   // the product of the form asked for and fits the device; it is FP64, so a mixed request then needs no refinement.
   // (Without iterations there is no system to form: its structure alone took 0.03 ms at 7 cameras and 0.35 at
   // 1,500 and 1.8M observations, of calls of 0.21 and 5.9 ms.)
-  const Tracks tracks = ctl->iterations == 0 ? Tracks() : (io.plan ? io.plan->tracks : count_pairs(index + 2 * size_t(M), P));
+  const Tracks tracks = ctl->iterations == 0 ? Tracks() : (io.plan ? io.plan->tracks : survey(C, P, M, index));
   const uint64_t npairs = tracks.pairs;
   // (The product's error asked of a mixed request is the FP32 product's.)
   const bool keep_product = ctl->precision == TBA_PRECISION_MIXED && (ctl->flags & TBA_FLAG_PRODUCT_ERROR) != 0;
@@ -2141,8 +2199,9 @@ void solve_vjp(tba_device* d, const tba_vjp_control* vc, const HostChecks* check
   // The explicit reduced system in place of the product over the cross blocks, where it costs less and
   // fits the device.  (With one variable camera there is nothing to gain: its preconditioner is the inverse, and
   // a call of two cameras took 0.21 ms instead of 0.19 for the system's structure.)
-  const uint64_t npairs = count_pairs(index + 2 * size_t(M), P).pairs;
-  bool schur = C - fixed > 1 && prefer_schur(C, M, Tracks{npairs, 0}, vc->max_cg, 64, vc->max_cg, false);
+  const Tracks tracks = survey(C, P, M, index);
+  const uint64_t npairs = tracks.pairs;
+  bool schur = C - fixed > 1 && prefer_schur(C, M, Tracks{npairs, 0, tracks.spread}, vc->max_cg, 64, vc->max_cg, false);
   Chunks chunks;
   if (checks && (checks->camera_ends || checks->camera_offsets)) schur = false;  // no chunks; the checks will fail
   if (schur) chunks = build_chunks(index + 2 * size_t(M) + P + 1, C, chunk_size(M, d->sms));
@@ -2850,7 +2909,9 @@ tba_status tba_scene_create(tba_device* d, const tba_control* shape, const doubl
     r = new tba_scene();
     r->device = d;
     r->shape = *shape;
-    r->plan = new HostPlan(make_plan(shape, index, d->sms));
+    HostPlan* plan = new HostPlan(make_plan(shape, index, d->sms));
+    r->plan = plan;
+    plan->tracks = survey(shape->cameras, shape->points, shape->observations, index);
     std::vector<uint32_t> flat;
     for (const std::vector<uint32_t>* v : static_cast<HostPlan*>(r->plan)->sections()) flat.insert(flat.end(), v->begin(), v->end());
     // (an explicit system's buffer that the handle keeps from its last solve makes room for the scene)
