@@ -249,9 +249,9 @@ typedef struct {
 
 /* Options shared by every problem of a batch (tba_control's meaning).  `schedule` picks the
  * launch shape: k >= 1 forces shape k - 1 of tba_batch_shape (the last is the kernels over all
- * problems at once, which run in FP64); 0 takes that last shape where its memory fits and the tracks
- * are no longer than about 64 observations, and else lets the autotuner choose among the persistent
- * ones (timed trial launches the first time a batch shape is seen on the handle, cached afterwards). */
+ * problems at once, which run in FP64); 0 takes that last shape where its memory fits, the tracks
+ * are no longer than about 64 observations and the reduced systems are not large for what the problems
+ * observe, and else lets the autotuner choose among the persistent ones (timed trial launches the first time a batch shape is seen on the handle, cached afterwards). */
 typedef struct {
   uint32_t iterations;
   uint32_t max_cg;

@@ -242,3 +242,19 @@ def test_an_adjoint_of_one_variable_camera_forms_no_system(device, fixed, system
     # (differences of 1e-7: the residuals' distances to the Huber threshold are larger)
     want, _ = Problem(sc.C, sc.P, sc.M, s, i).vjp(g, h=1e-7)
     assert np.linalg.norm(ybar - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("kind,count,cameras,points,track,grid", [
+    ("scattered", 2, 60, 400, 5, True), ("scattered", 2, 144, 250, 12, False), ("scattered", 2, 144, 4000, 5, True),
+    ("scattered", 150, 144, 300, 5, False), ("arc", 2, 144, 600, 5, True)])
+def test_windows_of_large_systems_run_on_the_persistent_launch(device, kind, count, cameras, points, track, grid):
+    base = [scattered(cameras, points, track, seed=k) if kind == "scattered" else
+            S.arc_scene(seed=k, cameras=cameras, points=points, track=(track - 1, track + 1)) for k in range(2)]
+    probs = [B.PackedProblem(sc.C, sc.P, sc.M, *sc.packed(), sc.anchor, sc.scale_view) for sc in base] * (count // 2)
+    kw = dict(iterations=3, max_cg=256, tolerance=1e-9)
+    recs, rep = B.batch_adjust(device, probs, precision="fp64", **kw)
+    assert (rep["schedule"] == 4) == grid
+    for sc, rec in zip(base, recs):
+        out, _ = solve(device, sc, **kw)
+        n = 12 * sc.C + 3 * sc.P
+        assert abs(rec[n + 6] - out[n + 6]) <= 1e-9 * out[n + 6]

@@ -90,9 +90,9 @@ def batch_adjust(device: ShadeDevice, problems: list[PackedProblem] | PackedBatc
                  schedule: int = 0, output: np.ndarray | None = None):
     """Solve every problem; returns (list of result records, report dict).
 
-    ``schedule`` 0 solves all problems side by side on the last shape, in FP64, where its memory fits and
-    the tracks are no longer than about 64 observations, and else lets the library's autotuner pick a
-    persistent shape; k >= 1 forces shape k - 1 of ``batch_shapes``.
+    ``schedule`` 0 solves all problems side by side on the last shape, in FP64, where its memory fits, the
+    tracks are no longer than about 64 observations and the reduced systems are not large for what the
+    problems observe, and else lets the library's autotuner pick a persistent shape; k >= 1 forces shape k - 1 of ``batch_shapes``.
     ``max_cg`` defaults to the reference's default for the largest problem (bundle-host.ts:49-65).
     """
     lib = _lib.load()

@@ -445,17 +445,21 @@ constexpr double kFarSystem = 110e6;  // bytes of S beyond which a step no longe
 double spread_blocks(uint32_t C, uint32_t P, uint32_t M, const uint32_t* index) {
   constexpr uint32_t kSamples = 2048, kStep = 256, kPlaces = 4096;
   const uint32_t* ps = index + 2 * size_t(M);
-  const auto point = [&](uint32_t k) { return uint32_t(uint64_t(P) * (k * 1229 % kSamples) / kSamples); };
+  const uint32_t samples = std::min(kSamples, P);
+  // Golden-ratio steps along the list, so that any first few of them lie evenly.
+  const auto point = [&](uint32_t k) { return uint32_t(uint64_t(P) * (k * 1265 % kSamples) / kSamples); };
   std::vector<uint64_t> key(kPlaces, UINT64_MAX);
-  std::vector<uint32_t> met(kPlaces, 0);
-  uint32_t one[kStep], two[kStep];
+  std::vector<uint32_t> met(kPlaces, 0), last(kPlaces, UINT32_MAX);
+  uint32_t one[kStep], two[kStep], from[kStep];
   uint64_t sampled = 0, agreed = 0, random = 88172645463325252ull;
   double blocks = 0;
-  for (uint32_t k0 = 0; k0 < kSamples; k0 += kStep) {
-    for (uint32_t k = 0; k < kStep; k++) __builtin_prefetch(ps + point(k0 + k));
-    for (uint32_t k = 0; k < kStep; k++) {
+  for (uint32_t k0 = 0; k0 < samples; k0 += kStep) {
+    const uint32_t take = std::min(kStep, samples - k0);
+    for (uint32_t k = 0; k < take; k++) __builtin_prefetch(ps + point(k0 + k));
+    for (uint32_t k = 0; k < take; k++) {
       const uint32_t p = point(k0 + k), b = ps[p], e = ps[p + 1];
       one[k] = two[k] = 0;
+      from[k] = p;
       if (e > M || uint64_t(e) < uint64_t(b) + 2) continue;
       random = random * 6364136223846793005ull + 1442695040888963407ull;
       const uint32_t n = e - b, i = uint32_t((random >> 33) % n);
@@ -464,12 +468,14 @@ double spread_blocks(uint32_t C, uint32_t P, uint32_t M, const uint32_t* index) 
       __builtin_prefetch(index + one[k]);
       __builtin_prefetch(index + two[k]);
     }
-    for (uint32_t k = 0; k < kStep; k++) {
+    for (uint32_t k = 0; k < take; k++) {
       const uint32_t c = index[one[k]], d = index[two[k]];
       if (one[k] == two[k] || c == d) continue;
       const uint64_t pair = (uint64_t(std::min(c, d)) << 32) | std::max(c, d);
       uint32_t at = uint32_t((pair * 0x9e3779b97f4a7c15ull) >> 52);
       while (key[at] != UINT64_MAX && key[at] != pair) at = (at + 1) % kPlaces;
+      if (last[at] == from[k]) continue;  // the same point again
+      last[at] = from[k];
       key[at] = pair;
       agreed += met[at]++;
       sampled++;
@@ -1745,6 +1751,37 @@ bool batch_on_grid(tba_device* d, const tba_batch_control* bc, const tba_batch_p
   return true;
 }
 
+// Whether the windows' PCG steps cost less on the systems, one block a window, than on the block solver: there
+// 14 us and 11.5 ns an observation; here 5 us, 80 ns a camera and 4.2 ns a block of S, or, where the S of the windows
+// in flight (one an SM) do not stay in the L2, their bytes from DRAM.  The blocks are the bound's, or where that
+// says no, those that a window's camera pairs spread over.  Whole batches, six iterations, every camera sharing
+// points with any other, block solver and systems, ms: 1 window of 60 cameras / 2,000 observations 8.5 and 4.8,
+// 100 / 3,000 12.1 and 10.4, 144 / 3,000 12.5 and 13.8, 144 / 25,000 47.6 and 18.4; 148 windows of 60 / 2,000 with the
+// focal unknown 11.0 and 13.8, of 144 / 3,000 16.1 and 30.8.
+bool systems_pay(const tba_batch_problem* probs, uint32_t count, const std::vector<WindowPlan>& plans,
+                 const uint32_t* index, int sms) {
+  double product = 0, cameras = 0, bound = 0;
+  for (uint32_t k = 0; k < count; k++) {
+    product += 14 + 11.5e-3 * double(probs[k].observations);
+    cameras += 5 + 0.08 * probs[k].cameras;
+    bound += double(schur_block_bound(probs[k].cameras, plans[k].pairs));
+  }
+  const auto pay = [&](double blocks) {
+    // (the windows in flight read their systems together, at 4.5 TB/s)
+    const double flight = 288 * blocks * std::min(1.0, double(sms) / count);
+    return cameras + std::max(4.2e-3 * blocks, flight > 100e6 ? flight / 4.5e6 * count : 0) < product;
+  };
+  if (pay(bound)) return true;
+  double found = 0, of = 0;  // at most eight of the windows tell for all
+  for (uint32_t k = 0; k < count; k += (count + 7) / 8) {
+    const tba_batch_problem& q = probs[k];
+    const double most = double(schur_block_bound(q.cameras, plans[k].pairs));
+    found += std::min(most, spread_blocks(q.cameras, q.points, q.observations, index + q.index_offset));
+    of += most;
+  }
+  return pay(bound * found / of);
+}
+
 void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_problem* probs, uint32_t count,
                  const double* scene, size_t scene_len, const uint32_t* index, size_t index_len, double* output,
                  size_t output_len, tba_batch_report* report) {
@@ -1914,7 +1951,8 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
   };
   // The grid kernels unless another shape is asked for.  They form each reduced system, at a cost that
   // grows with the pairs of observations of a point; beyond tracks of about 64 that is more than the
-  // block solver's passes over the observations, and they need the memory for them.
+  // block solver's passes over the observations, and they need the memory for them.  Nor are they taken
+  // where the systems are large for what the windows observe.
   if (auto_shape || grid_forced) {
     uint64_t pairs = 0;
     bool fits = true;
@@ -1924,7 +1962,7 @@ void solve_batch(tba_device* d, const tba_batch_control* bc, const tba_batch_pro
     }
     double* dout = nullptr;
     const std::function<void()> whole = check_whole;
-    if (fits && (grid_forced || pairs <= 32 * M_all) &&
+    if (fits && (grid_forced || (pairs <= 32 * M_all && systems_pay(probs, count, plans, index, d->sms))) &&
         batch_on_grid(d, bc, probs, count, plans, order, scene, scene_len, index, index_len, output_len, e1, e0, ran, dout, h2d,
                       checked ? nullptr : static_cast<const std::function<void()>*>(&whole))) {
       finish(dout);
